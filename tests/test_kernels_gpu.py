@@ -201,6 +201,20 @@ def test_gemm_simt(ops, dtype, M, N, K):
         assert rel_err(host(out32), plain.linear(a, w)) < 2e-5
 
 
+@pytest.mark.parametrize("tile,splits", [(t, c) for t in range(3) for c in (1, 2, 4, 8)])
+@pytest.mark.parametrize("M,N,K", [(17, 1, 1), (33, 65, 37), (129, 63, 260), (64, 64, 1024), (97, 200, 1504)])
+def test_float_products_in_every_tiling(ops, tile, splits, M, N, K):
+    """Tiles' edges, widths whose rows are no whole 16-byte pieces, splits that get no slice of k; a row stride above the row."""
+    from tiny_inference_engine_b200.ops.library import call
+    rng = np.random.default_rng(M + N + K)
+    a, w = rng.standard_normal((M, K + 4)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    da, dw, out = dev(a), dev(w), torch.full((M, N + 3), -7.0, device="cuda")
+    call("tie_gemm_f32_tiled", da.data_ptr(), dw.data_ptr(), out.data_ptr(), M, N, K, K + 4, K, N + 3, tile, splits,
+         torch.cuda.current_stream().cuda_stream)
+    assert rel_err(host(out)[:, :N], plain.linear(a[:, :K], w)) < TOL["float32"]
+    assert (host(out)[:, N:] == -7.0).all()
+
+
 def dense_reference(q, k, v, Hq, Hkv, Dh, n_new, window=0):
     """The last n_new rows of causal attention over all of k, v."""
     n = k.shape[0]
