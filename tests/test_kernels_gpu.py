@@ -254,6 +254,29 @@ def test_paged_attention_rows_and_split(ops, dtype, Hq, Hkv, Dh, page, window):
     assert not host(out2)[:n_multi].any()
 
 
+@pytest.mark.parametrize("Hq,Hkv,Dh,page,window,new,ctx", [
+    (4, 2, 128, 16, 0, [16, 3, 40], [16, 70, 40]), (2, 1, 64, 8, 0, [1, 15, 33], [97, 15, 64]), (3, 3, 32, 12, 9, [31, 17], [31, 90]),
+    (2, 2, 128, 4, 33, [50], [140])])
+def test_float_rows_by_tiles(ops, Hq, Hkv, Dh, page, window, new, ctx):
+    """Tiles of 16 rows and 32 keys with several sequences in one, portions behind cached keys, windows; and a token with NaN values
+    leaves the rows before it, and the other sequences, as they are."""
+    rng = np.random.default_rng(Hq * Dh + window)
+    kc, vc, bt, ks, vs = paged_cache(rng, "float32", ctx, Hkv, Dh, page, 60 * 16 // page)
+    T, qs = sum(new), np.concatenate([[0], np.cumsum(new)])
+    q = rng.standard_normal((T, Hq * Dh)).astype(np.float32) * 3
+    want = np.concatenate([dense_reference(q[qs[i]:qs[i + 1]], ks[i], vs[i], Hq, Hkv, Dh, new[i], window) for i in range(len(new))])
+    args = (dev(np.repeat(np.arange(len(new)), new), torch.int32), dev(qs, torch.int32), dev(np.array(ctx), torch.int32), dev(bt, torch.int32))
+    out = torch.full((T, Hq * Dh), float("nan"), device="cuda")
+    ops.attention_rows(dev(q), dev(kc), dev(vc), out, *args, Hq, Hkv, Dh, 1.0 / np.sqrt(Dh), window)
+    assert rel_err(host(out), want) < TOL["float32"]
+    sick = ctx[-1] - 2                                 # the second last token of the last sequence
+    vc = vc.copy()
+    vc[bt[len(new) - 1, sick // page], :, sick % page] = np.nan
+    ops.attention_rows(dev(q), dev(kc), dev(vc), out, *args, Hq, Hkv, Dh, 1.0 / np.sqrt(Dh), window)
+    assert rel_err(host(out)[:T - 2], want[:T - 2]) < TOL["float32"]
+    assert np.isnan(host(out)[T - 2:]).all()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("far", [0, 15, 16, 31, 32, 255, 256, 257, 511, 512, 1022, 1023])
 def test_one_far_key_among_a_thousand_is_found(ops, dtype, far):

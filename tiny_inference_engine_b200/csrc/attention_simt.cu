@@ -212,6 +212,176 @@ __global__ void __launch_bounds__(128) attention_rows_kernel(AttnArgs a) {
   }
 }
 
+// Rows of prompt portions in float, heads of 32, 64 or 128, plain scores (a window at most): 16 rows of a query head a block, keys in
+// tiles of 32 through two buffers in shared memory (cp.async), so that a key row is read from L2 once per 16 rows instead of once a
+// row, with whole lines in flight (a lane of the rows kernel walks a key row of its own). A half warp holds two rows: scores of two
+// keys a lane, then a sixteenth of the output row a lane. What bounds it is shared memory into registers. Rows of
+// several sequences in one tile are worked through sequence by sequence.
+constexpr int kTileRows = 16, kTileKeys = 32;
+
+template <int DH>
+__global__ void __launch_bounds__(128) attention_rows_tiled_kernel(AttnArgs a) {
+  pdl_sync();
+  constexpr int LD = DH + 4, PIECES = DH / 4, OWN = DH / 16;      // rows 16 bytes apart modulo the banks' 128
+  extern __shared__ __align__(16) float tiles[];
+  float* const qs = tiles;                             // [kTileRows][LD]
+  float* const ring = qs + kTileRows * LD;             // 2 x (keys [kTileKeys][LD], values [kTileKeys][LD])
+  float* const ps = ring + 4 * kTileKeys * LD;         // [kTileRows][kTileKeys + 4]
+  const int t0 = blockIdx.x * kTileRows, h = blockIdx.y, kvh = h / (a.q_heads / a.kv_heads);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r0 = (tid >> 4) * 2, c = tid & 15;
+  const int t_end = min(t0 + kTileRows, a.rows);
+  const float* q = static_cast<const float*>(a.q);
+  const float* kc = static_cast<const float*>(a.k_cache);
+  const float* vc = static_cast<const float*>(a.v_cache);
+  for (int i = tid; i < kTileRows * PIECES; i += 128) {
+    const int r = i / PIECES, d = (i % PIECES) * 4;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (t0 + r < t_end) load4(q + (t0 + r) * a.q_stride + h * DH + d, v);
+    store4(qs + r * LD + d, v);
+  }
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, acc[2][OWN] = {};
+  for (int begin = t0; begin < t_end;) {
+    const int s = a.seq_of_row[begin], end = min(t_end, a.query_start[s + 1]);
+    const int* table = a.block_tables + static_cast<long long>(s) * a.max_blocks;
+    const int shift = a.context_lens[s] - a.query_start[s + 1];      // position of row t: t + shift
+    const int lo = a.window > 0 ? max(0, begin + shift - a.window + 1) : 0, hi = end - 1 + shift;
+    auto fetch = [&](int tile) {
+      const int key0 = lo + tile * kTileKeys;
+      float* kt = ring + (tile & 1) * 2 * kTileKeys * LD;
+      if (key0 <= hi) {
+        for (int i = warp; i < kTileKeys; i += 4) {        // a warp a row
+          const int j = min(key0 + i, hi);
+          const long long row = (static_cast<long long>(table[j / a.page_size]) * a.kv_heads + kvh) * a.page_size + j % a.page_size;
+          if (lane < PIECES) {
+            const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(kt + i * LD + lane * 4));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(kc + row * DH + lane * 4) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + kTileKeys * LD * 4), "l"(vc + row * DH + lane * 4) : "memory");
+          }
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncthreads();                                       // the rows are in place; nobody reads the ring of the sequence before
+    fetch(0);
+    for (int tile = 0; lo + tile * kTileKeys <= hi; ++tile) {
+      fetch(tile + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      const float* kt = ring + (tile & 1) * 2 * kTileKeys * LD;
+      const float* vt = kt + kTileKeys * LD;
+      const int key0 = lo + tile * kTileKeys;
+      float dot[2][2][2] = {};
+#pragma unroll 8
+      for (int d = 0; d < DH; d += 4) {
+        float x[2][4], y[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) load4(qs + (r0 + i) * LD + d, x[i]), load4(kt + (c + 16 * i) * LD + d, y[i]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dot[i][j][e & 1] = fmaf(x[i][e], y[j][e], dot[i][j][e & 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = t0 + r0 + i, pos = t + shift;
+        const bool mine = t >= begin && t < end;
+        const int from = a.window > 0 ? pos - a.window + 1 : 0;
+        float sc[2], top = -INFINITY;
+        bool seen[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int key = key0 + c + 16 * j;
+          seen[j] = mine && key <= pos && key >= from;
+          sc[j] = seen[j] ? a.scale * (dot[i][j][0] + dot[i][j][1]) : -INFINITY;
+          top = fmaxf(top, sc[j]);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float m_new = fmaxf(m[i], top);
+        const float corr = m_new == m[i] ? 1.0f : expf(m[i] - m_new);      // (both -inf: nothing seen yet, nothing to scale)
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float p = seen[j] ? expf(sc[j] - m_new) : 0.0f;
+          ps[(r0 + i) * (kTileKeys + 4) + c + 16 * j] = p;
+          sum += p;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        l[i] = fmaf(l[i], corr, sum);
+        m[i] = m_new;
+#pragma unroll
+        for (int e = 0; e < OWN; ++e) acc[i][e] *= corr;
+      }
+      __syncwarp();                                        // a row's weights are written and read by one half warp
+      // A weight of 0 must not touch a value that the row does not see (0 times a NaN of another request is a NaN): where all
+      // rows see all keys of the tile there is none.
+      const bool whole = begin == t0 && end == t_end && key0 + kTileKeys - 1 <= begin + shift && (a.window <= 0 || key0 >= hi - a.window + 1);
+      auto add = [&](float (&o)[OWN], float p, const float (&v)[OWN]) {
+        if (!whole && p == 0.0f) return;
+#pragma unroll
+        for (int x = 0; x < OWN; ++x) o[x] = fmaf(p, v[x], o[x]);
+      };
+#pragma unroll 2
+      for (int j = 0; j < kTileKeys; j += 4) {
+        float p[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) load4(ps + (r0 + i) * (kTileKeys + 4) + j, p[i]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float v[OWN];
+          const float* vr = vt + (j + e) * LD;
+          if constexpr (DH >= 64) {
+#pragma unroll
+            for (int x = 0; x < OWN; x += 4) {
+              float v4[4];
+              load4(vr + x * 16 + c * 4, v4);
+#pragma unroll
+              for (int y = 0; y < 4; ++y) v[x + y] = v4[y];
+            }
+          } else {
+#pragma unroll
+            for (int x = 0; x < OWN; ++x) v[x] = vr[c * OWN + x];
+          }
+          add(acc[0], p[0][e], v);
+          add(acc[1], p[1][e], v);
+        }
+      }
+      __syncthreads();                                     // through with this buffer: the tile after the next goes there
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    begin = end;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int t = t0 + r0 + i;
+    if (t >= t_end) continue;
+    const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+    float* out = static_cast<float*>(a.out) + (static_cast<long long>(t) * a.q_heads + h) * DH;
+#pragma unroll
+    for (int e = 0; e < OWN; ++e) out[DH >= 64 ? (e >> 2) * 64 + c * 4 + (e & 3) : c * OWN + e] = acc[i][e] * inv;
+  }
+}
+
+// What the tiled kernel takes; everything else is the rows kernel's. (A tile wants rows to share it: few rows run a warp each.)
+inline bool rows_tiled_takes(const AttnArgs& a) {
+  return (a.head_dim == 32 || a.head_dim == 64 || a.head_dim == 128) && a.rows >= kTileRows && a.q_heads <= 65535 && a.q_stride % 4 == 0 &&
+         (reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) % 16 == 0;
+}
+
+template <int DH>
+int launch_rows_tiled(const AttnArgs& a, cudaStream_t s) {
+  constexpr int smem = ((kTileRows + 4 * kTileKeys) * (DH + 4) + kTileRows * (kTileKeys + 4)) * static_cast<int>(sizeof(float));
+  if (cudaFuncSetAttribute(attention_rows_tiled_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    set_error("attention: cannot reserve %d bytes of shared memory", smem);
+    return kCudaError;
+  }
+  TIE_LAUNCH((attention_rows_tiled_kernel<DH>), dim3(ceil_div(a.rows, kTileRows), a.q_heads), 128, smem, s, a);
+  TIE_RETURN_LAUNCH("attention_rows_tiled");
+}
+
 // Split kernel: sequences listed in `seq_list` (each brings exactly one query row).
 // scratch: [n_list, q_heads, max_splits, v_dim + 2] floats (acc, then m, l).
 template <typename T, int DPL>
@@ -573,6 +743,8 @@ TIE_API int tie_attention_rows(int dtype, const void* q, long long q_stride, con
   const AttnArgs a{q, k_cache, v_cache, out, seq_of_row, query_start, context_lens, block_tables, q_stride, max_blocks,
                    rows, seqs, q_heads, kv_heads, head_dim, page_size, window, scale, head_dim};
   if (const int st = check_attn(a)) return st;
+  if (dtype == TIE_F32 && rows_tiled_takes(a))
+    return head_dim == 32 ? launch_rows_tiled<32>(a, s) : head_dim == 64 ? launch_rows_tiled<64>(a, s) : launch_rows_tiled<128>(a, s);
   if (dtype == TIE_F32) return launch_attention<float>(a, nullptr, nullptr, 0, 0, 0, nullptr, 1, s);
   if (dtype == TIE_BF16) return launch_attention<__nv_bfloat16>(a, nullptr, nullptr, 0, 0, 0, nullptr, 1, s);
   set_error("attention: unknown dtype code %d", dtype);
