@@ -1060,3 +1060,63 @@ def test_gemm_with_silu_epilogue(ops, M, I, K):
     out = torch.full((M, I), float("nan"), device="cuda", dtype=torch.bfloat16)
     ops.gemm_silu(dev(a, torch.bfloat16), w, out)
     assert rel_err(host(out), plain.swiglu(plain.linear(a, gate), plain.linear(a, up))) < TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("mode", ["delta", "channel", "head"])
+@pytest.mark.parametrize("H,G,dim,vdim,lens", [(2, 2, 128, 128, [1, 16, 33]), (4, 2, 64, 64, [15, 17]), (3, 3, 128, 20, [50])])
+def test_recurrence_in_chunks(ops, mode, H, G, dim, vdim, lens):
+    """The three recurrences sixteen tokens at a time against the plain loop in float64: chunks that end in the middle, single tokens, value
+    heads that fill no block of columns, decays down to zero; the convolution's inputs as the kernel that walks token by token leaves them;
+    and a token with a NaN leaves the tokens ahead of it in its chunk, and the other sequences, as they are."""
+    from types import SimpleNamespace
+    from tiny_inference_engine_b200.engine.workspace import Workspace
+    if mode == "channel":
+        G = H
+    rng = np.random.default_rng(H * dim + vdim + len(lens))
+    T, per, taps = sum(lens), H // G, 4
+    q, k = rng.standard_normal((T, G, dim)), rng.standard_normal((T, G, dim))
+    q, k = q / np.linalg.norm(q, axis=-1, keepdims=True), k / np.linalg.norm(k, axis=-1, keepdims=True)
+    v = rng.standard_normal((T, H, vdim))
+    beta = rng.uniform(0.1, 1.0, (T, H)) if mode != "channel" else None
+    decay = rng.uniform(0.3, 1.0, (T, H) if mode == "head" else (T, H, dim))
+    decay.reshape(T, H, -1)[T // 2] = 0.0                      # a token that forgets everything
+    S0 = rng.standard_normal((len(lens), H, dim, vdim))
+    C = 2 * G * dim + H * vdim
+    qs = np.concatenate([[0], np.cumsum(lens)])
+
+    def plain_loop(v):
+        out, S = np.zeros((T, H, vdim)), S0.copy()
+        for s, n in enumerate(lens):
+            for t in range(qs[s], qs[s] + n):
+                for h in range(H):
+                    S[s, h] *= decay[t, h] if mode == "head" else decay[t, h][:, None]
+                    u = v[t, h] * (1.0 if beta is None else beta[t, h])
+                    if mode == "delta":
+                        u = u - beta[t, h] * (S[s, h].T @ k[t, h // per])
+                    S[s, h] += np.outer(k[t, h // per], u)
+                    out[t, h] = S[s, h].T @ q[t, h // per]
+        return out, S
+
+    proj = dev(rng.standard_normal((T, C)), torch.bfloat16)
+    state0 = dev(np.concatenate([S0.reshape(len(lens), -1), rng.standard_normal((len(lens), (taps - 1) * C))], axis=1))
+
+    def engine(v, chunked):
+        rows = [dev(x.reshape(T, -1)) for x in (q, k, v)]
+        state, out = state0.clone(), torch.empty(T, H * vdim, device="cuda")
+        ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=10 ** 6 if chunked else 1, max_seqs=len(lens))
+        ops.delta_rule(*rows, None if beta is None else dev(beta), dev(decay.reshape(T, -1)), state, H * dim * vdim, proj, 0, G * dim, 2 * G * dim,
+                       dev(qs, torch.int32), dev(np.arange(len(lens)), torch.int32), len(lens), H, G, dim, vdim, taps, out, plain=mode != "delta",
+                       decay_per_head=mode == "head", chunks=ops.RecurrenceChunks(ctx))
+        return host(out), host(state)
+
+    want, S = plain_loop(v)
+    out, state = engine(v, True)
+    _, by_token = engine(v, False)
+    assert rel_err(out, want.reshape(T, -1)) < TOL["float32"]
+    assert rel_err(state[:, :H * dim * vdim], S.reshape(len(lens), -1)) < TOL["float32"]
+    assert np.array_equal(state[:, H * dim * vdim:], by_token[:, H * dim * vdim:])
+    sick = T - 2
+    v = v.copy()
+    v[sick] = np.nan
+    out, _ = engine(v, True)
+    assert rel_err(out[:sick], want.reshape(T, -1)[:sick]) < TOL["float32"] and np.isnan(out[sick:]).all()

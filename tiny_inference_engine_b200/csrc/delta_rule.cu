@@ -23,13 +23,9 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "delta_state.cuh"
 
 namespace tie {
-
-struct DeltaShape {
-  int heads, kv_heads, dim, vdim, taps;
-  int channels() const { return 2 * kv_heads * dim + heads * vdim; }
-};
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
@@ -478,23 +474,8 @@ __global__ void __launch_bounds__(kDeltaCols * LANES) delta_rule_kernel(
       if (col0 + c < vdim) S[static_cast<long long>(r) * vdim + col0 + c] = stage[r * kDeltaPad + c];
     }
   }
-  // The convolution's last taps - 1 inputs after this step: from the step's rows where it brought enough, else
-  // what the slot held moves up. Every block of the sequence takes a slice of the channels.
-  if (sh.taps > 1) {
-    const int C = 2 * nqk + nv, keep = sh.taps - 1;
-    const int blocks = gridDim.y * gridDim.z, mine = blockIdx.y * gridDim.z + blockIdx.z;
-    const int per = (C + blocks - 1) / blocks;
-    const int c_end = min(C, (mine + 1) * per);
-    float* tail = state + slot * state_stride + conv_state_off;
-    for (int c = mine * per + threadIdx.x; c < c_end; c += blockDim.x) {
-      const int pc = c < nqk ? q_off + c : (c < 2 * nqk ? k_off + (c - nqk) : v_off + (c - 2 * nqk));
-      for (int i = 0; i < keep; ++i) {
-        const int from = n - keep + i;        // offset in the step of the token that lands at place i
-        tail[static_cast<long long>(i) * C + c] = from >= 0 ? ld(proj + (t0 + from) * proj_stride + pc)
-                                                            : tail[static_cast<long long>(n + i) * C + c];
-      }
-    }
-  }
+  move_conv_tail(sh, state + slot * state_stride + conv_state_off, proj, proj_stride, q_off, k_off, v_off, t0, n,
+                 blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z);
 }
 
 template <typename T>

@@ -722,16 +722,37 @@ def delta_prep(proj, q_off: int, k_off: int, v_off: int, b_off: int, conv_w, sta
          _stream())
 
 
+def chunks_pay(longest: int, seqs: int) -> bool:
+    """Whether a step's recurrence is faster in chunks. Token by token, a portion of n tokens is a chain of n steps (0.25 us each with the
+    delta rule, 0.16 and 0.11 us without, heads of 128); in chunks it is n / 16 steps of 1.6 to 2 us behind a launch of its own. The two meet at
+    about 90 tokens (64: 22 against 31 us, 2,048: 514 against 305). Sequences that bring one token cost either kernel the trip of
+    their state, the chunked one about a microsecond each more (128 tokens beside 30 of them: 98 against 109 us)."""
+    return longest >= 88 + 8 * seqs
+
+
+class RecurrenceChunks:
+    """What `delta_rule` needs to go through a step in chunks: the step's workspace and how many tokens its longest portion brings."""
+
+    def __init__(self, ctx):
+        self.ws, self.longest, self.max_seqs = ctx.ws, ctx.multi_max_queries, ctx.max_seqs
+
+    def scratch(self, lib, tokens: int, seqs: int, heads: int, dim: int, plain: bool) -> torch.Tensor:
+        most = lib.tie_delta_chunk_scratch(self.ws.max_rows, self.max_seqs, heads, dim, int(plain))
+        return self.ws.flat("delta.chunks", lib.tie_delta_chunk_scratch(tokens, seqs, heads, dim, int(plain)), torch.float32, most)
+
+
 def delta_rule(qn, kn, vn, beta, decay, state, conv_state_off: int, proj, q_off: int, k_off: int, v_off: int,
                query_start, state_slots, seqs: int, heads: int, kv_heads: int, dim: int, vdim: int, taps: int, out,
-               plain: bool = False, decay_per_head: bool = False, single: bool = False) -> None:
+               plain: bool = False, decay_per_head: bool = False, single: bool = False, chunks=None) -> None:
     """The recurrence over each sequence's tokens of the step: per head S <- decay S; u = beta (v - S^T k);
     S <- S + k u^T; o = S^T q, with `decay` float32 [T, >= heads * dim] per head and key channel (`delta_prep`).
     S [heads, dim, vdim] sits at the start of the sequence's row of `state` and is updated; so are the convolution's
     last inputs (from the q, k, v columns of `proj`). out float32 [T, heads * vdim].
     `plain`: no correction, u = beta v (beta None: u = v), which is the recurrence of gated linear attention and of
     state-space layers, S <- diag(decay) S + k u^T. `decay_per_head`: decay is float32 [T, >= heads], one factor for
-    all key channels of a head. `single`: every sequence brings one token (a hint: how the launch is cut, not what it computes)."""
+    all key channels of a head. `single`: every sequence brings one token (a hint: how the launch is cut, not what it computes).
+    `chunks` (a `RecurrenceChunks`): the rows qn, kn, vn and decay are the caller's to lose, and a step with a long enough portion may
+    go through it sixteen tokens at a time; they are then overwritten."""
     _dev(qn, kn, vn, beta, decay, state, proj, query_start, state_slots, out)
     T = proj.shape[0]
     _need(beta is not None or plain, "delta_rule: the delta rule needs beta")
@@ -741,6 +762,16 @@ def delta_rule(qn, kn, vn, beta, decay, state, conv_state_off: int, proj, q_off:
     _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1 and conv_state_off >= heads * dim * vdim,
           "delta_rule: state rows too short")
     _need(query_start.numel() >= seqs + 1 and state_slots.numel() >= seqs, "delta_rule: index tensors too short")
+    if chunks is not None and not single and chunks_pay(chunks.longest, seqs):
+        lib = library.library()
+        scratch = chunks.scratch(lib, T, seqs, heads, dim, plain)
+        if lib.tie_delta_chunk_takes(heads, kv_heads, dim, vdim, int(plain), int(decay_per_head), decay.stride(0), state.stride(0), qn.data_ptr(),
+                                     kn.data_ptr(), vn.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), scratch.data_ptr()):
+            call("tie_delta_rule_chunked", dtype_code(proj), qn.data_ptr(), kn.data_ptr(), vn.data_ptr(), _ptr(beta), decay.data_ptr(),
+                 decay.stride(0), state.data_ptr(), state.stride(0), conv_state_off, proj.data_ptr(), proj.stride(0), q_off, k_off, v_off,
+                 query_start.data_ptr(), state_slots.data_ptr(), seqs, T, heads, kv_heads, dim, vdim, taps, out.data_ptr(), 1 if plain else 0,
+                 1 if decay_per_head else 0, scratch.data_ptr(), _stream())
+            return
     call("tie_delta_rule", dtype_code(proj), qn.data_ptr(), kn.data_ptr(), vn.data_ptr(), _ptr(beta), decay.data_ptr(),
          decay.stride(0), state.data_ptr(), state.stride(0), conv_state_off, proj.data_ptr(), proj.stride(0), q_off, k_off, v_off,
          query_start.data_ptr(), state_slots.data_ptr(), seqs, heads, kv_heads, dim, vdim, taps, out.data_ptr(),

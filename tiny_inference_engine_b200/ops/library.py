@@ -50,6 +50,7 @@ _SIGNATURES = {
     "tie_scale_rows": [P, L, I, I, F, P],
     "tie_qkv_span_prep": [I, P, L, I, I, I, P, P, P, P, P, F, P, P, I, I, P, P, P, P, I, I, I, I, I, I, I, I, P, P, P],
     "tie_delta_prep": [I, P, L, I, I, I, I, P, P, L, L, P, P, P, I, I, I, I, I, I, F, F, P, P, P, P, P, L, P, P, P],
+    "tie_delta_rule_chunked": [I, P, P, P, P, P, L, P, L, L, P, L, I, I, I, P, P, I, I, I, I, I, I, I, P, I, I, P, P],
     "tie_delta_rule": [I, P, P, P, P, P, L, P, L, L, P, L, I, I, I, P, P, I, I, I, I, I, I, P, I, I, I, P],
     "tie_delta_out": [I, P, P, L, P, F, P, I, I, I, P],
     "tie_gemm_simt_batched": [I, I, P, P, P, I, I, I, L, L, L, I, L, L, L, P],
@@ -150,6 +151,10 @@ def library() -> ctypes.CDLL:
         lib.tie_attention_mixed_tc_takes.argtypes = [c_int, c_int, c_int, c_int]
         lib.tie_gemm_heads_mma_takes.restype = c_int
         lib.tie_gemm_heads_mma_takes.argtypes = [P, L, I, P, P, L, I, I, I]
+        lib.tie_delta_chunk_takes.restype = c_int
+        lib.tie_delta_chunk_takes.argtypes = [I, I, I, I, I, I, L, L, P, P, P, P, P, P, P]
+        lib.tie_delta_chunk_scratch.restype = c_longlong
+        lib.tie_delta_chunk_scratch.argtypes = [I, I, I, I, I]
         lib.tie_moe_max_tiles.restype = c_int
         lib.tie_moe_max_tiles.argtypes = [c_int, c_int, c_int]
         lib.tie_replay_launcher_id.restype = c_int
