@@ -1120,3 +1120,75 @@ def test_recurrence_in_chunks(ops, mode, H, G, dim, vdim, lens):
     v[sick] = np.nan
     out, _ = engine(v, True)
     assert rel_err(out[:sick], want.reshape(T, -1)[:sick]) < TOL["float32"] and np.isnan(out[sick:]).all()
+
+
+def softmax_reference(q, k, v, scale, window, sink, start):
+    """q [n, H, d], k [m, G, d], v [m, G, e] in float64; row i sits at start + i. Returns [n, H, e]."""
+    n, H, G = q.shape[0], q.shape[1], k.shape[1]
+    far = (start + np.arange(n))[:, None] - np.arange(k.shape[0])[None, :]
+    seen = (far >= 0) & ((far < window) if window else (far >= 0))
+    out = np.zeros((n, H, v.shape[2]))
+    for h in range(H):
+        z = np.where(seen, scale * (q[:, h] @ k[:, h // (H // G)].T), -np.inf)
+        top = z.max(-1, keepdims=True) if sink is None else np.maximum(z.max(-1, keepdims=True), sink[h])
+        e = np.exp(z - top)
+        total = e.sum(-1, keepdims=True) + (0.0 if sink is None else np.exp(sink[h] - top))
+        out[:, h] = (e / total) @ v[:, h // (H // G)]
+    return out
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv,page,window,new,ctx,sinks", [
+    (4, 2, 16, 0, [129, 64], [129, 400], False), (3, 3, 64, 100, [300], [333], True), (8, 1, 8, 0, [33, 2, 17], [33, 65, 700], True),
+    (2, 2, 16, 0, [513], [513], False)])
+def test_exact_prompt_attention_on_tcgen05(ops, Dh, Hq, Hkv, page, window, new, ctx, sinks):
+    """Rows and keys that end inside tiles, portions behind cached keys, windows, sinks, one and two row tiles a CTA; weights in two
+    bfloat16 terms, so the rounding of the output is what is left of the error."""
+    rng = np.random.default_rng(Hq * Dh + sum(ctx))
+    kc, vc, bt, ks, vs = paged_cache(rng, "bfloat16", ctx, Hkv, Dh, page, 90 * 16 // page + 8)
+    T, qs = sum(new), np.concatenate([[0], np.cumsum(new)])
+    q = as_stored(rng.standard_normal((T, Hq * Dh)) * 2, "bfloat16")
+    sink = rng.uniform(-2, 6, Hq).astype(np.float32) if sinks else None
+    out = torch.full((T, Hq * Dh), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.attention_prompt_exact(dev(q, torch.bfloat16), dev(kc, torch.bfloat16), dev(vc, torch.bfloat16), out, dev(qs, torch.int32),
+                               dev(np.array(ctx), torch.int32), dev(bt, torch.int32), len(new), max(new), Hq, Hkv, Dh, Dh ** -0.5, window,
+                               None if sink is None else dev(sink))
+    want = np.concatenate([softmax_reference(q[qs[i]:qs[i + 1]].reshape(-1, Hq, Dh).astype(np.float64), ks[i].astype(np.float64),
+                                             vs[i].astype(np.float64), Dh ** -0.5, window, sink, ctx[i] - new[i]) for i in range(len(new))])
+    assert rel_err(host(out), want.reshape(T, -1)) < TOL["bfloat16"]
+    # 2-norm: one rounding to bfloat16 is 2^-9 / sqrt(3) = 1.1e-3 of a value at most; weights in one term would add 1.1e-3 of their own
+    assert np.linalg.norm(host(out) - want.reshape(T, -1)) < 2.0e-3 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("H,page,window,new,ctx,sinks", [(2, 16, 0, [200, 65], [200, 65], True), (3, 8, 90, [130, 64], [260, 321], False),
+                                                         (1, 64, 0, [300], [450], True)])
+def test_latent_attention_over_expanded_keys(ops, H, page, window, new, ctx, sinks):
+    """Gathered latents (each sequence padded to whole tiles with zeros), and attention over keys and values per head beside a rotated part that all
+    heads share."""
+    rng = np.random.default_rng(H + sum(ctx))
+    rank, kd = 64, 128
+    kc, _, bt, ks, _ = paged_cache(rng, "bfloat16", ctx, 1, kd, page, 60 * 16 // page + 8)
+    T, qs = sum(new), np.concatenate([[0], np.cumsum(new)])
+    index = (dev(qs, torch.int32), dev(np.array(ctx), torch.int32))
+    rows = ops.latent_expanded_rows(ctx, new, window)
+    latents = torch.full((rows, kd), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.latent_gather(dev(kc, torch.bfloat16), *index, dev(bt, torch.int32), len(new), window, latents)
+    firsts = [max(0, c - n - window + 1) // 64 * 64 if window else 0 for c, n in zip(ctx, new)]
+    want_rows = np.concatenate([np.concatenate([k[f:, 0], np.zeros((-(len(k) - f) % 64, kd))]) for k, f in zip(ks, firsts)])
+    assert np.array_equal(host(latents), want_rows)
+    kv = as_stored(rng.standard_normal((rows, H * 256)), "bfloat16")
+    q = as_stored(rng.standard_normal((T, H * 192)) * 1.5, "bfloat16")
+    sink = rng.uniform(-2, 6, H).astype(np.float32) if sinks else None
+    out = torch.full((T, H * 128), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.attention_latent_expanded(dev(q, torch.bfloat16), latents, dev(kv, torch.bfloat16), out, *index, len(new), max(new), H, 192 ** -0.5, window,
+                                  None if sink is None else dev(sink))
+    want, base = [], 0
+    for i, (n, c) in enumerate(zip(new, ctx)):
+        m = c - firsts[i]
+        k = np.concatenate([kv[base:base + m, :H * 128].reshape(m, H, 128), np.repeat(want_rows[base:base + m, None, rank:], H, axis=1)], axis=-1)
+        v = kv[base:base + m, H * 128:].reshape(m, H, 128)
+        want.append(softmax_reference(q[qs[i]:qs[i + 1]].reshape(n, H, 192).astype(np.float64), k.astype(np.float64), v.astype(np.float64), 192 ** -0.5,
+                                      window, sink, c - n - firsts[i]))
+        base += -(-m // 64) * 64
+    want = np.concatenate(want).reshape(T, -1)
+    assert np.linalg.norm(host(out) - want) < 2.0e-3 * np.linalg.norm(want)

@@ -46,44 +46,6 @@ struct UmmaPromptArgs {
   int cta_rows;   // 256: a CTA works on two row tiles side by side; 128: on one (more CTAs when there are few rows)
 };
 
-// Descriptor of an operand stored with its MN extent contiguous (V as [key][head dim]): 64 elements of
-// MN per 128-byte row, 8 rows (k) per 1024-byte swizzle atom; `mn_block_bytes` apart lie successive blocks
-// of 64 along MN.
-__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t addr, uint32_t mn_block_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((addr >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>((mn_block_bytes >> 4) & 0x3FFF) << 16;   // leading byte offset
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                         // stride byte offset: next 8 k
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
-// D[tmem_d] (+)= A[tmem_a] . B: the A operand read from tensor memory (lane = row, a 32-bit column = two
-// consecutive k of 16 bits), B from shared memory.
-__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int DH, int STAGES>
 __global__ void __launch_bounds__(kUmmaAttnThreads, 1)
 attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, UmmaPromptArgs a) {

@@ -368,6 +368,58 @@ def attention_prompt_umma(q, k_cache, v_cache, out, query_start, context_lens, b
          max_queries, q_heads, kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], int(window), float(scale), _stream())
 
 
+def attention_prompt_exact(q, k_cache, v_cache, out, query_start, context_lens, block_tables, n_seqs: int, max_queries: int,
+                           q_heads, kv_heads, head_dim, scale: float, window: int = 0, sink=None) -> None:
+    """As attention_prompt_tma with `exact_weights`, on tcgen05 (head sizes 64 and 128; what `attention_prompt_umma_takes` says). `sink`
+    (float32 [q_heads] or None): exp(sink) is one more term of a softmax's denominator."""
+    _dev(q, k_cache, v_cache, out, query_start, context_lens, block_tables, sink)
+    _attn_common(q, k_cache, v_cache, out, query_start, context_lens, block_tables, q_heads, kv_heads, head_dim)
+    _need(out.is_contiguous(), "attention: out must be contiguous")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == q_heads), "attention: sink must be float32 [q_heads]")
+    call("tie_attention_prompt_exact", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
+         query_start.data_ptr(), context_lens.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], n_seqs, max_queries, q_heads,
+         kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], int(window), float(scale), _ptr(sink), _stream())
+
+
+EXPANDED_KEY, EXPANDED_ROT, EXPANDED_VALUE = 128, 64, 128      # sizes of a head that the expanded latent attention is made for
+EXPANDED_TILE = 64
+
+
+def latent_expanded_rows(contexts, queries, window: int) -> int:
+    """Rows of multiplied-out keys that portions of these sequences need (host numbers): each from the first key that one of its rows sees,
+    rounded down to a whole tile of 64, to its last, rounded up."""
+    rows = 0
+    for context, n in zip(contexts, queries):
+        first = max(0, int(context) - int(n) - window + 1) // EXPANDED_TILE * EXPANDED_TILE if window > 0 else 0
+        rows += -(-(int(context) - first) // EXPANDED_TILE) * EXPANDED_TILE
+    return rows
+
+
+def latent_gather(k_cache, query_start, context_lens, block_tables, n_seqs: int, window: int, out) -> None:
+    """out [rows, key_dim] bfloat16: the cached rows (k_cache [pages, 1, page_size, key_dim]) that the portions of sequences 0..n_seqs-1 see,
+    in order, padded with zeros to whole tiles (`latent_expanded_rows`)."""
+    _dev(k_cache, query_start, context_lens, block_tables, out)
+    _need(k_cache.dim() == 4 and k_cache.is_contiguous() and k_cache.shape[1] == 1 and k_cache.dtype == torch.bfloat16 and out.dim() == 2 and
+          out.is_contiguous() and out.dtype == torch.bfloat16 and out.shape[1] == k_cache.shape[3], "latent_gather: bfloat16 key plane and rows")
+    call("tie_latent_gather", k_cache.data_ptr(), query_start.data_ptr(), context_lens.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+         n_seqs, int(window), k_cache.shape[2], k_cache.shape[3], out.shape[0], out.data_ptr(), _stream())
+
+
+def attention_latent_expanded(q, latents, kv, out, query_start, context_lens, n_seqs: int, max_queries: int, heads: int, scale: float,
+                              window: int = 0, sink=None) -> None:
+    """Attention of the portions of sequences 0..n_seqs-1 over multiplied-out latents: q [T, heads * 192] (128 and 64 rotated), latents
+    [rows, key_dim] from `latent_gather` (the rotated key part in its last 64 columns), kv [rows, heads * 256] (every head's key, then every
+    head's value), out [T, heads * 128]. Softmax weights as in `attention_prompt_exact`."""
+    _dev(q, latents, kv, out, query_start, context_lens, sink)
+    _need(all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 for t in (q, latents, kv, out)) and latents.is_contiguous() and
+          kv.is_contiguous() and out.is_contiguous() and q.shape[1] >= heads * 192 and kv.shape == (latents.shape[0], heads * 256) and
+          out.shape == (q.shape[0], heads * 128), "latent attention: bfloat16 q [T, heads * 192], kv [rows, heads * 256], out [T, heads * 128]")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == heads), "latent attention: sink must be float32 [heads]")
+    call("tie_attention_latent_expanded", q.data_ptr(), q.stride(0), latents.data_ptr(), latents.shape[1], kv.data_ptr(), kv.shape[0],
+         out.data_ptr(), query_start.data_ptr(), context_lens.data_ptr(), n_seqs, max_queries, heads, int(window), float(scale), _ptr(sink),
+         _stream())
+
+
 CLUSTER_SPLITS = (2, 4, 8, 16)      # how many splits the decode attention merges as one thread-block cluster
 
 

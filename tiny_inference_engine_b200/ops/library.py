@@ -50,6 +50,9 @@ _SIGNATURES = {
     "tie_scale_rows": [P, L, I, I, F, P],
     "tie_qkv_span_prep": [I, P, L, I, I, I, P, P, P, P, P, F, P, P, I, I, P, P, P, P, I, I, I, I, I, I, I, I, P, P, P],
     "tie_delta_prep": [I, P, L, I, I, I, I, P, P, L, L, P, P, P, I, I, I, I, I, I, F, F, P, P, P, P, P, L, P, P, P],
+    "tie_attention_prompt_exact": [P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, P],
+    "tie_latent_gather": [P, P, P, P, I, I, I, I, I, I, P, P],
+    "tie_attention_latent_expanded": [P, L, P, I, P, I, P, P, P, I, I, I, I, F, P, P],
     "tie_delta_rule_chunked": [I, P, P, P, P, P, L, P, L, L, P, L, I, I, I, P, P, I, I, I, I, I, I, I, P, I, I, P, P],
     "tie_delta_rule": [I, P, P, P, P, P, L, P, L, L, P, L, I, I, I, P, P, I, I, I, I, I, I, P, I, I, I, P],
     "tie_delta_out": [I, P, P, L, P, F, P, I, I, I, P],

@@ -163,8 +163,11 @@ class GatedWindowAttention(Mixer):
         as two bfloat16 terms (`exact_weights`), so that they keep 16 bits of mantissa."""
         H, G, Dh = self.heads, self.kv_heads, self.head_dim
         if ctx.multi_rows > 0:
-            ops.attention_prompt_tma(q, cache.k, cache.v, attn, ctx.query_start, ctx.context_lens, g.block_tables, ctx.multi_seqs,
-                                     ctx.multi_max_queries, H, G, Dh, self.scale, self.window, exact_weights=True)
+            index = (ctx.query_start, ctx.context_lens, g.block_tables, ctx.multi_seqs, ctx.multi_max_queries)
+            if ops.attention_prompt_umma_takes(q, H, G, Dh, cache.k.shape[2], ctx.multi_max_queries):
+                ops.attention_prompt_exact(q, cache.k, cache.v, attn, *index, H, G, Dh, self.scale, self.window)
+            else:
+                ops.attention_prompt_tma(q, cache.k, cache.v, attn, *index, H, G, Dh, self.scale, self.window, exact_weights=True)
         if ctx.single_count > 0:
             longest = ctx.single_max_context if self.window <= 0 else min(ctx.single_max_context, self.window)
             page = cache.k.shape[2]

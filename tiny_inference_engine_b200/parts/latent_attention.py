@@ -33,6 +33,13 @@ LATENT_SPLIT_KEYS = 128     # least keys per split of a sequence that brings one
 LATENT_ROWS = 32            # (token, head) rows of a block of that kernel; one block an SM
 
 
+# Portions multiply the cached latents out into keys and values per head (csrc/attention_prompt_exact.cu) where these cost less than the folded
+# queries' 576 + 512 dimensions a pair: from EXPAND_MIN_TOKENS tokens on (one layer of 32 heads of 128 + 64, 2,048 tokens: 1,940 us
+# folded, products and all, about 150 expanded), and up to EXPAND_MAX_KEYS keys in all, which bounds what the step keeps for it (16 KB a key with 32 heads).
+EXPAND_MIN_TOKENS = 64
+EXPAND_MAX_KEYS = 16384
+
+
 def latent_split_keys(longest: int, sequences: int, heads: int) -> int:
     """Keys per split: as few splits as give every SM a block (what a split leaves for the merge is `rank` floats a head), in whole
     tiles of 64 keys, at least LATENT_SPLIT_KEYS."""
@@ -115,6 +122,12 @@ class LatentAttention(Mixer):
         # per head: q' = Wuk_h^T q_plain (weights [heads, rank, dim]) and out_h = Wuv_h ctx_h (weights [heads, vdim, rank])
         self.w_fold = to_compute(get(n("uk")), self.dtype).view(H, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = to_compute(get(n("uv")), self.dtype).view(H, self.vdim, self.rank).contiguous()
+        # for portions, the same two maps as one product over the latents: every head's key dimensions, then every head's value
+        self.gemm_kv = None
+        if self.dtype == torch.bfloat16 and self.rank % 8 == 0 and \
+                (self.dim, self.rot, self.vdim) == (ops.EXPANDED_KEY, ops.EXPANDED_ROT, ops.EXPANDED_VALUE):
+            self.gemm_kv = ops.bound_gemm(torch.cat([to_compute(get(n(leaf)), self.dtype) for leaf in ("uk", "uv")], dim=0).contiguous(),
+                                          split_many=False)
         self.gemm_o = ops.bound_gemm(to_compute(get(n("o")), self.dtype).contiguous(), split_many=True)
         self.w_o = self.gemm_o.w
         self.wq_norm = get(n("dq.norm")).to(torch.float32).contiguous()
@@ -144,13 +157,15 @@ class LatentAttention(Mixer):
                         table, ctx.positions, g.slots, cq, cache.k, neighbours)
         q = ctx.ws.rows("lattn.q", T, H * (self.dim + self.rot), self.dtype)
         self.gemm_uq(cq, q)
-        folded = ctx.ws.rows("lattn.folded", T, H * self.key_dim, self.dtype)
-        ops.gemm_heads(q, self.w_fold, folded, H)
-        ops.latent_query_rot(q, self.dim, self.rot, table, ctx.positions, folded, self.rank, H, neighbours)
-        mixed = ctx.ws.rows("lattn.mixed", T, H * self.rank, self.dtype)       # per head: the weighted sum of latents
-        self._attend(folded, mixed, ctx, g, cache)
         attn = ctx.ws.rows("lattn.out", T, H * self.vdim, self.dtype)
-        ops.gemm_heads(mixed, self.w_uv, attn, H)
+        done = self._attend_expanded(q, attn, table, neighbours, ctx, g, cache)      # rows of portions, or none
+        if done < T:
+            folded = ctx.ws.rows("lattn.folded", T, H * self.key_dim, self.dtype)
+            ops.gemm_heads(q[done:], self.w_fold, folded[done:], H)
+            ops.latent_query_rot(q[done:], self.dim, self.rot, table, ctx.positions[done:T], folded[done:], self.rank, H, neighbours)
+            mixed = ctx.ws.rows("lattn.mixed", T, H * self.rank, self.dtype)       # per head: the weighted sum of latents
+            self._attend(folded, mixed, ctx, g, cache, ctx.multi_rows - done)
+            ops.gemm_heads(mixed[done:], self.w_uv, attn[done:], H)
         gate = proj[:, self.g_off:self.g_off + self.gates]
         if self.output_gate == "head":
             ops.head_gate_mul(attn, gate, H, self.vdim)
@@ -161,11 +176,35 @@ class LatentAttention(Mixer):
             self._capacity = ops.partial_capacity(ctx.ws.max_rows, self.gemm_o.N, self.gemm_o.K)
         return self.gemm_o(attn, out, lambda m: ctx.ws.flat("mixer.out.partial", m, torch.float32, self._capacity))
 
-    def _attend(self, folded, mixed, ctx, g, cache):
+    def _attend_expanded(self, q, attn, table, neighbours, ctx, g, cache) -> int:
+        """The rows of portions over keys and values multiplied out of the latents they see (q's rotated part is rotated in place).
+        Returns how many rows it took: all of the portions', or none."""
+        n, S = ctx.multi_rows, ctx.multi_seqs
+        if self.gemm_kv is None or n < EXPAND_MIN_TOKENS or cache.k.dtype != torch.bfloat16:
+            return 0
+        key = ("latent_expanded_rows", self.window)
+        rows = ctx.memo.get(key)
+        if rows is None:
+            starts = ctx.host.query_start
+            rows = ctx.memo[key] = ops.latent_expanded_rows(ctx.host.context_lens[:S], starts[1:S + 1] - starts[:S], self.window)
+        if rows > EXPAND_MAX_KEYS:
+            return 0
+        H, wide = self.heads, self.heads * (self.dim + self.vdim)
+        most = min(EXPAND_MAX_KEYS, 2 * ctx.ws.max_rows)
+        latents = ctx.ws.flat("lattn.latents", rows * self.key_dim, self.dtype, most * self.key_dim)[:rows * self.key_dim].view(rows, self.key_dim)
+        kv = ctx.ws.flat("lattn.kv", rows * wide, self.dtype, most * wide)[:rows * wide].view(rows, wide)
+        ops.latent_gather(cache.k, ctx.query_start, ctx.context_lens, g.block_tables, S, self.window, latents)
+        self.gemm_kv(latents[:, :self.rank], kv)
+        ops.latent_query_rot(q[:n], self.dim, self.rot, table, ctx.positions[:n], q[:n], self.dim, H, neighbours)
+        ops.attention_latent_expanded(q[:n], latents, kv, attn[:n], ctx.query_start, ctx.context_lens, S, ctx.multi_max_queries, H, self.scale,
+                                      self.window, self.sink)
+        return n
+
+    def _attend(self, folded, mixed, ctx, g, cache, n):
         """One kv head of `key_dim` for all query heads; a value is the first `rank` elements of its key. bfloat16 with
-        sizes in whole MMA steps runs on the tensor cores, everything else (float32 above all) on the CUDA cores."""
+        sizes in whole MMA steps runs on the tensor cores, everything else (float32 above all) on the CUDA cores. n: the rows of
+        portions that are still to do (all or none)."""
         H = self.heads
-        n = ctx.multi_rows
         if ops.attention_latent_mma_takes(folded, cache.k, self.key_dim, self.rank):
             if n > 0:
                 ops.attention_latent_prompt(folded, cache.k, mixed, ctx.query_start, ctx.context_lens, g.block_tables, ctx.multi_seqs,
