@@ -1192,3 +1192,22 @@ def test_latent_attention_over_expanded_keys(ops, H, page, window, new, ctx, sin
         base += -(-m // 64) * 64
     want = np.concatenate(want).reshape(T, -1)
     assert np.linalg.norm(host(out) - want) < 2.0e-3 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv,page,window,new,ctx", [
+    (4, 2, 16, 0, [130], [2600]), (8, 2, 16, 0, [300, 3], [2351, 40]), (4, 4, 64, 700, [700], [1500]), (32, 8, 8, 0, [260], [2119])])
+def test_keys_shared_out_over_a_cluster(ops, Dh, Hq, Hkv, page, window, new, ctx):
+    """Few rows behind many keys: two and four CTAs share out the key tiles of 256 rows; a short sequence beside the long one leaves CTAs without
+    keys, the last rows of a portion leave row tiles without any."""
+    rng = np.random.default_rng(Hq * Dh + sum(ctx))
+    kc, vc, bt, ks, vs = paged_cache(rng, "bfloat16", ctx, Hkv, Dh, page, 180 * 16 // page + 8)
+    T, qs = sum(new), np.concatenate([[0], np.cumsum(new)])
+    q = as_stored(rng.standard_normal((T, Hq * Dh)) * 2, "bfloat16")
+    out = torch.full((T, Hq * Dh), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.attention_prompt_umma(dev(q, torch.bfloat16), dev(kc, torch.bfloat16), dev(vc, torch.bfloat16), out, dev(qs, torch.int32),
+                              dev(np.array(ctx), torch.int32), dev(bt, torch.int32), len(new), max(new), Hq, Hkv, Dh, Dh ** -0.5, window,
+                              max_keys=4096)
+    want = np.concatenate([softmax_reference(q[qs[i]:qs[i + 1]].reshape(-1, Hq, Dh).astype(np.float64), ks[i].astype(np.float64),
+                                             vs[i].astype(np.float64), Dh ** -0.5, window, None, ctx[i] - new[i]) for i in range(len(new))])
+    assert rel_err(host(out), want.reshape(T, -1)) < TOL["bfloat16"]

@@ -23,7 +23,9 @@
 //   9         one thread issues the MMAs: Q K^T of tile i + 1 ahead of P V of tile i.
 // Barriers: kv_full/kv_empty per stage, and for each row tile s_full (scores written), s_empty
 // (scores read), p_full[2] (P written, O rescaled), p_empty[2] (P V retired). Every wait is bounded.
-// grid = (kv heads, row tiles, sequences): CTAs start in that order with the last row tiles first, so the
+// Where the rows are few and the keys many, 2 or 4 CTAs of a thread-block cluster share out the keys of 256 rows and put their sums
+// together through distributed shared memory.
+// grid = (kv heads, row tiles, sequences x splits): CTAs start in that order with the last row tiles first, so the
 // tiles with the most keys of every kv head run first.
 #include "attention_mma.cuh"
 #include "umma.cuh"
@@ -32,6 +34,8 @@
 namespace tie {
 
 constexpr int kUmmaAttnThreads = 320;
+constexpr int kUmmaMaxSplits = 4;
+constexpr int kUmmaSplitKeys = 2049;
 
 struct UmmaPromptArgs {
   const __nv_bfloat16* q;
@@ -43,6 +47,7 @@ struct UmmaPromptArgs {
   long long q_stride;
   int max_blocks, q_heads, kv_heads, page_size, page_shift, window;
   float scale_log2;
+  int splits;     // CTAs of a cluster that share out the keys of 256 rows (1: no cluster)
   int cta_rows;   // 256: a CTA works on two row tiles side by side; 128: on one (more CTAs when there are few rows)
 };
 
@@ -74,7 +79,7 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int seq = blockIdx.z, kvh = blockIdx.x;
+  const int seq = blockIdx.z / a.splits, rank = blockIdx.z % a.splits, kvh = blockIdx.x;
   const int G = a.q_heads / a.kv_heads;
   const int t0 = a.query_start[seq];
   const int nq = a.query_start[seq + 1] - t0;
@@ -94,7 +99,18 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
     first[q] = a.window > 0 ? max(0, lo_pos - a.window + 1) / kKeysPerTile : 0;
     last[q] = hi_pos / kKeysPerTile;
   }
-  const int kt_first = first[0], kt_last = has[1] ? last[1] : last[0];
+  int kt_first = first[0], kt_last = has[1] ? last[1] : last[0];
+  if (a.splits > 1) {             // this CTA's share of the key tiles
+    const int per = (kt_last - kt_first + a.splits) / a.splits;
+    kt_first += rank * per;
+    kt_last = min(kt_last, kt_first + per - 1);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      first[q] = max(first[q], kt_first);
+      last[q] = min(last[q], kt_last);
+      has[q] = has[q] && first[q] <= last[q];
+    }
+  }
   const int n_tiles = kt_last - kt_first + 1;
 
   if (threadIdx.x == 0) {
@@ -362,25 +378,95 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
     }
     if (ok && my_tiles > 0) {
       ok = __all_sync(0xffffffffu, mbar_wait(p_empty + 2 * q + ((my_tiles - 1) & 1), ((my_tiles - 1) >> 1) & 1, abort_flag, a.status, 13) ? 1 : 0) != 0;
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-        __nv_bfloat16* o_row = row < rows ? a.out + (static_cast<long long>(t0 + row / G) * a.q_heads + kvh * G + row % G) * DH : nullptr;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    const bool mine = ok && my_tiles > 0;
+    if (a.splits > 1) {
+      // The CTAs of the cluster leave their sums, references and row sums in shared memory (once neither row tile's products read there any
+      // more); every CTA puts together a slice of the columns of all rows.
+      float* const sums = reinterpret_cast<float*>(smem) + (128 * q + rr) * (DH + 4);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (mine) {
 #pragma unroll 1
         for (int c0 = 0; c0 < DH; c0 += 16) {
           uint32_t o[16];
           tmem_ld16(o_tmem + c0, o);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (o_row) {
-            uint32_t w[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = pack_bf16(__uint_as_float(o[2 * e]) * inv, __uint_as_float(o[2 * e + 1]) * inv);
-            *reinterpret_cast<uint4*>(o_row + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4*>(o_row + c0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-          }
+          for (int e = 0; e < 16; e += 4) *reinterpret_cast<uint4*>(sums + c0 + e) = make_uint4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+        }
+      }
+      sums[DH] = mine ? m_used : -INFINITY;
+      sums[DH + 1] = l;
+    } else if (mine) {
+      const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+      __nv_bfloat16* o_row = row < rows ? a.out + (static_cast<long long>(t0 + row / G) * a.q_heads + kvh * G + row % G) * DH : nullptr;
+#pragma unroll 1
+      for (int c0 = 0; c0 < DH; c0 += 16) {
+        uint32_t o[16];
+        tmem_ld16(o_tmem + c0, o);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (o_row) {
+          uint32_t w[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[e] = pack_bf16(__uint_as_float(o[2 * e]) * inv, __uint_as_float(o[2 * e + 1]) * inv);
+          *reinterpret_cast<uint4*>(o_row + c0) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(o_row + c0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
         }
       }
     }
+  }
+  if (a.splits > 1) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp < 8) {
+      const int row = row0 + threadIdx.x;
+      const uint32_t here = smem_u32(reinterpret_cast<float*>(smem) + threadIdx.x * (DH + 4));
+      auto peer = [&](int r, int column) {
+        uint32_t at;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(here + column * 4), "r"(r));
+        return at;
+      };
+      float top = -INFINITY, f[kUmmaMaxSplits], total = 0.0f;
+#pragma unroll
+      for (int r = 0; r < kUmmaMaxSplits; ++r) {
+        f[r] = -INFINITY;
+        if (r < a.splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f[r]) : "r"(peer(r, DH)));
+        top = fmaxf(top, f[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < kUmmaMaxSplits; ++r) {
+        float l = 0.0f;
+        if (r < a.splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l) : "r"(peer(r, DH + 1)));
+        f[r] = f[r] == -INFINITY ? 0.0f : ex2(f[r] - top);
+        if (f[r] > 0.0f) total = fmaf(l, f[r], total);
+      }
+      const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+      const int cols = DH / a.splits;
+      if (row < rows) {
+        __nv_bfloat16* dst = a.out + (static_cast<long long>(t0 + row / G) * a.q_heads + kvh * G + row % G) * DH;
+        for (int c = rank * cols; c < (rank + 1) * cols; c += 8) {
+          float v[8] = {};
+#pragma unroll
+          for (int r = 0; r < kUmmaMaxSplits; ++r) {
+            if (r >= a.splits || !(f[r] > 0.0f)) continue;      // (what a CTA without keys for the row left is not read)
+#pragma unroll
+            for (int e = 0; e < 8; e += 4) {
+              float x[4];
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(peer(r, c + e)));
+#pragma unroll
+              for (int y = 0; y < 4; ++y) v[e + y] = fmaf(x[y], f[r] * inv, v[e + y]);
+            }
+          }
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody leaves while its sums are read
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -409,7 +495,26 @@ static int launch_prompt_umma(const CUtensorMap& km, const CUtensorMap& vm, cons
     }
     configured = true;
   }
-  TIE_LAUNCH((attn_prompt_umma_kernel<DH, STAGES>), dim3(a.kv_heads, ceil_div(max_rows, a.cta_rows), n_seqs), kUmmaAttnThreads, smem, s, km, vm, a);
+  static_assert(smem >= 256 * (DH + 4) * 4 + (2 * STAGES + 12) * 8 + 16 + 1024, "the sums of a CTA's rows");
+  const dim3 grid(a.kv_heads, ceil_div(max_rows, a.cta_rows), n_seqs * a.splits);
+  if (a.splits == 1) {
+    TIE_LAUNCH((attn_prompt_umma_kernel<DH, STAGES>), grid, kUmmaAttnThreads, smem, s, km, vm, a);
+    return kOk;
+  }
+  // clusters of CTAs that hold tensor memory are not started beside the kernel ahead
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kUmmaAttnThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = a.splits;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, attn_prompt_umma_kernel<DH, STAGES>, km, vm, a);
   return kOk;
 }
 
@@ -418,12 +523,12 @@ static int launch_prompt_umma(const CUtensorMap& km, const CUtensorMap& vm, cons
 using namespace tie;
 
 // Rows [0, rows) of the step belong to sequences 0..n_seqs-1, each bringing several tokens;
-// max_queries is the largest number of tokens one of them brings; pages is the number of pages
-// of the cache planes.
+// max_queries is the largest number of tokens one of them brings, max_keys the longest context of one; pages is the
+// number of pages of the cache planes.
 TIE_API int tie_attention_prompt_umma(const void* q, long long q_stride, const void* k_cache, const void* v_cache, void* out,
                                       const int* query_start, const int* context_lens, const int* block_tables,
                                       int max_blocks, int n_seqs, int max_queries, int q_heads, int kv_heads, int head_dim,
-                                      int page_size, int pages, int window, float scale, cudaStream_t s) {
+                                      int page_size, int pages, int window, float scale, int max_keys, cudaStream_t s) {
   TIE_REQUIRE(head_dim == 64 || head_dim == 128, "attention_prompt_umma: head_dim %d is not 64 or 128", head_dim);
   TIE_REQUIRE(q_heads > 0 && kv_heads > 0 && q_heads % kv_heads == 0 && q_heads / kv_heads <= 16,
               "attention_prompt_umma: %d query heads over %d kv heads (at most 16 per group)", q_heads, kv_heads);
@@ -443,12 +548,20 @@ TIE_API int tie_attention_prompt_umma(const void* q, long long q_stride, const v
               "attention_prompt_umma: cuTensorMapEncodeTiled failed");
   TIE_REQUIRE(status_word() != nullptr, "attention_prompt_umma: cannot allocate the status word");
   UmmaPromptArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(out), query_start, context_lens, block_tables,
-                   status_word(), q_stride, max_blocks, q_heads, kv_heads, page_size, shift, window, scale * 1.4426950408889634f, 256};
+                   status_word(), q_stride, max_blocks, q_heads, kv_heads, page_size, shift, window, scale * 1.4426950408889634f, 1, 256};
   const int max_rows = max_queries * (q_heads / kv_heads);
   // Few rows: with two row tiles a CTA, half of the SMs or more would have none
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  if (static_cast<long long>(kv_heads) * ceil_div(max_rows, 256) * n_seqs * 2 <= sms) a.cta_rows = 128;
+  // ...; with many keys they share out the keys instead: what bounds either is the keys and values that L2 feeds the SMs, and tiles of
+  // 256 rows read them half as often (512 tokens of 32 heads over 8, 16,384 keys: 239 -> 165 us; 6,000: 94 -> 74; 2,048: 38 -> 39;
+  // 1,024: 24 -> 29: the merge costs about 8 us)
+  const long long ctas = static_cast<long long>(kv_heads) * ceil_div(max_rows, 256) * n_seqs;
+  const int keys = window > 0 && window + max_queries < max_keys ? window + max_queries : max_keys;
+  if (ctas * 2 <= sms) {
+    if (keys >= kUmmaSplitKeys) a.splits = ctas * 4 <= sms ? 4 : 2;
+    else a.cta_rows = 128;
+  }
   const int st = head_dim == 64 ? launch_prompt_umma<64>(km, vm, a, n_seqs, max_rows, s) : launch_prompt_umma<128>(km, vm, a, n_seqs, max_rows, s);
   if (st != kOk) return st;
   TIE_RETURN_LAUNCH("attention_prompt_umma");

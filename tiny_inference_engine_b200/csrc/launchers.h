@@ -75,4 +75,4 @@ TIE_API int tie_attention_decode_prep(const void* qkv, long long qkv_stride, con
 TIE_API int tie_attention_prompt_umma(const void* q, long long q_stride, const void* k_cache, const void* v_cache, void* out,
                                       const int* query_start, const int* context_lens, const int* block_tables,
                                       int max_blocks, int n_seqs, int max_queries, int q_heads, int kv_heads, int head_dim,
-                                      int page_size, int pages, int window, float scale, cudaStream_t s);
+                                      int page_size, int pages, int window, float scale, int max_keys, cudaStream_t s);

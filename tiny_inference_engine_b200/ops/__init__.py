@@ -357,15 +357,15 @@ def attention_prompt_umma_takes(q: torch.Tensor, q_heads: int, kv_heads: int, he
 
 
 def attention_prompt_umma(q, k_cache, v_cache, out, query_start, context_lens, block_tables, n_seqs: int, max_queries: int,
-                          q_heads, kv_heads, head_dim, scale: float, window: int = 0) -> None:
+                          q_heads, kv_heads, head_dim, scale: float, window: int = 0, max_keys: int = 0) -> None:
     """As attention_prompt_tma with both products on tcgen05 and the accumulators in tensor memory
-    (head sizes 64 and 128)."""
+    (head sizes 64 and 128). `max_keys`: the longest context of one of the portions (how the launch is cut, not what it computes)."""
     _dev(q, k_cache, v_cache, out, query_start, context_lens, block_tables)
     _attn_common(q, k_cache, v_cache, out, query_start, context_lens, block_tables, q_heads, kv_heads, head_dim)
     _need(out.is_contiguous(), "attention: out must be contiguous")
     call("tie_attention_prompt_umma", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
          query_start.data_ptr(), context_lens.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], n_seqs,
-         max_queries, q_heads, kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], int(window), float(scale), _stream())
+         max_queries, q_heads, kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], int(window), float(scale), int(max_keys), _stream())
 
 
 def attention_prompt_exact(q, k_cache, v_cache, out, query_start, context_lens, block_tables, n_seqs: int, max_queries: int,

@@ -40,7 +40,7 @@ _SIGNATURES = {
     "tie_attention_decode_prep": [P, L, P, L, I, L, P, P, F, F, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P, I, I, I, I, P, P, I, P],
     "tie_attention_prompt_tma": [P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P],
     "tie_attention_prompt_tma_exact": [P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P],
-    "tie_attention_prompt_umma": [P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P],
+    "tie_attention_prompt_umma": [P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P],
     "tie_attention_merge": [I, P, P, P, I, I, I, P, I, I, I, P, P, P],
     "tie_attention_rows_dv": [I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, P],
     "tie_attention_split_dv": [I, P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, I, I, I, P, I, P, P],

@@ -156,11 +156,12 @@ class GQAttention(Mixer):
             n = ctx.multi_rows
             if tc:
                 tma = ops.attention_decode_tma_takes(q, Hq, Hkv, Dh, cache.k.shape[2])
-                fn = ops.attention_prompt_tma if tma else ops.attention_prompt_tc
+                args = (q, cache.k, cache.v, attn, ctx.query_start, ctx.context_lens, g.block_tables, ctx.multi_seqs,
+                        ctx.multi_max_queries, Hq, Hkv, Dh, self.scale, self.window)
                 if tma and ops.attention_prompt_umma_takes(q, Hq, Hkv, Dh, cache.k.shape[2], ctx.multi_max_queries):
-                    fn = ops.attention_prompt_umma
-                fn(q, cache.k, cache.v, attn, ctx.query_start, ctx.context_lens, g.block_tables, ctx.multi_seqs,
-                   ctx.multi_max_queries, Hq, Hkv, Dh, self.scale, self.window)
+                    ops.attention_prompt_umma(*args, max_keys=portion_keys(ctx))
+                else:
+                    (ops.attention_prompt_tma if tma else ops.attention_prompt_tc)(*args)
             else:
                 ops.attention_rows(q[:n], cache.k, cache.v, attn[:n], ctx.seq_of_row[:n], ctx.query_start,
                                    ctx.context_lens, g.block_tables, Hq, Hkv, Dh, self.scale, self.window)
@@ -210,6 +211,14 @@ class GQAttention(Mixer):
         fn = ops.attention_decode_tc if tc else ops.attention_split
         fn(q, cache.k, cache.v, attn, ctx.query_start, ctx.context_lens, g.block_tables, Hq, Hkv, Dh, self.scale,
            ctx.single_seqs, ctx.single_count, split_keys, max_splits, scratch, self.window)
+
+
+def portion_keys(ctx) -> int:
+    """The longest context among the step's portions, rounded up to 1,024 (steps alike make the same launches)."""
+    keys = ctx.memo.get("portion_keys")
+    if keys is None:
+        keys = ctx.memo["portion_keys"] = -(-int(ctx.host.context_lens[:ctx.multi_seqs].max()) // 1024) * 1024
+    return keys
 
 
 def decode_splits(longest: int, sequences: int, kv_heads: int, page_size: int, contexts=None) -> tuple[int, int]:
