@@ -630,3 +630,40 @@ def test_products_batched_over_heads(shape, dtype):
     tol = 2e-2 if dtype == torch.bfloat16 else 1e-4
     assert torch.allclose(out.view(T, H, N + room)[:, :, :N].float(), want, rtol=tol, atol=tol)
     assert (out.view(T, H, N + room)[:, :, N:] == 0).all()                  # what lies behind a head's result is left alone
+
+
+@pytest.mark.parametrize("tokens,E,top,D,I", [(1, 5, 2, 40, 24), (16, 32, 4, 136, 72), (40, 6, 3, 200, 136)])
+@pytest.mark.parametrize("block_m", [4, 8])
+def test_few_rows_of_experts_on_the_tensor_cores(tokens, E, top, D, I, block_m):
+    """Tiles of 4 and 8 pairs over weights in k-blocks: the first product with and without the gated unit, the second with its weights; sizes that
+    end inside a warp's sixteen rows and inside a k-block, an expert with several tiles, experts without any."""
+    from tiny_inference_engine_b200 import ops
+    g = torch.Generator().manual_seed(tokens + E)
+    h = torch.randn((tokens, D), generator=g).to(torch.bfloat16).cuda()
+    w1 = (torch.randn((E, 2 * I, D), generator=g) * 3 / D ** 0.5).to(torch.bfloat16).cuda()
+    w2 = (torch.randn((E, D, I), generator=g) / I ** 0.5).to(torch.bfloat16).cuda()
+    b1, b2 = ops.pack_k_blocks(w1.view(E * 2 * I, D)), ops.pack_k_blocks(w2.view(E * D, I))
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(tokens)]).to(torch.int32).cuda()
+    ids[: tokens // 2, 0] = 1
+    weights = torch.rand((tokens, top), generator=g).cuda()
+    tiles = ops.moe_max_tiles(tokens * top, E, block_m)
+    sorted_pairs = torch.empty(tiles * block_m, dtype=torch.int32, device="cuda")
+    tile_expert = torch.empty(tiles, dtype=torch.int32, device="cuda")
+    meta = torch.zeros(4, dtype=torch.int32, device="cuda")
+    ops.moe_align(ids, E, block_m, sorted_pairs, tile_expert, meta)
+    lists = (sorted_pairs, tile_expert, meta, tiles)
+    sums = torch.stack([w1[int(ids[t, s])].double() @ h[t].double() for t in range(tokens) for s in range(top)])
+    first = torch.full((tokens * top, 2 * I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.moe_gemm(h, b1, first, top, block_m, *lists, blocks_of=(2 * I, D))
+    act = torch.full((tokens * top, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.moe_gemm_glu(h, b1, act, top, block_m, *lists, I, 2.5, 1.702, 1.0)
+    partial = torch.full((top, tokens, D), float("nan"), device="cuda")
+    ops.moe_gemm(act, b2, None, top, block_m, *lists, second=True, partial=partial.view(-1), weights=weights.view(-1), blocks_of=(D, I))
+    gate, up = sums[:, :I].clamp(max=2.5), sums[:, I:].clamp(-2.5, 2.5)
+    rounding = 2.0 ** -8                                   # one rounding to bfloat16 (2^-9 of a value), and as much again for float sums
+    assert (first.double() - sums).abs().max() <= rounding * sums.abs().max()
+    want = gate * torch.sigmoid(1.702 * gate) * (up + 1.0)
+    assert (act.double() - want).abs().max() <= rounding * want.abs().max()
+    want = torch.stack([torch.stack([weights[t, s].double() * (w2[int(ids[t, s])].double() @ act[t * top + s].double()) for t in range(tokens)])
+                        for s in range(top)])
+    assert (partial.double() - want).abs().max() <= 2e-6 * want.abs().max()

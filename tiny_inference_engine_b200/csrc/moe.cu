@@ -9,9 +9,9 @@
 //               that is a whole number of tiles of `block_m` rows, and lists the pairs in that order (-1 pads a
 //               tile). Also says which expert each tile belongs to and how many tiles there are, all on the
 //               device: nothing of a step's routing is read by the host, so a step can be a captured graph.
-//   moe_gemv, moe_gemv_blocks   the same products for tiles of 4 pairs (decode: an expert has a row or two): the
-//               expert's weight rows are streamed once, a warp per output column (row-major weights) or per four
-//               columns (weights in k-blocks).
+//   moe_gemv, moe_mma_blocks   the same products for tiles of 4 or 8 pairs (decode: an expert has a row or two): the
+//               expert's weight rows are streamed once, a warp per output column (row-major weights, 4 pairs) or per
+//               sixteen (bfloat16 weights in k-blocks, on the tensor cores).
 //   moe_gather, moe_combine   for prompts in bfloat16: rows copied into the listed order ahead of the grouped products
 //               on the tensor cores (gemm_tc.cu, tiles of 128 rows), and the weighted results back to their tokens.
 //   moe_gemm    grouped products on the CUDA cores, one block per (tile of rows, 64 output columns): rows are
@@ -23,7 +23,7 @@
 
 #include <type_traits>
 
-#include "common.cuh"
+#include "attention_mma.cuh"
 
 namespace tie {
 
@@ -147,16 +147,26 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
   __syncthreads();
   for (int i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(&count[ids[i]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int row = 0;
-    for (int e = 0; e < experts; ++e) {
-      cursor[e] = row;
-      const int tiles = (count[e] + block_m - 1) / block_m;
-      for (int i = 0; i < tiles; ++i) tile_expert[row / block_m + i] = e;
-      row += tiles * block_m;
+  if (threadIdx.x < 32) {                  // the experts' tiles one after the other, 32 experts at a time
+    const int lane = threadIdx.x;
+    int before = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane, tiles = e < experts ? (count[e] + block_m - 1) / block_m : 0;
+      int end = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int left = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += left;
+      }
+      const int first = before + end - tiles;
+      if (e < experts) cursor[e] = first * block_m;
+      for (int i = 0; i < tiles; ++i) tile_expert[first + i] = e;
+      before += __shfl_sync(0xffffffffu, end, 31);
     }
-    total_rows = row;
-    meta[0] = row / block_m;
+    if (lane == 0) {
+      total_rows = before * block_m;
+      meta[0] = before;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < total_rows; i += blockDim.x) sorted[i] = -1;
@@ -322,60 +332,83 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const int* __restric
   }
 }
 
-// The same for bfloat16 weights stored in k-blocks, [ceil(K / 64)][w_rows][64] (this expert's rows at expert * N): a
-// warp takes four neighbouring output columns, eight lanes a column, so that one load instruction of the warp is 512
-// consecutive bytes of a k-block (four rows' 64 elements) and a block's eight warps read 4 KB in a row; a lane sums its
-// eighth of every k-block, and the eight lanes of a column add up at the end.
-template <bool SECOND>
-__global__ void __launch_bounds__(256) moe_gemv_blocks_kernel(const __nv_bfloat16* __restrict__ a, long long lda,
-                                                              const __nv_bfloat16* __restrict__ w, int w_rows,
-                                                              __nv_bfloat16* __restrict__ out, long long ldo,
-                                                              float* __restrict__ partial, long long part_stride,
-                                                              const float* __restrict__ weights, const int* __restrict__ sorted,
-                                                              const int* __restrict__ tile_expert, const int* __restrict__ meta,
-                                                              int top, int N, int K) {
+// The same for bfloat16 weights stored in k-blocks, [ceil(K / 64)][w_rows][64] (this expert's rows at expert * N), on the tensor cores:
+// a warp takes 16 weight rows as the A operand of mma.sync m16n8k16 and the tile's pairs (up to eight) as its columns. Both operands come
+// straight from memory in their fragments' layout: a lane loads 16 bytes in a row of a weight row and of a pair's row, and since the
+// order of k is free as long as both agree, its eight elements are its share of two MMAs. Per 64 k a warp issues four loads of
+// weights (2 KB in whole 128-byte lines), two of activations (from L1) and four MMAs, and what bounds the kernel is the weight
+// stream. (A lane a column's eighth on FFMA, with eight conversions a load, was bound by issue slots at 3.0 TB/s: 119 us for the
+// first product of 64 pairs over 32 experts of 1,536 x 2,048; 55 us with the unit on top now.)
+// KIND 0: out[pair, n] = w[n] . a[pair / top].   1: the gated unit on top: the warp's rows are eight gate rows and the up rows that
+// go with them, out[pair, n] = g' sigmoid(slope g') (u' + up_shift) as glu_clamped forms it, from the float sums.
+// 2: partial[pair % top][pair / top][n] = weights[pair] * (w[n] . a[pair]).
+struct ClampedUnit {
+  float limit, slope, up_shift;
+};
+
+__device__ __forceinline__ uint4 load_stream(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(256, 3) moe_mma_blocks_kernel(const __nv_bfloat16* __restrict__ a, long long lda,
+                                                               const __nv_bfloat16* __restrict__ w, int w_rows,
+                                                               __nv_bfloat16* __restrict__ out, long long ldo,
+                                                               float* __restrict__ partial, long long part_stride,
+                                                               const float* __restrict__ weights, const int* __restrict__ sorted,
+                                                               const int* __restrict__ tile_expert, const int* __restrict__ meta,
+                                                               int block_m, int top, int N, int K, ClampedUnit unit) {
   pdl_sync();
-  constexpr int MT = 4;
   const int tile = blockIdx.y;
   if (tile >= meta[0]) return;
-  const int lane = threadIdx.x & 31, sub = lane >> 3, piece = lane & 7;
-  const int n = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4 + sub;
-  const bool live = n < N;
-  int pair[MT];
-  const __nv_bfloat16* arow[MT];
-#pragma unroll
-  for (int i = 0; i < MT; ++i) {
-    pair[i] = sorted[tile * MT + i];
-    arow[i] = pair[i] < 0 ? nullptr : a + static_cast<long long>(SECOND ? pair[i] : pair[i] / top) * lda + piece * 8;
-  }
-  const __nv_bfloat16* wr = w + (static_cast<long long>(tile_expert[tile]) * N + (live ? n : 0)) * 64 + piece * 8;
+  constexpr int COLS = KIND == 1 ? 8 : 16;                // output columns of a warp
+  const int lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+  const int n0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * COLS;
+  if (n0 >= N) return;
+  const int last = N - 1, expert = tile_expert[tile];
+  // rows beyond the last are read as the last and not written
+  const long long base = static_cast<long long>(expert) * (KIND == 1 ? 2 * N : N);
+  const __nv_bfloat16* w0 = w + (base + min(n0 + g, last)) * 64 + tq * 8;
+  const __nv_bfloat16* w1 = w + (base + (KIND == 1 ? N + min(n0 + g, last) : min(n0 + g + 8, last))) * 64 + tq * 8;
+  const int pair = g < block_m ? sorted[tile * block_m + g] : -1;
+  const __nv_bfloat16* x = pair < 0 ? nullptr : a + static_cast<long long>(KIND == 2 ? pair : pair / top) * lda + tq * 8;
   const long long kb_stride = static_cast<long long>(w_rows) * 64;
-  float acc[MT] = {};
-  const int k_blocks = (K + 63) >> 6;
-#pragma unroll 4
+  const int k_blocks = (K + 63) >> 6, k_mine = K - tq * 8;
+  float acc[2][4] = {};
+#pragma unroll 2
   for (int kb = 0; kb < k_blocks; ++kb) {
-    if (kb * 64 + piece * 8 >= K) break;                 // the last k-block may be short (K in whole vectors)
-    Vec16<__nv_bfloat16> wv;
-    wv.load(wr + kb * kb_stride);
+    uint4 r0[2], r1[2], v[2];
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      if (arow[i] != nullptr) {
-        Vec16<__nv_bfloat16> av;
-        av.load(arow[i] + kb * 64);
+    for (int h = 0; h < 2; ++h) {
+      r0[h] = load_stream(w0 + kb * kb_stride + h * 32);
+      r1[h] = load_stream(w1 + kb * kb_stride + h * 32);
+      v[h] = x != nullptr && kb * 64 + h * 32 < k_mine ? *reinterpret_cast<const uint4*>(x + kb * 64 + h * 32) : make_uint4(0u, 0u, 0u, 0u);
+    }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i] = fmaf(av.v[j], wv.v[j], acc[i]);
-      }
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t lo[4] = {r0[h].x, r1[h].x, r0[h].y, r1[h].y}, hi[4] = {r0[h].z, r1[h].z, r0[h].w, r1[h].w};
+      mma_bf16(acc[0], lo, v[h].x, v[h].y);
+      mma_bf16(acc[1], hi, v[h].z, v[h].w);
     }
   }
+  // columns 2 tq and 2 tq + 1 of the tile; rows g and g + 8 of the warp's sixteen
 #pragma unroll
-  for (int i = 0; i < MT; ++i) {
-    float v = acc[i];
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    if (piece == 0 && live && pair[i] >= 0) {
-      if (SECOND) partial[(pair[i] % top) * part_stride + static_cast<long long>(pair[i] / top) * N + n] = weights[pair[i]] * v;
-      else out[static_cast<long long>(pair[i]) * ldo + n] = __float2bfloat16_rn(v);
+  for (int c = 0; c < 2; ++c) {
+    const int to = __shfl_sync(0xffffffffu, pair, (2 * tq + c) * 4);      // (lane 4 g holds pair g)
+    if (to < 0) continue;
+    const float top_row = acc[0][c] + acc[1][c], low_row = acc[0][2 + c] + acc[1][2 + c];
+    if (KIND == 1) {
+      const float gate = fminf(top_row, unit.limit), up = fminf(fmaxf(low_row, -unit.limit), unit.limit);
+      if (n0 + g < N) out[static_cast<long long>(to) * ldo + n0 + g] = __float2bfloat16_rn((gate / (1.0f + expf(-unit.slope * gate))) * (up + unit.up_shift));
+    } else if (KIND == 0) {
+      if (n0 + g < N) out[static_cast<long long>(to) * ldo + n0 + g] = __float2bfloat16_rn(top_row);
+      if (n0 + g + 8 < N) out[static_cast<long long>(to) * ldo + n0 + g + 8] = __float2bfloat16_rn(low_row);
+    } else {
+      float* dst = partial + (to % top) * part_stride + static_cast<long long>(to / top) * N + n0 + g;
+      if (n0 + g < N) dst[0] = weights[to] * top_row;
+      if (n0 + g + 8 < N) dst[8] = weights[to] * low_row;
     }
   }
 }
@@ -423,7 +456,7 @@ TIE_API int tie_moe_route(const float* logits, long long ld_logits, int tokens, 
 
 TIE_API int tie_moe_align(const int* ids, int pairs, int experts, int block_m, int* sorted, int* tile_expert, int* meta,
                           cudaStream_t s) {
-  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 16 || block_m == 64 || block_m == 128),
+  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 8 || block_m == 16 || block_m == 64 || block_m == 128),
               "moe_align: bad sizes experts=%d block_m=%d", experts, block_m);
   if (pairs <= 0) return kOk;
   TIE_LAUNCH(moe_align_kernel, 1, 1024, 2 * experts * sizeof(int), s, ids, pairs, experts, block_m, sorted, tile_expert, meta);
@@ -441,19 +474,18 @@ static int launch_moe_gemm(int second, int block_m, const void* a, long long lda
                            void* out, long long ldo, float* partial, long long part_stride, const float* weights,
                            const int* sorted, const int* tile_expert, const int* meta, int max_tiles, int top, int N, int K,
                            int w_rows, cudaStream_t s) {
-  if (block_m == 4 && w_rows > 0) {
+  if (w_rows > 0) {
     if constexpr (std::is_same<TI, __nv_bfloat16>::value) {
-      const dim3 grid(ceil_div(N, 32), max_tiles);
-      const __nv_bfloat16* ap = static_cast<const __nv_bfloat16*>(a);
-      const __nv_bfloat16* wp = static_cast<const __nv_bfloat16*>(w);
-      if (second) {
-        TIE_LAUNCH((moe_gemv_blocks_kernel<true>), grid, 256, 0, s, ap, lda, wp, w_rows, static_cast<__nv_bfloat16*>(out), ldo, partial,
-                   part_stride, weights, sorted, tile_expert, meta, top, N, K);
-      } else {
-        TIE_LAUNCH((moe_gemv_blocks_kernel<false>), grid, 256, 0, s, ap, lda, wp, w_rows, static_cast<__nv_bfloat16*>(out), ldo, partial,
-                   part_stride, weights, sorted, tile_expert, meta, top, N, K);
-      }
-      TIE_RETURN_LAUNCH("moe_gemv_blocks");
+      const dim3 grid(ceil_div(N, 128), max_tiles);
+      const __nv_bfloat16 *ap = static_cast<const __nv_bfloat16*>(a), *wp = static_cast<const __nv_bfloat16*>(w);
+      __nv_bfloat16* op = static_cast<__nv_bfloat16*>(out);
+      if (second)
+        TIE_LAUNCH((moe_mma_blocks_kernel<2>), grid, 256, 0, s, ap, lda, wp, w_rows, op, ldo, partial, part_stride, weights, sorted, tile_expert,
+                   meta, block_m, top, N, K, ClampedUnit{});
+      else
+        TIE_LAUNCH((moe_mma_blocks_kernel<0>), grid, 256, 0, s, ap, lda, wp, w_rows, op, ldo, partial, part_stride, weights, sorted, tile_expert,
+                   meta, block_m, top, N, K, ClampedUnit{});
+      TIE_RETURN_LAUNCH("moe_mma_blocks");
     } else {
       set_error("moe_gemm: weights in k-blocks are bfloat16");
       return kBadArgument;
@@ -486,21 +518,22 @@ static int launch_moe_gemm(int second, int block_m, const void* a, long long lda
 }
 
 // second 0: out[pair, :N] = w[expert] a[pair / top]; second 1: partial[pair % top][pair / top][:N] = weights[pair] * (w[expert] a[pair]).
-// w is [experts, N, K] (an expert's rows K apart, experts w_expert_stride apart), or with w_rows > 0 (tiles of 4 rows only)
+// w is [experts, N, K] (an expert's rows K apart, experts w_expert_stride apart), or with w_rows > 0 (tiles of 4 and 8 rows only)
 // the same rows one expert after the other stored in k-blocks, [ceil(K / 64)][w_rows][64].
 TIE_API int tie_moe_gemm(int dtype, int second, int block_m, const void* a, long long lda, const void* w,
                          long long w_expert_stride, void* out, long long ldo, float* partial, long long part_stride,
                          const float* weights, const int* sorted, const int* tile_expert, const int* meta, int max_tiles,
                          int top, int N, int K, int w_rows, cudaStream_t s) {
-  TIE_REQUIRE(w_rows == 0 || (block_m == 4 && w_rows % N == 0), "moe_gemm: weights in k-blocks are read by the tiles of 4 rows only");
-  TIE_REQUIRE(N > 0 && K > 0 && top > 0 && (block_m == 4 || block_m == 16 || block_m == 64) && max_tiles >= 0 && max_tiles <= 65535,
+  TIE_REQUIRE(N > 0 && K > 0 && top > 0, "moe_gemm: bad sizes N=%d K=%d top=%d", N, K, top);
+  TIE_REQUIRE(w_rows == 0 || ((block_m == 4 || block_m == 8) && w_rows % N == 0), "moe_gemm: weights in k-blocks are read by the tiles of 4 and 8 rows only");
+  TIE_REQUIRE((block_m == 4 || (block_m == 8 && w_rows > 0) || block_m == 16 || block_m == 64) && max_tiles >= 0 && max_tiles <= 65535,
               "moe_gemm: bad sizes N=%d K=%d top=%d block_m=%d tiles=%d", N, K, top, block_m, max_tiles);
   if (max_tiles == 0) return kOk;
-  if (block_m == 4) {
+  if (block_m <= 8) {
     const int v = dtype == TIE_BF16 ? 8 : 4;
     TIE_REQUIRE(K % v == 0 && lda % v == 0 && w_expert_stride % v == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0 &&
                     reinterpret_cast<uintptr_t>(w) % 16 == 0,
-                "moe_gemm: tiles of 4 rows need K=%d and the row strides in whole 16-byte vectors", K);
+                "moe_gemm: tiles of 4 and 8 rows need K=%d and the row strides in whole 16-byte vectors", K);
   }
   if (dtype == TIE_F32)
     return launch_moe_gemm<float, float>(second, block_m, a, lda, w, w_expert_stride, out, ldo, partial, part_stride, weights, sorted,
@@ -510,4 +543,20 @@ TIE_API int tie_moe_gemm(int dtype, int second, int block_m, const void* a, long
                                                          weights, sorted, tile_expert, meta, max_tiles, top, N, K, w_rows, s);
   set_error("unknown dtype code %d", dtype);
   return kBadArgument;
+}
+
+// The first product with the clamped gated unit on top: w holds every expert's `inter` gate rows and its `inter` up rows in k-blocks,
+// out[pair, :inter] = unit(gate, up) of a[pair / top]. Tiles of 4 or 8 pairs.
+TIE_API int tie_moe_gemm_glu(int block_m, const void* a, long long lda, const void* w, int w_rows, void* out, long long ldo, const int* sorted,
+                             const int* tile_expert, const int* meta, int max_tiles, int top, int inter, int K, float limit, float slope,
+                             float up_shift, cudaStream_t s) {
+  TIE_REQUIRE(inter > 0 && K > 0 && top > 0 && (block_m == 4 || block_m == 8) && max_tiles >= 0 && max_tiles <= 65535 && w_rows % (2 * inter) == 0,
+              "moe_gemm_glu: bad sizes inter=%d K=%d top=%d block_m=%d tiles=%d", inter, K, top, block_m, max_tiles);
+  TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0,
+              "moe_gemm_glu: needs K=%d and the row stride in whole 16-byte vectors", K);
+  if (max_tiles == 0) return kOk;
+  TIE_LAUNCH((moe_mma_blocks_kernel<1>), dim3(ceil_div(inter, 64), max_tiles), 256, 0, s, static_cast<const __nv_bfloat16*>(a), lda,
+             static_cast<const __nv_bfloat16*>(w), w_rows, static_cast<__nv_bfloat16*>(out), ldo, nullptr, 0, nullptr, sorted, tile_expert, meta,
+             block_m, top, inter, K, ClampedUnit{limit, slope, up_shift});
+  TIE_RETURN_LAUNCH("moe_gemm_glu");
 }

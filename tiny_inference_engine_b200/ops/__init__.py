@@ -1128,14 +1128,14 @@ def moe_gemm(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, meta,
              partial=None, weights=None, blocks_of=None) -> None:
     """Grouped products by expert. w [experts, N, K]. First (second False): a [T, K], out [T * top, N] = w[expert] a[token]
     per pair. Second: a [T * top, K], partial float32 [top, T, N] gets weights[pair] * (w[expert] a[pair]). With
-    `blocks_of` = (N, K) and block_m 4, w is the experts' rows one after the other in k-blocks (`pack_k_blocks`)."""
+    `blocks_of` = (N, K) and block_m 4 or 8, w is the experts' rows one after the other in k-blocks (`pack_k_blocks`)."""
     _dev(a, w, out, partial, weights, sorted_pairs, tile_expert, meta)
     w_rows = 0
     if blocks_of is not None:
         N, K = blocks_of
-        _need(block_m == 4 and w.dim() == 3 and w.is_contiguous() and w.shape[2] == 64 and w.shape[0] == (K + 63) // 64 and
+        _need(block_m in (4, 8) and w.dim() == 3 and w.is_contiguous() and w.shape[2] == 64 and w.shape[0] == (K + 63) // 64 and
               w.shape[1] % N == 0 and a.dim() == 2 and a.stride(1) == 1 and a.shape[1] == K and a.dtype == w.dtype,
-              "moe_gemm: weights in k-blocks of [experts * N, K] go with tiles of 4 rows")
+              "moe_gemm: weights in k-blocks of [experts * N, K] go with tiles of 4 or 8 rows")
         w_rows = w.shape[1]
     else:
         _need(w.dim() == 3 and w.is_contiguous() and a.dim() == 2 and a.stride(1) == 1 and a.shape[1] == w.shape[2] and a.dtype == w.dtype,
@@ -1153,6 +1153,19 @@ def moe_gemm(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, meta,
     call("tie_moe_gemm", dtype_code(a), 1 if second else 0, block_m, a.data_ptr(), a.stride(0), w.data_ptr(), N * K,
          _ptr(out), out.stride(0) if out is not None else 0, _ptr(partial), T * N if second else 0, _ptr(weights),
          sorted_pairs.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(), max_tiles, top, N, K, w_rows, _stream())
+
+
+def moe_gemm_glu(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, meta, max_tiles: int, inter: int, limit: float, slope: float,
+                 up_shift: float) -> None:
+    """The first product and the clamped gated unit behind it (`glu_clamped`) in one: a [T, K] bfloat16, w every expert's `inter` gate and
+    `inter` up rows in k-blocks, out [T * top, inter]. The unit works on the float sums. Tiles of 4 or 8 pairs."""
+    _dev(a, w, out, sorted_pairs, tile_expert, meta)
+    K = a.shape[1]
+    _need(w.dim() == 3 and w.is_contiguous() and w.shape[2] == 64 and w.shape[0] == (K + 63) // 64 and w.shape[1] % (2 * inter) == 0 and
+          a.stride(1) == 1 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.stride(1) == 1 and
+          out.shape == (a.shape[0] * top, inter), "moe_gemm_glu: bfloat16 a [T, K], w in k-blocks, out [T * top, inter]")
+    call("tie_moe_gemm_glu", block_m, a.data_ptr(), a.stride(0), w.data_ptr(), w.shape[1], out.data_ptr(), out.stride(0), sorted_pairs.data_ptr(),
+         tile_expert.data_ptr(), meta.data_ptr(), max_tiles, top, inter, K, float(limit), float(slope), float(up_shift), _stream())
 
 
 GROUPED_TILE = 128      # rows of a tile of the grouped product on the tensor cores

@@ -70,6 +70,7 @@ _SIGNATURES = {
     "tie_glu_biased": [I, P, P, P, P, I, I, I, I, P],
     "tie_moe_route": [P, L, I, I, I, I, I, I, P, I, I, F, P, P, P, P],
     "tie_moe_align": [P, I, I, I, P, P, P, P],
+    "tie_moe_gemm_glu": [I, P, L, P, I, P, L, P, P, P, I, I, I, I, F, F, F, P],
     "tie_moe_gemm": [I, I, I, P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, P],
     "tie_moe_gather": [I, P, L, P, P, I, I, P, I, I, P],
     "tie_moe_combine": [I, P, P, P, I, I, P, P, L, I, I, P],

@@ -113,16 +113,16 @@ class RoutedExperts(FeedForward):
                       correction=self.correction, group_top=self.group_top, renorm=self.renorm, weight_scale=self.weight_scale,
                       bias=self.router_bias)
         pairs = T * top
-        few = pairs <= 8 * E      # an expert has a few rows: a warp per output column streams its weights once
+        few = pairs <= 8 * E      # an expert has a few rows: its weights are streamed once
         if self.in_blocks:
-            block_m = 4 if few else ops.GROUPED_TILE
+            block_m = 8 if few else ops.GROUPED_TILE
         elif few and D % 4 == 0 and I % 4 == 0 and self.dtype == torch.float32:
             block_m = 4
         else:
             block_m = 16 if pairs <= 16 * E else 64
         rows_cap = ctx.ws.max_rows * top
         tiles_cap = max(ops.moe_max_tiles(rows_cap, E, 4), 1)
-        sorted_pairs = ctx.ws.flat("moe.sorted", max(ops.moe_max_tiles(rows_cap, E, m) * m for m in (4, 16, 64, 128)), torch.int32)
+        sorted_pairs = ctx.ws.flat("moe.sorted", max(ops.moe_max_tiles(rows_cap, E, m) * m for m in (4, 8, 16, 64, 128)), torch.int32)
         tile_expert = ctx.ws.flat("moe.tile_expert", tiles_cap, torch.int32)
         meta = ctx.ws.flat("moe.meta", 4, torch.int32)
         ops.moe_align(ids, E, block_m, sorted_pairs, tile_expert, meta)
@@ -143,11 +143,13 @@ class RoutedExperts(FeedForward):
             ops.gemm_grouped(act, self.w_down, y, D, I, meta, tile_expert)
             ops.moe_combine(y, sorted_pairs, meta, top, weights.view(-1), partial, T)
             return ops.SplitSum(partial, top, T, D)
-        gu = ctx.ws.rows("moe.gate_up", T, top * 2 * I, self.dtype).view(pairs, 2 * I)
-        ops.moe_gemm(h, self.w_gate_up, gu, top, block_m, sorted_pairs, tile_expert, meta, max_tiles,
-                     blocks_of=(2 * I, D) if self.in_blocks else None)
         act = ctx.ws.rows("moe.act", T, top * I, self.dtype).view(pairs, I)
-        ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
+        if self.in_blocks:
+            ops.moe_gemm_glu(h, self.w_gate_up, act, top, block_m, sorted_pairs, tile_expert, meta, max_tiles, I, self.limit, self.slope, self.up_shift)
+        else:
+            gu = ctx.ws.rows("moe.gate_up", T, top * 2 * I, self.dtype).view(pairs, 2 * I)
+            ops.moe_gemm(h, self.w_gate_up, gu, top, block_m, sorted_pairs, tile_expert, meta, max_tiles)
+            ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
         ops.moe_gemm(act, self.w_down, None, top, block_m, sorted_pairs, tile_expert, meta, max_tiles, second=True,
                      partial=partial, weights=weights.view(-1), blocks_of=(D, I) if self.in_blocks else None)
         return ops.SplitSum(partial, top, T, D)
