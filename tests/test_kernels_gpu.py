@@ -201,6 +201,21 @@ def test_gemm_simt(ops, dtype, M, N, K):
         assert rel_err(host(out32), plain.linear(a, w)) < 2e-5
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 2048), (4, 7, 1016), (5, 33, 2056), (8, 300, 1024), (16, 32, 2048), (9, 600, 512), (16, 1184, 4096)])
+def test_few_rows_with_k_shared_by_warps(ops, dtype, M, N, K):
+    """One, two, four and eight warps a column: columns that leave warps over, k's that give the last warps less or nothing.
+    A row's sums do not depend on how many rows there are."""
+    rng = np.random.default_rng(M + N + K)
+    a, w = as_stored(rng.standard_normal((M, K)), dtype), as_stored(rng.standard_normal((N, K)), dtype)
+    da, dw = dev(a, DT[dtype]), dev(w, DT[dtype])
+    out, row = torch.full((M, N), float("nan"), device="cuda"), torch.empty(1, N, device="cuda")
+    ops.gemm_simt(da, dw, out)
+    assert rel_err(host(out), plain.linear(a, w)) < 2e-5
+    ops.gemm_simt(da[-1:], dw, row)
+    assert torch.equal(row[0], out[-1])
+
+
 @pytest.mark.parametrize("tile,splits", [(t, c) for t in range(3) for c in (1, 2, 4, 8)])
 @pytest.mark.parametrize("M,N,K", [(17, 1, 1), (33, 65, 37), (129, 63, 260), (64, 64, 1024), (97, 200, 1504)])
 def test_float_products_in_every_tiling(ops, tile, splits, M, N, K):
