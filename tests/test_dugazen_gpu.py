@@ -442,3 +442,37 @@ def test_configurations_drawn_at_random(tmp_path, seed, dtype):
         rows.update(hs.step([("a", a[i:i + 1], [0])]))
     close(np.stack([rows[("a", i)] for i in range(83)]), want_a, dtype, f"seed {seed} in portions and decoded")
     close(np.stack([rows[("b", i)] for i in range(31)]), want_b, dtype, f"seed {seed} the request beside it")
+
+
+def _on_gpu(rng, *shape, scale=1.0):
+    return torch.from_numpy((rng.standard_normal(shape) * scale).astype(np.float32)).cuda()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim", [4, 72, 260, 2048, 8192, 8196, 16384, 16388])
+@pytest.mark.parametrize("splits,biased,picked", [(0, False, False), (0, True, True), (3, True, False), (5, False, True)])
+def test_normed_sublayer_outputs_join_the_stream(dim, splits, biased, picked, dtype):
+    """Rows held in registers, two and four pieces a thread, and the widest rows; a tensor or partial sums; all rows or some. The sums
+    of squares are good to dim 2^-24 at worst and to a few 2^-24 as trees; an output is rounded once to its type."""
+    from tiny_inference_engine_b200 import ops
+    rng = np.random.default_rng(dim + splits)
+    T, eps = 5, 1e-5
+    x, wb, w, bias = _on_gpu(rng, T, dim), _on_gpu(rng, dim), _on_gpu(rng, dim), _on_gpu(rng, dim)
+    if splits:
+        part = _on_gpu(rng, splits * T * dim)
+        delta, y = ops.SplitSum(part, splits, T, dim), part.double().cpu().view(splits, T, dim).sum(0)
+    else:
+        delta = _on_gpu(rng, T, dim).to(dtype)
+        y = delta.double().cpu()
+    norm = lambda v, e: v / torch.sqrt((v * v).mean(-1, keepdim=True) + e)
+    y = y + (bias.double().cpu() if biased else 0.0)
+    rows = torch.tensor([3, 0, 4], dtype=torch.int32, device="cuda") if picked else None
+    before = x.double().cpu()
+    stream = before + 0.7 * norm(y, 1e-6) * wb.double().cpu()
+    want = norm(stream, eps) * w.double().cpu()
+    out = torch.empty(3 if picked else T, dim, device="cuda", dtype=dtype)
+    ops.add_normed_rmsnorm(x, ops.NormedDelta(delta, wb, 1e-6, 0.7, bias if biased else None), w, eps, out, rows=rows)
+    assert rel_err(x.double().cpu().numpy(), (before if picked else stream).numpy()) < 2e-6
+    if picked:
+        want = want[[3, 0, 4]]
+    assert rel_err(out.double().cpu().numpy(), want.numpy()) < (2e-6 if dtype == torch.float32 else 2.0 ** -8)

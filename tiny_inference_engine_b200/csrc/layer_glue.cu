@@ -140,6 +140,77 @@ __global__ void __launch_bounds__(1024) add_normed_rmsnorm_vec4_kernel(float* __
   }
 }
 
+// The same with a row held in registers, NV pieces of four a thread: the stream and both norms' weights are read with the delta, so
+// that only the two sums stand between the loads and the stores. Bound by latency for few rows, by the passes over memory for many:
+// 2,048 rows of 2,048 22.5 -> 13.5 us (the row in shared memory, the stream read after the first sum, before); a decode step of 8 rows
+// with 16 of these, 632 -> 619 us (646 with two pieces a thread).
+template <typename T, int NV>
+__global__ void __launch_bounds__(1024) add_normed_rmsnorm_regs_kernel(float* __restrict__ x, const T* __restrict__ delta,
+                                                                      const float* __restrict__ part, long long part_stride,
+                                                                      int splits, const float* __restrict__ bias,
+                                                                      const float* __restrict__ wb, float eps_b, float mult,
+                                                                      const int* __restrict__ rows, const float* __restrict__ w,
+                                                                      float eps, T* __restrict__ out, int dim) {
+  pdl_sync();
+  __shared__ float scratch[2][33];
+  const int t = blockIdx.x;
+  const size_t src = static_cast<size_t>(rows ? rows[t] : t) * dim;
+  float xv[NV][4], y[NV][4], gb[NV][4], g[NV][4];
+  float ss = 0.0f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (n * blockDim.x + threadIdx.x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[n][i] = xv[n][i] = gb[n][i] = g[n][i] = 0.0f;
+    if (k >= dim) continue;
+    if (delta) load4(delta + src + k, y[n]);
+    load4(x + src + k, xv[n]);
+    load4(wb + k, gb[n]);
+    load4(w + k, g[n]);
+    if (!delta) {                                           // split by split: each element adds in split order
+#pragma unroll 4
+      for (int z = 0; z < splits; ++z) {
+        float p[4];
+        load4(part + src + static_cast<long long>(z) * part_stride + k, p);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[n][i] += p[i];
+      }
+    }
+    if (bias) {
+      float b[4];
+      load4(bias + k, b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[n][i] += b[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss += y[n][i] * y[n][i];
+  }
+  ss = block_sum(ss, scratch[0]);
+  const float inv_y = 1.0f / sqrtf(ss / static_cast<float>(dim) + eps_b);
+  float sx = 0.0f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (n * blockDim.x + threadIdx.x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      xv[n][i] = xv[n][i] + mult * ((y[n][i] * inv_y) * gb[n][i]);
+      sx += k < dim ? xv[n][i] * xv[n][i] : 0.0f;
+    }
+    if (rows == nullptr && k < dim) store4(x + src + k, xv[n]);
+  }
+  sx = block_sum(sx, scratch[1]);
+  const float inv_x = 1.0f / sqrtf(sx / static_cast<float>(dim) + eps);
+  T* o = out + static_cast<size_t>(t) * dim;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (n * blockDim.x + threadIdx.x);
+    if (k >= dim) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xv[n][i] = (xv[n][i] * inv_x) * g[n][i];
+    store4(o + k, xv[n]);
+  }
+}
+
 template <typename T>
 __global__ void glu_clamped_kernel(const T* __restrict__ gu, T* __restrict__ out, int inter, long long total, float limit,
                                    float slope, float up_shift) {
@@ -297,6 +368,16 @@ int launch_add_normed_rmsnorm(float* x, const void* delta, const float* part, lo
   const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (dim % 4 == 0 && part_stride % 4 == 0 && aligned(x) && aligned(delta) && aligned(part) && aligned(bias) && aligned(wb) &&
       aligned(w) && aligned(out)) {
+    if (dim <= 16384) {
+      // a piece a thread where few rows leave the SMs to themselves (the longest chain of loads counts), else two; wide rows take
+      // what 1024 threads need
+      const int pieces = dim > 8192 ? 4 : dim > 4096 || n >= 148 ? 2 : 1;
+      auto regs = pieces == 1 ? add_normed_rmsnorm_regs_kernel<T, 1>
+                              : pieces == 2 ? add_normed_rmsnorm_regs_kernel<T, 2> : add_normed_rmsnorm_regs_kernel<T, 4>;
+      TIE_LAUNCH(regs, n, 32 * ceil_div(dim, 128 * pieces), 0, s, x, static_cast<const T*>(delta), part, part_stride, splits, bias, wb,
+                 eps_b, mult, rows, w, eps, static_cast<T*>(out), dim);
+      TIE_RETURN_LAUNCH("add_normed_rmsnorm");
+    }
     auto vec = add_normed_rmsnorm_vec4_kernel<T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     TIE_LAUNCH(vec, n, dim >= 8192 ? 1024 : (dim >= 2048 ? 512 : (dim >= 1024 ? 256 : 128)), smem, s, x, static_cast<const T*>(delta),
