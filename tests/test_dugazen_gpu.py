@@ -449,6 +449,45 @@ def _on_gpu(rng, *shape, scale=1.0):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(16, 16, 128, 128), (48, 24, 20, 36), (40, 20, 200, 132)])
+@pytest.mark.parametrize("lengths", [[1], [3, 1, 2, 5], [1, 2, 3, 4, 0, 6, 500], [253, 1, 1, 4]])
+def test_inputs_of_the_recurrence_several_tokens_a_warp(lengths, heads, kv_heads, dim, vdim, dtype):
+    """Sequences that begin anywhere in a warp's four tokens, with earlier inputs in their state slot or none; a last warp that is
+    not full; heads that fill part of a warp or take a second piece. Four products and a unit norm in float32: rounding stays below
+    (4 + 256 / 2) 2^-24 of a head's largest value, and sigmoid and exp are good to a few units more."""
+    from tiny_inference_engine_b200 import ops
+    rng = np.random.default_rng(sum(lengths) + dim)
+    T, seqs, nqk, nv = sum(lengths), len(lengths), kv_heads * dim, heads * vdim
+    C = 2 * nqk + nv
+    proj = _on_gpu(rng, T, C + heads + 4 - heads % 4).to(dtype)
+    conv, state = _on_gpu(rng, C, 4, scale=0.5), _on_gpu(rng, seqs + 1, 8 + 3 * C)
+    slots = torch.from_numpy(np.where(np.arange(seqs) % 3 == 2, -1, np.arange(seqs)[::-1])).int()
+    starts = torch.tensor([0] + lengths).cumsum(0).int()
+    seq_of_row = torch.repeat_interleave(torch.arange(seqs), torch.tensor(lengths)).int()
+    decay, bias, a_log = _on_gpu(rng, T, heads * dim + 8), _on_gpu(rng, heads * dim), _on_gpu(rng, heads, scale=0.3)
+    raw = decay.double().cpu()
+    qn, kn, vn, beta = (torch.full((T, n), float("nan"), device="cuda") for n in (nqk, nqk, nv, heads))
+    ops.delta_prep(proj, 0, nqk, 2 * nqk, C, conv, state, 8, seq_of_row.cuda(), starts[:seqs].cuda(), slots.cuda(), heads, kv_heads, dim,
+                   vdim, 4, 1e-6, 0.25, qn, kn, vn, beta, decay, bias, a_log)
+    p, w, st = proj.double().cpu(), conv.double().cpu(), state.double().cpu()
+    y = torch.empty(T, C, dtype=torch.float64)
+    for s, n in enumerate(lengths):
+        slot, t0 = int(slots[s]), int(starts[s])
+        tail = st[slot, 8:].view(3, C) if slot >= 0 else torch.zeros(3, C, dtype=torch.float64)
+        seen = torch.cat([tail, p[t0:t0 + n, :C]])
+        y[t0:t0 + n] = sum(seen[i:i + n] * w[:, i] for i in range(4))
+    y = y * torch.sigmoid(y)
+    unit = lambda z: (z.view(T, kv_heads, dim) / torch.sqrt((z.view(T, kv_heads, dim) ** 2).sum(-1, keepdim=True) + 1e-6)).reshape(T, nqk)
+    want = {"q": (qn, unit(y[:, :nqk]) * 0.25), "k": (kn, unit(y[:, nqk:2 * nqk])), "v": (vn, y[:, 2 * nqk:]),
+            "beta": (beta, torch.sigmoid(p[:, C:C + heads]))}
+    rate = torch.exp(a_log.double().cpu()).repeat_interleave(dim)
+    want["decay"] = (decay[:, :heads * dim], torch.exp(-rate * torch.nn.functional.softplus(raw[:, :heads * dim] + bias.double().cpu())))
+    for name, (got, ref) in want.items():
+        assert rel_err(got.double().cpu().numpy(), ref.numpy()) < 2e-5, name
+    assert torch.equal(decay[:, heads * dim:].double().cpu(), raw[:, heads * dim:])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("dim", [4, 72, 260, 2048, 8192, 8196, 16384, 16388])
 @pytest.mark.parametrize("splits,biased,picked", [(0, False, False), (0, True, True), (3, True, False), (5, False, True)])
 def test_normed_sublayer_outputs_join_the_stream(dim, splits, biased, picked, dtype):
