@@ -1226,3 +1226,50 @@ def test_keys_shared_out_over_a_cluster(ops, Dh, Hq, Hkv, page, window, new, ctx
     want = np.concatenate([softmax_reference(q[qs[i]:qs[i + 1]].reshape(-1, Hq, Dh).astype(np.float64), ks[i].astype(np.float64),
                                              vs[i].astype(np.float64), Dh ** -0.5, window, None, ctx[i] - new[i]) for i in range(len(new))])
     assert rel_err(host(out), want.reshape(T, -1)) < TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv,new,ctx", [(4, 2, 130, 2600), (64, 8, 150, 2900)])
+@pytest.mark.parametrize("sick", ["query", "key", "value", "value of no weight", "infinite"])
+def test_what_is_not_a_number_survives_shared_out_keys(ops, Dh, Hq, Hkv, new, ctx, sick):
+    """Four and two CTAs a tile. A NaN in a query row, a key, a value (one whose share of the keys has a factor of zero as well) or an infinite
+    score shows in the rows that see it as it does when one CTA goes through all keys, and every other row stays as it was."""
+    rng = np.random.default_rng(Hq * Dh + ctx)
+    page = 16
+    kc, vc, bt, ks, vs = paged_cache(rng, "bfloat16", [ctx], Hkv, Dh, page, 180 * 16 // page + 8)
+    q = rng.standard_normal((new, Hq * Dh)) * 2
+    at = ctx - new + 40                                    # a key that rows 40 and up see
+    rows = np.zeros((new, Hq), bool)
+    if sick == "value of no weight":
+        q *= 64                                            # scores of hundreds, but for the first half of the keys and a little more
+        for p in range((ctx // 2 + 64) // page):
+            kc[bt[0, p]] *= 0.01
+            ks[0][p * page:(p + 1) * page] *= 0.01
+    if sick == "query":
+        q[5, 3 * Dh + 1] = np.nan
+        rows[5, 3] = True
+    elif sick == "infinite":
+        q[5, 3 * Dh + 1], rows[5, 3] = np.inf, True        # scores of both infinities
+    elif sick == "key":
+        kc[bt[0, at // page], 1, at % page, 2] = np.nan
+        rows[40:, Hq // Hkv:2 * Hq // Hkv] = True
+    else:
+        where = at if sick == "value" else 5
+        vc[bt[0, where // page], 1, where % page] = np.nan
+        rows[40 if sick == "value" else 0:, Hq // Hkv:2 * Hq // Hkv] = True
+    args = (dev(as_stored(q, "bfloat16"), torch.bfloat16), dev(kc, torch.bfloat16), dev(vc, torch.bfloat16))
+    index = (dev(np.array([0, new]), torch.int32), dev(np.array([ctx]), torch.int32), dev(bt, torch.int32), 1, new, Hq, Hkv, Dh, Dh ** -0.5, 0)
+    got = []
+    for max_keys in (0, ctx):
+        out = torch.full((new, Hq * Dh), 7.0, device="cuda", dtype=torch.bfloat16)
+        ops.attention_prompt_umma(*args, out, *index, max_keys=max_keys)
+        got.append(host(out).reshape(new, Hq, Dh))
+    for out in got:
+        assert np.isnan(out[rows]).all()
+    # a tile's masked values are multiplied with weights of zero, so rows that do not see a sick value may be lost with either
+    clean = ~np.isnan(got[0]).any(-1)
+    assert clean.sum() > 0 and (sick.startswith("value") or np.array_equal(clean, ~rows))
+    assert np.isfinite(got[1][clean]).all()
+    want = softmax_reference(as_stored(np.nan_to_num(q, posinf=0.0), "bfloat16").reshape(-1, Hq, Dh).astype(np.float64),
+                             ks[0].astype(np.float64), vs[0].astype(np.float64), Dh ** -0.5, 0, None, ctx - new)
+    assert rel_err(got[1][clean], want[clean]) < TOL["bfloat16"]

@@ -397,7 +397,7 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
         }
       }
       sums[DH] = mine ? m_used : -INFINITY;
-      sums[DH + 1] = l;
+      sums[DH + 1] = mine ? l : 0.0f;
     } else if (mine) {
       const float inv = l > 0.0f ? 1.0f / l : 0.0f;
       __nv_bfloat16* o_row = row < rows ? a.out + (static_cast<long long>(t0 + row / G) * a.q_heads + kvh * G + row % G) * DH : nullptr;
@@ -427,19 +427,25 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(here + column * 4), "r"(r));
         return at;
       };
-      float top = -INFINITY, f[kUmmaMaxSplits], total = 0.0f;
+      // A share that met no key of the row (reference -inf, row sum 0) is left out; every other one counts, whatever its factor: a share
+      // whose scores were NaN has the reference -inf too, but a NaN row sum, and one with a NaN among its values may have a factor
+      // that came to zero. Both leave NaN, as without shares.
+      float top = -INFINITY, f[kUmmaMaxSplits], l[kUmmaMaxSplits], total = 0.0f;
 #pragma unroll
       for (int r = 0; r < kUmmaMaxSplits; ++r) {
-        f[r] = -INFINITY;
-        if (r < a.splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f[r]) : "r"(peer(r, DH)));
+        f[r] = -INFINITY, l[r] = 0.0f;
+        if (r < a.splits) {
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f[r]) : "r"(peer(r, DH)));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[r]) : "r"(peer(r, DH + 1)));
+        }
         top = fmaxf(top, f[r]);
       }
+      bool left_out[kUmmaMaxSplits];
 #pragma unroll
       for (int r = 0; r < kUmmaMaxSplits; ++r) {
-        float l = 0.0f;
-        if (r < a.splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l) : "r"(peer(r, DH + 1)));
-        f[r] = f[r] == -INFINITY ? 0.0f : ex2(f[r] - top);
-        if (f[r] > 0.0f) total = fmaf(l, f[r], total);
+        left_out[r] = f[r] == -INFINITY && l[r] == 0.0f;
+        f[r] = f[r] == -INFINITY ? l[r] : ex2(f[r] - top);      // (-inf with a row sum: that is NaN)
+        if (!left_out[r]) total = fmaf(l[r], f[r], total);
       }
       const float inv = total > 0.0f ? 1.0f / total : 0.0f;
       const int cols = DH / a.splits;
@@ -449,7 +455,7 @@ attn_prompt_umma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
           float v[8] = {};
 #pragma unroll
           for (int r = 0; r < kUmmaMaxSplits; ++r) {
-            if (r >= a.splits || !(f[r] > 0.0f)) continue;      // (what a CTA without keys for the row left is not read)
+            if (left_out[r]) continue;      // (its sums were not written)
 #pragma unroll
             for (int e = 0; e < 8; e += 4) {
               float x[4];
