@@ -1189,7 +1189,9 @@ def test_latent_attention_over_expanded_keys(ops, H, page, window, new, ctx, sin
     latents = torch.full((rows, kd), float("nan"), device="cuda", dtype=torch.bfloat16)
     ops.latent_gather(dev(kc, torch.bfloat16), *index, dev(bt, torch.int32), len(new), window, latents)
     firsts = [max(0, c - n - window + 1) // 64 * 64 if window else 0 for c, n in zip(ctx, new)]
-    want_rows = np.concatenate([np.concatenate([k[f:, 0], np.zeros((-(len(k) - f) % 64, kd))]) for k, f in zip(ks, firsts)])
+    edges = [max(0, c - n - window + 1) if window else 0 for c, n in zip(ctx, new)]      # ahead of the first key seen: zeros too
+    want_rows = np.concatenate([np.concatenate([np.zeros((e - f, kd)), k[e:, 0], np.zeros((-(len(k) - f) % 64, kd))])
+                                for k, f, e in zip(ks, firsts, edges)])
     assert np.array_equal(host(latents), want_rows)
     kv = as_stored(rng.standard_normal((rows, H * 256)), "bfloat16")
     q = as_stored(rng.standard_normal((T, H * 192)) * 1.5, "bfloat16")
@@ -1273,3 +1275,32 @@ def test_what_is_not_a_number_survives_shared_out_keys(ops, Dh, Hq, Hkv, new, ct
     want = softmax_reference(as_stored(np.nan_to_num(q, posinf=0.0), "bfloat16").reshape(-1, Hq, Dh).astype(np.float64),
                              ks[0].astype(np.float64), vs[0].astype(np.float64), Dh ** -0.5, 0, None, ctx - new)
     assert rel_err(got[1][clean], want[clean]) < TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("page,window,new,ctx", [(16, 100, [70, 64], [300, 513]), (8, 90, [64], [1000]), (64, 40, [65], [300])])
+def test_pages_behind_a_window_are_not_gathered(ops, page, window, new, ctx):
+    """Pages below a window have been given back: the table names page 0 there, which is another request's by then. Tiles begin below the
+    window's first key, so NaN in page 0 must not reach the rows gathered, nor the attention over them."""
+    rng = np.random.default_rng(page + window)
+    H, kd = 2, 128
+    kc, _, bt, ks, _ = paged_cache(rng, "bfloat16", ctx, 1, kd, page, 100 * 16 // page + 8)
+    kc = np.concatenate([np.full_like(kc[:1], np.nan), kc])        # page 0: someone else's
+    bt = bt + 1
+    edges = [c - n - window + 1 for c, n in zip(ctx, new)]           # first key that the sequence's first row sees
+    for s, edge in enumerate(edges):
+        bt[s, :edge // page] = 0
+        bt[s, -(-ctx[s] // page):] = 0
+    qs = np.concatenate([[0], np.cumsum(new)])
+    index = (dev(qs, torch.int32), dev(np.array(ctx), torch.int32))
+    rows = ops.latent_expanded_rows(ctx, new, window)
+    latents = torch.full((rows, kd), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.latent_gather(dev(kc, torch.bfloat16), *index, dev(bt, torch.int32), len(new), window, latents)
+    want = [np.zeros((0, kd))]
+    for k, c, edge in zip(ks, ctx, edges):
+        first = edge // 64 * 64
+        want += [np.zeros((edge - first, kd)), k[edge:, 0], np.zeros((-(c - first) % 64, kd))]
+    assert np.array_equal(host(latents), np.concatenate(want))
+    q = dev(as_stored(rng.standard_normal((sum(new), H * 192)), "bfloat16"), torch.bfloat16)
+    out = torch.full((sum(new), H * 128), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.attention_latent_expanded(q, latents, latents.repeat(1, H * 256 // kd), out, *index, len(new), max(new), H, 192 ** -0.5, window)
+    assert torch.isfinite(out.float()).all()

@@ -380,7 +380,8 @@ static int launch_prompt_exact(const CUtensorMap& km, const CUtensorMap& vm, con
 }
 
 // The latents and rotated key parts that the portions' rows see, from the pages into rows [.., kd] one after the other (what
-// expanded_first and expanded_rows say), zeros behind a sequence's last key. A warp a row.
+// expanded_first and expanded_rows say), zeros behind a sequence's last key and ahead of the first key that the window leaves its first
+// row: pages there have been given back, and what the table names in their place belongs to others. A warp a row.
 __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ keys, const int* __restrict__ query_start,
                                                            const int* __restrict__ context_lens, const int* __restrict__ block_tables,
                                                            int max_blocks, int n_seqs, int window, int page_size, int kd, int rows,
@@ -394,8 +395,13 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16*
     if (at < n) break;
     at -= n;
   }
-  const int key = s < n_seqs ? expanded_first(context_lens[s], query_start[s + 1] - query_start[s], window) + at : 0;
-  const bool there = s < n_seqs && key < context_lens[s];
+  int key = 0;
+  bool there = false;
+  if (s < n_seqs) {
+    const int context = context_lens[s], queries = query_start[s + 1] - query_start[s];
+    key = expanded_first(context, queries, window) + at;
+    there = key < context && (window <= 0 || key > context - queries - window);
+  }
   const __nv_bfloat16* src = keys;
   if (there) src += (static_cast<long long>(block_tables[static_cast<long long>(s) * max_blocks + key / page_size]) * page_size + key % page_size) * kd;
   for (int c = lane; c < kd / 8; c += 32)
