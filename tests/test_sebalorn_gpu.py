@@ -210,6 +210,40 @@ def test_whole_prompts_decoding_and_portions(tmp_path, truth, name, dtype):
     close(np.stack([rows[("m", i)] for i in range(100, 150)]), want[100:], dtype, f"{name} prompt then decoding")
 
 
+def test_latent_layers_of_the_size_that_is_multiplied_out(tmp_path, monkeypatch):
+    """Latent layers of heads of 128 + 64 with values of 128: portions over multiplied-out keys in a prompt, behind cached tokens and beside
+    decoding requests, against the plain rows. A document in portions outgrows the buffer of these keys once, and the workspace
+    keeps one; where the device has no room for it the folded form gives the same rows."""
+    cfg = plain.make_config([LA(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=64, q_rank=48, base=100.0, mlp=plain.dense(64)),
+                             LA(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=72, q_rank=40, mlp=None)], vocab=60, width=64)
+    w = plain.random_weights(cfg, 3)
+    toks, other = tokens_of(cfg, 500, 1), tokens_of(cfg, 90, 2)
+    want, beside = reference(w, cfg, toks), reference(w, cfg, other)
+    from tiny_inference_engine_b200.engine.workspace import Workspace
+    from tiny_inference_engine_b200.parts import latent_attention
+    taken = []
+    inner = latent_attention.LatentAttention._attend_expanded
+    monkeypatch.setattr(latent_attention.LatentAttention, "_attend_expanded", lambda self, *a: taken.append(inner(self, *a)) or taken[-1])
+    for room in (True, False):
+        if not room:
+            monkeypatch.setattr(Workspace, "_free_bytes", lambda self: 0)
+        hs = Harness(tmp_path / str(room), cfg, w, "bfloat16", max_tokens=132)
+        taken.clear()
+        close(hs.in_portions("p", toks, [70, 130, 64, 100, 131]), want, "bfloat16", f"in portions, room {room}")
+        assert taken == [n if room else 0 for n in (70, 130, 64, 100, 131, 5) for _ in range(2)][:10] + [0, 0]
+        rows = hs.step([("b", other[:40], range(40))])
+        rows.update(hs.step([("a", toks[:100], range(100)), ("b", other[40:41], [0])]))
+        rows.update(hs.step([("b", other[41:42], [0]), ("a", toks[100:228], range(128))]))
+        rows.update(hs.step([("b", other[42:82], range(40)), ("a", toks[228:318], range(90))]))
+        close(np.stack([rows[("a", i)] for i in range(318)]), want[:318], "bfloat16", f"beside a request that decodes, room {room}")
+        close(np.stack([rows[("b", i)] for i in range(82)]), beside[:82], "bfloat16", f"the request that decodes, room {room}")
+        ws = hs.runner.ws
+        assert not ws._retired
+        if room:
+            most = max(latent_attention.expanded_capacity(h, r + 64) * 2 * (h * 256 + r + 64) for h, r in ((3, 64), (2, 72)))
+            assert sum(t.numel() * 2 for k, t in ws._flat.items() if "expanded" in k[0]) <= most
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["mixed", "odd", "square"])
 def test_mixed_batches_on_a_small_pool_with_two_state_slots(tmp_path, truth, name, dtype):

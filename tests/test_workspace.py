@@ -1,0 +1,31 @@
+"""Workspace buffers on the CPU: which are kept, which are let go, and what happens when the device is short of memory."""
+import torch
+
+from tiny_inference_engine_b200.engine.workspace import Workspace
+from tiny_inference_engine_b200.parts import latent_attention
+
+
+def test_spare_buffers_are_outgrown_without_a_trace_and_refused_when_memory_is_short():
+    ws = Workspace(8, "cpu")
+    free = [1 << 20]
+    ws._free_bytes = lambda: free[0]
+    a = ws.spare("x", 100, torch.bfloat16, 128)
+    assert a.numel() == 128 and ws.spare("x", 128, torch.bfloat16, 500) is a
+    b = ws.spare("x", 129, torch.bfloat16, 1000)
+    assert b.numel() == 1000 and ws.bytes() == 2000                # the outgrown one is gone
+    free[0] = 8000
+    assert ws.spare("x", 1001, torch.bfloat16, 2001) is None       # 4,002 bytes: more than half of what is left
+    assert ws.spare("x", 1000, torch.bfloat16) is b                # what is there stays
+    free[0] = 1 << 20
+    assert ws.spare("x", 1001, torch.bfloat16) is None             # asked once, not at every step
+    kept = ws.flat("y", 10, torch.float32)
+    ws.flat("y", 11, torch.float32)
+    assert ws.bytes() == 2000 + 40 + 80 and kept.numel() == 10     # a captured graph may still use it
+
+
+def test_expanded_keys_stay_within_their_bytes():
+    for heads, key_dim in ((1, 128), (16, 576), (32, 576), (33, 576), (64, 320), (128, 576), (500, 512)):
+        keys = latent_attention.expanded_capacity(heads, key_dim)
+        assert 0 < keys <= latent_attention.EXPAND_MAX_KEYS
+        assert keys * 2 * (heads * 256 + key_dim) <= latent_attention.EXPAND_MAX_BYTES
+    assert latent_attention.expanded_capacity(32, 576) == 16384 and latent_attention.expanded_capacity(128, 576) == 4528

@@ -3,8 +3,10 @@
 Row buffers are allocated once at their largest size. A flat buffer grows when a step asks for more
 than any step before it; the smaller buffer it replaces is kept, never given back, because a
 captured CUDA graph may still write to its address (and read from it in the same graph). Callers
-that know their largest need say so (`capacity`), so that growth is the exception. Steady-state
-stepping allocates nothing (the reference's arena: src/model/qwen3.cpp:109-146).
+that know their largest need say so (`capacity`), so that growth is the exception. Buffers of steps
+that are never captured (`spare`) are let go when they are outgrown, and are not to be had where the
+device is short of memory. Steady-state stepping allocates nothing (the reference's arena:
+src/model/qwen3.cpp:109-146).
 """
 from __future__ import annotations
 
@@ -18,6 +20,7 @@ class Workspace:
         self._rows: dict[tuple, torch.Tensor] = {}
         self._flat: dict[tuple, torch.Tensor] = {}
         self._retired: list[torch.Tensor] = []      # outgrown buffers: captured graphs may still use them
+        self._refused: dict[tuple, int] = {}        # spare buffers that there was no room for, and their smallest size
 
     def rows(self, name: str, n: int, width: int, dtype: torch.dtype) -> torch.Tensor:
         """[n, width] view of a buffer that holds max_rows rows."""
@@ -42,6 +45,28 @@ class Workspace:
             buf = make(max(numel, capacity, 2 * buf.numel() if buf is not None else 0))
             self._flat[key] = buf
         return buf
+
+    def spare(self, name: str, numel: int, dtype: torch.dtype, capacity: int = 0) -> torch.Tensor | None:
+        """At least `numel` elements for a step that is not captured and that has another way if there are none: None where the
+        buffer would take more than half of what the device has left (the buffers that other steps will ask for are not
+        there yet). An outgrown buffer goes back to the allocator; the stream's order keeps it whole until the steps that use it are done."""
+        key = (name, dtype, "spare")
+        buf = self._flat.get(key)
+        if buf is not None and buf.numel() >= numel:
+            return buf
+        if numel >= self._refused.get(key, numel + 1):
+            return None
+        size = max(numel, capacity)
+        if size * dtype.itemsize > self._free_bytes() // 2:
+            self._refused[key] = numel
+            return None
+        self._flat.pop(key, None)
+        del buf
+        self._flat[key] = buf = torch.empty(size, dtype=dtype, device=self.device)
+        return buf
+
+    def _free_bytes(self) -> int:
+        return torch.cuda.mem_get_info(self.device)[0]
 
     def zeros(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that is zero when first handed out (kernels that use it leave it zero)."""

@@ -35,9 +35,16 @@ LATENT_ROWS = 32            # (token, head) rows of a block of that kernel; one 
 
 # Portions multiply the cached latents out into keys and values per head (csrc/attention_prompt_exact.cu) where these cost less than the folded
 # queries' 576 + 512 dimensions a pair: from EXPAND_MIN_TOKENS tokens on (one layer of 32 heads of 128 + 64, 2,048 tokens: 1,940 us
-# folded, products and all, about 150 expanded), and up to EXPAND_MAX_KEYS keys in all, which bounds what the step keeps for it (16 KB a key with 32 heads).
+# folded, products and all, about 150 expanded), and up to as many keys in all as EXPAND_MAX_BYTES hold (`expanded_capacity`): the
+# latents and 512 bytes a head and key, 16,384 keys of 32 heads and 4,528 of 128. The step's workspace keeps one such buffer for all layers.
 EXPAND_MIN_TOKENS = 64
 EXPAND_MAX_KEYS = 16384
+EXPAND_MAX_BYTES = 288 << 20
+
+
+def expanded_capacity(heads: int, key_dim: int) -> int:
+    """The most keys that a step multiplies out for a layer of `heads` heads over latents of `key_dim` (bfloat16)."""
+    return min(EXPAND_MAX_KEYS, EXPAND_MAX_BYTES // (2 * (heads * (ops.EXPANDED_KEY + ops.EXPANDED_VALUE) + key_dim)))
 
 
 def latent_split_keys(longest: int, sequences: int, heads: int) -> int:
@@ -187,12 +194,17 @@ class LatentAttention(Mixer):
         if rows is None:
             starts = ctx.host.query_start
             rows = ctx.memo[key] = ops.latent_expanded_rows(ctx.host.context_lens[:S], starts[1:S + 1] - starts[:S], self.window)
-        if rows > EXPAND_MAX_KEYS:
+        H, per_key = self.heads, self.heads * (self.dim + self.vdim) + self.key_dim
+        most = expanded_capacity(H, self.key_dim)
+        if rows > most:
             return 0
-        H, wide = self.heads, self.heads * (self.dim + self.vdim)
-        most = min(EXPAND_MAX_KEYS, 2 * ctx.ws.max_rows)
-        latents = ctx.ws.flat("lattn.latents", rows * self.key_dim, self.dtype, most * self.key_dim)[:rows * self.key_dim].view(rows, self.key_dim)
-        kv = ctx.ws.flat("lattn.kv", rows * wide, self.dtype, most * wide)[:rows * wide].view(rows, wide)
+        # whole prompts and what precedes a first portion or two fit twice a step's rows; later portions take the most at once
+        small = min(most, 2 * ctx.ws.max_rows)
+        both = ctx.ws.spare("lattn.expanded", rows * per_key, self.dtype, (small if rows <= small else most) * per_key)
+        if both is None:
+            return 0
+        latents = both[:rows * self.key_dim].view(rows, self.key_dim)
+        kv = both[rows * self.key_dim:rows * per_key].view(rows, per_key - self.key_dim)
         ops.latent_gather(cache.k, ctx.query_start, ctx.context_lens, g.block_tables, S, self.window, latents)
         self.gemm_kv(latents[:, :self.rank], kv)
         ops.latent_query_rot(q[:n], self.dim, self.rot, table, ctx.positions[:n], q[:n], self.dim, H, neighbours)
