@@ -1,4 +1,5 @@
-"""Workspace buffers on the CPU: which are kept, which are let go, and what happens when the device is short of memory."""
+"""Workspace buffers on the CPU: which are kept, which are let go, and what happens when the device is short of memory; and which steps
+ask for the largest of them."""
 import torch
 
 from tiny_inference_engine_b200.engine.workspace import Workspace
@@ -29,3 +30,15 @@ def test_expanded_keys_stay_within_their_bytes():
         assert 0 < keys <= latent_attention.EXPAND_MAX_KEYS
         assert keys * 2 * (heads * 256 + key_dim) <= latent_attention.EXPAND_MAX_BYTES
     assert latent_attention.expanded_capacity(32, 576) == 16384 and latent_attention.expanded_capacity(128, 576) == 4528
+
+
+def test_latents_are_multiplied_out_where_many_queries_share_a_key():
+    pays = latent_attention.expanding_pays
+    assert pays([64], [64], 0) == 64 and pays([2048], [2048], 0) == 2048 and pays([16384], [64], 0) == 16384
+    assert pays([500] * 32, [2] * 32, 0) == 0 and pays([1000] * 16, [8] * 16, 0) == 0 and pays([500] * 16, [16] * 16, 0) == 0
+    assert pays([300] * 4, [24] * 4, 0) == 4 * 320
+    for context, n, window in ((70, 64, 0), (300, 64, 100), (90, 64, 40), (130, 64, 100), (5000, 65, 1024), (64, 64, 1)):
+        pairs = sum(min(i + 1, window or 1 << 30) for i in range(context - n, context))
+        rows = latent_attention.ops.latent_expanded_rows([context], [n], window)
+        keys = context - max(0, context - n - window + 1 if window else 0)
+        assert pays([context], [n], window) == (rows if pairs >= latent_attention.EXPAND_PAIRS_PER_KEY * keys else 0), (context, n, window)

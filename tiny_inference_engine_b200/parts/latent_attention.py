@@ -33,11 +33,15 @@ LATENT_SPLIT_KEYS = 128     # least keys per split of a sequence that brings one
 LATENT_ROWS = 32            # (token, head) rows of a block of that kernel; one block an SM
 
 
-# Portions multiply the cached latents out into keys and values per head (csrc/attention_prompt_exact.cu) where these cost less than the folded
-# queries' 576 + 512 dimensions a pair: from EXPAND_MIN_TOKENS tokens on (one layer of 32 heads of 128 + 64, 2,048 tokens: 1,940 us
-# folded, products and all, about 150 expanded), and up to as many keys in all as EXPAND_MAX_BYTES hold (`expanded_capacity`): the
-# latents and 512 bytes a head and key, 16,384 keys of 32 heads and 4,528 of 128. The step's workspace keeps one such buffer for all layers.
+# Portions multiply the cached latents out into keys and values per head (csrc/attention_prompt_exact.cu) where that costs less than the
+# folded queries' 576 + 512 dimensions a pair (`expanding_pays`): from EXPAND_MIN_TOKENS tokens on, with EXPAND_PAIRS_PER_KEY pairs of a
+# query and a key for each key that is multiplied out. Measured, folded with all its products against expanded, 32 heads of 128 + 64: 2,048
+# tokens 1,940 us against about 150; 64 tokens behind none 38 / 31, behind 448 85 / 46, behind 16,320 1,707 / 540 (32 to 64 pairs a key); 4 x 24
+# tokens at 300 (22 pairs) 67 / 54, with 128 heads 157 / 157; 16 x 16 at 500 (15 pairs) 155 / 216; 32 x 2 at 500 (2 pairs) 85 / 376.
+# And up to as many keys in all as EXPAND_MAX_BYTES hold (`expanded_capacity`): the latents and 512 bytes a head and key, 16,384 keys of
+# 32 heads and 4,528 of 128. The step's workspace keeps one such buffer for all layers.
 EXPAND_MIN_TOKENS = 64
+EXPAND_PAIRS_PER_KEY = 20
 EXPAND_MAX_KEYS = 16384
 EXPAND_MAX_BYTES = 288 << 20
 
@@ -45,6 +49,17 @@ EXPAND_MAX_BYTES = 288 << 20
 def expanded_capacity(heads: int, key_dim: int) -> int:
     """The most keys that a step multiplies out for a layer of `heads` heads over latents of `key_dim` (bfloat16)."""
     return min(EXPAND_MAX_KEYS, EXPAND_MAX_BYTES // (2 * (heads * (ops.EXPANDED_KEY + ops.EXPANDED_VALUE) + key_dim)))
+
+
+def expanding_pays(contexts, queries, window: int) -> int:
+    """How many rows of multiplied-out keys portions of these sequences need (host numbers), or 0 where the folded form is faster."""
+    pairs = keys = 0
+    for context, n in zip(contexts, queries):
+        context, n = int(context), int(n)
+        short = min(n, max(0, window - (context - n))) if window > 0 else n      # queries that see all keys ahead of them
+        pairs += short * (context - n) + short * (short + 1) // 2 + (n - short) * window
+        keys += context - (max(0, context - n - window + 1) if window > 0 else 0)
+    return ops.latent_expanded_rows(contexts, queries, window) if pairs >= EXPAND_PAIRS_PER_KEY * keys else 0
 
 
 def latent_split_keys(longest: int, sequences: int, heads: int) -> int:
@@ -189,14 +204,14 @@ class LatentAttention(Mixer):
         n, S = ctx.multi_rows, ctx.multi_seqs
         if self.gemm_kv is None or n < EXPAND_MIN_TOKENS or cache.k.dtype != torch.bfloat16:
             return 0
-        key = ("latent_expanded_rows", self.window)
+        key = ("expanding_pays", self.window)
         rows = ctx.memo.get(key)
         if rows is None:
             starts = ctx.host.query_start
-            rows = ctx.memo[key] = ops.latent_expanded_rows(ctx.host.context_lens[:S], starts[1:S + 1] - starts[:S], self.window)
+            rows = ctx.memo[key] = expanding_pays(ctx.host.context_lens[:S], starts[1:S + 1] - starts[:S], self.window)
         H, per_key = self.heads, self.heads * (self.dim + self.vdim) + self.key_dim
         most = expanded_capacity(H, self.key_dim)
-        if rows > most:
+        if rows == 0 or rows > most:
             return 0
         # whole prompts and what precedes a first portion or two fit twice a step's rows; later portions take the most at once
         small = min(most, 2 * ctx.ws.max_rows)
