@@ -1304,3 +1304,16 @@ def test_pages_behind_a_window_are_not_gathered(ops, page, window, new, ctx):
     out = torch.full((sum(new), H * 128), float("nan"), device="cuda", dtype=torch.bfloat16)
     ops.attention_latent_expanded(q, latents, latents.repeat(1, H * 256 // kd), out, *index, len(new), max(new), H, 192 ** -0.5, window)
     assert torch.isfinite(out.float()).all()
+
+
+def test_rows_behind_the_last_query_end(ops):
+    """More rows than the sequences' queries: each takes the place that its number says, as in the kernel without tiles, and the walk over a tile's
+    sequences ends."""
+    Hq, Hkv, Dh, page, ctx, queries, T = 2, 1, 64, 16, 20, 16, 20
+    rng = np.random.default_rng(3)
+    kc, vc, bt, ks, vs = paged_cache(rng, "float32", [ctx + T - queries], Hkv, Dh, page, 8)
+    q = rng.standard_normal((T, Hq * Dh)).astype(np.float32)
+    out = torch.full((T, Hq * Dh), float("nan"), device="cuda")
+    ops.attention_rows(dev(q), dev(kc), dev(vc), out, dev(np.zeros(T), torch.int32), dev(np.array([0, queries]), torch.int32),
+                       dev(np.array([ctx]), torch.int32), dev(bt, torch.int32), Hq, Hkv, Dh, Dh ** -0.5)
+    assert rel_err(host(out), dense_reference(q, ks[0], vs[0], Hq, Hkv, Dh, T)) < TOL["float32"]

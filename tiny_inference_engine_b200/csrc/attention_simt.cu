@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(128) attention_rows_tiled_kernel(AttnArgs a) {
   }
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, acc[2][OWN] = {};
   for (int begin = t0; begin < t_end;) {
-    const int s = a.seq_of_row[begin], end = min(t_end, a.query_start[s + 1]);
+    const int s = a.seq_of_row[begin], end = min(t_end, max(begin + 1, a.query_start[s + 1]));      // (a row at least: the walk ends whatever the indexes say)
     const int* table = a.block_tables + static_cast<long long>(s) * a.max_blocks;
     const int shift = a.context_lens[s] - a.query_start[s + 1];      // position of row t: t + shift
     const int lo = a.window > 0 ? max(0, begin + shift - a.window + 1) : 0, hi = end - 1 + shift;
