@@ -1317,3 +1317,19 @@ def test_rows_behind_the_last_query_end(ops):
     ops.attention_rows(dev(q), dev(kc), dev(vc), out, dev(np.zeros(T), torch.int32), dev(np.array([0, queries]), torch.int32),
                        dev(np.array([ctx]), torch.int32), dev(bt, torch.int32), Hq, Hkv, Dh, Dh ** -0.5)
     assert rel_err(host(out), dense_reference(q, ks[0], vs[0], Hq, Hkv, Dh, T)) < TOL["float32"]
+
+
+@pytest.mark.parametrize("Dh,new,ctx", [(32, 20, 20), (64, 40, 100), (128, 33, 64)])
+def test_a_value_that_is_not_a_number_counts_at_any_weight(ops, Dh, new, ctx):
+    """Key 0 scores 200 below the others, so its weight is zero in float32; its value is NaN and every row sees it. (One tile of keys and
+    several, the last one seen in part.)"""
+    u = np.ones(Dh, np.float32)
+    page = 16
+    kc, vc, bt, ks, vs = paged_cache(np.random.default_rng(1), "float32", [ctx], 1, Dh, page, 12)
+    for j in range(ctx):
+        kc[bt[0, j // page], 0, j % page] = (-u if j == 0 else u) * 100 / Dh
+    vc[bt[0, 0], 0, 0] = np.nan
+    out = torch.zeros((new, Dh), device="cuda")
+    ops.attention_rows(dev(np.tile(u, (new, 1))), dev(kc), dev(vc), out, dev(np.zeros(new), torch.int32), dev(np.array([0, new]), torch.int32),
+                       dev(np.array([ctx]), torch.int32), dev(bt, torch.int32), 1, 1, Dh, 1.0)
+    assert np.isnan(host(out)).all()
