@@ -1333,3 +1333,22 @@ def test_a_value_that_is_not_a_number_counts_at_any_weight(ops, Dh, new, ctx):
     ops.attention_rows(dev(np.tile(u, (new, 1))), dev(kc), dev(vc), out, dev(np.zeros(new), torch.int32), dev(np.array([0, new]), torch.int32),
                        dev(np.array([ctx]), torch.int32), dev(bt, torch.int32), 1, 1, Dh, 1.0)
     assert np.isnan(host(out)).all()
+
+
+def test_short_portions_do_not_share_tiles(ops):
+    """Twenty portions of two or three tokens: a tile of 16 rows would go through the keys of eight of them one after the other, so they run
+    row by row as a portion alone does, to the last bit."""
+    Hq, Hkv, Dh, page = 4, 2, 64, 16
+    rng = np.random.default_rng(5)
+    new, ctx = [2 + i % 2 for i in range(20)], [90 + 7 * i for i in range(20)]
+    kc, vc, bt, ks, vs = paged_cache(rng, "float32", ctx, Hkv, Dh, page, 330)
+    qs = np.concatenate([[0], np.cumsum(new)])
+    q = dev(rng.standard_normal((sum(new), Hq * Dh)))
+    planes, heads = (dev(kc), dev(vc)), (Hq, Hkv, Dh, Dh ** -0.5)
+
+    def rows(lo, hi):
+        out = torch.empty((qs[hi] - qs[lo], Hq * Dh), device="cuda")
+        ops.attention_rows(q[qs[lo]:qs[hi]], *planes, out, dev(np.repeat(np.arange(hi - lo), new[lo:hi]), torch.int32), dev(qs[lo:hi + 1] - qs[lo], torch.int32),
+                           dev(np.array(ctx[lo:hi]), torch.int32), dev(bt[lo:hi], torch.int32), *heads)
+        return out
+    assert torch.equal(rows(0, 20), torch.cat([rows(i, i + 1) for i in range(20)]))

@@ -34,7 +34,7 @@ struct AttnArgs {
   long long q_stride;
   int max_blocks;
   int rows;                 // T
-  int seqs;                 // S
+  int seqs;                 // sequences (rows kernels: those that the rows belong to)
   int q_heads, kv_heads, head_dim, page_size;
   int window;               // 0 = all keys
   float scale;
@@ -365,9 +365,12 @@ __global__ void __launch_bounds__(128) attention_rows_tiled_kernel(AttnArgs a) {
   }
 }
 
-// What the tiled kernel takes; everything else is the rows kernel's. (A tile wants rows to share it: few rows run a warp each.)
+// What the tiled kernel takes; everything else is the rows kernel's. A tile wants rows to share it: few rows run a warp each, and so do
+// portions of two or three tokens, whose keys a block goes through portion by portion. A call of 8 heads over 2 of 128, rows kernel
+// against tiles: 30 portions of 2 tokens at 2,000 keys 997 / 1,541 us, 16 of 4 at 1,000 491 / 396, 16 of 8 454 / 203, one of 16 at 2,000
+// 760 / 198; 16 heads over 8 of 64: 30 of 2 1,248 / 1,275, 16 of 4 625 / 329.
 inline bool rows_tiled_takes(const AttnArgs& a) {
-  return (a.head_dim == 32 || a.head_dim == 64 || a.head_dim == 128) && a.rows >= kTileRows && a.q_heads <= 65535 && a.q_stride % 4 == 0 &&
+  return (a.head_dim == 32 || a.head_dim == 64 || a.head_dim == 128) && a.rows >= kTileRows && a.rows >= 4ll * a.seqs && a.q_heads <= 65535 && a.q_stride % 4 == 0 &&
          (reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) % 16 == 0;
 }
 

@@ -261,15 +261,16 @@ def _attn_common(q, k_cache, v_cache, out, query_start, context_lens, block_tabl
 
 
 def attention_rows(q, k_cache, v_cache, out, seq_of_row, query_start, context_lens, block_tables, q_heads, kv_heads,
-                   head_dim, scale: float, window: int = 0) -> None:
-    """Causal attention of every row of the step over the paged cache (CUDA cores)."""
+                   head_dim, scale: float, window: int = 0, portions: int | None = None) -> None:
+    """Causal attention of every row of the step over the paged cache (CUDA cores). `portions`: how many sequences the rows belong to, where
+    these are not all (a hint: which kernel is launched, not what it computes)."""
     _dev(q, k_cache, v_cache, out, seq_of_row, query_start, context_lens, block_tables)
     S = _attn_common(q, k_cache, v_cache, out, query_start, context_lens, block_tables, q_heads, kv_heads, head_dim)
     _need(seq_of_row.dtype == torch.int32 and seq_of_row.numel() == q.shape[0], "attention: seq_of_row must be int32 [T]")
     call("tie_attention_rows", dtype_code(q), q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
          out.data_ptr(), seq_of_row.data_ptr(), query_start.data_ptr(), context_lens.data_ptr(), block_tables.data_ptr(),
-         block_tables.shape[1], q.shape[0], S, q_heads, kv_heads, head_dim, k_cache.shape[2], int(window), float(scale),
-         _stream())
+         block_tables.shape[1], q.shape[0], S if portions is None else int(portions), q_heads, kv_heads, head_dim, k_cache.shape[2],
+         int(window), float(scale), _stream())
 
 
 def attention_split_scratch_floats(n_list: int, q_heads: int, head_dim: int, max_splits: int) -> int:

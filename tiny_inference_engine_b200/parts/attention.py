@@ -164,7 +164,7 @@ class GQAttention(Mixer):
                     (ops.attention_prompt_tma if tma else ops.attention_prompt_tc)(*args)
             else:
                 ops.attention_rows(q[:n], cache.k, cache.v, attn[:n], ctx.seq_of_row[:n], ctx.query_start,
-                                   ctx.context_lens, g.block_tables, Hq, Hkv, Dh, self.scale, self.window)
+                                   ctx.context_lens, g.block_tables, Hq, Hkv, Dh, self.scale, self.window, portions=ctx.multi_seqs)
         if ctx.single_count > 0:
             self.attend_single(q, attn, ctx, g, cache, tc)
 
