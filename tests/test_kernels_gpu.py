@@ -1352,3 +1352,33 @@ def test_short_portions_do_not_share_tiles(ops):
                            dev(np.array(ctx[lo:hi]), torch.int32), dev(bt[lo:hi], torch.int32), *heads)
         return out
     assert torch.equal(rows(0, 20), torch.cat([rows(i, i + 1) for i in range(20)]))
+
+
+@pytest.mark.parametrize("mode", ["delta", "channel", "head"])
+def test_sequences_without_tokens_keep_their_state(ops, mode, monkeypatch):
+    """A step in chunks in which the first, a middle and the last sequence bring nothing: their rows of the state stay to the last bit, and the
+    others' outputs are those of the walk token by token."""
+    from types import SimpleNamespace
+    from tiny_inference_engine_b200.engine.workspace import Workspace
+    H, dim, vdim, lens, taps = 2, 64, 64, [0, 100, 0, 33, 0], 4
+    rng = np.random.default_rng(4)
+    T, C = sum(lens), 2 * H * dim + H * vdim
+    q, k = (x / np.linalg.norm(x, axis=-1, keepdims=True) for x in rng.standard_normal((2, T, H, dim)))
+    v, beta = rng.standard_normal((T, H * vdim)), rng.uniform(0.1, 1.0, (T, H)) if mode != "channel" else None
+    decay = rng.uniform(0.3, 1.0, (T, H if mode == "head" else H * dim))
+    state0, proj = dev(rng.standard_normal((len(lens), H * dim * vdim + (taps - 1) * C))), dev(rng.standard_normal((T, C)))
+    qs = dev(np.concatenate([[0], np.cumsum(lens)]), torch.int32)
+    got = {}
+    for chunked in (True, False):
+        monkeypatch.setattr(ops, "chunks_pay", lambda *a: chunked)
+        rows = [dev(x.reshape(T, -1)) for x in (q, k, v)]
+        state, out = state0.clone(), torch.empty(T, H * vdim, device="cuda")
+        ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=max(lens), max_seqs=len(lens))
+        ops.delta_rule(*rows, None if beta is None else dev(beta), dev(decay), state, H * dim * vdim, proj, 0, H * dim, 2 * H * dim, qs,
+                       dev(np.arange(len(lens)), torch.int32), len(lens), H, H, dim, vdim, taps, out, plain=mode != "delta",
+                       decay_per_head=mode == "head", chunks=ops.RecurrenceChunks(ctx))
+        got[chunked] = host(out), host(state)
+    for s, n in enumerate(lens):
+        if n == 0:
+            assert np.array_equal(got[True][1][s, :H * dim * vdim], host(state0)[s, :H * dim * vdim])
+    assert rel_err(got[True][0], got[False][0]) < TOL["float32"] and rel_err(got[True][1], got[False][1]) < TOL["float32"]

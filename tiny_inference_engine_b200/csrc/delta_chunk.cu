@@ -409,8 +409,8 @@ __global__ void __launch_bounds__(DELTA ? 256 : 128) chunk_walk_kernel(ChunkWalk
   extern __shared__ __align__(16) float smem[];
   const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kChunkCols;
   const int slot = a.state_slots[s];
-  if (slot < 0) return;
   const int t0 = a.query_start[s], n = a.query_start[s + 1] - t0, base = chunk_base(a.query_start, s);
+  if (slot < 0 || n <= 0) return;            // a sequence without tokens keeps its state as it is
   const int vdim = sh.vdim, nv = sh.heads * vdim;
   const int tid = threadIdx.x, warp = (tid >> 5) & 3, lane = tid & 31;
   const bool corrects = DELTA && tid < 128;      // the warps that multiply with W
