@@ -1079,7 +1079,7 @@ def test_gemm_with_silu_epilogue(ops, M, I, K):
 
 @pytest.mark.parametrize("mode", ["delta", "channel", "head"])
 @pytest.mark.parametrize("H,G,dim,vdim,lens", [(2, 2, 128, 128, [1, 16, 33]), (4, 2, 64, 64, [15, 17]), (3, 3, 128, 20, [50])])
-def test_recurrence_in_chunks(ops, mode, H, G, dim, vdim, lens):
+def test_recurrence_in_chunks(ops, mode, H, G, dim, vdim, lens, monkeypatch):
     """The three recurrences sixteen tokens at a time against the plain loop in float64: chunks that end in the middle, single tokens, value
     heads that fill no block of columns, decays down to zero; the convolution's inputs as the kernel that walks token by token leaves them;
     and a token with a NaN leaves the tokens ahead of it in its chunk, and the other sequences, as they are."""
@@ -1118,7 +1118,8 @@ def test_recurrence_in_chunks(ops, mode, H, G, dim, vdim, lens):
     def engine(v, chunked):
         rows = [dev(x.reshape(T, -1)) for x in (q, k, v)]
         state, out = state0.clone(), torch.empty(T, H * vdim, device="cuda")
-        ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=10 ** 6 if chunked else 1, max_seqs=len(lens))
+        monkeypatch.setattr(ops, "chunks_pay", lambda *a: chunked)
+        ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=max(lens), max_seqs=len(lens))
         ops.delta_rule(*rows, None if beta is None else dev(beta), dev(decay.reshape(T, -1)), state, H * dim * vdim, proj, 0, G * dim, 2 * G * dim,
                        dev(qs, torch.int32), dev(np.arange(len(lens)), torch.int32), len(lens), H, G, dim, vdim, taps, out, plain=mode != "delta",
                        decay_per_head=mode == "head", chunks=ops.RecurrenceChunks(ctx))

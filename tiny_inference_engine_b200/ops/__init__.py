@@ -775,12 +775,23 @@ def delta_prep(proj, q_off: int, k_off: int, v_off: int, b_off: int, conv_w, sta
          _stream())
 
 
-def chunks_pay(longest: int, seqs: int) -> bool:
-    """Whether a step's recurrence is faster in chunks. Token by token, a portion of n tokens is a chain of n steps (0.25 us each with the
-    delta rule, 0.16 and 0.11 us without, heads of 128); in chunks it is n / 16 steps of 1.6 to 2 us behind a launch of its own. The two meet at
-    about 90 tokens (64: 22 against 31 us, 2,048: 514 against 305). Sequences that bring one token cost either kernel the trip of
-    their state, the chunked one about a microsecond each more (128 tokens beside 30 of them: 98 against 109 us)."""
-    return longest >= 88 + 8 * seqs
+def chunks_pay(longest: int, seqs: int, blocks: int, dim: int, plain: bool, decay_per_head: bool) -> bool:
+    """Whether a step's recurrence is faster in chunks; `blocks`: sequences x heads x column tiles of 16, `dim` key channels a head. Token by
+    token, a portion of n tokens is a chain of n steps (0.25 us each with the delta rule, 0.16 us with a decay a channel, 0.11 us with
+    one a head, heads of 128); in chunks it is n / 16 steps of 1.6 to 2 us behind a launch of its own. Sequences that bring one token cost
+    the chunked kernel about a microsecond each more. Token by token against chunks, us, 16 heads of 128 / 128 where nothing else is said:
+      delta rule          96 tokens 33.8 / 33.8, 128 43.0 / 35.8, 1,024 264 / 167; heads of 64: 128 34.8 / 31.7, 1,024 205 / 116;
+      a decay a channel   96 tokens 24.6 / 27.6, 128 30.7 / 29.5, 256 49.2 / 43.0; heads of 64: 128 22.5 / 23.6, 256 35.2 / 33.7;
+      a decay a head      the shortest chain, so only what it costs several blocks an SM pays: 128 blocks 256 tokens 38.9 / 44.0, 2,048
+                          240 / 247; 256 blocks 2 x 256 62 / 54, 1,021 + 510 213 / 161, 32 heads 2,048 414 / 327; 3 x 128 49 / 42; heads of 64
+                          64 heads 2,048 291 / 296, 2 x 1,021 277 / 220; 2 x 128 tokens 43 / 46."""
+    if longest < 88 + 8 * seqs:
+        return False
+    if not plain:
+        return longest >= 112
+    if not decay_per_head:
+        return longest >= 160 or blocks * dim * longest >= 4 << 20
+    return blocks * dim >= 1 << 15 and blocks * dim * longest >= 6 << 20
 
 
 class RecurrenceChunks:
@@ -815,7 +826,7 @@ def delta_rule(qn, kn, vn, beta, decay, state, conv_state_off: int, proj, q_off:
     _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1 and conv_state_off >= heads * dim * vdim,
           "delta_rule: state rows too short")
     _need(query_start.numel() >= seqs + 1 and state_slots.numel() >= seqs, "delta_rule: index tensors too short")
-    if chunks is not None and not single and chunks_pay(chunks.longest, seqs):
+    if chunks is not None and not single and chunks_pay(chunks.longest, seqs, seqs * heads * ((vdim + 15) // 16), dim, plain, decay_per_head):
         lib = library.library()
         scratch = chunks.scratch(lib, T, seqs, heads, dim, plain)
         if lib.tie_delta_chunk_takes(heads, kv_heads, dim, vdim, int(plain), int(decay_per_head), decay.stride(0), state.stride(0), qn.data_ptr(),
