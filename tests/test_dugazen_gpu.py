@@ -491,7 +491,7 @@ def test_inputs_of_the_recurrence_several_tokens_a_warp(lengths, heads, kv_heads
 @pytest.mark.parametrize("dim", [4, 72, 260, 2048, 8192, 8196, 16384, 16388])
 @pytest.mark.parametrize("splits,biased,picked", [(0, False, False), (0, True, True), (3, True, False), (5, False, True)])
 def test_normed_sublayer_outputs_join_the_stream(dim, splits, biased, picked, dtype):
-    """Rows held in registers, two and four pieces a thread, and the widest rows; a tensor or partial sums; all rows or some. The sums
+    """Rows held in registers, one and two pieces a thread, and in shared memory; a tensor or partial sums; all rows or some. The sums
     of squares are good to dim 2^-24 at worst and to a few 2^-24 as trees; an output is rounded once to its type."""
     from tiny_inference_engine_b200 import ops
     rng = np.random.default_rng(dim + splits)
@@ -515,3 +515,17 @@ def test_normed_sublayer_outputs_join_the_stream(dim, splits, biased, picked, dt
     if picked:
         want = want[[3, 0, 4]]
     assert rel_err(out.double().cpu().numpy(), want.numpy()) < (2e-6 if dtype == torch.float32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("dim", [12232, 12285, 12288])
+def test_rows_that_just_fill_the_shared_memory_a_block_has_unasked(dim):
+    """48 KB of row beside the few bytes of the sums."""
+    from tiny_inference_engine_b200 import ops
+    rng = np.random.default_rng(dim)
+    x, delta, wb, w = _on_gpu(rng, 3, dim), _on_gpu(rng, 3, dim), _on_gpu(rng, dim), _on_gpu(rng, dim)
+    norm = lambda v, e: v / torch.sqrt((v * v).mean(-1, keepdim=True) + e)
+    stream = x.double() + 0.7 * norm(delta.double(), 1e-6) * wb.double()
+    out = torch.empty(3, dim, device="cuda")
+    ops.add_normed_rmsnorm(x, ops.NormedDelta(delta, wb, 1e-6, 0.7, None), w, 1e-5, out)
+    assert rel_err(x.cpu().numpy(), stream.cpu().numpy()) < 2e-6
+    assert rel_err(out.cpu().numpy(), (norm(stream, 1e-5) * w.double()).cpu().numpy()) < 2e-6

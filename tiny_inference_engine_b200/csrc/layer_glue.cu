@@ -358,8 +358,9 @@ int launch_add_normed_rmsnorm(float* x, const void* delta, const float* part, lo
                               const float* w, float eps, void* out, int n, int dim, cudaStream_t s) {
   if (n == 0) return kOk;
   const size_t smem = static_cast<size_t>(dim) * sizeof(float);
+  const bool wide = smem > 47 * 1024;      // beside the sums' few bytes, more than a block has unless it asks
   auto kernel = add_normed_rmsnorm_kernel<T>;
-  if (smem > 48 * 1024) {
+  if (wide) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
       set_error("add_normed_rmsnorm: rows of %d floats do not fit shared memory", dim);
       return kBadArgument;
@@ -368,19 +369,19 @@ int launch_add_normed_rmsnorm(float* x, const void* delta, const float* part, lo
   const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (dim % 4 == 0 && part_stride % 4 == 0 && aligned(x) && aligned(delta) && aligned(part) && aligned(bias) && aligned(wb) &&
       aligned(w) && aligned(out)) {
-    if (dim <= 16384) {
-      // a piece a thread where few rows leave the SMs to themselves (the longest chain of loads counts), else two; wide rows take
-      // what 1024 threads need
-      const int pieces = dim > 8192 ? 4 : dim > 4096 || n >= 148 ? 2 : 1;
-      auto regs = pieces == 1 ? add_normed_rmsnorm_regs_kernel<T, 1>
-                              : pieces == 2 ? add_normed_rmsnorm_regs_kernel<T, 2> : add_normed_rmsnorm_regs_kernel<T, 4>;
+    if (dim <= 8192) {
+      // a piece a thread where few rows leave the SMs to themselves (the longest chain of loads counts), else two. (Rows above 8,192
+      // would take four pieces a thread, which spill at 1,024 threads: 2,048 rows of 8,196 90.1 us against 82.1 with the row in shared
+      // memory, of 16,384 130 / 127.)
+      const int pieces = dim > 4096 || n >= 148 ? 2 : 1;
+      auto regs = pieces == 1 ? add_normed_rmsnorm_regs_kernel<T, 1> : add_normed_rmsnorm_regs_kernel<T, 2>;
       TIE_LAUNCH(regs, n, 32 * ceil_div(dim, 128 * pieces), 0, s, x, static_cast<const T*>(delta), part, part_stride, splits, bias, wb,
                  eps_b, mult, rows, w, eps, static_cast<T*>(out), dim);
       TIE_RETURN_LAUNCH("add_normed_rmsnorm");
     }
     auto vec = add_normed_rmsnorm_vec4_kernel<T>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    TIE_LAUNCH(vec, n, dim >= 8192 ? 1024 : (dim >= 2048 ? 512 : (dim >= 1024 ? 256 : 128)), smem, s, x, static_cast<const T*>(delta),
+    if (wide) cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    TIE_LAUNCH(vec, n, 1024, smem, s, x, static_cast<const T*>(delta),
                part, part_stride, splits, bias, wb, eps_b, mult, rows, w, eps, static_cast<T*>(out), dim);
     TIE_RETURN_LAUNCH("add_normed_rmsnorm");
   }
