@@ -672,3 +672,20 @@ def test_heads_normed_without_a_weight_and_gated(dtype, H, vdim):
     want = y.double() * torch.sigmoid(wide[:, :H].double()).repeat_interleave(vdim, dim=1)
     ops.head_gate_mul(y, wide[:, :H], H, vdim)
     assert (y.double() - want).abs().max() < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_queries_rotated_in_place(dtype):
+    """The rotated part of a query over itself, bit for bit what goes elsewhere; the rest of the head stays. More pairs than a warp has lanes."""
+    from tiny_inference_engine_b200 import ops
+    draw, H, dim = _draw(6), 3, 24
+    pos = torch.tensor(POSITIONS, device="cuda", dtype=torch.int32)
+    for rot in (10, 64, 140):
+        q = draw(4, H * (dim + rot)).to(dtype)
+        for part, _, _ in _rotations(50.0, rot):
+            table, neighbours = part.rotation()
+            apart, inside = torch.zeros_like(q), q.clone()
+            ops.latent_query_rot(q, dim, rot, table, pos, apart, dim, H, neighbours)
+            ops.latent_query_rot(inside, dim, rot, table, pos, inside, dim, H, neighbours)
+            heads = [x.view(4, H, dim + rot) for x in (q, apart, inside)]
+            assert torch.equal(heads[2][..., dim:], heads[1][..., dim:]) and torch.equal(heads[2][..., :dim], heads[0][..., :dim])

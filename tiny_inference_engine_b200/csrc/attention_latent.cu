@@ -60,9 +60,10 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(const T* __restrict__ 
   }
 }
 
+// `folded` may be `q` itself (rank = dim): a lane reads both elements of its pair before it writes them, and no lane reads another's.
 template <typename T>
-__global__ void __launch_bounds__(128) latent_query_rot_kernel(const T* __restrict__ q, long long q_stride, int dim, int rot,
-                                                               Rotation turn, const int* __restrict__ positions, T* __restrict__ folded,
+__global__ void __launch_bounds__(128) latent_query_rot_kernel(const T* q, long long q_stride, int dim, int rot,
+                                                               Rotation turn, const int* __restrict__ positions, T* folded,
                                                                long long folded_stride, int rank, int heads,
                                                                long long items) {
   pdl_sync();

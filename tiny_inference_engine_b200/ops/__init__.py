@@ -965,7 +965,8 @@ def latent_prep(proj, q_off: int, q_rank: int, kv_off: int, rank: int, rot: int,
 
 
 def latent_query_rot(q, dim: int, rot: int, table, positions, folded, rank: int, heads: int, neighbours: bool = False) -> None:
-    """folded[t, h, rank : rank + rot] = rotation of q[t, h, dim : dim + rot] (heads of dim + rot in q, of rank + rot in folded)."""
+    """folded[t, h, rank : rank + rot] = rotation of q[t, h, dim : dim + rot] (heads of dim + rot in q, of rank + rot in folded). In place
+    with `folded` the very q and rank = dim."""
     _dev(q, positions, folded)
     T = q.shape[0]
     _need(q.dim() == 2 and q.stride(1) == 1 and q.shape[1] >= heads * (dim + rot) and folded.dim() == 2 and folded.stride(1) == 1
