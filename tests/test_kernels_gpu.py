@@ -1383,3 +1383,14 @@ def test_sequences_without_tokens_keep_their_state(ops, mode, monkeypatch):
         if n == 0:
             assert np.array_equal(got[True][1][s, :H * dim * vdim], host(state0)[s, :H * dim * vdim])
     assert rel_err(got[True][0], got[False][0]) < TOL["float32"] and rel_err(got[True][1], got[False][1]) < TOL["float32"]
+
+
+@pytest.mark.parametrize("M,N", [(17, 65535 * 64 + 65), (65535 * 64 + 65, 17)])
+def test_float_products_of_more_tiles_than_a_grid_has_in_one_direction(ops, M, N):
+    """Above 65,535 tiles of columns or of rows; k of 4, so that every output can be looked at."""
+    g = torch.Generator("cuda").manual_seed(M)
+    a, w = torch.randn(M, 4, generator=g, device="cuda"), torch.randn(N, 4, generator=g, device="cuda")
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_simt(a, w, out)
+    want = sum(a[:, i:i + 1] * w[:, i] for i in range(4))
+    assert (out - want).abs().max() <= 8 * 2.0 ** -24 * 4 * want.abs().max()      # four products, each rounded, in another order
