@@ -1394,3 +1394,17 @@ def test_float_products_of_more_tiles_than_a_grid_has_in_one_direction(ops, M, N
     ops.gemm_simt(a, w, out)
     want = sum(a[:, i:i + 1] * w[:, i] for i in range(4))
     assert (out - want).abs().max() <= 8 * 2.0 ** -24 * 4 * want.abs().max()      # four products, each rounded, in another order
+
+
+def test_refused_sizes_take_no_scratch_for_chunks(ops):
+    """Heads that the chunked kernels do not take, in a step that would pay: nothing is allocated for them."""
+    from types import SimpleNamespace
+    from tiny_inference_engine_b200.engine.workspace import Workspace
+    H, dim, T = 2, 32, 400
+    ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=T, max_seqs=1)
+    rows = [torch.randn(T, H * dim, device="cuda") for _ in range(3)]
+    state, out = torch.zeros(1, H * dim * dim + 9 * H * dim, device="cuda"), torch.full((T, H * dim), float("nan"), device="cuda")
+    ops.delta_rule(*rows, torch.rand(T, H, device="cuda"), torch.rand(T, H * dim, device="cuda"), state, H * dim * dim, torch.randn(T, 3 * H * dim, device="cuda"),
+                   0, H * dim, 2 * H * dim, torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), 1, H, H, dim,
+                   dim, 4, out, chunks=ops.RecurrenceChunks(ctx))
+    assert ctx.ws.bytes() == 0 and not torch.isnan(out).all()

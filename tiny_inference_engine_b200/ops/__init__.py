@@ -828,9 +828,9 @@ def delta_rule(qn, kn, vn, beta, decay, state, conv_state_off: int, proj, q_off:
     _need(query_start.numel() >= seqs + 1 and state_slots.numel() >= seqs, "delta_rule: index tensors too short")
     if chunks is not None and not single and chunks_pay(chunks.longest, seqs, seqs * heads * ((vdim + 15) // 16), dim, plain, decay_per_head):
         lib = library.library()
-        scratch = chunks.scratch(lib, T, seqs, heads, dim, plain)
         if lib.tie_delta_chunk_takes(heads, kv_heads, dim, vdim, int(plain), int(decay_per_head), decay.stride(0), state.stride(0), qn.data_ptr(),
-                                     kn.data_ptr(), vn.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), scratch.data_ptr()):
+                                     kn.data_ptr(), vn.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), 0):
+            scratch = chunks.scratch(lib, T, seqs, heads, dim, plain)
             call("tie_delta_rule_chunked", dtype_code(proj), qn.data_ptr(), kn.data_ptr(), vn.data_ptr(), _ptr(beta), decay.data_ptr(),
                  decay.stride(0), state.data_ptr(), state.stride(0), conv_state_off, proj.data_ptr(), proj.stride(0), q_off, k_off, v_off,
                  query_start.data_ptr(), state_slots.data_ptr(), seqs, T, heads, kv_heads, dim, vdim, taps, out.data_ptr(), 1 if plain else 0,
