@@ -1408,3 +1408,25 @@ def test_refused_sizes_take_no_scratch_for_chunks(ops):
                    0, H * dim, 2 * H * dim, torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), 1, H, H, dim,
                    dim, 4, out, chunks=ops.RecurrenceChunks(ctx))
     assert ctx.ws.bytes() == 0 and not torch.isnan(out).all()
+
+
+@pytest.mark.parametrize("per_head", [True, False])
+def test_what_a_recurrence_in_chunks_overwrites(ops, per_head, monkeypatch):
+    """One decay a head: q, k, v and the decays stay to the last bit (a state-space layer reads its values again, constant decays are a model's own tensor
+    read with a stride of zero). A decay a channel: q and k are the kernels' to change, v and the decays stay."""
+    from types import SimpleNamespace
+    from tiny_inference_engine_b200.engine.workspace import Workspace
+    H, dim, T, taps = 2, 64, 200, 4
+    monkeypatch.setattr(ops, "chunks_pay", lambda *a: True)
+    g = torch.Generator("cuda").manual_seed(2)
+    q, k, v = (torch.randn(T, H * dim, generator=g, device="cuda") / 8 for _ in range(3))
+    decay = torch.rand(H, generator=g, device="cuda").expand(T, H) if per_head else torch.rand(T, H * dim, generator=g, device="cuda")
+    before = [x.clone() for x in (q, k, v, decay)]
+    state, out = torch.zeros(1, H * dim * dim + (taps - 1) * 3 * H * dim, device="cuda"), torch.empty(T, H * dim, device="cuda")
+    ctx = SimpleNamespace(ws=Workspace(T, "cuda"), multi_max_queries=T, max_seqs=1)
+    ops.delta_rule(q, k, v, None, decay, state, H * dim * dim, torch.randn(T, 3 * H * dim, generator=g, device="cuda"), 0, H * dim, 2 * H * dim,
+                   torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), 1, H, H, dim, dim, taps, out,
+                   plain=True, decay_per_head=per_head, chunks=ops.RecurrenceChunks(ctx))
+    assert ctx.ws.bytes() > 0
+    same = [torch.equal(x, y) for x, y in zip((q, k, v, decay), before)]
+    assert same == ([True] * 4 if per_head else [False, False, True, True])

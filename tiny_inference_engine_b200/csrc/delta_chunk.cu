@@ -653,7 +653,8 @@ TIE_API long long tie_delta_chunk_scratch(int tokens, int seqs, int heads, int d
   return numbers * heads * (dim > 2 * kChunk ? dim : 2 * kChunk) + (plain ? 0 : 2ll * tokens * heads * dim);
 }
 
-// tie_delta_rule for steps with portions, in chunks. q, k (plain, a decay a channel), decay and v (delta rule) are overwritten.
+// tie_delta_rule for steps with portions, in chunks. Overwritten are v and decay (delta rule), q and k (plain, a decay a channel), nothing with a
+// decay a head: callers rely on it.
 TIE_API int tie_delta_rule_chunked(int dtype, float* qn, float* kn, float* vn, const float* beta, float* decay, long long decay_stride,
                                    float* state, long long state_stride, long long conv_state_off, const void* proj, long long proj_stride,
                                    int q_off, int k_off, int v_off, const int* query_start, const int* state_slots, int seqs, int tokens,

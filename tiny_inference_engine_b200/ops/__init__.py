@@ -815,8 +815,9 @@ def delta_rule(qn, kn, vn, beta, decay, state, conv_state_off: int, proj, q_off:
     `plain`: no correction, u = beta v (beta None: u = v), which is the recurrence of gated linear attention and of
     state-space layers, S <- diag(decay) S + k u^T. `decay_per_head`: decay is float32 [T, >= heads], one factor for
     all key channels of a head. `single`: every sequence brings one token (a hint: how the launch is cut, not what it computes).
-    `chunks` (a `RecurrenceChunks`): the rows qn, kn, vn and decay are the caller's to lose, and a step with a long enough portion may
-    go through it sixteen tokens at a time; they are then overwritten."""
+    `chunks` (a `RecurrenceChunks`): a step with a long enough portion may go through it sixteen tokens at a time. Of its inputs that
+    overwrites, with the delta rule, vn and decay; without it and with a decay a channel, qn and kn; with `decay_per_head` none (callers
+    read their values again, and decays may be a model's own tensor). The caller of the first two has rows to lose."""
     _dev(qn, kn, vn, beta, decay, state, proj, query_start, state_slots, out)
     T = proj.shape[0]
     _need(beta is not None or plain, "delta_rule: the delta rule needs beta")
