@@ -1410,6 +1410,30 @@ def test_refused_sizes_take_no_scratch_for_chunks(ops):
     assert ctx.ws.bytes() == 0 and not torch.isnan(out).all()
 
 
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv,page,window,new,ctx", [
+    (4, 2, 16, 1900, [300], [3000]), (32, 8, 64, 2000, [150, 49], [2900, 2100]), (4, 4, 8, 1950, [100, 2], [2049, 90]), (16, 8, 16, 1500, [600], [4000])])
+def test_windows_of_keys_shared_out_over_a_cluster(ops, Dh, Hq, Hkv, page, window, new, ctx):
+    """Windows long enough for four and two shares: each row tile's first key tile is clipped to a share, and a share may hold tiles of one
+    row tile alone, or none (the last row tile of a portion, a short sequence beside a long one)."""
+    rng = np.random.default_rng(Hq * Dh + sum(ctx))
+    tiles = -(-max(new) * (Hq // Hkv) // 256) * Hkv * len(new)
+    assert tiles * 2 <= 148 and window + max(new) >= 2049            # what the launcher looks at
+    kc, vc, bt, ks, vs = paged_cache(rng, "bfloat16", ctx, Hkv, Dh, page, 330 * 16 // page + 8)
+    T, qs = sum(new), np.concatenate([[0], np.cumsum(new)])
+    q = as_stored(rng.standard_normal((T, Hq * Dh)) * 2, "bfloat16")
+    want = np.concatenate([softmax_reference(q[qs[i]:qs[i + 1]].reshape(-1, Hq, Dh).astype(np.float64), ks[i].astype(np.float64),
+                                             vs[i].astype(np.float64), Dh ** -0.5, window, None, ctx[i] - new[i]) for i in range(len(new))])
+    got = []
+    for max_keys in (0, max(ctx)):
+        out = torch.full((T, Hq * Dh), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.attention_prompt_umma(dev(q, torch.bfloat16), dev(kc, torch.bfloat16), dev(vc, torch.bfloat16), out, dev(qs, torch.int32),
+                                  dev(np.array(ctx), torch.int32), dev(bt, torch.int32), len(new), max(new), Hq, Hkv, Dh, Dh ** -0.5, window, max_keys=max_keys)
+        got.append(host(out))
+        assert rel_err(got[-1], want.reshape(T, -1)) < TOL["bfloat16"]
+    assert not np.array_equal(*got)                                  # (another order of sums: the keys were shared out)
+
+
 @pytest.mark.parametrize("per_head", [True, False])
 def test_what_a_recurrence_in_chunks_overwrites(ops, per_head, monkeypatch):
     """One decay a head: q, k, v and the decays stay to the last bit (a state-space layer reads its values again, constant decays are a model's own tensor
