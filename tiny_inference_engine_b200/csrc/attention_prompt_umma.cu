@@ -22,9 +22,10 @@
 //   8         TMA producer: lane b fetches box b (a page, or 64 keys of a larger page) of every tile.
 //   9         one thread issues the MMAs: Q K^T of tile i + 1 ahead of P V of tile i.
 // Barriers: kv_full/kv_empty per stage, and for each row tile s_full (scores written), s_empty
-// (scores read), p_full[2] (P written, O rescaled), p_empty[2] (P V retired). Every wait is bounded.
+// (scores read), p_full[2] (P written, O rescaled), p_empty[2] (P V retired). Every wait on an mbarrier is bounded.
 // Where the rows are few and the keys many, 2 or 4 CTAs of a thread-block cluster share out the keys of 256 rows and put their sums
-// together through distributed shared memory.
+// together through distributed shared memory. (The cluster's two barriers have no limit; every path of a CTA reaches them, one that
+// gave up a wait too, and the CTAs of a cluster leave ahead of them together or not at all.)
 // grid = (kv heads, row tiles, sequences x splits): CTAs start in that order with the last row tiles first, so the
 // tiles with the most keys of every kv head run first.
 #include "attention_mma.cuh"
@@ -560,8 +561,10 @@ TIE_API int tie_attention_prompt_umma(const void* q, long long q_stride, const v
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
   // ...; with many keys they share out the keys instead: what bounds either is the keys and values that L2 feeds the SMs, and tiles of
-  // 256 rows read them half as often (512 tokens of 32 heads over 8, 16,384 keys: 239 -> 165 us; 6,000: 94 -> 74; 2,048: 38 -> 39;
-  // 1,024: 24 -> 29: the merge costs about 8 us)
+  // 256 rows read them half as often. 128 rows a CTA against shares, us: two shares, 512 tokens of 32 heads over 8, heads of 128: 2,100
+  // keys 45 / 43, 3,000 57 / 51, 8,192 131 / 100, 16,384 246 / 175 (at 1,024 24 / 29: the merge costs about 8 us); heads of 64 37 / 37,
+  // 47 / 45, 111 / 92, 207 / 164. Four shares, 128 tokens: heads of 128 2,100 keys 43 / 37, 3,000 55 / 41, 8,192 126 / 65; 16 heads of 64 over
+  // 4 35 / 31, 45 / 35, 104 / 57; 8 over 8 of 128 41 / 29, 53 / 31, 124 / 49.
   const long long ctas = static_cast<long long>(kv_heads) * ceil_div(max_rows, 256) * n_seqs;
   const int keys = window > 0 && window + max_queries < max_keys ? window + max_queries : max_keys;
   if (ctas * 2 <= sms) {

@@ -8,8 +8,10 @@
 // and sees keys 0..pos (with a window w > 0: keys pos-w+1..pos); query head h reads kv head
 // h / (Hq/Hkv); online softmax of scale * q.k; out = acc / l.
 //
-// Two kernels share the inner loop:
-//   rows kernel   one warp per (row, head) over all of its keys: prompt portions.
+// Two kernels share the inner loop, a third has tiles:
+//   rows kernel   one warp per (row, head) over all of its keys: prompt portions in bfloat16, of a few rows, of two or three tokens each,
+//                 and of every head size and score that the tiles do not take.
+//   tiled rows    float32 prompt portions, heads of 32, 64 and 128: 16 rows share tiles of 32 keys and values.
 //   split kernel  one warp per (sequence, head, split of the keys) for sequences that bring
 //                 one token: each split of `split_keys` keys leaves (max, sum, acc) in
 //                 scratch memory and a merge kernel combines them in split order. The split

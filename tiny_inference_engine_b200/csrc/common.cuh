@@ -1,11 +1,11 @@
 // Shared device helpers: element types, 16-byte vectors, warp and block reductions.
 #pragma once
 
-#include <atomic>
-
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
 
 namespace tie {
 
@@ -129,8 +129,9 @@ inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b -
 // until the kernels before it in the stream have completed and their writes are visible,
 // then lets the kernel after it be scheduled. So the next kernel's blocks are already resident
 // (launch latency, block scheduling and whatever they do before their own pdl_sync() are hidden
-// behind this kernel) and start the moment this one is done. Nothing may touch global memory
-// before pdl_sync().
+// behind this kernel) and start the moment this one is done. Nothing may read or write global
+// memory before pdl_sync(); asking for lines to be brought into L2 is no read (gemm_small_m_kernel
+// asks for its weight's).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() {
