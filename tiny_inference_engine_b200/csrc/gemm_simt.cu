@@ -94,8 +94,7 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 8 ? 2 : 1) gemm_f32_k
   extern __shared__ __align__(16) float ring[];
   const int product = blockIdx.z / splits, rank = blockIdx.z % splits;
   a += product * sa, w += product * sw, out += product * so;
-  // row and column tiles numbered together, so that neither has a grid's limit of 65,535; those of one stretch of the weight run side by side
-  const int m_tiles = (M + BM - 1) / BM, m0 = static_cast<int>(blockIdx.x % m_tiles) * BM, n0 = static_cast<int>(blockIdx.x / m_tiles) * BN;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;      // (the row tiles of one stretch of the weight run side by side)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int slices = (K + kSliceK - 1) / kSliceK, per = (slices + splits - 1) / splits;
   const int first = min(rank * per, slices), count = min(per, slices - first);
@@ -202,7 +201,7 @@ int launch_f32_tile(const float* a, const float* w, float* out, int M, int N, in
     return kCudaError;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(M, BM)) * ceil_div(N, BN), 1, batch * splits);
+  cfg.gridDim = dim3(ceil_div(M, BM), 0, batch * splits);
   cfg.blockDim = dim3(32 * WM * WN);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -220,7 +219,13 @@ int launch_f32_tile(const float* a, const float* w, float* out, int M, int N, in
     attrs[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
-  cudaLaunchKernelEx(&cfg, kernel, a, w, out, M, N, K, lda, ldw, ldo, sa, sw, so, splits);
+  // A grid has 65,535 tiles of columns: a launch for as many columns each. (Tiles numbered in one direction cost the kernel two per cent.)
+  constexpr int most = 65535 * BN;
+  for (int n0 = 0; n0 < N; n0 = N - n0 > most ? n0 + most : N) {
+    const int n = N - n0 < most ? N - n0 : most;
+    cfg.gridDim.y = ceil_div(n, BN);
+    cudaLaunchKernelEx(&cfg, kernel, a, w + n0 * ldw, out + n0, M, n, K, lda, ldw, ldo, sa, sw, so, splits);
+  }
   TIE_RETURN_LAUNCH("gemm_f32");
 }
 
