@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(128) attention_rows_tiled_kernel(AttnArgs a) {
         float sum = 0.0f;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const float p = seen[j] ? expf(sc[j] - m_new) : 0.0f;
-          ps[(r0 + i) * (kTileKeys + 4) + c + 16 * j] = seen[j] ? p : -1.0f;
+          const float p = seen[j] ? expf(sc[j] - m_new) : -0.0f;
+          ps[(r0 + i) * (kTileKeys + 4) + c + 16 * j] = p;
           sum += p;
         }
 #pragma unroll
@@ -318,11 +318,11 @@ __global__ void __launch_bounds__(128) attention_rows_tiled_kernel(AttnArgs a) {
         for (int e = 0; e < OWN; ++e) acc[i][e] *= corr;
       }
       __syncwarp();                                        // a row's weights are written and read by one half warp
-      // A value that the row does not see (its place holds -1) must not be touched: 0 times a NaN of another request is a NaN. One
+      // A value that the row does not see (its weight is -0, which no exponential is) must not be touched: 0 times a NaN of another request is a NaN. One
       // that it sees counts however small its weight. Where all rows see all keys of the tile nothing has to be looked at.
       const bool whole = begin == t0 && end == t_end && key0 + kTileKeys - 1 <= begin + shift && (a.window <= 0 || key0 >= hi - a.window + 1);
       auto add = [&](float (&o)[OWN], float p, const float (&v)[OWN]) {
-        if (!whole && p < 0.0f) return;
+        if (!whole && __float_as_uint(p) == 0x80000000u) return;
 #pragma unroll
         for (int x = 0; x < OWN; ++x) o[x] = fmaf(p, v[x], o[x]);
       };
