@@ -366,8 +366,7 @@ static int launch_prompt_exact(const CUtensorMap& km, const CUtensorMap& vm, con
   constexpr size_t smem = 2 * KH * 128 * 128 + static_cast<size_t>(STAGES) * (KH + VH) * 64 * 128 + (2 * STAGES + 12) * 8 + 16 + 1024;
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
   auto kernel = attn_prompt_exact_kernel<KH, VH, PAGED, STAGES>;
-  static std::atomic<unsigned long long> reserved;
-  if (!reserve_shared(reserved, reinterpret_cast<const void*>(kernel), static_cast<int>(smem))) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
     set_error("attention_prompt_exact: cannot reserve %zu bytes of shared memory", smem);
     return kCudaError;
   }

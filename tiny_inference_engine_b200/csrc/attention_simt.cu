@@ -379,8 +379,7 @@ inline bool rows_tiled_takes(const AttnArgs& a) {
 template <int DH>
 int launch_rows_tiled(const AttnArgs& a, cudaStream_t s) {
   constexpr int smem = ((kTileRows + 4 * kTileKeys) * (DH + 4) + kTileRows * (kTileKeys + 4)) * static_cast<int>(sizeof(float));
-  static std::atomic<unsigned long long> reserved;
-  if (!reserve_shared(reserved, reinterpret_cast<const void*>(attention_rows_tiled_kernel<DH>), smem)) {
+  if (cudaFuncSetAttribute(attention_rows_tiled_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     set_error("attention: cannot reserve %d bytes of shared memory", smem);
     return kCudaError;
   }

@@ -5,8 +5,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
-
 namespace tie {
 
 // Error codes that launchers return to Python (0 = launched).
@@ -168,17 +166,6 @@ inline void launch_kernel_alone(void (*kernel)(KArgs...), dim3 grid, dim3 block,
   cfg.stream = stream;
   cfg.numAttrs = 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
-// Asks for more shared memory than the 48 KB that a kernel's blocks have unasked, once a device: `done` has a bit a device, one
-// variable a kernel. (The call costs the host as much as a fifth of a launch.)
-inline bool reserve_shared(std::atomic<unsigned long long>& done, const void* kernel, int bytes) {
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device > 63) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-  if (done.load(std::memory_order_relaxed) >> device & 1) return true;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
-  done.fetch_or(1ull << device, std::memory_order_relaxed);
-  return true;
 }
 
 }  // namespace tie

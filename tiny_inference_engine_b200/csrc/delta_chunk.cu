@@ -598,21 +598,19 @@ int launch_chunk_prep(const float* q, const float* k, float* v, const float* bet
   const size_t rows = kChunk * DIM * sizeof(float), pairs = kChunk * kChunk * sizeof(float), values = kChunk * sh.vdim * sizeof(float);
   const size_t smem = decay_per_head ? rows + pairs + kChunk * sizeof(float) + values : plain ? 3 * rows + pairs + values : 4 * rows + 3 * pairs + 2 * values;
   const long long own = static_cast<long long>(sh.heads) * DIM;
-  static std::atomic<unsigned long long> reserved[3];
-  const auto ready = [&](int which, auto kernel) {      // as much as values of 256 need
-    constexpr int most = (4 * kChunk * DIM + 3 * kChunk * kChunk + 2 * kChunk * 256) * static_cast<int>(sizeof(float));
-    return smem <= 48 * 1024 || reserve_shared(reserved[which], reinterpret_cast<const void*>(kernel), most);
+  auto ready = [&](auto kernel) {
+    return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess;
   };
   bool ok = true;
   if (decay_per_head) {
-    if ((ok = ready(0, chunk_prep_scalar_kernel<CH>)))
+    if ((ok = ready(chunk_prep_scalar_kernel<CH>)))
       TIE_LAUNCH((chunk_prep_scalar_kernel<CH>), grid, 256, smem, s, q, k, v, beta, decay, decay_stride, query_start, seqs, sh, gc_out, out);
   } else if (plain) {
-    if ((ok = ready(1, chunk_prep_channel_kernel<CH, false>)))
+    if ((ok = ready(chunk_prep_channel_kernel<CH, false>)))
       TIE_LAUNCH((chunk_prep_channel_kernel<CH, false>), grid, 256, smem, s, q, k, v, beta, decay, decay_stride, query_start, seqs, sh,
                  const_cast<float*>(q), const_cast<float*>(k), own, nullptr, gc_out, out);
   } else {
-    if ((ok = ready(2, chunk_prep_channel_kernel<CH, true>)))
+    if ((ok = ready(chunk_prep_channel_kernel<CH, true>)))
       TIE_LAUNCH((chunk_prep_channel_kernel<CH, true>), grid, 256, smem, s, q, k, v, beta, decay, decay_stride, query_start, seqs, sh, q_out,
                  decay, decay_stride, w_out, gc_out, out);
   }
@@ -629,8 +627,7 @@ int launch_chunk_walk(const ChunkWalk& a, const void* proj, long long proj_strid
   constexpr int DIM = 32 * CH, stage = (DELTA ? 3 : 2) * kChunk * DIM + 2 * kChunk * (kChunkCols + 4) + (SCALAR ? 2 * kChunk : DIM) + kChunk;
   constexpr int smem = (2 * stage + 4 * 128) * static_cast<int>(sizeof(float));
   auto kernel = chunk_walk_kernel<T, CH, DELTA, SCALAR>;
-  static std::atomic<unsigned long long> reserved;
-  if (!reserve_shared(reserved, reinterpret_cast<const void*>(kernel), smem)) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     set_error("delta_chunk: cannot reserve %d bytes of shared memory", smem);
     return kCudaError;
   }

@@ -195,8 +195,7 @@ int launch_f32_tile(const float* a, const float* w, float* out, int M, int N, in
   const bool wide = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && sa % 4 == 0 && sw % 4 == 0 &&
                     reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
   auto kernel = wide ? gemm_f32_kernel<WM, WN, true> : gemm_f32_kernel<WM, WN, false>;
-  static std::atomic<unsigned long long> reserved[2];
-  if (!reserve_shared(reserved[wide], reinterpret_cast<const void*>(kernel), smem)) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     set_error("gemm_simt: cannot reserve %d bytes of shared memory", smem);
     return kCudaError;
   }
