@@ -6,19 +6,24 @@ from tiny_inference_engine_b200.engine.workspace import Workspace
 from tiny_inference_engine_b200.parts import latent_attention
 
 
-def test_spare_buffers_are_outgrown_without_a_trace_and_refused_when_memory_is_short():
+def test_spare_buffers_are_outgrown_without_a_trace_and_refused_when_memory_is_short(monkeypatch):
+    monkeypatch.setattr(Workspace, "_free_bytes", lambda self: 8000)
     ws = Workspace(8, "cpu")
-    free = [1 << 20]
-    ws._free_bytes = lambda: free[0]
     a = ws.spare("x", 100, torch.bfloat16, 128)
     assert a.numel() == 128 and ws.spare("x", 128, torch.bfloat16, 500) is a
     b = ws.spare("x", 129, torch.bfloat16, 1000)
     assert b.numel() == 1000 and ws.bytes() == 2000                # the outgrown one is gone
-    free[0] = 8000
-    assert ws.spare("x", 1001, torch.bfloat16, 2001) is None       # 4,002 bytes: more than half of what is left
+    assert ws.spare("x", 1001, torch.bfloat16, 2001) is None       # 4,002 bytes: more than half of what was left
     assert ws.spare("x", 1000, torch.bfloat16) is b                # what is there stays
-    free[0] = 1 << 20
-    assert ws.spare("x", 1001, torch.bfloat16) is None             # asked once, not at every step
+    full = torch.empty
+
+    def short(*a, **k):
+        raise torch.cuda.OutOfMemoryError("no more")
+    monkeypatch.setattr(torch, "empty", short)
+    assert ws.spare("x", 1500, torch.bfloat16) is None and ws.bytes() == 0
+    monkeypatch.setattr(torch, "empty", full)
+    assert ws.spare("x", 1500, torch.bfloat16) is None             # not tried again at every step
+    assert ws.spare("x", 1000, torch.bfloat16).numel() == 1000
     kept = ws.flat("y", 10, torch.float32)
     ws.flat("y", 11, torch.float32)
     assert ws.bytes() == 2000 + 40 + 80 and kept.numel() == 10     # a captured graph may still use it

@@ -20,7 +20,7 @@ class Workspace:
         self._rows: dict[tuple, torch.Tensor] = {}
         self._flat: dict[tuple, torch.Tensor] = {}
         self._retired: list[torch.Tensor] = []      # outgrown buffers: captured graphs may still use them
-        self._refused: dict[tuple, int] = {}        # spare buffers that there was no room for, and their smallest size
+        self._spare_bytes = self._free_bytes() // 2 # what a spare buffer may take (asking the device costs 0.1 ms: asked once)
 
     def rows(self, name: str, n: int, width: int, dtype: torch.dtype) -> torch.Tensor:
         """[n, width] view of a buffer that holds max_rows rows."""
@@ -48,25 +48,27 @@ class Workspace:
 
     def spare(self, name: str, numel: int, dtype: torch.dtype, capacity: int = 0) -> torch.Tensor | None:
         """At least `numel` elements for a step that is not captured and that has another way if there are none: None where the
-        buffer would take more than half of what the device has left (the buffers that other steps will ask for are not
-        there yet). An outgrown buffer goes back to the allocator; the stream's order keeps it whole until the steps that use it are done."""
+        buffer would take more than half of what the device had left when this workspace was made (behind weights and cache; the
+        buffers of other steps were still to come), or where it has no more. An outgrown buffer goes back to the allocator; the
+        stream's order keeps it whole until the steps that use it are done."""
         key = (name, dtype, "spare")
         buf = self._flat.get(key)
         if buf is not None and buf.numel() >= numel:
             return buf
-        if numel >= self._refused.get(key, numel + 1):
-            return None
         size = max(numel, capacity)
-        if size * dtype.itemsize > self._free_bytes() // 2:
-            self._refused[key] = numel
+        if size * dtype.itemsize > self._spare_bytes:
             return None
         self._flat.pop(key, None)
         del buf
-        self._flat[key] = buf = torch.empty(size, dtype=dtype, device=self.device)
+        try:
+            self._flat[key] = buf = torch.empty(size, dtype=dtype, device=self.device)
+        except torch.cuda.OutOfMemoryError:
+            self._spare_bytes = size * dtype.itemsize - 1
+            return None
         return buf
 
     def _free_bytes(self) -> int:
-        return torch.cuda.mem_get_info(self.device)[0]
+        return torch.cuda.mem_get_info(self.device)[0] if torch.device(self.device).type == "cuda" else 1 << 62
 
     def zeros(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that is zero when first handed out (kernels that use it leave it zero)."""
