@@ -311,6 +311,23 @@ def test_a_key_just_inside_and_just_outside_the_window(tmp_path, dtype, sizes):
         close(hs.in_portions("c", toks, [at, 1] + [1] * 60), ref, dtype, f"token by token over the edge, page {page}")
 
 
+def test_windows_of_the_size_that_is_multiplied_out(tmp_path):
+    """Latent layers of heads of 128 + 64 with values of 128 in windows, in portions whose pages are given back behind them, while another
+    request holds page 0, which the tables name in their place, with NaN in it: no row of the document may notice."""
+    cfg = plain.make_config([L(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=64, q_rank=48, window=100, mlp=plain.dense(64)),
+                             L(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=128, q_rank=40, window=70, mlp=None)], vocab=60)
+    w = plain.random_weights(cfg, 3)
+    toks = tokens_of(cfg, 460, 1)
+    want = reference(w, cfg, toks)
+    for page in (8, 16):
+        hs = Harness(tmp_path / f"p{page}", cfg, w, "bfloat16", page=page, pages=512 // page, max_tokens=132)
+        hs.step([("x", tokens_of(cfg, 5, 2), [])])
+        assert all(t.ids[0] == 0 for t in hs.live["x"][0].tables)
+        for i in range(2):
+            hs.cache.layer_cache(i, False).k[0] = float("nan")
+        close(hs.in_portions("a", toks, [90, 70, 131, 64, 2, 100]), want, "bfloat16", f"in portions, page {page}")
+
+
 def _far_memory(kind):
     """One recurrent layer with decays close to one in which one key channel answers to one token alone: what that
     token wrote at place 3 stays in the state, and every later query reads it."""
