@@ -57,10 +57,10 @@ def test_recurrences_go_in_chunks_where_that_was_measured_to_be_faster():
     assert not pays("delta", [64], 16, 128, 128) and not pays("delta", [96], 8, 128, 256) and not pays("delta", [128] + [1] * 30, 16, 128, 128)
     assert pays("delta", [128], 16, 64, 64) and pays("delta", [2048], 16, 128, 128) and pays("delta", [160] * 8, 16, 128, 128)
     assert not pays("channel", [96], 16, 128, 128) and not pays("channel", [128], 16, 64, 64) and not pays("channel", [128] * 2, 16, 64, 64)
-    assert pays("channel", [256], 16, 128, 128) and pays("channel", [128], 32, 128, 128) and pays("channel", [256], 16, 64, 64) and pays("channel", [160] * 8, 16, 64, 64)
-    for lens, heads, dim, vdim in (([256], 16, 128, 128), ([2048], 16, 128, 128), ([4096], 32, 128, 64), ([2048], 32, 64, 64), ([128] * 2, 64, 64, 64),
-                                   ([128], 32, 128, 128), ([200] * 4, 16, 64, 64)):
+    assert pays("channel", [128], 16, 128, 128) and pays("channel", [256], 16, 64, 64) and pays("channel", [160] * 8, 16, 64, 64)
+    for lens, heads, dim, vdim in (([256], 16, 128, 128), ([2048], 16, 128, 128), ([4096], 32, 128, 64), ([2048], 32, 64, 64), ([96], 32, 128, 128),
+                                   ([200] * 4, 16, 64, 64)):
         assert not pays("head", lens, heads, dim, vdim), (lens, heads, dim, vdim)
     for lens, heads, dim, vdim in (([2048], 32, 128, 128), ([1021, 510], 16, 128, 128), ([128] * 3, 16, 128, 128), ([1024] + [1] * 8, 16, 64, 64),
-                                   ([1021] * 2, 64, 64, 64), ([256], 64, 128, 128)):
+                                   ([1021] * 2, 64, 64, 64), ([256], 64, 128, 128), ([128] * 2, 64, 64, 64), ([128], 32, 128, 128)):
         assert pays("head", lens, heads, dim, vdim), (lens, heads, dim, vdim)

@@ -779,19 +779,20 @@ def chunks_pay(longest: int, seqs: int, blocks: int, dim: int, plain: bool, deca
     """Whether a step's recurrence is faster in chunks; `blocks`: sequences x heads x column tiles of 16, `dim` key channels a head. Token by
     token, a portion of n tokens is a chain of n steps (0.25 us each with the delta rule, 0.16 us with a decay a channel, 0.11 us with
     one a head, heads of 128); in chunks it is n / 16 steps of 1.6 to 2 us behind a launch of its own. Sequences that bring one token cost
-    the chunked kernel about a microsecond each more. Token by token against chunks, us, 16 heads of 128 / 128 where nothing else is said:
-      delta rule          96 tokens 33.8 / 33.8, 128 43.0 / 35.8, 1,024 264 / 167; heads of 64: 128 34.8 / 31.7, 1,024 205 / 116;
-      a decay a channel   96 tokens 24.6 / 27.6, 128 30.7 / 29.5, 256 49.2 / 43.0; heads of 64: 128 22.5 / 23.6, 256 35.2 / 33.7;
-      a decay a head      the shortest chain, so only what it costs several blocks an SM pays: 128 blocks 256 tokens 38.9 / 44.0, 2,048
-                          240 / 247; 256 blocks 2 x 256 62 / 54, 1,021 + 510 213 / 161, 32 heads 2,048 414 / 327; 3 x 128 49 / 42; heads of 64
-                          64 heads 2,048 291 / 296, 2 x 1,021 277 / 220; 2 x 128 tokens 43 / 46."""
+    the chunked kernel about a microsecond each more. Token by token against chunks, us, inputs in L2 (from memory chunks cost up to a tenth
+    more), 16 heads of 128 / 128 where nothing else is said:
+      delta rule          96 tokens 29.3 / 32.0 (from memory 33.8 / 33.8), 1,024 from memory 264 / 167; heads of 64: 96 23.2 / 21.4;
+      a decay a channel   96 tokens 21.1 / 19.6 (from memory 24.6 / 27.6), 128 25.2 / 23.4; heads of 64: 96 14.9 / 18.5, 128 19.0 / 18.4;
+      a decay a head      the shortest chain, so only what it costs several blocks an SM pays: 128 blocks 256 tokens 35.5 / 37.7, 512
+                          63.3 / 64.5, 2,048 234 / 228, 32 heads of 128 / 64 236 / 278; 256 blocks 2 x 128 32.1 / 28.8, 32 heads 128 32.2 / 28.5;
+                          heads of 64: 32 heads 3 x 128 31.3 / 31.6, 64 heads 256 41.5 / 40.0."""
     if longest < 88 + 8 * seqs:
         return False
     if not plain:
         return longest >= 112
     if not decay_per_head:
-        return longest >= 160 or blocks * dim * longest >= 4 << 20
-    return blocks * dim >= 1 << 15 and blocks * dim * longest >= 6 << 20
+        return longest >= 160 or blocks * dim * longest >= 2 << 20
+    return blocks * dim >= 1 << 15 and blocks * dim * longest >= 4 << 20
 
 
 class RecurrenceChunks:
