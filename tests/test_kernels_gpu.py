@@ -554,6 +554,56 @@ def test_pair_kernel_at_every_tile_width(ops, bn):
     assert rel_err(host(out), plain.swiglu(plain.linear(a, gate), plain.linear(a, up))) < TOL["bfloat16"]
 
 
+@pytest.mark.parametrize("M,N,K,transposed,bn,splits", [(65, 264, 72, 1, 64, 1), (129, 1001, 1096, 1, 160, 3), (256, 4992, 520, 1, 256, 1),
+                                                        (200, 515, 1992, 0, 96, 4), (600, 260, 4096, 0, 64, 5), (1, 300, 136, 1, 32, 2)])
+def test_pair_kernel_on_either_side_and_with_split_k(ops, M, N, K, transposed, bn, splits):
+    """Pairs of SMs with the tokens or the weights on the 256-row side, k whole or split (the sums left for a consumer, or added),
+    sizes that end inside a tile, rows that TMA can store and rows that it cannot (odd widths and offsets)."""
+    from tiny_inference_engine_b200.ops import gemm_select
+    rng = np.random.default_rng(M + N + K)
+    a, w = as_stored(rng.standard_normal((M, K)), "bfloat16"), as_stored(rng.standard_normal((N, K)), "bfloat16")
+    want = plain.linear(a, w)
+    ta, tw = dev(a, torch.bfloat16), dev(w, torch.bfloat16)
+    for dtype, offset in ((torch.float32, 8), (torch.bfloat16, 8), (torch.bfloat16, 3)):
+        wide = torch.full((M, N + 16), 7.0, device="cuda", dtype=dtype)
+        scratch = torch.full((splits * M * N + 16,), float("nan"), device="cuda")
+        gemm_select._call("tie_gemm_tc2", int(dtype == torch.bfloat16), ta.data_ptr(), tw.data_ptr(), wide[:, offset:].data_ptr(), M, N, K, K, K,
+                          N + 16, 0, 0, 0, bn, transposed, splits, scratch.data_ptr(), 1, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        gemm_select.check_status()
+        assert rel_err(host(wide[:, offset:offset + N]), want) < (TOL["bfloat16"] if dtype == torch.bfloat16 else 2e-5), (dtype, offset)
+        assert (wide[:, :offset] == 7).all() and (wide[:, offset + N:] == 7).all()
+        real = gemm_select._library().tie_gemm_tc_real_splits(K, splits) if splits > 1 else 0
+        assert torch.isnan(scratch[real * M * N:]).all()
+        if real:
+            assert rel_err(scratch[:real * M * N].view(real, M, N).sum(0).cpu().numpy(), want) < 2e-5
+
+
+@pytest.mark.parametrize("transposed", [0, 1])
+def test_silu_epilogue_from_the_smallest_to_the_largest_gates(ops, transposed):
+    """act(gate) * up against 64 bits where the exponential is 1, rounds away, and overflows; in float output, within four
+    roundings of 32 bits (exp, sum, quotient, product) and the exponential's own two units."""
+    from tiny_inference_engine_b200.ops import gemm_select
+    gates = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 0.3, -0.3, 5.0, -5.0, 17.0, -17.0, 40.0, -40.0, -43.0, -60.0, 88.0, -88.0, -88.5, -89.0,
+                          -200.0, 1e38, -1e38]).to(torch.bfloat16)      # times 3 at most: below 3.4e38
+    M, I, K = 100, 32, 16
+    a = torch.zeros(M, K, dtype=torch.bfloat16)
+    a[:, 0], a[:, 1] = gates.repeat(5)[:M], 1.5
+    gate, up = torch.zeros(I, K, dtype=torch.bfloat16), torch.zeros(I, K, dtype=torch.bfloat16)
+    gate[:, 0], up[:, 1] = 1.0, torch.linspace(-2, 2, I).to(torch.bfloat16)
+    out = torch.full((M, I), float("nan"), device="cuda")
+    w = ops.interleave_gate_up(gate.cuda(), up.cuda())
+    gemm_select._call("tie_gemm_tc2", 0, a.cuda().data_ptr(), w.data_ptr(), out.data_ptr(), M, 2 * I, K, K, K, I, 1, 0, 0, 128 if transposed else 64,
+                      transposed, 1, 0, 1, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    gemm_select.check_status()
+    g = a[:, 0].double()
+    want = (g / (1.0 + torch.exp(-g)))[:, None] * (1.5 * up[:, 1].double())[None]
+    got = out.double().cpu()
+    near = want.abs() > 1e-36                      # below, 32 bits have no full mantissa
+    assert ((got - want).abs()[near] <= 6 * 2.0 ** -24 * want.abs()[near] * 2).all() and (got - want).abs()[~near].max() < 2e-36
+
+
 @pytest.mark.parametrize("M", [5, 300, 640])
 def test_silu_product_and_split_sums_with_the_weight_in_k_blocks(ops, M):
     from tiny_inference_engine_b200.ops import gemm_select

@@ -118,8 +118,24 @@ __device__ __forceinline__ float squared_relu(float v) {
   return r * r;
 }
 
+// g / (1 + exp(-g)). An epilogue evaluates sixteen and more of these side by side, and the branches of `/` keep them from
+// overlapping (the gate/up product of 2,048 tokens waited for its epilogue), so the quotient is formed without any: the
+// hardware's approximate reciprocal, one Newton-Raphson step on it, and one on the quotient by its residual. Denominators
+// above 2^60 are scaled down first, so that no reciprocal is subnormal; where exp(-g) overflows, g * 0 is what g / inf is.
+__device__ __forceinline__ float silu(float g) {
+  const float e = expf(-g);
+  const float scale = e > 1.152921504606847e18f ? 5.421010862427522e-20f : 1.0f;      // 2^60, 2^-64
+  const float d = (1.0f + fminf(e, 3.402823466e38f)) * scale, n = g * scale;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(r, fmaf(-d, r, 1.0f), r);
+  float q = n * r;
+  q = fmaf(r, fmaf(-d, q, n), q);
+  return e > 3.402823466e38f ? g * 0.0f : q;
+}
+
 // The activation of a gated product's epilogue: 1 the SiLU, 2 the ReLU.
-__device__ __forceinline__ float gate_act(float g, int act) { return act == 2 ? fmaxf(g, 0.0f) : g / (1.0f + expf(-g)); }
+__device__ __forceinline__ float gate_act(float g, int act) { return act == 2 ? fmaxf(g, 0.0f) : silu(g); }
 
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 

@@ -52,6 +52,20 @@ bool make_map_bf16(CUtensorMap* map, const void* base, long long rows, long long
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_map_rows(CUtensorMap* map, const void* base, bool is_float, long long rows, long long cols, long long ld, int planes,
+                   int box_cols, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  const int size = is_float ? 4 : 2;
+  if (fn == nullptr || reinterpret_cast<uintptr_t>(base) % 16 != 0 || (ld * size) % 16 != 0) return false;
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(planes)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * size, static_cast<cuuint64_t>(ld) * size * rows};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1};
+  const cuuint32_t elem[3] = {1, 1, 1};
+  return fn(map, is_float ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
+            elem, CU_TENSOR_MAP_INTERLEAVE_NONE, is_float ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static int* g_status_host = nullptr;
 static int* g_status_dev = nullptr;
 

@@ -404,6 +404,17 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& my, void* out, fl
   return kOk;
 }
 
+void launch_splitk_reduce(int out_dtype, const float* partial, long long part_stride, int splits, void* out, long long ldo, int N,
+                          long long total, int epilogue, cudaStream_t s) {
+  if (out_dtype == TIE_BF16) {
+    TIE_LAUNCH((splitk_reduce_kernel<__nv_bfloat16>), ceil_div(total, 256), 256, 0, s, partial, part_stride, splits,
+               static_cast<__nv_bfloat16*>(out), ldo, N, total, epilogue);
+  } else {
+    TIE_LAUNCH((splitk_reduce_kernel<float>), ceil_div(total, 256), 256, 0, s, partial, part_stride, splits, static_cast<float*>(out), ldo, N,
+               total, epilogue);
+  }
+}
+
 }  // namespace tie
 
 using namespace tie;
@@ -479,18 +490,7 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
 #undef TIE_TC_ARGS
 #undef TIE_TC_CASE
   if (st != kOk) return st;
-  if (splits > 1 && reduce) {
-    const int k_blocks = ceil_div(K, kBK);
-    const int real_splits = ceil_div(k_blocks, ceil_div(k_blocks, splits));
-    const long long total = part_stride;
-    if (out_dtype == TIE_BF16) {
-      TIE_LAUNCH((splitk_reduce_kernel<__nv_bfloat16>), ceil_div(total, 256), 256, 0, s, 
-          partial, part_stride, real_splits, static_cast<__nv_bfloat16*>(out), ldo, N, total, silu);
-    } else {
-      TIE_LAUNCH((splitk_reduce_kernel<float>), ceil_div(total, 256), 256, 0, s, partial, part_stride, real_splits,
-                                                                      static_cast<float*>(out), ldo, N, total, silu);
-    }
-  }
+  if (splits > 1 && reduce) launch_splitk_reduce(out_dtype, partial, part_stride, tie_gemm_tc_real_splits(K, splits), out, ldo, N, part_stride, silu, s);
   TIE_RETURN_LAUNCH("gemm_tc");
 }
 

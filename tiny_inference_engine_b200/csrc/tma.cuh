@@ -88,6 +88,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 bool make_map_bf16(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_cols,
                    int box_rows);
 
+// [planes, rows, cols] bfloat16 or float, row stride ld elements, for TMA stores of box_cols x box_rows: box rows of 64 bytes with
+// the 64-byte swizzle (bfloat16, 32 columns) or of 128 bytes with the 128-byte one (float, 32 columns). False if rows or base
+// are not 16-byte aligned.
+bool make_map_rows(CUtensorMap* map, const void* base, bool is_float, long long rows, long long cols, long long ld, int planes,
+                   int box_cols, int box_rows);
+
 // Device pointer of the status word (pinned, mapped host memory): kernels write a code there when a
 // bounded wait runs out; the host reads and clears it with tie_kernel_status(). Null if it could
 // not be allocated.

@@ -110,24 +110,24 @@ def partial_capacity(max_rows: int, N: int, K: int, split_many: bool = True) -> 
     return most
 
 
-PAIR_MIN_ROWS = 512     # from this many tokens on, 256 x 256 tiles on pairs of SMs (cta_group::2)
-
+# Pairs of SMs (cta_group::2): from 65 tokens on; up to 64 the weights stream through two CTAs an SM (`plan`).
+PAIR_FROM, PAIR_MIN_COLUMNS = 64, 256
 
 _NO_PAIR = os.environ.get("TIE_NO_PAIR_GEMM") == "1"
 _ops = None
 
-
-def pair_takes(M: int, N: int) -> bool:
-    """Pairs of SMs once the 128 x 128 tiles of the product are more than one wave of CTAs."""
-    return M >= PAIR_MIN_ROWS and N >= 256 and not _NO_PAIR and math.ceil(M / 128) * math.ceil(N / 128) > NUM_SMS
-
-
-PAIR_WIDTHS = (256, 224, 192, 160, 128)
-# Microseconds of a 256 x width tile per 64-deep k-block, measured at Qwen3-8B's widths: the MMAs of the full width,
-# and what staging the operands from L2 costs at any width (the 256 rows of `a` are fetched whatever the width:
-# narrow tiles are bound by that, which is why they only pay where they save a whole wave); and per tile the
-# prologue and epilogue that nothing hides.
-_PAIR_US_MMA, _PAIR_US_FEED, _PAIR_US_TILE = 0.45, 0.33, 3.0
+PAIR_WIDTHS = (256, 224, 192, 160, 128, 96, 64)
+# Microseconds on one B200, fitted to a sweep of 15 products of Qwen3's and the other designs' widths at 72 to 2,048 tokens, every
+# tile width and up to eight splits (2,300 launches, 6 % error; the estimate's choice costs 0.5 % more than the best of each on
+# average): a 64-deep k-block of a tile of 256 rows by `width` columns (2 cycles a column on the tensor cores from 192 columns on;
+# narrower tiles wait for their operands, 66 bytes a cycle and SM from L2), a tile's own cost, the last tile's epilogue, a million
+# float partial sums on their way out. _REDUCE_*: adding them up again, in the kernel that consumes them or in one of its own.
+_PAIR_US_K_BLOCK = {64: 0.190, 96: 0.199, 128: 0.205, 160: 0.213, 192: 0.253, 224: 0.278, 256: 0.321}
+_PAIR_US_LAUNCH, _PAIR_US_TILE, _PAIR_US_TAIL, _PAIR_US_MEGA_PARTIAL = 3.55, 0.92, 1.12, 0.367
+_REDUCE_US_MEGA_CONSUMER, _REDUCE_US_MEGA, _REDUCE_US_LAUNCH = 0.35, 0.6, 2.2
+# The same for one CTA a tile of 128 rows (`plan`), from the same sweep.
+_SINGLE_US_K_BLOCK, _SINGLE_US_WAVE = {128: 0.237, 256: 0.414}, {128: 1.3, 256: 3.9}
+_SINGLE_US_LAUNCH, _SINGLE_US_MEGA_PARTIAL = 3.5, 0.48
 _pairs = None
 
 
@@ -142,18 +142,64 @@ def resident_pairs() -> int:
     return _pairs
 
 
+def _reduce_cost(M: int, N: int, splits: int, consumer: bool) -> float:
+    mega = splits * M * N / 1e6
+    return 0.0 if splits == 1 else mega * _REDUCE_US_MEGA_CONSUMER if consumer else _REDUCE_US_LAUNCH + mega * _REDUCE_US_MEGA
+
+
+def _pair_cost(M: int, N: int, K: int, pairs: int, transposed: int, bn: int, splits: int) -> float:
+    """Estimated time of the pair kernel: its work items (tiles x splits) go round the pairs in waves."""
+    rows, cols = (N, M) if transposed else (M, N)
+    waves = math.ceil(math.ceil(rows / 256) * math.ceil(cols / bn) * splits / pairs)
+    per = math.ceil(math.ceil(K / 64) / splits)
+    out = _PAIR_US_TAIL * bn / 256 + (_PAIR_US_TAIL * bn / 256 + _PAIR_US_MEGA_PARTIAL * splits * M * N / 1e6 if splits > 1 else 0.0)
+    # of two that come out alike the wider one: fewer bytes from L2, which counts once the power limit sets the clock
+    return (_PAIR_US_LAUNCH + waves * (per * _PAIR_US_K_BLOCK[bn] + _PAIR_US_TILE) + out) * (1.0 + 1e-4 * (256 - bn))
+
+
+def _single_cost(M: int, N: int, K: int, bn: int, splits: int) -> float:
+    per = math.ceil(math.ceil(K / 64) / splits)
+    real = math.ceil(math.ceil(K / 64) / per)
+    tiles = math.ceil(M / 128) * math.ceil(N / bn)
+    ctas = tiles if tiles * real <= NUM_SMS else max(1, NUM_SMS // real)
+    waves = math.ceil(tiles / min(ctas, tiles))
+    return _SINGLE_US_LAUNCH + waves * (per * _SINGLE_US_K_BLOCK[bn] + _SINGLE_US_WAVE[bn]) + (_SINGLE_US_MEGA_PARTIAL * real * M * N / 1e6 if real > 1 else 0.0)
+
+
 @functools.lru_cache(maxsize=None)
+def pair_plan(M: int, N: int, K: int, pairs: int, split: bool, consumer: bool = False) -> tuple | None:
+    """(transposed, tile width, splits) of the pair kernel for out[M, N] = a[M, K] w^T, or None where `plan`'s one CTA a tile is
+    as good: up to 64 tokens, few columns, and where its row tiles of 128 save more than pairs do (257 to 384 tokens).
+
+    Up to 256 tokens the weights may fill the 256-row side of a tile and the tokens the other (`transposed`). With `split` k may be
+    cut so that every pair has work; `consumer`: whoever reads the product adds the splits (else a kernel of its own does)."""
+    if M <= PAIR_FROM or N < PAIR_MIN_COLUMNS or _NO_PAIR:
+        return None
+    k_blocks, best = math.ceil(K / 64), None
+    most = plan(M, N, K, split)[2] if split else 1        # as many sums as one CTA a tile would leave: what their buffers are made for
+    for transposed in ((1, 0) if M <= 256 else (0,)):
+        for bn in PAIR_WIDTHS:
+            if transposed and (bn >= M + 32 or 2 * bn < M):
+                continue
+            tiles = math.ceil(N / 256) * math.ceil(M / bn) if transposed else math.ceil(M / 256) * math.ceil(N / bn)
+            for splits in range(1, most + 1):
+                if splits > 1 and (tiles * splits > pairs or k_blocks // splits < 6):
+                    break
+                if math.ceil(k_blocks / math.ceil(k_blocks / splits)) != splits:
+                    continue
+                cost = _pair_cost(M, N, K, pairs, transposed, bn, splits) + _reduce_cost(M, N, splits, consumer)
+                if best is None or cost < best[0] - 1e-9:
+                    best = (cost, transposed, bn, splits)
+    if M > 128:
+        _, bn, splits = plan(M, N, K, split)
+        if _single_cost(M, N, K, bn, splits) + _reduce_cost(M, N, splits, consumer) < best[0]:
+            return None
+    return best[1:]
+
+
 def pair_width(M: int, N: int, K: int, pairs: int) -> int:
-    """The tile width of the pair kernel for out[M, N] = a[M, K] w^T: the one whose waves of tiles over `pairs` pairs
-    of SMs take the least time by the estimate above; the widest on a tie."""
-    tiles_m, k_blocks = math.ceil(M / 256), math.ceil(K / 64)
-    best = None
-    for bn in PAIR_WIDTHS:
-        waves = math.ceil(tiles_m * math.ceil(N / bn) / pairs)
-        cost = waves * (k_blocks * max(_PAIR_US_MMA * bn / 256, _PAIR_US_FEED) + _PAIR_US_TILE)
-        if best is None or cost < best[0] - 1e-9:
-            best = (cost, bn)
-    return best[1]
+    """The tile width of the pair kernel with whole k and the tokens on the 256-row side; the widest on a tie."""
+    return min(PAIR_WIDTHS, key=lambda bn: (_pair_cost(M, N, K, pairs, 0, bn, 1), -bn))
 
 
 def _gated(epilogue) -> bool:
@@ -177,13 +223,18 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
     _need(a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1, "gemm: last axes must be contiguous")
     _need(checked or tc_takes(a, w, out),
           "gemm_tc: operands must be bfloat16 with K and row strides multiples of 8, 16-byte aligned")
-    if pair is None:
-        pair = transposed is None and bn is None and splits is None and pair_takes(M, N)
-    if pair:
+    forced = not (transposed is None and bn is None and splits is None)
+    p = None if forced or pair is False else pair_plan(M, N, K, resident_pairs(), not silu and K > 0, partial_scratch is not None)
+    if pair and p is None:
+        p = (transposed or 0, bn or pair_width(M, N, K, resident_pairs()), splits or 1)
+    if p is not None:
+        t, bn, splits = p
+        leave = splits > 1 and partial_scratch is not None
+        if splits > 1:
+            scratch = partial_scratch(splits * M * N) if leave else scratch if scratch is not None else _scratch_for(splits * M * N, a.device)
         _call("tie_gemm_tc2", dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
-              w.stride(0), out.stride(0), int(silu), 0, 0, bn if bn in PAIR_WIDTHS else pair_width(M, N, K, resident_pairs()),
-              _stream())
-        return out
+              w.stride(0), out.stride(0), int(silu), 0, 0, bn, t, splits, scratch.data_ptr() if splits > 1 else 0, 0 if leave else 1, _stream())
+        return SplitSum(scratch, _library().tie_gemm_tc_real_splits(K, splits), M, N) if leave else out
     t, b, s = plan(M, N, K)
     transposed = t if transposed is None else int(transposed)
     bn = b if bn is None else bn
@@ -283,18 +334,20 @@ class BoundGemm:
         from . import unpack_k_blocks
         return unpack_k_blocks(self.w, self.K)[self.row0:self.row0 + self.N]
 
-    def _plan(self, M: int):
-        pair = pair_takes(M, self.N)
-        t, bn, splits = plan(M, self.N, self.K, self.split_many)
+    def _plan(self, M: int, consumer: bool):
+        # up to 128 tokens k may be split for anyone, above for those who did not ask for the finished product
+        pair = pair_plan(M, self.N, self.K, resident_pairs(), not self.silu and (self.split_many or M <= 128), consumer)
+        if pair is not None:
+            t, bn, splits = pair
+        else:
+            t, bn, splits = plan(M, self.N, self.K, self.split_many)
         if self.gated:
             splits = 1
             if not t:
                 bn = max(bn, 32)
         real = _library().tie_gemm_tc_real_splits(self.K, splits) if splits > 1 else 1
-        if pair:
-            bn = pair_width(M, self.N, self.K, resident_pairs())
-        p = (pair, t, bn, splits, int(not t or bn >= 128), real)
-        self._plans[M] = p
+        p = (pair is not None, t, bn, splits, int(not t or bn >= 128), real)
+        self._plans[M, consumer] = p
         return p
 
     def __call__(self, a: torch.Tensor, out: torch.Tensor, partial_scratch=None):
@@ -319,13 +372,10 @@ class BoundGemm:
             from . import SplitSum, _need, _stream, dtype_code
             _ops = (SplitSum, _need, _stream, dtype_code)
         SplitSum, _, _stream, dtype_code = _ops
-        pair, t, bn, splits, deep, real = self._plans.get(M) or self._plan(M)
+        consumer = partial_scratch is not None and not self.silu
+        pair, t, bn, splits, deep, real = self._plans.get((M, consumer)) or self._plan(M, consumer)
         code = 1 if out.dtype == torch.bfloat16 else 0
-        if pair:
-            _call("tie_gemm_tc2", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw,
-                  out.stride(0), self.silu, self.packed_rows, self.row0, bn, _stream())
-            return out
-        leave = splits > 1 and partial_scratch is not None and not self.silu
+        leave = splits > 1 and consumer
         scratch = 0
         if leave:
             buf = partial_scratch(splits * M * self.N)
@@ -333,8 +383,12 @@ class BoundGemm:
         elif splits > 1:
             buf = _scratch_for(splits * M * self.N, a.device)
             scratch = buf.data_ptr()
-        _call("tie_gemm_tc", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0),
-              t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0, _stream())
+        if pair:
+            _call("tie_gemm_tc2", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw,
+                  out.stride(0), self.silu, self.packed_rows, self.row0, bn, t, splits, scratch, 0 if leave else 1, _stream())
+        else:
+            _call("tie_gemm_tc", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0),
+                  t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0, _stream())
         if leave:
             return SplitSum(buf, real, M, self.N)
         return out
