@@ -230,6 +230,44 @@ def test_float_products_in_every_tiling(ops, tile, splits, M, N, K):
     assert (host(out)[:, N:] == -7.0).all()
 
 
+@pytest.mark.parametrize("bn,splits", [(32, 1), (32, 8), (64, 1), (64, 4), (96, 1), (96, 2), (96, 8)])
+@pytest.mark.parametrize("M,N,K,pad", [(1, 1, 64, 0), (129, 97, 130, 4), (128, 96, 1024, 0), (300, 200, 1031, 1)])
+def test_float_products_by_three_terms(ops, bn, splits, M, N, K, pad):
+    """Edges of tiles, k-blocks that end early, splits that get no k-block, rows that are no whole 16-byte pieces. The error against 64 bits
+    is 1.0 to 1.4e-7 (a rounding a block of 64 k's, and the tensor core's truncation, 2^-24 a step); FFMAs are at 1.1e-7 (k = 64) to 4.1e-7."""
+    from tiny_inference_engine_b200.ops.library import call
+    rng = np.random.default_rng(M + N + K)
+    a, w = rng.standard_normal((M, K + pad)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    da, dw, out = dev(a), dev(w), torch.full((M, N + 3), -7.0, device="cuda")
+    call("tie_gemm_f32_split", da.data_ptr(), dw.data_ptr(), out.data_ptr(), M, N, K, K + pad, K, N + 3, bn, splits,
+         torch.cuda.current_stream().cuda_stream)
+    want = a[:, :K].astype(np.float64) @ w.astype(np.float64).T
+    got = host(out)
+    assert np.linalg.norm(got[:, :N] - want) < 2.2e-7 * np.linalg.norm(want) and (got[:, N:] == -7.0).all()
+
+
+@pytest.mark.parametrize("bn,splits", [(64, 1), (96, 4)])
+def test_float_products_by_three_terms_of_infinities_and_large_values(ops, bn, splits):
+    """An infinity, a NaN or a value that bfloat16 would round to an infinity reaches exactly the outputs it belongs to."""
+    from tiny_inference_engine_b200.ops.library import call
+    rng = np.random.default_rng(bn)
+    M, N, K = 200, 150, 520
+    a, w = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    w[w == 0] = 1.0
+    w[3, 40] = 1.0
+    a[5, 40], a[130, 300], a[7, 519], w[60, 65], a[9, :], a[9, 2] = np.inf, -np.inf, np.nan, np.inf, 0.0, 3.4e38
+    w[:, 2] = np.clip(w[:, 2], -0.5, 0.5)
+    da, dw, out = dev(a), dev(w), torch.empty(M, N, device="cuda")
+    call("tie_gemm_f32_split", da.data_ptr(), dw.data_ptr(), out.data_ptr(), M, N, K, K, K, N, bn, splits, torch.cuda.current_stream().cuda_stream)
+    got, want = host(out).astype(np.float64), torch.from_numpy(a).double() @ torch.from_numpy(w).double().T
+    want = want.numpy()
+    odd = ~np.isfinite(want)
+    assert odd.sum() > 400 and ((got[odd] == want[odd]) | (np.isnan(got[odd]) & np.isnan(want[odd]))).all()
+    rest = (~odd) & (np.arange(M) != 9)[:, None]
+    assert np.linalg.norm(got[rest] - want[rest]) < 1e-6 * np.linalg.norm(want[rest])
+    assert (np.abs(got[9] - want[9])[~odd[9]] <= 1e-6 * np.abs(want[9])[~odd[9]]).all()
+
+
 def dense_reference(q, k, v, Hq, Hkv, Dh, n_new, window=0):
     """The last n_new rows of causal attention over all of k, v."""
     n = k.shape[0]

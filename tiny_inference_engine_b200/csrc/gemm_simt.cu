@@ -1,8 +1,8 @@
 // Matrix products on the CUDA cores: out[M, N] = a[M, K] . w[N, K]^T with float accumulation.
 //
-// These are the kernels of the true 32-bit path (float in, float out, FFMA only, no tensor
-// cores and so no reduced-precision matrix mode), and they take every size; the bfloat16
-// instantiations serve sizes that the tensor-core kernels refuse. The reference's
+// These are the FFMA kernels of the true 32-bit path (float in, float out; no reduced-precision matrix mode): few rows,
+// batches and short k. Its large products run on the tensor cores without giving precision up (gemm_f32_split.cu). They
+// take every size; the bfloat16 instantiations serve sizes that the tensor-core kernels refuse. The reference's
 // counterpart is its dot-product matmul (src/backend/cpu/cpu_backend.cpp:78-139): weights
 // in the checkpoint's [out, in] layout, y = x . W^T, no bias.
 #include <type_traits>
@@ -11,6 +11,9 @@
 #include "launchers.h"
 
 namespace tie {
+
+int launch_gemm_f32_split_chosen(const float* a, const float* w, float* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
+                                 cudaStream_t s);      // gemm_f32_split.cu
 
 // ---------------------------------------------------------------------------------------------
 // Tiled kernel for any M, N, K (bfloat16 operands): 64 x 64 output tile, 16-deep k slices, 256 threads, 4 x 4
@@ -338,6 +341,9 @@ int launch_gemm(const void* a, const void* w, void* out, int M, int N, int K, lo
 #undef TIE_SMALL_M_ROWS
 #undef TIE_SMALL_M
   } else if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+    // one product of more than 16 rows by three bfloat16 terms on the tensor cores: a half to a quarter of the FFMAs' time at every size
+    // tried (17 to 1,000 rows, 32 to 32,000 columns, k from 64 on), and nearer to 64 bits; below 64 k's a block is mostly padding
+    if (batch == 1 && M > 16 && K >= 64) return launch_gemm_f32_split_chosen(ap, wp, op, M, N, K, lda, ldw, ldo, s);
     return launch_gemm_f32(ap, wp, op, M, N, K, lda, ldw, ldo, s, batch, sa, sw, so, -1, 1);
   } else {
     TIE_LAUNCH((gemm_tiled_kernel<TI, TO>), dim3(ceil_div(N, 64), ceil_div(M, 64), batch), 256, 0, s, ap, wp, op, M, N, K, lda, ldw,

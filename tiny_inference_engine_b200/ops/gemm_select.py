@@ -1,6 +1,7 @@
 """Which matrix-product kernel runs for which operands, and with which tiling.
 
-float32 always runs on the CUDA cores: the 32-bit path has no reduced-precision matrix mode.
+float32 has no reduced-precision matrix mode: few rows run on the CUDA cores, more as exact sums of bfloat16 terms
+(csrc/gemm_f32_split.cu), with smaller errors than FFMAs.
 bfloat16 runs on the tensor cores (tcgen05) whenever TMA can address the operands (K and the
 row strides multiples of 8 elements, 16-byte aligned bases), else on the CUDA cores.
 """

@@ -26,6 +26,7 @@ _SIGNATURES = {
     "tie_kv_append": [I, P, P, L, L, P, P, P, I, I, I, I, P],
     "tie_qk_norm_rope_append": [I, P, L, P, L, I, L, P, P, F, F, P, I, P, P, P, P, I, I, I, I, I, I, P],
     "tie_gemm_f32_tiled": [P, P, P, I, I, I, L, L, L, I, I, P],
+    "tie_gemm_f32_split": [P, P, P, I, I, I, L, L, L, I, I, P],
     "tie_gemm_simt": [I, I, P, P, P, I, I, I, L, L, L, P],
     "tie_attention_rows": [I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P],
     "tie_attention_split": [I, P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P, I, I, I, P, P],
