@@ -606,7 +606,8 @@ def test_pair_kernel_on_either_side_and_with_split_k(ops, M, N, K, transposed, b
         wide = torch.full((M, N + 16), 7.0, device="cuda", dtype=dtype)
         scratch = torch.full((splits * M * N + 16,), float("nan"), device="cuda")
         gemm_select._call("tie_gemm_tc2", int(dtype == torch.bfloat16), ta.data_ptr(), tw.data_ptr(), wide[:, offset:].data_ptr(), M, N, K, K, K,
-                          N + 16, 0, 0, 0, bn, transposed, splits, scratch.data_ptr(), 1, torch.cuda.current_stream().cuda_stream)
+                          N + 16, 0, 0, 0, bn, transposed, splits, scratch.data_ptr(), 1, 0, 0, 0.0, 1.0, 0.0, 0,
+                          torch.cuda.current_stream().cuda_stream)
         torch.cuda.synchronize()
         gemm_select.check_status()
         assert rel_err(host(wide[:, offset:offset + N]), want) < (TOL["bfloat16"] if dtype == torch.bfloat16 else 2e-5), (dtype, offset)
@@ -632,7 +633,7 @@ def test_silu_epilogue_from_the_smallest_to_the_largest_gates(ops, transposed):
     out = torch.full((M, I), float("nan"), device="cuda")
     w = ops.interleave_gate_up(gate.cuda(), up.cuda())
     gemm_select._call("tie_gemm_tc2", 0, a.cuda().data_ptr(), w.data_ptr(), out.data_ptr(), M, 2 * I, K, K, K, I, 1, 0, 0, 128 if transposed else 64,
-                      transposed, 1, 0, 1, torch.cuda.current_stream().cuda_stream)
+                      transposed, 1, 0, 1, 0, 0, 0.0, 1.0, 0.0, 0, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     gemm_select.check_status()
     g = a[:, 0].double()
@@ -640,6 +641,36 @@ def test_silu_epilogue_from_the_smallest_to_the_largest_gates(ops, transposed):
     got = out.double().cpu()
     near = want.abs() > 1e-36                      # below, 32 bits have no full mantissa
     assert ((got - want).abs()[near] <= 6 * 2.0 ** -24 * want.abs()[near] * 2).all() and (got - want).abs()[~near].max() < 2e-36
+
+
+@pytest.mark.parametrize("act", [4, 5, 6])
+@pytest.mark.parametrize("M,I,K", [(5, 48, 1024), (64, 496, 2048), (100, 48, 72), (200, 352, 264), (640, 176, 136)])
+def test_gated_units_in_the_epilogue(ops, M, I, K, act):
+    """The clamped unit and the ones with biases, the columns of a one and zeros behind them: k split (the unit formed where the sums are
+    added), the weights or the tokens on the row side, one CTA or a pair a tile, sizes that end inside a tile."""
+    from tiny_inference_engine_b200.ops import gemm_select
+    rng = np.random.default_rng(M + act)
+    a = as_stored(rng.standard_normal((M, K)), "bfloat16")
+    gate, up = (as_stored(rng.standard_normal((I, K)) * 3 / K ** 0.5, "bfloat16") for _ in range(2))
+    bg, bu = rng.standard_normal(I).astype(np.float32), rng.standard_normal(I).astype(np.float32)
+    ones = 0 if act == 4 else 8
+    unit = gemm_select.GatedUnit(2.0, 1.702, 1.0) if act == 4 else gemm_select.GatedUnit(bias_gate=dev(bg), bias_up=dev(bu), ones=ones)
+    product = ops.bound_gemm(ops.interleave_gate_up(dev(gate, torch.bfloat16), dev(up, torch.bfloat16)), silu=act, unit=unit)
+    wide = torch.full((M, I + ones + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    product(dev(a, torch.bfloat16), wide[:, :I])
+    torch.cuda.synchronize()
+    gemm_select.check_status()
+    g, u = plain.linear(a, gate).astype(np.float64), plain.linear(a, up).astype(np.float64)
+    if act == 4:
+        g, u = np.minimum(g, 2.0), np.clip(u, -2.0, 2.0)
+        want = g / (1 + np.exp(-1.702 * g)) * (u + 1.0)
+    else:
+        g, u = g + bg, u + bu
+        want = u * (g / (1 + np.exp(-g)) if act == 5 else 0.5 * g * (1 + np.tanh(np.sqrt(2 / np.pi) * (g + 0.044715 * g ** 3))))
+    assert rel_err(host(wide[:, :I]), want) < TOL["bfloat16"]
+    if ones:
+        assert (wide[:, I] == 1).all() and (wide[:, I + 1:I + ones] == 0).all()
+    assert (wide[:, I + ones:] == 7).all()
 
 
 @pytest.mark.parametrize("M", [5, 300, 640])

@@ -118,12 +118,12 @@ __device__ __forceinline__ float squared_relu(float v) {
   return r * r;
 }
 
-// g / (1 + exp(-g)). An epilogue evaluates sixteen and more of these side by side, and the branches of `/` keep them from
+// g / (1 + exp(-slope g)). An epilogue evaluates sixteen and more of these side by side, and the branches of `/` keep them from
 // overlapping (the gate/up product of 2,048 tokens waited for its epilogue), so the quotient is formed without any: the
 // hardware's approximate reciprocal, one Newton-Raphson step on it, and one on the quotient by its residual. Denominators
 // above 2^60 are scaled down first, so that no reciprocal is subnormal; where exp(-g) overflows, g * 0 is what g / inf is.
-__device__ __forceinline__ float silu(float g) {
-  const float e = expf(-g);
+__device__ __forceinline__ float silu(float g, float slope = 1.0f) {
+  const float e = expf(-slope * g);
   const float scale = e > 1.152921504606847e18f ? 5.421010862427522e-20f : 1.0f;      // 2^60, 2^-64
   const float d = (1.0f + fminf(e, 3.402823466e38f)) * scale, n = g * scale;
   float r;
@@ -134,8 +134,50 @@ __device__ __forceinline__ float silu(float g) {
   return e > 3.402823466e38f ? g * 0.0f : q;
 }
 
-// The activation of a gated product's epilogue: 1 the SiLU, 2 the ReLU.
-__device__ __forceinline__ float gate_act(float g, int act) { return act == 2 ? fmaxf(g, 0.0f) : silu(g); }
+__device__ __forceinline__ float gelu_tanh_f(float z) {
+  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
+}
+
+// A gated unit in a product's epilogue (the weight's rows in blocks of 16 gate and 16 up rows; the output half as wide): 1 SiLU(g) u,
+// 2 ReLU(g) u, 4 the clamped unit g' sigmoid(slope g') (u' + up_shift) with g' = min(g, limit), u' = clamp(u, +-limit), 5 and 6 SiLU or the
+// tanh form of GELU of g + bias_gate, times u + bias_up. `ones` > 0: that many more columns behind the unit's, a one and zeros (for a
+// product whose weight carries its bias as that column).
+constexpr int kEpilogueClamped = 4, kEpilogueBiasedSilu = 5, kEpilogueBiasedGelu = 6;
+struct GatedUnit {
+  const float *bias_gate, *bias_up;
+  float limit, slope, up_shift;
+  int ones;
+};
+__host__ __device__ constexpr bool gated_epilogue(int e) { return e != 0 && e != kEpilogueSquaredRelu; }
+// N of them at once, the kind of unit chosen outside the loop: g and u as their bits, bias_gate and bias_up the biases of the first (of all of
+// them with `same`: N rows of one output column).
+template <int N, bool same = false>
+__device__ __forceinline__ void gated_values(const uint32_t* g, const uint32_t* u, float (&v)[N], int act, const GatedUnit& unit,
+                                             const float* bias_gate, const float* bias_up) {
+  if (act == 1) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = silu(__uint_as_float(g[e])) * __uint_as_float(u[e]);
+  } else if (act == 2) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = fmaxf(__uint_as_float(g[e]), 0.0f) * __uint_as_float(u[e]);
+  } else if (act == kEpilogueClamped) {
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      v[e] = silu(fminf(__uint_as_float(g[e]), unit.limit), unit.slope) *
+             (fminf(fmaxf(__uint_as_float(u[e]), -unit.limit), unit.limit) + unit.up_shift);
+  } else {
+    float a[N], b[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) a[e] = __uint_as_float(g[e]) + bias_gate[same ? 0 : e], b[e] = __uint_as_float(u[e]) + bias_up[same ? 0 : e];
+    if (act == kEpilogueBiasedSilu) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) v[e] = silu(a[e]) * b[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < N; ++e) v[e] = gelu_tanh_f(a[e]) * b[e];
+    }
+  }
+}
 
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 

@@ -63,7 +63,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, OutT* __restrict__ out,
                float* __restrict__ partial, long long part_stride, long long ldp, int rows_x, int rows_y, int k_blocks,
                int k_blocks_per_split, long long ldo, int transposed, int silu, int tiles_x, int n_tiles, int* status,
-               int w_rows, int w_row0, const int* __restrict__ group_meta, const int* __restrict__ group_of_tile) {
+               int w_rows, int w_row0, const int* __restrict__ group_meta, const int* __restrict__ group_of_tile,
+               const __grid_constant__ GatedUnit unit) {
   pdl_launch_dependents();   // the next kernel may get resident now; it waits for this one at its own pdl_wait()
   // Grouped (plain tiling only): the row operand is `group_meta[0]` tiles of 128 rows, fewer than the grid was sized
   // for, and row tile t multiplies the weight rows of group `group_of_tile[t]` (`rows_y` rows each, one after the
@@ -228,9 +229,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + buf * BN;
       const int i = i0 + warp * 32 + lane;
-      if (silu != 0 && silu != kEpilogueSquaredRelu) {
+      if (gated_epilogue(silu) && part == nullptr) {
         // The weight rows come in blocks of 16 gate rows followed by their 16 up rows; the output is
-        // act(gate) * up (act 1: the SiLU, 2: the ReLU), half as wide as the product: out[token, 16 * block + r].
+        // that of a gated unit (GatedUnit), half as wide as the product: out[token, 16 * block + r].
         if (transposed) {
           // lanes 0-15 of a warp hold gate rows, lanes 16-31 the matching up rows: exchange, then
           // the lower half finishes columns 0-7 of each chunk and the upper half columns 8-15
@@ -242,16 +243,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             uint32_t r[16];
             tmem_ld16(tmem_acc + (static_cast<uint32_t>(warp * 32) << 16) + c0, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int j1 = j0 + c0 + (upper ? 8 : 0);
+            uint32_t g[8], u[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               // the lower lane sends its gate of column e + 8 and receives the up of column e;
               // the upper lane sends its up of column e and receives the gate of column e + 8
               const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? r[e] : r[e + 8], 16);
-              const float g = __uint_as_float(upper ? got : r[e]);
-              const float u = __uint_as_float(upper ? r[e + 8] : got);
-              const int j = j0 + c0 + e + (upper ? 8 : 0);
-              if (j < rows_y && o < (rows_x >> 1)) st(out + static_cast<long long>(j) * ldo + o, gate_act(g, silu) * u);
+              g[e] = upper ? got : r[e];
+              u[e] = upper ? r[e + 8] : got;
             }
+            if (o < (rows_x >> 1)) {
+              float v[8];
+              gated_values<8, true>(g, u, v, silu, unit, unit.bias_gate + o, unit.bias_up + o);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (j1 + e < rows_y) st(out + static_cast<long long>(j1 + e) * ldo + o, v[e]);
+            }
+            if (unit.ones > 0 && i0 + kBM >= rows_x) store_ones(out, ldo, rows_x >> 1, unit.ones, j0 + c0, min(16, rows_y - (j0 + c0)), warp * 32 + lane);
           }
         } else {
 #pragma unroll 1
@@ -263,11 +272,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (i < rows_x) {
               float v[16];
-#pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const float gv = __uint_as_float(g[e]);
-                v[e] = gate_act(gv, silu) * __uint_as_float(u[e]);
-              }
+              const int column = (j0 + c0) >> 1;
+              gated_values<16>(g, u, v, silu, unit, unit.bias_gate + column, unit.bias_up + column);
               const long long at = static_cast<long long>(i) * ldo + ((j0 + c0) >> 1);
               if (((at * sizeof(OutT)) & 15) == 0 && sizeof(OutT) == 2) {
                 uint32_t w[8];
@@ -284,6 +290,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
               }
             }
           }
+          if (unit.ones > 0 && j0 + BN >= rows_y) store_ones(out, ldo, rows_y >> 1, unit.ones, i0 + warp * 32, min(32, rows_x - (i0 + warp * 32)), lane);
         }
       } else {
 #pragma unroll 1
@@ -371,13 +378,37 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, long lon
   st(out + (idx / N) * ldo + idx % N, epilogue == kEpilogueSquaredRelu ? squared_relu(acc) : acc);
 }
 
+// The same for a gated unit: out[m, c] from the sums of its gate and its up column, and the columns behind the unit's. A thread
+// an output.
+template <typename OutT>
+__global__ void splitk_gated_kernel(const float* __restrict__ partial, long long part_stride, int splits, OutT* __restrict__ out, long long ldo,
+                                    int N, int rows, int act, GatedUnit unit) {
+  pdl_sync();
+  const int inter = N / 2, width = inter + unit.ones;
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= static_cast<long long>(rows) * width) return;
+  const long long m = idx / width;
+  const int c = static_cast<int>(idx - m * width);
+  if (c >= inter) {
+    st(out + m * ldo + c, c == inter ? 1.0f : 0.0f);
+    return;
+  }
+  const float* at = partial + m * N + (c >> 4) * 32 + (c & 15);
+  float g = at[0], u = at[16];
+  for (int z = 1; z < splits; ++z) g += at[z * part_stride], u += at[z * part_stride + 16];
+  const uint32_t gb = __float_as_uint(g), ub = __float_as_uint(u);
+  float v[1];
+  gated_values<1>(&gb, &ub, v, act, unit, unit.bias_gate + c, unit.bias_up + c);
+  st(out + m * ldo + c, v[0]);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Host side
 
 template <int BN, typename OutT, bool DEEP>
 static int launch_tc(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* partial, long long part_stride,
                      long long ldp, int rows_x, int rows_y, int K, long long ldo, int transposed, int silu, int splits, int w_rows,
-                     int w_row0, cudaStream_t s, const int* group_meta = nullptr, const int* group_of_tile = nullptr) {
+                     int w_row0, cudaStream_t s, const GatedUnit& unit, const int* group_meta = nullptr, const int* group_of_tile = nullptr) {
   using C = TcConfig<BN, DEEP>;
   static bool configured = false;
   if (!configured) {
@@ -400,7 +431,7 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& my, void* out, fl
   const dim3 grid(min(ctas, n_tiles), 1, z);
   TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
              rows_x, rows_y, k_blocks, per_split, ldo, transposed, silu, tiles_x, n_tiles, status_word(), w_rows, w_row0, group_meta,
-             group_of_tile);
+             group_of_tile, unit);
   return kOk;
 }
 
@@ -424,7 +455,7 @@ using namespace tie;
 // with tie_gemm_tc_scratch_floats floats: the float partial sums [splits, M, N]; with reduce == 0
 // they are left there for a consumer that adds them itself (tie_gemm_tc_real_splits says how
 // many there are). silu != 0: w holds blocks of 16 gate rows followed by their 16 up rows and
-// out[M, N / 2] = act(gate) * up, act the SiLU (1) or the ReLU (2); silu == 3: out[M, N] = max(product, 0)^2, with split k
+// out[M, N / 2] is a gated unit's (1, 2, 4, 5, 6: GatedUnit); silu == 3: out[M, N] = max(product, 0)^2, with split k
 // applied by the reduction (reduce != 0). deep != 0: the deepest shared-memory ring (one CTA per SM), else
 // a ring of about 100 KB (two CTAs per SM). Returns kBadArgument
 // with a message for sizes it does not take (K or a row stride not a multiple of 8, unaligned
@@ -443,7 +474,8 @@ TIE_API long long tie_gemm_tc_scratch_floats(int M, int N, int splits) {
 // w_row0 .. w_row0 + N - 1; ldw is then ignored.
 TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
                         long long ldw, long long ldo, int transposed, int bn, int splits, float* scratch, int silu,
-                        int reduce, int deep, int w_rows, int w_row0, cudaStream_t s) {
+                        int reduce, int deep, int w_rows, int w_row0, const float* bias_gate, const float* bias_up, float limit,
+                        float slope, float up_shift, int ones, cudaStream_t s) {
   TIE_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_tc: bad sizes M=%d N=%d K=%d", M, N, K);
   TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && (w_rows > 0 || ldw % 8 == 0), "gemm_tc: K=%d and the row strides must be multiples of 8", K);
   TIE_REQUIRE(w_rows == 0 || (w_row0 >= 0 && w_row0 + N <= w_rows), "gemm_tc: rows %d..%d of a weight of %d rows", w_row0, w_row0 + N, w_rows);
@@ -452,10 +484,11 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
   TIE_REQUIRE(bn == 16 || bn == 32 || bn == 64 || bn == 128 || bn == 256, "gemm_tc: tile width %d", bn);
   TIE_REQUIRE(splits >= 1 && (splits == 1 || scratch != nullptr), "gemm_tc: splits=%d needs scratch memory", splits);
   TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc: output dtype code %d", out_dtype);
-  TIE_REQUIRE(silu >= 0 && silu <= kEpilogueSquaredRelu && (silu != kEpilogueSquaredRelu || splits == 1 || reduce),
+  TIE_REQUIRE(silu >= 0 && silu <= kEpilogueBiasedGelu && (silu != kEpilogueSquaredRelu || splits == 1 || reduce),
               "gemm_tc: epilogue %d (the squared ReLU of a split product needs the reduction here)", silu);
-  TIE_REQUIRE(silu == 0 || silu == kEpilogueSquaredRelu || (splits == 1 && N % 32 == 0 && (transposed || bn >= 32)),
-              "gemm_tc: the SiLU epilogue needs unsplit k and weight rows in blocks of 16 gate + 16 up (N=%d)", N);
+  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (bias_gate != nullptr && bias_up != nullptr), "gemm_tc: epilogue %d needs biases", silu);
+  TIE_REQUIRE(!gated_epilogue(silu) || ((splits == 1 || reduce) && N % 32 == 0 && (transposed || bn >= 32)),
+              "gemm_tc: a gated unit needs unsplit k (or the reduction here) and weight rows in blocks of 16 gate + 16 up (N=%d)", N);
   TIE_REQUIRE(status_word() != nullptr, "gemm_tc: cannot allocate the status word");
   // row operand X (128 per tile) and column operand Y (bn per tile)
   const void* x = transposed ? w : a;
@@ -471,7 +504,8 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
   const long long part_stride = static_cast<long long>(M) * N;
   const long long ldp = N;
   int st = kOk;
-#define TIE_TC_ARGS mx, my, out, partial, part_stride, ldp, rows_x, rows_y, K, ldo, transposed, silu, splits, w_rows, w_row0, s
+  const GatedUnit unit{bias_gate, bias_up, limit, slope, up_shift, gated_epilogue(silu) ? ones : 0};
+#define TIE_TC_ARGS mx, my, out, partial, part_stride, ldp, rows_x, rows_y, K, ldo, transposed, silu, splits, w_rows, w_row0, s, unit
 #define TIE_TC_CASE(B)                                                                                     \
   case B:                                                                                                  \
     if (deep) {                                                                                            \
@@ -490,7 +524,14 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
 #undef TIE_TC_ARGS
 #undef TIE_TC_CASE
   if (st != kOk) return st;
-  if (splits > 1 && reduce) launch_splitk_reduce(out_dtype, partial, part_stride, tie_gemm_tc_real_splits(K, splits), out, ldo, N, part_stride, silu, s);
+  if (splits > 1 && gated_epilogue(silu)) {
+    const int real = tie_gemm_tc_real_splits(K, splits);
+    const unsigned blocks = ceil_div(static_cast<long long>(M) * (N / 2 + unit.ones), 256);
+    if (out_dtype == TIE_BF16)
+      TIE_LAUNCH((splitk_gated_kernel<__nv_bfloat16>), blocks, 256, 0, s, partial, part_stride, real, static_cast<__nv_bfloat16*>(out), ldo, N, M, silu, unit);
+    else
+      TIE_LAUNCH((splitk_gated_kernel<float>), blocks, 256, 0, s, partial, part_stride, real, static_cast<float*>(out), ldo, N, M, silu, unit);
+  } else if (splits > 1 && reduce) launch_splitk_reduce(out_dtype, partial, part_stride, tie_gemm_tc_real_splits(K, splits), out, ldo, N, part_stride, silu, s);
   TIE_RETURN_LAUNCH("gemm_tc");
 }
 
@@ -511,7 +552,7 @@ TIE_API int tie_gemm_tc_grouped(int out_dtype, const void* a, const void* w, voi
   TIE_REQUIRE(make_map_bf16(&mx, a, M_cap, K, lda, kBK, kBM) && make_map_bf16(&my, w, kb_rows, kBK, kBK, kBK, bn),
               "gemm_tc_grouped: cuTensorMapEncodeTiled failed (rows %d, K %d)", M_cap, K);
   int st = kOk;
-#define TIE_TCG_ARGS mx, my, out, nullptr, 0, N, M_cap, N, K, ldo, 0, 0, 1, w_rows, 0, s, meta, group_of_tile
+#define TIE_TCG_ARGS mx, my, out, nullptr, 0, N, M_cap, N, K, ldo, 0, 0, 1, w_rows, 0, s, GatedUnit{}, meta, group_of_tile
   if (bn == 128) st = out_dtype == TIE_BF16 ? launch_tc<128, __nv_bfloat16, true>(TIE_TCG_ARGS) : launch_tc<128, float, true>(TIE_TCG_ARGS);
   else st = out_dtype == TIE_BF16 ? launch_tc<256, __nv_bfloat16, true>(TIE_TCG_ARGS) : launch_tc<256, float, true>(TIE_TCG_ARGS);
 #undef TIE_TCG_ARGS

@@ -102,6 +102,7 @@ struct PairArgs {
   int transposed;          // x are the weights and the epilogue writes the tile's transpose
   int epilogue, by_tma;    // by_tma: a tensor map describes the output (or the sums), else rows are stored element by element
   int w_rows, w_row0;
+  GatedUnit unit;
   int* status;
 };
 
@@ -260,7 +261,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   } else {
     // ---- epilogue (both CTAs): rows i0 .. i0 + 127 of the pair's tile, all its columns
     const int group = warp >> 2, quarter = warp & 3;
-    const bool gated = g.epilogue != 0 && g.epilogue != kEpilogueSquaredRelu;
+    const bool gated = gated_epilogue(g.epilogue);
     const bool squared = g.epilogue == kEpilogueSquaredRelu && g.partial == nullptr;
     int local = 0;
     for (int work = pair; work < g.n_work; work += pairs, ++local) {
@@ -291,18 +292,27 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
           uint32_t r[16];
           tmem_ld16(acc + c0, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (gated && g.unit.ones > 0 && i0 < g.rows_x && i0 + 128 >= g.rows_x) store_ones(static_cast<OutT*>(g.out), g.ldo, g.rows_x >> 1, g.unit.ones, j0 + c0, min(16, g.rows_y - (j0 + c0)), quarter * 32 + lane);
           if (gated) {
             // lanes 0-15 hold 16 gate rows, lanes 16-31 the matching up rows: exchange, then the lower half finishes
             // columns 0-7 and the upper half columns 8-15
             const bool upper = lane >= 16;
             const int o = (i0 >> 1) + quarter * 16 + (lane & 15);
+            const int c1 = j0 + c0 + (upper ? 8 : 0);
+            uint32_t gv[8], uv[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? r[e] : r[e + 8], 16);
-              const float gv = __uint_as_float(upper ? got : r[e]);
-              const float u = __uint_as_float(upper ? r[e + 8] : got);
-              const int j = j0 + c0 + e + (upper ? 8 : 0);
-              if (j < g.rows_y && o < (g.rows_x >> 1)) st(static_cast<OutT*>(g.out) + static_cast<long long>(j) * g.ldo + o, gate_act(gv, g.epilogue) * u);
+              gv[e] = upper ? got : r[e];
+              uv[e] = upper ? r[e + 8] : got;
+            }
+            if (o < (g.rows_x >> 1)) {
+              float v[8];
+              gated_values<8, true>(gv, uv, v, g.epilogue, g.unit, g.unit.bias_gate + o, g.unit.bias_up + o);
+              OutT* at = static_cast<OutT*>(g.out) + static_cast<long long>(c1) * g.ldo + o;
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (c1 + e < g.rows_y) st(at + e * g.ldo, v[e]);
             }
           } else if (i < g.rows_x) {
             const int n = min(16, g.rows_y - (j0 + c0));
@@ -360,8 +370,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (gated) {
               float v[16];
-#pragma unroll
-              for (int e = 0; e < 16; ++e) v[e] = gate_act(__uint_as_float(r[e]), g.epilogue) * __uint_as_float(r[e + 16]);
+              const int column = ((j0 + c0) >> 1) + h * 16;
+              gated_values<16>(r, r + 16, v, g.epilogue, g.unit, g.unit.bias_gate + column, g.unit.bias_up + column);
               const int next = h + 1 < halves ? c0 + 32 : c0 + 2 * per;
               if (next < end) tmem_ld32(acc + next, r);
               else release();
@@ -392,6 +402,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             __syncwarp();
           }
         }
+        if (gated && g.unit.ones > 0 && j0 + bn >= g.rows_y && group == 0 && i1 < g.rows_x)
+          store_ones(static_cast<OutT*>(g.out), g.ldo, g.rows_y >> 1, g.unit.ones, i1, min(32, g.rows_x - i1), lane);
         if (last) {
           if (waiting > 0) store_boxes(base, (j0 + group * per) >> (gated ? 1 : 0), waiting);
         } else {      // what the next tile writes into the 4 KB has left them by then
@@ -495,8 +507,8 @@ using namespace tie;
 // How many pairs of SMs hold the kernel at once: what the host counts waves of tiles with.
 TIE_API int tie_gemm_tc2_pairs() { return resident_pairs(); }
 
-// out[M, N] (or, with silu 1 or 2, out[M, N / 2] = act(gate) * up, act the SiLU or the ReLU, for w in blocks of 16 gate + 16 up
-// rows; with 3, out[M, N] = max(product, 0)^2)
+// out[M, N] (or, with a gated unit, silu 1, 2, 4, 5, 6, out[M, N / 2] for w in blocks of 16 gate + 16 up rows: GatedUnit;
+// with 3, out[M, N] = max(product, 0)^2)
 // = a[M, K] . w[N, K]^T on pairs of SMs. a, w bfloat16 with K and row strides multiples of 8. w_rows > 0: w is
 // stored in k-blocks, [ceil(K / 64)][w_rows][64], and the product uses its rows w_row0 .. w_row0 + N - 1 (gemm_tc.cu).
 // transposed != 0: the weights fill the tiles' 256-row side. bn: the other side, a multiple of 32 up to 256 (0: 256).
@@ -504,7 +516,8 @@ TIE_API int tie_gemm_tc2_pairs() { return resident_pairs(); }
 // into out by a second kernel, or with reduce == 0 left there for a consumer that adds them itself.
 TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
                          long long ldw, long long ldo, int silu, int w_rows, int w_row0, int bn, int transposed, int splits,
-                         float* scratch, int reduce, cudaStream_t s) {
+                         float* scratch, int reduce, const float* bias_gate, const float* bias_up, float limit, float slope, float up_shift,
+                         int ones, cudaStream_t s) {
   if (bn == 0) bn = 256;
   TIE_REQUIRE(bn >= 32 && bn <= 256 && bn % 32 == 0, "gemm_tc2: tile width %d", bn);
   TIE_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_tc2: bad sizes M=%d N=%d K=%d", M, N, K);
@@ -513,8 +526,9 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   TIE_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0,
               "gemm_tc2: operands must be 16-byte aligned");
   TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc2: output dtype code %d", out_dtype);
-  TIE_REQUIRE(silu >= 0 && silu <= kEpilogueSquaredRelu, "gemm_tc2: epilogue %d", silu);
-  TIE_REQUIRE(silu == 0 || silu == kEpilogueSquaredRelu || N % 32 == 0, "gemm_tc2: the SiLU epilogue needs weight rows in blocks of 16 gate + 16 up (N=%d)", N);
+  TIE_REQUIRE(silu >= 0 && silu <= kEpilogueBiasedGelu, "gemm_tc2: epilogue %d", silu);
+  TIE_REQUIRE(!gated_epilogue(silu) || N % 32 == 0, "gemm_tc2: a gated unit needs weight rows in blocks of 16 gate + 16 up (N=%d)", N);
+  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (bias_gate != nullptr && bias_up != nullptr), "gemm_tc2: epilogue %d needs biases", silu);
   TIE_REQUIRE(splits >= 1 && (splits == 1 || scratch != nullptr), "gemm_tc2: splits=%d needs scratch memory", splits);
   TIE_REQUIRE(splits == 1 || silu == 0 || (silu == kEpilogueSquaredRelu && reduce),
               "gemm_tc2: epilogue %d of a split product (the squared ReLU needs the reduction here)", silu);
@@ -539,6 +553,7 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   g.ldp = N;
   g.ldo = ldo;
   g.epilogue = silu;
+  g.unit = GatedUnit{bias_gate, bias_up, limit, slope, up_shift, gated_epilogue(silu) ? ones : 0};
   g.w_rows = w_rows;
   g.w_row0 = w_row0;
   g.status = status_word();
@@ -548,7 +563,7 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
                                : make_map_bf16(&mw, w, N, K, ldw, k2BK, rows_of_w);
   TIE_REQUIRE(make_map_bf16(&ma, a, M, K, lda, k2BK, rows_of_a) && w_ok, "gemm_tc2: cuTensorMapEncodeTiled failed (M %d, N %d, K %d)", M, N, K);
   const bool as_float = scratch != nullptr || out_dtype == TIE_F32;
-  g.by_tma = !transposed && make_map_rows(&mo, scratch != nullptr ? scratch : out, as_float, M, silu == 1 || silu == 2 ? N / 2 : N,
+  g.by_tma = !transposed && make_map_rows(&mo, scratch != nullptr ? scratch : out, as_float, M, gated_epilogue(silu) ? N / 2 : N,
                                           scratch != nullptr ? N : ldo, scratch != nullptr ? real : 1, 32, 32);
   if (!g.by_tma) mo = ma;
   const CUtensorMap &mx = transposed ? mw : ma, &my = transposed ? ma : mw;

@@ -34,10 +34,6 @@ __global__ void __launch_bounds__(256) add_concat_kernel(float* __restrict__ x, 
   }
 }
 
-__device__ __forceinline__ float gelu_tanh_f(float z) {
-  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
-
 template <typename T>
 __global__ void glu_biased_kernel(const T* __restrict__ gu, const float* __restrict__ bg, const float* __restrict__ bu,
                                   T* __restrict__ out, int inter, int out_width, int act, long long total) {

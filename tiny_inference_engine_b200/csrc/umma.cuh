@@ -105,6 +105,13 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// The columns behind a gated unit's (GatedUnit::ones) of `rows` rows from row0 on, a row a lane id.
+template <typename OutT>
+__device__ __forceinline__ void store_ones(OutT* out, long long ldo, int first, int ones, int row0, int rows, int id) {
+  if (id < rows)
+    for (int e = 0; e < ones; ++e) st(out + (row0 + id) * ldo + first + e, e == 0 ? 1.0f : 0.0f);
+}
+
 // out[m, n] = the sum over splits of partial[split][m, n], in split order, with the epilogue of a product (gemm_tc.cu).
 void launch_splitk_reduce(int out_dtype, const float* partial, long long part_stride, int splits, void* out, long long ldo, int N,
                           long long total, int epilogue, cudaStream_t s);

@@ -539,7 +539,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, partial_scratch=No
     return gemm_select.gemm(a, w, out, partial_scratch)
 
 
-def bound_gemm(w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True):
+def bound_gemm(w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True, unit=None):
     """A matrix product bound to one weight (gemm_select.BoundGemm): checked once, called every step.
     `silu`: an epilogue. Of a gated unit, True or GATED_SILU: silu(gate) * up, GATED_RELU: max(gate, 0) * up; SQUARED_RELU: max(., 0)^2.
     `split_many` False: above 128 tokens k is never split (the consumer wants the finished product). With `pack`
@@ -547,7 +547,7 @@ def bound_gemm(w: torch.Tensor, silu=False, split_many: bool = True, pack: bool 
     keeps that copy (`.w`) and the caller lets go of its own. `.rows(a, b)` is the product with rows a..b-1 of
     the same weight, without a copy."""
     from . import gemm_select
-    return gemm_select.BoundGemm(w, silu, split_many, pack)
+    return gemm_select.BoundGemm(w, silu, split_many, pack, unit=unit or gemm_select.GatedUnit())
 
 
 def partial_capacity(max_rows: int, N: int, K: int, split_many: bool = True) -> int:
@@ -616,8 +616,8 @@ def glu_clamped(gate_up: torch.Tensor, out: torch.Tensor, limit: float, slope: f
          float(up_shift), _stream())
 
 
-# The epilogues of a product: 1, 2 act(gate) * up of a gated unit; 3 max(product, 0)^2.
-GATED_SILU, GATED_RELU, SQUARED_RELU = 1, 2, 3
+# The epilogues of a product: 1, 2, 4, 5, 6 a gated unit's (act(gate) * up, clamped, with biases: gemm_select.GatedUnit); 3 max(product, 0)^2.
+GATED_SILU, GATED_RELU, SQUARED_RELU, GATED_CLAMPED, GATED_BIASED_SILU, GATED_BIASED_GELU = 1, 2, 3, 4, 5, 6
 
 
 def sigmoid_gate_mul(y: torch.Tensor, gate: torch.Tensor) -> None:

@@ -204,12 +204,26 @@ def pair_width(M: int, N: int, K: int, pairs: int) -> int:
 
 
 def _gated(epilogue) -> bool:
-    """Whether an epilogue is that of a gated unit (1, 2): the output is half as wide as the product, and k stays whole."""
-    return int(epilogue) in (1, 2)
+    """Whether an epilogue is that of a gated unit: the output is half as wide as the product, and k stays whole."""
+    return int(epilogue) in (1, 2, 4, 5, 6)
+
+
+class GatedUnit:
+    """What a gated unit in a product's epilogue takes beside its code: the clamped unit's limit, slope and shift, the biases of
+    the biased ones (float32 [N / 2]), and how many columns stand behind the unit's in the output's rows, a one and zeros."""
+
+    def __init__(self, limit: float = 0.0, slope: float = 1.0, up_shift: float = 0.0, bias_gate=None, bias_up=None, ones: int = 0):
+        self.biases = (bias_gate, bias_up)               # (their memory)
+        self.ones = int(ones)
+        self.args = (0 if bias_gate is None else bias_gate.data_ptr(), 0 if bias_up is None else bias_up.data_ptr(), float(limit), float(slope),
+                     float(up_shift), self.ones)
+
+
+_PLAIN_UNIT = GatedUnit()
 
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None, bn=None, splits=None, scratch=None,
-            silu=False, partial_scratch=None, deep=None, pair=None, checked: bool = False):
+            silu=False, partial_scratch=None, deep=None, pair=None, checked: bool = False, unit: GatedUnit = _PLAIN_UNIT):
     """The tensor-core product; the tiling can be forced (tests). Returns `out`, or a SplitSum when
     `partial_scratch` is given and k is split."""
     global _ops
@@ -234,7 +248,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
         if splits > 1:
             scratch = partial_scratch(splits * M * N) if leave else scratch if scratch is not None else _scratch_for(splits * M * N, a.device)
         _call("tie_gemm_tc2", dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
-              w.stride(0), out.stride(0), int(silu), 0, 0, bn, t, splits, scratch.data_ptr() if splits > 1 else 0, 0 if leave else 1, _stream())
+              w.stride(0), out.stride(0), int(silu), 0, 0, bn, t, splits, scratch.data_ptr() if splits > 1 else 0, 0 if leave else 1, *unit.args, _stream())
         return SplitSum(scratch, _library().tie_gemm_tc_real_splits(K, splits), M, N) if leave else out
     t, b, s = plan(M, N, K)
     transposed = t if transposed is None else int(transposed)
@@ -251,7 +265,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
         scratch = _scratch_for(splits * M * N, a.device)
     _call("tie_gemm_tc", dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
           w.stride(0), out.stride(0), transposed, bn, splits, scratch.data_ptr() if splits > 1 else 0, int(silu),
-          0 if leave else 1, int(deep if deep is not None else (not transposed or bn >= 128)), 0, 0, _stream())
+          0 if leave else 1, int(deep if deep is not None else (not transposed or bn >= 128)), 0, 0, *unit.args, _stream())
     if leave:
         return SplitSum(scratch, _library().tie_gemm_tc_real_splits(K, splits), M, N)
     return out
@@ -281,12 +295,12 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, partial_scratch=No
     return out
 
 
-def gemm_silu(a: torch.Tensor, w_blocks: torch.Tensor, out: torch.Tensor, act: int = 1) -> None:
+def gemm_silu(a: torch.Tensor, w_blocks: torch.Tensor, out: torch.Tensor, act: int = 1, unit: GatedUnit = _PLAIN_UNIT) -> None:
     from . import _need
     _need(w_blocks.shape[0] % 32 == 0 and tc_takes(a, w_blocks, out),
           "gemm_silu: needs bfloat16 operands TMA can address and gate/up rows in blocks of 16")
     if a.shape[0] > 0:
-        gemm_tc(a, w_blocks, out, silu=act)
+        gemm_tc(a, w_blocks, out, silu=act, unit=unit)
 
 
 class BoundGemm:
@@ -301,8 +315,9 @@ class BoundGemm:
     [ceil(K / 64), rows, 64] and `packed_rows` its number of rows; `.rows(a, b)` gives the product with a slice of
     its rows (the q rows of a stacked q/k/v weight) over the same memory."""
 
-    def __init__(self, w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True, _slice=None):
-        self.silu, self.split_many = int(silu), split_many      # 0: none, 1: the SiLU, 2: the ReLU of a gated unit, 3: the squared ReLU
+    def __init__(self, w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True, _slice=None, unit: GatedUnit = _PLAIN_UNIT):
+        self.silu, self.split_many = int(silu), split_many      # 0: none, 3: the squared ReLU, else a gated unit
+        self.unit = unit
         self.gated = _gated(silu)
         if _slice is not None:              # rows [row0, row0 + N) of a packed weight
             parent, row0, n = _slice
@@ -343,7 +358,9 @@ class BoundGemm:
         else:
             t, bn, splits = plan(M, self.N, self.K, self.split_many)
         if self.gated:
-            splits = 1
+            # few tokens: k split like any product's, the unit formed where the sums are added (Dugazen's 12,288 columns at 8 tokens:
+            # 96 tiles; whole k 2.5 us slower than three splits, their sum and the unit in kernels of their own)
+            splits = splits if M <= PAIR_FROM else 1
             if not t:
                 bn = max(bn, 32)
         real = _library().tie_gemm_tc_real_splits(self.K, splits) if splits > 1 else 1
@@ -360,7 +377,7 @@ class BoundGemm:
                 and out.shape[0] == M and out.dtype in (torch.bfloat16, torch.float32)):
             w = self.row_major()
             if self.gated:
-                gemm_silu(a, w, out, self.silu)
+                gemm_silu(a, w, out, self.silu, self.unit)
                 return out
             if self.silu:                   # the squared ReLU behind whichever product takes the operands
                 from . import squared_relu
@@ -386,10 +403,11 @@ class BoundGemm:
             scratch = buf.data_ptr()
         if pair:
             _call("tie_gemm_tc2", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw,
-                  out.stride(0), self.silu, self.packed_rows, self.row0, bn, t, splits, scratch, 0 if leave else 1, _stream())
+                  out.stride(0), self.silu, self.packed_rows, self.row0, bn, t, splits, scratch, 0 if leave else 1,
+                  *self.unit.args, _stream())
         else:
             _call("tie_gemm_tc", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0),
-                  t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0, _stream())
+                  t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0, *self.unit.args, _stream())
         if leave:
             return SplitSum(buf, real, M, self.N)
         return out

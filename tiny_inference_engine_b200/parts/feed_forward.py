@@ -7,6 +7,7 @@ import torch
 
 from .. import ops
 from ..weights.loader import TensorNeed
+from ..ops.gemm_select import GatedUnit
 from .base import FeedForward, register_part, to_compute
 
 
@@ -85,17 +86,26 @@ class ClampedGLU(FeedForward):
 
     def bind(self, get):
         gate, up = (to_compute(get(n), self.dtype) for n in self.names[:2])
-        self.gate_up = ops.bound_gemm(torch.cat([gate, up], dim=0).contiguous(), split_many=False)
+        # as in SwiGLU: on the tensor-core path the unit is the product's epilogue
+        self.fused = self.dtype == torch.bfloat16 and self.inter % 16 == 0 and self.hidden % 8 == 0
+        if self.fused:
+            self.gate_up = ops.bound_gemm(ops.interleave_gate_up(gate, up), silu=ops.GATED_CLAMPED,
+                                          unit=GatedUnit(self.limit, self.slope, self.up_shift))
+        else:
+            self.gate_up = ops.bound_gemm(torch.cat([gate, up], dim=0).contiguous(), split_many=False)
         del gate, up
         self.down = ops.bound_gemm(to_compute(get(self.names[2]), self.dtype).contiguous())
         self.w_gate_up, self.w_down = self.gate_up.w, self.down.w
 
     def forward(self, h, ctx):
         T = h.shape[0]
-        gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
-        self.gate_up(h, gu)
         act = ctx.ws.rows("ffn.act", T, self.inter, self.dtype)
-        ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
+        if self.fused:
+            self.gate_up(h, act)
+        else:
+            gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
+            self.gate_up(h, gu)
+            ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
         out = ctx.ws.rows("ffn.out", T, self.hidden, self.dtype)
         if self._partial_capacity is None:
             self._partial_capacity = ops.partial_capacity(ctx.ws.max_rows, self.down.N, self.down.K)
@@ -104,13 +114,14 @@ class ClampedGLU(FeedForward):
 
 class BiasedGLU(FeedForward):
     """A gated unit whose three products have biases: down(act(gate(h) + b_gate) * (up(h) + b_up)) + b_down, with `act`
-    "silu" or "gelu_tanh" (0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))). Gate and up are one stacked product; their
-    biases and the activation are one float kernel behind it. The down bias rides in the product: the unit's output
+    "silu" or "gelu_tanh" (0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))). Gate and up are one product; their
+    biases and the activation are its epilogue, or one float kernel behind it. The down bias rides in the product: the unit's output
     gets a column of ones (and zeros up to a multiple of 8) and the weight the bias as that column, so it is added
     inside the float accumulator and split products still hand on partial sums. params: `hidden_size`,
     `intermediate_size`, `activation`, and the tensors' names (`gate`, `up`, `down`; biases `<name>.b`) after `prefix`."""
     launches_only = False
     ACTIVATIONS = {"silu": ops.ACT_SILU, "gelu_tanh": ops.ACT_GELU_TANH}
+    EPILOGUES = {ops.ACT_SILU: ops.GATED_BIASED_SILU, ops.ACT_GELU_TANH: ops.GATED_BIASED_GELU}
 
     def __init__(self, spec, dtype, prefix: str = ""):
         p = spec.params
@@ -135,7 +146,13 @@ class BiasedGLU(FeedForward):
     def bind(self, get):
         g, u, d = self.names
         gate, up = (to_compute(get(n), self.dtype) for n in (g, u))
-        self.gate_up = ops.bound_gemm(torch.cat([gate, up], dim=0).contiguous(), split_many=False)
+        self.bias_gate, self.bias_up = (get(n + ".b").to(torch.float32).contiguous() for n in (g, u))
+        self.fused = self.dtype == torch.bfloat16 and self.inter % 16 == 0 and self.hidden % 8 == 0
+        if self.fused:
+            self.gate_up = ops.bound_gemm(ops.interleave_gate_up(gate, up), silu=self.EPILOGUES[self.act],
+                                          unit=GatedUnit(bias_gate=self.bias_gate, bias_up=self.bias_up, ones=self.padded - self.inter))
+        else:
+            self.gate_up = ops.bound_gemm(torch.cat([gate, up], dim=0).contiguous(), split_many=False)
         del gate, up
         down = to_compute(get(d), self.dtype)
         wide = torch.zeros((self.hidden, self.padded), dtype=self.dtype, device=down.device)
@@ -143,14 +160,16 @@ class BiasedGLU(FeedForward):
         wide[:, self.inter] = to_compute(get(d + ".b"), self.dtype)
         self.down = ops.bound_gemm(wide)
         self.w_gate_up, self.w_down = self.gate_up.w, self.down.w
-        self.bias_gate, self.bias_up = (get(n + ".b").to(torch.float32).contiguous() for n in (g, u))
 
     def forward(self, h, ctx):
         T = h.shape[0]
-        gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
-        self.gate_up(h, gu)
         act = ctx.ws.rows("ffn.act1", T, self.padded, self.dtype)
-        ops.glu_biased(gu, self.bias_gate, self.bias_up, act, self.act)
+        if self.fused:
+            self.gate_up(h, act[:, :self.inter])
+        else:
+            gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
+            self.gate_up(h, gu)
+            ops.glu_biased(gu, self.bias_gate, self.bias_up, act, self.act)
         out = ctx.ws.rows("ffn.out", T, self.hidden, self.dtype)
         if self._partial_capacity is None:
             self._partial_capacity = ops.partial_capacity(ctx.ws.max_rows, self.down.N, self.down.K)
