@@ -103,6 +103,9 @@ struct PairArgs {
   int epilogue, by_tma;    // by_tma: a tensor map describes the output (or the sums), else rows are stored element by element
   int w_rows, w_row0;
   GatedUnit unit;
+  // Grouped (tokens on the row side, k whole): x is group_meta[0] tiles of 256 rows, fewer than the grid was sized for, and row tile t
+  // multiplies the rows_y weight rows of group group_of_tile[t], one group's behind the other's in y. Null: one product.
+  const int *group_meta, *group_of_tile;
   int* status;
 };
 
@@ -185,6 +188,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_holder;
   pdl_wait();
+  int tiles_x = g.tiles_x, n_tiles = g.n_tiles, n_work = g.n_work;
+  if (g.group_meta != nullptr) {
+    const int tiles_y = n_tiles / tiles_x;
+    tiles_x = g.group_meta[0];
+    n_tiles = n_work = tiles_x * tiles_y;
+  }
 
   if (warp == k2EpilogueWarps) {
     // ---- TMA producer (both CTAs): own 128 rows of x, own half of the tile's rows of y; bytes count on the leader's
@@ -194,10 +203,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     bool ok = true;
     const uint32_t both = 2 * stage_bytes;
     const int x_blocks = g.transposed ? g.w_rows : 0, y_blocks = g.transposed ? 0 : g.w_rows;   // rows of an operand in k-blocks, else 0
-    for (int work = pair; work < g.n_work && ok; work += pairs) {
-      const int tile = work % g.n_tiles, z = work / g.n_tiles;
-      const int row_x = (tile % g.tiles_x) * 256 + static_cast<int>(rank) * 128 + (x_blocks ? g.w_row0 : 0);
-      const int row_y = (tile / g.tiles_x) * bn + static_cast<int>(rank) * (bn / 2) + (y_blocks ? g.w_row0 : 0);
+    for (int work = pair; work < n_work && ok; work += pairs) {
+      const int tile = work % n_tiles, z = work / n_tiles;
+      const int row_x = (tile % tiles_x) * 256 + static_cast<int>(rank) * 128 + (x_blocks ? g.w_row0 : 0);
+      const int row_y = (tile / tiles_x) * bn + static_cast<int>(rank) * (bn / 2) + (y_blocks ? g.w_row0 : 0) +
+                        (g.group_of_tile != nullptr ? g.group_of_tile[tile % tiles_x] * g.rows_y : 0);
       const int kb_end = min(g.k_blocks, (z + 1) * g.k_blocks_per_split);
       for (int kb = z * g.k_blocks_per_split; kb < kb_end; ++kb) {
         if (!__all_sync(0xffffffffu, mbar_wait(empty + s, parity, abort_flag, status, 1) ? 1 : 0)) {
@@ -226,8 +236,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       int s = 0, local = 0;
       uint32_t parity = 0;
       bool ok = true;
-      for (int work = pair; work < g.n_work && ok; work += pairs, ++local) {
-        const int buf = local & 1, z = work / g.n_tiles;
+      for (int work = pair; work < n_work && ok; work += pairs, ++local) {
+        const int buf = local & 1, z = work / n_tiles;
         const int kb_begin = z * g.k_blocks_per_split, kb_end = min(g.k_blocks, kb_begin + g.k_blocks_per_split);
         if (!__all_sync(0xffffffffu, mbar_wait(acc_empty + buf, ((local >> 1) & 1) ^ 1, abort_flag, status, 2) ? 1 : 0)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -264,17 +274,17 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const bool gated = gated_epilogue(g.epilogue);
     const bool squared = g.epilogue == kEpilogueSquaredRelu && g.partial == nullptr;
     int local = 0;
-    for (int work = pair; work < g.n_work; work += pairs, ++local) {
+    for (int work = pair; work < n_work; work += pairs, ++local) {
       const int buf = local & 1;
-      const int tile = work % g.n_tiles, z = work / g.n_tiles;
-      const int i0 = (tile % g.tiles_x) * 256 + static_cast<int>(rank) * 128, j0 = (tile / g.tiles_x) * bn;
+      const int tile = work % n_tiles, z = work / n_tiles;
+      const int i0 = (tile % tiles_x) * 256 + static_cast<int>(rank) * 128, j0 = (tile / tiles_x) * bn;
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full + buf, (local >> 1) & 1, abort_flag, status, 3) ? 1 : 0)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + buf * 256 + (static_cast<uint32_t>(quarter * 32) << 16);
       // This warp has read its last columns of the accumulator: the leader's MMA thread may reuse it once all have. Told
       // before the rows are stored: the arrive waits for stores ahead of it.
       // The last tile's need not be told.
-      const bool last = work + pairs >= g.n_work;
+      const bool last = work + pairs >= n_work;
       bool released = last;
       auto release = [&] {
         if (released) return;
@@ -571,4 +581,47 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   if (st != kOk) return st;
   if (scratch != nullptr && reduce) launch_splitk_reduce(out_dtype, scratch, g.part_stride, real, out, ldo, N, g.part_stride, silu, s);
   TIE_RETURN_LAUNCH("gemm_tc2");
+}
+
+// Grouped product: a [M_cap, K] holds `meta[0]` tiles of 256 rows (M_cap is what the buffers were sized for); tile t multiplies the N weight
+// rows of group `group_of_tile[t]`, and out[M_cap, N] (or, with a gated unit's epilogue, out[M_cap, N / 2]) gets the rows in the same order. w
+// is stored in k-blocks, [ceil(K / 64)][w_rows][64], group g's rows at g * N .. g * N + N - 1 (w_rows = groups * N). meta and group_of_tile
+// live on the device and may be written by the kernel right ahead of this one. (On single SMs, tiles of 128 rows, 6,124 pairs over 32
+// experts of 3,072 x 2,048 took 130 us.)
+TIE_API int tie_gemm_tc2_grouped(int out_dtype, const void* a, const void* w, void* out, int M_cap, int N, int K, long long lda, long long ldo,
+                                 int w_rows, int epilogue, float limit, float slope, float up_shift, const int* meta, const int* group_of_tile,
+                                 cudaStream_t s) {
+  TIE_REQUIRE(M_cap > 0 && M_cap % 256 == 0 && N > 0 && K > 0, "gemm_tc2_grouped: bad sizes M=%d (whole tiles of 256) N=%d K=%d", M_cap, N, K);
+  TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && w_rows >= N && w_rows % N == 0, "gemm_tc2_grouped: K=%d, lda and the weight's %d rows", K, w_rows);
+  TIE_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0, "gemm_tc2_grouped: operands must be 16-byte aligned");
+  TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc2_grouped: output dtype code %d", out_dtype);
+  TIE_REQUIRE((epilogue == 0 || epilogue == kEpilogueClamped) && (epilogue == 0 || N % 32 == 0), "gemm_tc2_grouped: epilogue %d (N=%d)", epilogue, N);
+  TIE_REQUIRE(meta != nullptr && group_of_tile != nullptr && status_word() != nullptr, "gemm_tc2_grouped: no tile list");
+  PairArgs g = {};
+  g.rows_x = M_cap;
+  g.rows_y = N;
+  g.bn = N >= 256 ? 256 : ceil_div(N, 32) * 32;
+  const int stage = k2StageX + (g.bn / 2) * k2BK * 2;
+  g.stages = k2Ring / stage < k2MaxStages ? k2Ring / stage : k2MaxStages;
+  g.k_blocks = g.k_blocks_per_split = ceil_div(K, k2BK);
+  g.tiles_x = M_cap / 256;
+  g.n_tiles = g.n_work = g.tiles_x * ceil_div(N, g.bn);
+  g.out = out;
+  g.ldo = ldo;
+  g.epilogue = epilogue;
+  g.w_rows = w_rows;
+  g.unit = GatedUnit{nullptr, nullptr, limit, slope, up_shift, 0};
+  g.group_meta = meta;
+  g.group_of_tile = group_of_tile;
+  g.status = status_word();
+  CUtensorMap ma, mw, mo;
+  TIE_REQUIRE(make_map_bf16(&ma, a, M_cap, K, lda, k2BK, 128) &&
+                  make_map_bf16(&mw, w, static_cast<long long>(g.k_blocks) * w_rows, k2BK, k2BK, k2BK, g.bn / 2),
+              "gemm_tc2_grouped: cuTensorMapEncodeTiled failed (rows %d, K %d)", M_cap, K);
+  const bool as_float = out_dtype == TIE_F32;
+  g.by_tma = make_map_rows(&mo, out, as_float, M_cap, epilogue ? N / 2 : N, ldo, 1, 32, 32);
+  if (!g.by_tma) mo = ma;
+  const int st = as_float ? launch_tc2<float>(ma, mw, mo, g, s) : launch_tc2<__nv_bfloat16>(ma, mw, mo, g, s);
+  if (st != kOk) return st;
+  TIE_RETURN_LAUNCH("gemm_tc2_grouped");
 }

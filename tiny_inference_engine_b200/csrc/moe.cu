@@ -13,7 +13,7 @@
 //               expert's weight rows are streamed once, a warp per output column (row-major weights, 4 pairs) or per
 //               sixteen (bfloat16 weights in k-blocks, on the tensor cores).
 //   moe_gather, moe_combine   for prompts in bfloat16: rows copied into the listed order ahead of the grouped products
-//               on the tensor cores (gemm_tc.cu, tiles of 128 rows), and the weighted results back to their tokens.
+//               on the tensor cores (gemm_tc2.cu, tiles of 256 rows), and the weighted results back to their tokens.
 //   moe_gemm    grouped products on the CUDA cores, one block per (tile of rows, 64 output columns): rows are
 //               gathered through the list, weights are the tile's expert's. `first` reads token rows and writes a
 //               row per pair; `second` reads a row per pair and writes weight * result as the pair's choice-th
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(256, 3) moe_mma_blocks_kernel(const __nv_bfloa
                                                                float* __restrict__ partial, long long part_stride,
                                                                const float* __restrict__ weights, const int* __restrict__ sorted,
                                                                const int* __restrict__ tile_expert, const int* __restrict__ meta,
-                                                               int block_m, int top, int N, int K, ClampedUnit unit) {
+                                                               int block_m, int top, int N, int K, int interleaved, ClampedUnit unit) {
   pdl_sync();
   const int tile = blockIdx.y;
   if (tile >= meta[0]) return;
@@ -370,8 +370,10 @@ __global__ void __launch_bounds__(256, 3) moe_mma_blocks_kernel(const __nv_bfloa
   const int last = N - 1, expert = tile_expert[tile];
   // rows beyond the last are read as the last and not written
   const long long base = static_cast<long long>(expert) * (KIND == 1 ? 2 * N : N);
-  const __nv_bfloat16* w0 = w + (base + min(n0 + g, last)) * 64 + tq * 8;
-  const __nv_bfloat16* w1 = w + (base + (KIND == 1 ? N + min(n0 + g, last) : min(n0 + g + 8, last))) * 64 + tq * 8;
+  // an expert's gate rows, then its up rows, or (interleaved) blocks of sixteen of either
+  const int r0_at = min(n0 + g, last), gate_at = interleaved ? (r0_at >> 4) * 32 + (r0_at & 15) : r0_at;
+  const __nv_bfloat16* w0 = w + (base + (KIND == 1 ? gate_at : r0_at)) * 64 + tq * 8;
+  const __nv_bfloat16* w1 = w + (base + (KIND == 1 ? gate_at + (interleaved ? 16 : N) : min(n0 + g + 8, last))) * 64 + tq * 8;
   const int pair = g < block_m ? sorted[tile * block_m + g] : -1;
   const __nv_bfloat16* x = pair < 0 ? nullptr : a + static_cast<long long>(KIND == 2 ? pair : pair / top) * lda + tq * 8;
   const long long kb_stride = static_cast<long long>(w_rows) * 64;
@@ -456,7 +458,7 @@ TIE_API int tie_moe_route(const float* logits, long long ld_logits, int tokens, 
 
 TIE_API int tie_moe_align(const int* ids, int pairs, int experts, int block_m, int* sorted, int* tile_expert, int* meta,
                           cudaStream_t s) {
-  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 8 || block_m == 16 || block_m == 64 || block_m == 128),
+  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 8 || block_m == 16 || block_m == 64 || block_m == 256),
               "moe_align: bad sizes experts=%d block_m=%d", experts, block_m);
   if (pairs <= 0) return kOk;
   TIE_LAUNCH(moe_align_kernel, 1, 1024, 2 * experts * sizeof(int), s, ids, pairs, experts, block_m, sorted, tile_expert, meta);
@@ -481,10 +483,10 @@ static int launch_moe_gemm(int second, int block_m, const void* a, long long lda
       __nv_bfloat16* op = static_cast<__nv_bfloat16*>(out);
       if (second)
         TIE_LAUNCH((moe_mma_blocks_kernel<2>), grid, 256, 0, s, ap, lda, wp, w_rows, op, ldo, partial, part_stride, weights, sorted, tile_expert,
-                   meta, block_m, top, N, K, ClampedUnit{});
+                   meta, block_m, top, N, K, 0, ClampedUnit{});
       else
         TIE_LAUNCH((moe_mma_blocks_kernel<0>), grid, 256, 0, s, ap, lda, wp, w_rows, op, ldo, partial, part_stride, weights, sorted, tile_expert,
-                   meta, block_m, top, N, K, ClampedUnit{});
+                   meta, block_m, top, N, K, 0, ClampedUnit{});
       TIE_RETURN_LAUNCH("moe_mma_blocks");
     } else {
       set_error("moe_gemm: weights in k-blocks are bfloat16");
@@ -549,7 +551,8 @@ TIE_API int tie_moe_gemm(int dtype, int second, int block_m, const void* a, long
 // out[pair, :inter] = unit(gate, up) of a[pair / top]. Tiles of 4 or 8 pairs.
 TIE_API int tie_moe_gemm_glu(int block_m, const void* a, long long lda, const void* w, int w_rows, void* out, long long ldo, const int* sorted,
                              const int* tile_expert, const int* meta, int max_tiles, int top, int inter, int K, float limit, float slope,
-                             float up_shift, cudaStream_t s) {
+                             float up_shift, int interleaved, cudaStream_t s) {
+  TIE_REQUIRE(!interleaved || inter % 16 == 0, "moe_gemm_glu: %d gate rows in blocks of sixteen", inter);
   TIE_REQUIRE(inter > 0 && K > 0 && top > 0 && (block_m == 4 || block_m == 8) && max_tiles >= 0 && max_tiles <= 65535 && w_rows % (2 * inter) == 0,
               "moe_gemm_glu: bad sizes inter=%d K=%d top=%d block_m=%d tiles=%d", inter, K, top, block_m, max_tiles);
   TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0,
@@ -557,6 +560,6 @@ TIE_API int tie_moe_gemm_glu(int block_m, const void* a, long long lda, const vo
   if (max_tiles == 0) return kOk;
   TIE_LAUNCH((moe_mma_blocks_kernel<1>), dim3(ceil_div(inter, 64), max_tiles), 256, 0, s, static_cast<const __nv_bfloat16*>(a), lda,
              static_cast<const __nv_bfloat16*>(w), w_rows, static_cast<__nv_bfloat16*>(out), ldo, nullptr, 0, nullptr, sorted, tile_expert, meta,
-             block_m, top, inter, K, ClampedUnit{limit, slope, up_shift});
+             block_m, top, inter, K, interleaved, ClampedUnit{limit, slope, up_shift});
   TIE_RETURN_LAUNCH("moe_gemm_glu");
 }

@@ -1171,7 +1171,8 @@ def moe_gemm(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, meta,
 
 
 def moe_gemm_glu(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, meta, max_tiles: int, inter: int, limit: float, slope: float,
-                 up_shift: float) -> None:
+                 up_shift: float,
+                 interleaved: bool = False) -> None:
     """The first product and the clamped gated unit behind it (`glu_clamped`) in one: a [T, K] bfloat16, w every expert's `inter` gate and
     `inter` up rows in k-blocks, out [T * top, inter]. The unit works on the float sums. Tiles of 4 or 8 pairs."""
     _dev(a, w, out, sorted_pairs, tile_expert, meta)
@@ -1180,10 +1181,10 @@ def moe_gemm_glu(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, m
           a.stride(1) == 1 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.stride(1) == 1 and
           out.shape == (a.shape[0] * top, inter), "moe_gemm_glu: bfloat16 a [T, K], w in k-blocks, out [T * top, inter]")
     call("tie_moe_gemm_glu", block_m, a.data_ptr(), a.stride(0), w.data_ptr(), w.shape[1], out.data_ptr(), out.stride(0), sorted_pairs.data_ptr(),
-         tile_expert.data_ptr(), meta.data_ptr(), max_tiles, top, inter, K, float(limit), float(slope), float(up_shift), _stream())
+         tile_expert.data_ptr(), meta.data_ptr(), max_tiles, top, inter, K, float(limit), float(slope), float(up_shift), int(interleaved), _stream())
 
 
-GROUPED_TILE = 128      # rows of a tile of the grouped product on the tensor cores
+GROUPED_TILE = 256      # rows of a tile of the grouped product on the tensor cores (a pair of SMs)
 
 
 def moe_gather(h, sorted_pairs, meta, top: int, out) -> None:
@@ -1210,18 +1211,20 @@ def gemm_grouped_takes(rows: int, N: int, K: int) -> bool:
     return K % 8 == 0 and N % 8 == 0 and rows % GROUPED_TILE == 0
 
 
-def gemm_grouped(a, w_blocks, out, N: int, K: int, meta, tile_group) -> None:
+def gemm_grouped(a, w_blocks, out, N: int, K: int, meta, tile_group, clamped=None) -> None:
     """out[r, :N] = w[group of r's tile] a[r] for the first meta[0] tiles of GROUPED_TILE rows of a; `w_blocks` is the
-    groups' weights one after the other, [groups * N, K], stored in k-blocks (`pack_k_blocks`)."""
+    groups' weights one after the other, [groups * N, K], stored in k-blocks (`pack_k_blocks`). `clamped`: (limit, slope, up_shift) of the
+    clamped gated unit on top (`glu_clamped`); a group's rows are then blocks of 16 gate and 16 up rows and out is [rows, N / 2]."""
     _dev(a, w_blocks, out, meta, tile_group)
     _need(a.dim() == 2 and a.stride(1) == 1 and a.shape[1] == K and a.dtype == torch.bfloat16 and a.shape[0] % GROUPED_TILE == 0,
           "gemm_grouped: a must be bfloat16 [whole tiles, K]")
     _need(w_blocks.dim() == 3 and w_blocks.is_contiguous() and w_blocks.shape[2] == 64 and w_blocks.shape[0] == (K + 63) // 64 and
           w_blocks.shape[1] % N == 0 and w_blocks.dtype == torch.bfloat16, "gemm_grouped: weights must be k-blocks of [groups * N, K]")
-    _need(out.dim() == 2 and out.stride(1) == 1 and out.shape == (a.shape[0], N), "gemm_grouped: out must be [rows, N]")
-    bn = 256 if N >= 256 else 128
-    call("tie_gemm_tc_grouped", dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(), a.shape[0], N, K, a.stride(0),
-         out.stride(0), bn, w_blocks.shape[1], meta.data_ptr(), tile_group.data_ptr(), _stream())
+    _need(out.dim() == 2 and out.stride(1) == 1 and out.shape == (a.shape[0], N if clamped is None else N // 2), "gemm_grouped: out must be [rows, N]")
+    limit, slope, up_shift = clamped if clamped is not None else (0.0, 1.0, 0.0)
+    call("tie_gemm_tc2_grouped", dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(), a.shape[0], N, K, a.stride(0), out.stride(0),
+         w_blocks.shape[1], 0 if clamped is None else GATED_CLAMPED, float(limit), float(slope), float(up_shift), meta.data_ptr(),
+         tile_group.data_ptr(), _stream())
 
 
 # -- layers whose sublayers read the stream side by side, and what stands around them (csrc/parallel_layer.cu)

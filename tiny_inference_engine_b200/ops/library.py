@@ -71,12 +71,12 @@ _SIGNATURES = {
     "tie_glu_biased": [I, P, P, P, P, I, I, I, I, P],
     "tie_moe_route": [P, L, I, I, I, I, I, I, P, I, I, F, P, P, P, P],
     "tie_moe_align": [P, I, I, I, P, P, P, P],
-    "tie_moe_gemm_glu": [I, P, L, P, I, P, L, P, P, P, I, I, I, I, F, F, F, P],
+    "tie_moe_gemm_glu": [I, P, L, P, I, P, L, P, P, P, I, I, I, I, F, F, F, I, P],
     "tie_moe_gemm": [I, I, I, P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, P],
     "tie_moe_gather": [I, P, L, P, P, I, I, P, I, I, P],
     "tie_moe_combine": [I, P, P, P, I, I, P, P, L, I, I, P],
     "tie_gemm_heads_mma": [P, L, I, P, P, L, I, I, I, I, I, P],
-    "tie_gemm_tc_grouped": [I, P, P, P, I, I, I, L, L, I, I, P, P, P],
+    "tie_gemm_tc2_grouped": [I, P, P, P, I, I, I, L, L, I, I, F, F, F, P, P, P],
     "tie_pair_hash_add": [I, P, P, P, P, P, P, P, P, I, L, L, I, I, P],
     "tie_add_row_vector": [P, P, I, I, P],
     "tie_group_norm_taps": [I, P, P, P, L, I, P, I, I, I, F, P, P, P, P, I, P, P, P, P, P, P, P, P, P, I, P],

@@ -88,10 +88,13 @@ class RoutedExperts(FeedForward):
             self.correction = get(self.prefix + "correction").to(torch.float32).contiguous()
         if self.has_router_bias:
             self.router_bias = get(self.prefix + "router.b").to(torch.float32).contiguous()
-        # [experts, 2 * inter, hidden]: an expert's gate rows, then its up rows; [experts, hidden, inter]
-        w_gate_up = torch.stack([torch.cat([to_compute(get(self._expert(e, "gate")), self.dtype),
-                                            to_compute(get(self._expert(e, "up")), self.dtype)], dim=0) for e in range(E)]).contiguous()
+        # [experts, 2 * inter, hidden]: an expert's gate rows, then its up rows (or blocks of 16 of either, where the unit is the
+        # epilogue of the grouped product); [experts, hidden, inter]
         w_down = torch.stack([to_compute(get(self._expert(e, "down")), self.dtype) for e in range(E)]).contiguous()
+        self.fused = self.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 16 == 0 and w_down.is_cuda
+        pair = ops.interleave_gate_up if self.fused else (lambda gate, up: torch.cat([gate, up], dim=0))
+        w_gate_up = torch.stack([pair(to_compute(get(self._expert(e, "gate")), self.dtype), to_compute(get(self._expert(e, "up")), self.dtype))
+                                 for e in range(E)]).contiguous()
         # bfloat16 with sizes in whole 16-byte vectors: the experts' rows one after the other in k-blocks, the layout
         # that the tensor-core product streams (prompts) and that the few-rows kernel reads as well (decode)
         self.in_blocks = self.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0 and w_down.is_cuda
@@ -122,7 +125,7 @@ class RoutedExperts(FeedForward):
             block_m = 16 if pairs <= 16 * E else 64
         rows_cap = ctx.ws.max_rows * top
         tiles_cap = max(ops.moe_max_tiles(rows_cap, E, 4), 1)
-        sorted_pairs = ctx.ws.flat("moe.sorted", max(ops.moe_max_tiles(rows_cap, E, m) * m for m in (4, 8, 16, 64, 128)), torch.int32)
+        sorted_pairs = ctx.ws.flat("moe.sorted", max(ops.moe_max_tiles(rows_cap, E, m) * m for m in (4, 8, 16, 64, ops.GROUPED_TILE)), torch.int32)
         tile_expert = ctx.ws.flat("moe.tile_expert", tiles_cap, torch.int32)
         meta = ctx.ws.flat("moe.meta", 4, torch.int32)
         ops.moe_align(ids, E, block_m, sorted_pairs, tile_expert, meta)
@@ -135,17 +138,21 @@ class RoutedExperts(FeedForward):
             cap = ops.moe_max_tiles(rows_cap, E, block_m) * block_m
             xs = ctx.ws.flat("moe.listed", cap * D, self.dtype)[:rows * D].view(rows, D)
             ops.moe_gather(h, sorted_pairs, meta, top, xs)
-            gu = ctx.ws.flat("moe.listed.gate_up", cap * 2 * I, self.dtype)[:rows * 2 * I].view(rows, 2 * I)
-            ops.gemm_grouped(xs, self.w_gate_up, gu, 2 * I, D, meta, tile_expert)
             act = ctx.ws.flat("moe.listed.act", cap * I, self.dtype)[:rows * I].view(rows, I)
-            ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
+            if self.fused:
+                ops.gemm_grouped(xs, self.w_gate_up, act, 2 * I, D, meta, tile_expert, clamped=(self.limit, self.slope, self.up_shift))
+            else:
+                gu = ctx.ws.flat("moe.listed.gate_up", cap * 2 * I, self.dtype)[:rows * 2 * I].view(rows, 2 * I)
+                ops.gemm_grouped(xs, self.w_gate_up, gu, 2 * I, D, meta, tile_expert)
+                ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
             y = xs                                          # the listed inputs are done with
             ops.gemm_grouped(act, self.w_down, y, D, I, meta, tile_expert)
             ops.moe_combine(y, sorted_pairs, meta, top, weights.view(-1), partial, T)
             return ops.SplitSum(partial, top, T, D)
         act = ctx.ws.rows("moe.act", T, top * I, self.dtype).view(pairs, I)
         if self.in_blocks:
-            ops.moe_gemm_glu(h, self.w_gate_up, act, top, block_m, sorted_pairs, tile_expert, meta, max_tiles, I, self.limit, self.slope, self.up_shift)
+            ops.moe_gemm_glu(h, self.w_gate_up, act, top, block_m, sorted_pairs, tile_expert, meta, max_tiles, I, self.limit, self.slope, self.up_shift,
+                             interleaved=self.fused)
         else:
             gu = ctx.ws.rows("moe.gate_up", T, top * 2 * I, self.dtype).view(pairs, 2 * I)
             ops.moe_gemm(h, self.w_gate_up, gu, top, block_m, sorted_pairs, tile_expert, meta, max_tiles)
