@@ -606,8 +606,7 @@ def test_pair_kernel_on_either_side_and_with_split_k(ops, M, N, K, transposed, b
         wide = torch.full((M, N + 16), 7.0, device="cuda", dtype=dtype)
         scratch = torch.full((splits * M * N + 16,), float("nan"), device="cuda")
         gemm_select._call("tie_gemm_tc2", int(dtype == torch.bfloat16), ta.data_ptr(), tw.data_ptr(), wide[:, offset:].data_ptr(), M, N, K, K, K,
-                          N + 16, 0, 0, 0, bn, transposed, splits, scratch.data_ptr(), 1, 0, 0, 0.0, 1.0, 0.0, 0,
-                          torch.cuda.current_stream().cuda_stream)
+                          N + 16, 0, 0, 0, bn, transposed, splits, scratch.data_ptr(), 1, torch.cuda.current_stream().cuda_stream)
         torch.cuda.synchronize()
         gemm_select.check_status()
         assert rel_err(host(wide[:, offset:offset + N]), want) < (TOL["bfloat16"] if dtype == torch.bfloat16 else 2e-5), (dtype, offset)
@@ -633,7 +632,7 @@ def test_silu_epilogue_from_the_smallest_to_the_largest_gates(ops, transposed):
     out = torch.full((M, I), float("nan"), device="cuda")
     w = ops.interleave_gate_up(gate.cuda(), up.cuda())
     gemm_select._call("tie_gemm_tc2", 0, a.cuda().data_ptr(), w.data_ptr(), out.data_ptr(), M, 2 * I, K, K, K, I, 1, 0, 0, 128 if transposed else 64,
-                      transposed, 1, 0, 1, 0, 0, 0.0, 1.0, 0.0, 0, torch.cuda.current_stream().cuda_stream)
+                      transposed, 1, 0, 1, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     gemm_select.check_status()
     g = a[:, 0].double()

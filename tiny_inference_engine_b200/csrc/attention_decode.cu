@@ -44,6 +44,8 @@ struct DecodeArgs {
   int* status;
   long long q_stride;
   int max_blocks, q_heads, kv_heads, page_size, page_shift, window, split_keys, max_splits;
+  int heads_first;       // a sequence's heads start together (grid x): with more CTAs than places and the longest contexts first in the list,
+                         // the last to start are the shortest; else the sequences of a head do (a step of one request 0.7 % faster)
   int exact_weights;     // != 0: the softmax weights enter the value product as two bfloat16 terms (pv_tile)
   float scale_log2;
   // Only for the kernel that prepares its heads itself (PREP): the output of the q/k/v product, [T, (q_heads + 2 kv_heads)
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(kDecThreads) attn_decode_tma_kernel(const __gr
   [[maybe_unused]] float* inbox = reinterpret_cast<float*>(flags + 4) + (PREP ? 2 * DH : 0);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int li = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+  const int li = a.heads_first ? blockIdx.y : blockIdx.x, kvh = a.heads_first ? blockIdx.x : blockIdx.y, split = blockIdx.z;
   const int seq = a.seq_list ? a.seq_list[li] : a.seq_first + li;
   const int G = a.q_heads / a.kv_heads;
   // Without a window a split's first key does not depend on the context length: the page ids of all the boxes the
@@ -526,7 +528,7 @@ static int launch_decode_tma(const CUtensorMap& km, const CUtensorMap& vm, const
   }
   if constexpr (CLUSTER) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_list, a.kv_heads, a.max_splits);
+    cfg.gridDim = a.heads_first ? dim3(a.kv_heads, n_list, a.max_splits) : dim3(n_list, a.kv_heads, a.max_splits);
     cfg.blockDim = dim3(kDecThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -554,7 +556,7 @@ static int launch_decode_tma(const CUtensorMap& km, const CUtensorMap& vm, const
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, km, vm, a);
   } else {
-    TIE_LAUNCH(kernel, dim3(n_list, a.kv_heads, a.max_splits), kDecThreads, smem, s, km, vm, a);
+    TIE_LAUNCH(kernel, a.heads_first ? dim3(a.kv_heads, n_list, a.max_splits) : dim3(n_list, a.kv_heads, a.max_splits), kDecThreads, smem, s, km, vm, a);
   }
   return kOk;
 }
@@ -594,6 +596,7 @@ static int decode_tma(DecodeArgs a, bool prep, bool cluster, const void* k_cache
   a.status = status_word();
   a.page_shift = shift;
   a.scale_log2 = scale * 1.4426950408889634f;
+  a.heads_first = static_cast<long long>(n_list) * kv_heads * max_splits > 2 * 148 && n_list <= 65535;
   // cluster: the splits of a sequence and kv head as one thread-block cluster (2, 4, 8 or 16 CTAs), which merges them
   // through shared memory. The caller asks for it where every CTA of the launch is resident at once (a split without
   // keys holds its place until its cluster is through). Else, or with TIE_NO_CLUSTER_ATTENTION=1: through scratch

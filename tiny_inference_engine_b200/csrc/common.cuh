@@ -138,6 +138,9 @@ __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 
+// The activation of a gated product's epilogue: 1 the SiLU, 2 the ReLU.
+__device__ __forceinline__ float gate_act(float g, int act) { return act == 2 ? fmaxf(g, 0.0f) : silu(g); }
+
 // A gated unit in a product's epilogue (the weight's rows in blocks of 16 gate and 16 up rows; the output half as wide): 1 SiLU(g) u,
 // 2 ReLU(g) u, 4 the clamped unit g' sigmoid(slope g') (u' + up_shift) with g' = min(g, limit), u' = clamp(u, +-limit), 5 and 6 SiLU or the
 // tanh form of GELU of g + bias_gate, times u + bias_up. `ones` > 0: that many more columns behind the unit's, a one and zeros (for a
@@ -150,16 +153,13 @@ struct GatedUnit {
 };
 __host__ __device__ constexpr bool gated_epilogue(int e) { return e != 0 && e != kEpilogueSquaredRelu; }
 // N of them at once, the kind of unit chosen outside the loop: g and u as their bits, bias_gate and bias_up the biases of the first (of all of
-// them with `same`: N rows of one output column).
-template <int N, bool same = false>
+// them with `same`: N rows of one output column). all: every kind, else the SiLU and the ReLU only (fewer registers).
+template <int N, bool same, bool all>
 __device__ __forceinline__ void gated_values(const uint32_t* g, const uint32_t* u, float (&v)[N], int act, const GatedUnit& unit,
                                              const float* bias_gate, const float* bias_up) {
-  if (act == 1) {
+  if (!all || act <= 2) {
 #pragma unroll
-    for (int e = 0; e < N; ++e) v[e] = silu(__uint_as_float(g[e])) * __uint_as_float(u[e]);
-  } else if (act == 2) {
-#pragma unroll
-    for (int e = 0; e < N; ++e) v[e] = fmaxf(__uint_as_float(g[e]), 0.0f) * __uint_as_float(u[e]);
+    for (int e = 0; e < N; ++e) v[e] = gate_act(__uint_as_float(g[e]), act) * __uint_as_float(u[e]);
   } else if (act == kEpilogueClamped) {
 #pragma unroll
     for (int e = 0; e < N; ++e)

@@ -58,7 +58,9 @@ template <int BN, bool DEEP> struct TcConfig {
 // output tiles blockIdx.x, blockIdx.x + gridDim.x, ... (tile t covers rows 128 * (t % tiles_x)
 // of the row operand and BN * (t / tiles_x) of the column operand); two accumulators in tensor
 // memory let the MMAs of the next tile run while the epilogue drains the last one.
-template <int BN, typename OutT, bool DEEP>
+// UNIT: gated units of every kind; else the SiLU and the ReLU only, with 40 registers fewer, which the kernel behind this one needs to
+// get resident beside two of its CTAs (decode steps of 1 and 8 requests were 1 % slower without them).
+template <int BN, typename OutT, bool DEEP, bool UNIT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, OutT* __restrict__ out,
                float* __restrict__ partial, long long part_stride, long long ldp, int rows_x, int rows_y, int k_blocks,
@@ -245,12 +247,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             }
             if (o < (rows_x >> 1)) {
               float v[8];
-              gated_values<8, true>(g, u, v, silu, unit, unit.bias_gate + o, unit.bias_up + o);
+              gated_values<8, true, UNIT>(g, u, v, silu, unit, unit.bias_gate + o, unit.bias_up + o);
 #pragma unroll
               for (int e = 0; e < 8; ++e)
                 if (j1 + e < rows_y) st(out + static_cast<long long>(j1 + e) * ldo + o, v[e]);
             }
-            if (unit.ones > 0 && i0 + kBM >= rows_x) store_ones(out, ldo, rows_x >> 1, unit.ones, j0 + c0, min(16, rows_y - (j0 + c0)), warp * 32 + lane);
+            if (UNIT && unit.ones > 0 && i0 + kBM >= rows_x) store_ones(out, ldo, rows_x >> 1, unit.ones, j0 + c0, min(16, rows_y - (j0 + c0)), warp * 32 + lane);
           }
         } else {
 #pragma unroll 1
@@ -263,7 +265,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             if (i < rows_x) {
               float v[16];
               const int column = (j0 + c0) >> 1;
-              gated_values<16>(g, u, v, silu, unit, unit.bias_gate + column, unit.bias_up + column);
+              gated_values<16, false, UNIT>(g, u, v, silu, unit, unit.bias_gate + column, unit.bias_up + column);
               const long long at = static_cast<long long>(i) * ldo + ((j0 + c0) >> 1);
               if (((at * sizeof(OutT)) & 15) == 0 && sizeof(OutT) == 2) {
                 uint32_t w[8];
@@ -280,7 +282,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
               }
             }
           }
-          if (unit.ones > 0 && j0 + BN >= rows_y) store_ones(out, ldo, rows_y >> 1, unit.ones, i0 + warp * 32, min(32, rows_x - (i0 + warp * 32)), lane);
+          if (UNIT && unit.ones > 0 && j0 + BN >= rows_y) store_ones(out, ldo, rows_y >> 1, unit.ones, i0 + warp * 32, min(32, rows_x - (i0 + warp * 32)), lane);
         }
       } else {
 #pragma unroll 1
@@ -388,21 +390,21 @@ __global__ void splitk_gated_kernel(const float* __restrict__ partial, long long
   for (int z = 1; z < splits; ++z) g += at[z * part_stride], u += at[z * part_stride + 16];
   const uint32_t gb = __float_as_uint(g), ub = __float_as_uint(u);
   float v[1];
-  gated_values<1>(&gb, &ub, v, act, unit, unit.bias_gate + c, unit.bias_up + c);
+  gated_values<1, false, true>(&gb, &ub, v, act, unit, unit.bias_gate + c, unit.bias_up + c);
   st(out + m * ldo + c, v[0]);
 }
 
 // ---------------------------------------------------------------------------------------------
 // Host side
 
-template <int BN, typename OutT, bool DEEP>
-static int launch_tc(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* partial, long long part_stride,
+template <int BN, typename OutT, bool DEEP, bool UNIT>
+static int launch_tc_of(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* partial, long long part_stride,
                      long long ldp, int rows_x, int rows_y, int K, long long ldo, int transposed, int silu, int splits, int w_rows,
                      int w_row0, cudaStream_t s, const GatedUnit& unit) {
   using C = TcConfig<BN, DEEP>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, OutT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, OutT, DEEP, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(C::kSmem)) != cudaSuccess) {
       set_error("gemm_tc: cannot reserve %zu bytes of shared memory", C::kSmem);
       return kCudaError;
@@ -419,9 +421,14 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& my, void* out, fl
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
   const int ctas = DEEP ? (n_tiles * z > sms ? max(1, sms / z) : n_tiles) : n_tiles;
   const dim3 grid(min(ctas, n_tiles), 1, z);
-  TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
+  TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP, UNIT>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
              rows_x, rows_y, k_blocks, per_split, ldo, transposed, silu, tiles_x, n_tiles, status_word(), w_rows, w_row0, unit);
   return kOk;
+}
+
+template <int BN, typename OutT, bool DEEP, typename... A>
+static int launch_tc(bool units, A... args) {
+  return units ? launch_tc_of<BN, OutT, DEEP, true>(args...) : launch_tc_of<BN, OutT, DEEP, false>(args...);
 }
 
 void launch_splitk_reduce(int out_dtype, const float* partial, long long part_stride, int splits, void* out, long long ldo, int N,
@@ -461,10 +468,9 @@ TIE_API long long tie_gemm_tc_scratch_floats(int M, int N, int splits) {
 
 // w_rows > 0: w is stored in k-blocks, [ceil(K / 64)][w_rows][64] (zeros beyond K), and the product uses its rows
 // w_row0 .. w_row0 + N - 1; ldw is then ignored.
-TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
-                        long long ldw, long long ldo, int transposed, int bn, int splits, float* scratch, int silu,
-                        int reduce, int deep, int w_rows, int w_row0, const float* bias_gate, const float* bias_up, float limit,
-                        float slope, float up_shift, int ones, cudaStream_t s) {
+static int gemm_tc_of(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
+                      int transposed, int bn, int splits, float* scratch, int silu, int reduce, int deep, int w_rows, int w_row0, GatedUnit unit,
+                      cudaStream_t s) {
   TIE_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_tc: bad sizes M=%d N=%d K=%d", M, N, K);
   TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && (w_rows > 0 || ldw % 8 == 0), "gemm_tc: K=%d and the row strides must be multiples of 8", K);
   TIE_REQUIRE(w_rows == 0 || (w_row0 >= 0 && w_row0 + N <= w_rows), "gemm_tc: rows %d..%d of a weight of %d rows", w_row0, w_row0 + N, w_rows);
@@ -475,7 +481,7 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
   TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc: output dtype code %d", out_dtype);
   TIE_REQUIRE(silu >= 0 && silu <= kEpilogueBiasedGelu && (silu != kEpilogueSquaredRelu || splits == 1 || reduce),
               "gemm_tc: epilogue %d (the squared ReLU of a split product needs the reduction here)", silu);
-  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (bias_gate != nullptr && bias_up != nullptr), "gemm_tc: epilogue %d needs biases", silu);
+  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (unit.bias_gate != nullptr && unit.bias_up != nullptr), "gemm_tc: epilogue %d needs biases", silu);
   TIE_REQUIRE(!gated_epilogue(silu) || ((splits == 1 || reduce) && N % 32 == 0 && (transposed || bn >= 32)),
               "gemm_tc: a gated unit needs unsplit k (or the reduction here) and weight rows in blocks of 16 gate + 16 up (N=%d)", N);
   TIE_REQUIRE(status_word() != nullptr, "gemm_tc: cannot allocate the status word");
@@ -493,8 +499,8 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
   const long long part_stride = static_cast<long long>(M) * N;
   const long long ldp = N;
   int st = kOk;
-  const GatedUnit unit{bias_gate, bias_up, limit, slope, up_shift, gated_epilogue(silu) ? ones : 0};
-#define TIE_TC_ARGS mx, my, out, partial, part_stride, ldp, rows_x, rows_y, K, ldo, transposed, silu, splits, w_rows, w_row0, s, unit
+  if (!gated_epilogue(silu)) unit.ones = 0;
+#define TIE_TC_ARGS silu > kEpilogueSquaredRelu, mx, my, out, partial, part_stride, ldp, rows_x, rows_y, K, ldo, transposed, silu, splits, w_rows, w_row0, s, unit
 #define TIE_TC_CASE(B)                                                                                     \
   case B:                                                                                                  \
     if (deep) {                                                                                            \
@@ -522,4 +528,19 @@ TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, 
       TIE_LAUNCH((splitk_gated_kernel<float>), blocks, 256, 0, s, partial, part_stride, real, static_cast<float*>(out), ldo, N, M, silu, unit);
   } else if (splits > 1 && reduce) launch_splitk_reduce(out_dtype, partial, part_stride, tie_gemm_tc_real_splits(K, splits), out, ldo, N, part_stride, silu, s);
   TIE_RETURN_LAUNCH("gemm_tc");
+}
+
+TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
+                        int transposed, int bn, int splits, float* scratch, int silu, int reduce, int deep, int w_rows, int w_row0,
+                        cudaStream_t s) {
+  return gemm_tc_of(out_dtype, a, w, out, M, N, K, lda, ldw, ldo, transposed, bn, splits, scratch, silu, reduce, deep, w_rows, w_row0, GatedUnit{}, s);
+}
+
+// The same with what a gated unit takes beside its code (GatedUnit).
+TIE_API int tie_gemm_tc_unit(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw,
+                             long long ldo, int transposed, int bn, int splits, float* scratch, int silu, int reduce, int deep, int w_rows,
+                             int w_row0, const float* bias_gate, const float* bias_up, float limit, float slope, float up_shift, int ones,
+                             cudaStream_t s) {
+  return gemm_tc_of(out_dtype, a, w, out, M, N, K, lda, ldw, ldo, transposed, bn, splits, scratch, silu, reduce, deep, w_rows, w_row0,
+                    GatedUnit{bias_gate, bias_up, limit, slope, up_shift, ones}, s);
 }

@@ -134,7 +134,7 @@ __device__ __forceinline__ void put_pieces(uint8_t* mine, int row, int first, co
 }
 
 template <typename OutT>
-__global__ void __launch_bounds__(k2Threads, 1)
+__global__ void __launch_bounds__(512, 1)      // (launched with 320 threads: 128 registers a thread leave the next kernel some)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                 const __grid_constant__ CUtensorMap map_out, const __grid_constant__ PairArgs g) {
   pdl_launch_dependents();
@@ -318,7 +318,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             }
             if (o < (g.rows_x >> 1)) {
               float v[8];
-              gated_values<8, true>(gv, uv, v, g.epilogue, g.unit, g.unit.bias_gate + o, g.unit.bias_up + o);
+              gated_values<8, true, true>(gv, uv, v, g.epilogue, g.unit, g.unit.bias_gate + o, g.unit.bias_up + o);
               OutT* at = static_cast<OutT*>(g.out) + static_cast<long long>(c1) * g.ldo + o;
 #pragma unroll
               for (int e = 0; e < 8; ++e)
@@ -381,7 +381,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (gated) {
               float v[16];
               const int column = ((j0 + c0) >> 1) + h * 16;
-              gated_values<16>(r, r + 16, v, g.epilogue, g.unit, g.unit.bias_gate + column, g.unit.bias_up + column);
+              gated_values<16, false, true>(r, r + 16, v, g.epilogue, g.unit, g.unit.bias_gate + column, g.unit.bias_up + column);
               const int next = h + 1 < halves ? c0 + 32 : c0 + 2 * per;
               if (next < end) tmem_ld32(acc + next, r);
               else release();
@@ -524,10 +524,9 @@ TIE_API int tie_gemm_tc2_pairs() { return resident_pairs(); }
 // transposed != 0: the weights fill the tiles' 256-row side. bn: the other side, a multiple of 32 up to 256 (0: 256).
 // splits > 1: k is cut, and float sums [real splits][M][N] go to scratch (tie_gemm_tc_real_splits says how many there are): added
 // into out by a second kernel, or with reduce == 0 left there for a consumer that adds them itself.
-TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
-                         long long ldw, long long ldo, int silu, int w_rows, int w_row0, int bn, int transposed, int splits,
-                         float* scratch, int reduce, const float* bias_gate, const float* bias_up, float limit, float slope, float up_shift,
-                         int ones, cudaStream_t s) {
+static int gemm_tc2_of(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
+                       int silu, int w_rows, int w_row0, int bn, int transposed, int splits, float* scratch, int reduce, GatedUnit unit,
+                       cudaStream_t s) {
   if (bn == 0) bn = 256;
   TIE_REQUIRE(bn >= 32 && bn <= 256 && bn % 32 == 0, "gemm_tc2: tile width %d", bn);
   TIE_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_tc2: bad sizes M=%d N=%d K=%d", M, N, K);
@@ -538,7 +537,7 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc2: output dtype code %d", out_dtype);
   TIE_REQUIRE(silu >= 0 && silu <= kEpilogueBiasedGelu, "gemm_tc2: epilogue %d", silu);
   TIE_REQUIRE(!gated_epilogue(silu) || N % 32 == 0, "gemm_tc2: a gated unit needs weight rows in blocks of 16 gate + 16 up (N=%d)", N);
-  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (bias_gate != nullptr && bias_up != nullptr), "gemm_tc2: epilogue %d needs biases", silu);
+  TIE_REQUIRE(silu < kEpilogueBiasedSilu || (unit.bias_gate != nullptr && unit.bias_up != nullptr), "gemm_tc2: epilogue %d needs biases", silu);
   TIE_REQUIRE(splits >= 1 && (splits == 1 || scratch != nullptr), "gemm_tc2: splits=%d needs scratch memory", splits);
   TIE_REQUIRE(splits == 1 || silu == 0 || (silu == kEpilogueSquaredRelu && reduce),
               "gemm_tc2: epilogue %d of a split product (the squared ReLU needs the reduction here)", silu);
@@ -563,7 +562,8 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   g.ldp = N;
   g.ldo = ldo;
   g.epilogue = silu;
-  g.unit = GatedUnit{bias_gate, bias_up, limit, slope, up_shift, gated_epilogue(silu) ? ones : 0};
+  g.unit = unit;
+  if (!gated_epilogue(silu)) g.unit.ones = 0;
   g.w_rows = w_rows;
   g.w_row0 = w_row0;
   g.status = status_word();
@@ -581,6 +581,19 @@ TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out,
   if (st != kOk) return st;
   if (scratch != nullptr && reduce) launch_splitk_reduce(out_dtype, scratch, g.part_stride, real, out, ldo, N, g.part_stride, silu, s);
   TIE_RETURN_LAUNCH("gemm_tc2");
+}
+
+TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
+                         int silu, int w_rows, int w_row0, int bn, int transposed, int splits, float* scratch, int reduce, cudaStream_t s) {
+  return gemm_tc2_of(out_dtype, a, w, out, M, N, K, lda, ldw, ldo, silu, w_rows, w_row0, bn, transposed, splits, scratch, reduce, GatedUnit{}, s);
+}
+
+// The same with what a gated unit takes beside its code (GatedUnit).
+TIE_API int tie_gemm_tc2_unit(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw,
+                              long long ldo, int silu, int w_rows, int w_row0, int bn, int transposed, int splits, float* scratch, int reduce,
+                              const float* bias_gate, const float* bias_up, float limit, float slope, float up_shift, int ones, cudaStream_t s) {
+  return gemm_tc2_of(out_dtype, a, w, out, M, N, K, lda, ldw, ldo, silu, w_rows, w_row0, bn, transposed, splits, scratch, reduce,
+                     GatedUnit{bias_gate, bias_up, limit, slope, up_shift, ones}, s);
 }
 
 // Grouped product: a [M_cap, K] holds `meta[0]` tiles of 256 rows (M_cap is what the buffers were sized for); tile t multiplies the N weight

@@ -28,12 +28,10 @@ TIE_API int tie_gemm_simt(int in_dtype, int out_dtype, const void* a, const void
                           long long lda, long long ldw, long long ldo, cudaStream_t s);
 TIE_API int tie_gemm_tc(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
                         long long ldw, long long ldo, int transposed, int bn, int splits, float* scratch, int silu,
-                        int reduce, int deep, int w_rows, int w_row0, const float* bias_gate, const float* bias_up, float limit,
-                        float slope, float up_shift, int ones, cudaStream_t s);
+                        int reduce, int deep, int w_rows, int w_row0, cudaStream_t s);
 TIE_API int tie_gemm_tc2(int out_dtype, const void* a, const void* w, void* out, int M, int N, int K, long long lda,
                          long long ldw, long long ldo, int silu, int w_rows, int w_row0, int bn, int transposed, int splits,
-                         float* scratch, int reduce, const float* bias_gate, const float* bias_up, float limit, float slope, float up_shift,
-                         int ones, cudaStream_t s);
+                         float* scratch, int reduce, cudaStream_t s);
 
 TIE_API int tie_attention_rows(int dtype, const void* q, long long q_stride, const void* k_cache, const void* v_cache,
                                void* out, const int* seq_of_row, const int* query_start, const int* context_lens,

@@ -79,7 +79,7 @@ class StepContext:
     context_lens: torch.Tensor
     logit_rows: torch.Tensor
     state_slots: torch.Tensor        # [S] slot of each sequence's fixed-size state
-    single_seqs: torch.Tensor        # [single_count] sequences that bring one token
+    single_seqs: torch.Tensor        # [single_count] sequences that bring one token; more than eight: the longest context first
     groups: list[GroupStep]
     multi_rows: int                  # rows [0, multi_rows) belong to sequences that bring several tokens
     multi_seqs: int                  # sequences [0, multi_seqs) are those
@@ -463,7 +463,8 @@ class StepRunner:
             r += 1
         single = sec("single_seqs")
         n_single = S - n_multi
-        single[:n_single] = np.arange(n_multi, S)
+        # the longest first, where there may be more than fit at once (parts/attention.py, decode_order)
+        single[:n_single] = np.arange(n_multi, S) if n_single <= 8 else n_multi + np.argsort(-context_lens[n_multi:S], kind="stable")
         if table_len is not None:
             single_max_ctx = MB * page               # a captured graph must hold for every context of its bucket
         else:

@@ -547,7 +547,7 @@ def bound_gemm(w: torch.Tensor, silu=False, split_many: bool = True, pack: bool 
     keeps that copy (`.w`) and the caller lets go of its own. `.rows(a, b)` is the product with rows a..b-1 of
     the same weight, without a copy."""
     from . import gemm_select
-    return gemm_select.BoundGemm(w, silu, split_many, pack, unit=unit or gemm_select.GatedUnit())
+    return gemm_select.BoundGemm(w, silu, split_many, pack, unit=unit)
 
 
 def partial_capacity(max_rows: int, N: int, K: int, split_many: bool = True) -> int:

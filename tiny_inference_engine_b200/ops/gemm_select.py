@@ -222,6 +222,11 @@ class GatedUnit:
 _PLAIN_UNIT = GatedUnit()
 
 
+def _entry(name: str, unit: GatedUnit, *args):
+    """The launcher's call: with the unit's own arguments where it has some (`<name>_unit`, the stream behind them)."""
+    return (name, *args) if unit is _PLAIN_UNIT else (name + "_unit", *args[:-1], *unit.args, args[-1])
+
+
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None, bn=None, splits=None, scratch=None,
             silu=False, partial_scratch=None, deep=None, pair=None, checked: bool = False, unit: GatedUnit = _PLAIN_UNIT):
     """The tensor-core product; the tiling can be forced (tests). Returns `out`, or a SplitSum when
@@ -247,8 +252,8 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
         leave = splits > 1 and partial_scratch is not None
         if splits > 1:
             scratch = partial_scratch(splits * M * N) if leave else scratch if scratch is not None else _scratch_for(splits * M * N, a.device)
-        _call("tie_gemm_tc2", dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
-              w.stride(0), out.stride(0), int(silu), 0, 0, bn, t, splits, scratch.data_ptr() if splits > 1 else 0, 0 if leave else 1, *unit.args, _stream())
+        _call(*_entry("tie_gemm_tc2", unit, dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), w.stride(0),
+                      out.stride(0), int(silu), 0, 0, bn, t, splits, scratch.data_ptr() if splits > 1 else 0, 0 if leave else 1, _stream()))
         return SplitSum(scratch, _library().tie_gemm_tc_real_splits(K, splits), M, N) if leave else out
     t, b, s = plan(M, N, K)
     transposed = t if transposed is None else int(transposed)
@@ -263,9 +268,9 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
         scratch = partial_scratch(splits * M * N)
     elif splits > 1 and scratch is None:
         scratch = _scratch_for(splits * M * N, a.device)
-    _call("tie_gemm_tc", dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
-          w.stride(0), out.stride(0), transposed, bn, splits, scratch.data_ptr() if splits > 1 else 0, int(silu),
-          0 if leave else 1, int(deep if deep is not None else (not transposed or bn >= 128)), 0, 0, *unit.args, _stream())
+    _call(*_entry("tie_gemm_tc", unit, dtype_code(out), a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0),
+                  w.stride(0), out.stride(0), transposed, bn, splits, scratch.data_ptr() if splits > 1 else 0, int(silu),
+                  0 if leave else 1, int(deep if deep is not None else (not transposed or bn >= 128)), 0, 0, _stream()))
     if leave:
         return SplitSum(scratch, _library().tie_gemm_tc_real_splits(K, splits), M, N)
     return out
@@ -315,9 +320,12 @@ class BoundGemm:
     [ceil(K / 64), rows, 64] and `packed_rows` its number of rows; `.rows(a, b)` gives the product with a slice of
     its rows (the q rows of a stacked q/k/v weight) over the same memory."""
 
-    def __init__(self, w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True, _slice=None, unit: GatedUnit = _PLAIN_UNIT):
+    unit = _PLAIN_UNIT      # (an attribute of its own only where it says something: what a layer holds is looked through every step)
+
+    def __init__(self, w: torch.Tensor, silu=False, split_many: bool = True, pack: bool = True, _slice=None, unit: GatedUnit | None = None):
         self.silu, self.split_many = int(silu), split_many      # 0: none, 3: the squared ReLU, else a gated unit
-        self.unit = unit
+        if unit is not None:
+            self.unit = unit
         self.gated = _gated(silu)
         if _slice is not None:              # rows [row0, row0 + N) of a packed weight
             parent, row0, n = _slice
@@ -358,9 +366,10 @@ class BoundGemm:
         else:
             t, bn, splits = plan(M, self.N, self.K, self.split_many)
         if self.gated:
-            # few tokens: k split like any product's, the unit formed where the sums are added (Dugazen's 12,288 columns at 8 tokens:
-            # 96 tiles; whole k 2.5 us slower than three splits, their sum and the unit in kernels of their own)
-            splits = splits if M <= PAIR_FROM else 1
+            # few tokens on few tiles: k split like any product's, the unit formed where the sums are added (12,288 columns at 8 tokens,
+            # 96 tiles: whole k 2.5 us slower than three splits, their sum and the unit in kernels of their own; 16,384 columns in two
+            # splits 3 us slower than whole k)
+            splits = splits if M <= PAIR_FROM and splits >= 3 else 1
             if not t:
                 bn = max(bn, 32)
         real = _library().tie_gemm_tc_real_splits(self.K, splits) if splits > 1 else 1
@@ -402,12 +411,16 @@ class BoundGemm:
             buf = _scratch_for(splits * M * self.N, a.device)
             scratch = buf.data_ptr()
         if pair:
-            _call("tie_gemm_tc2", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw,
-                  out.stride(0), self.silu, self.packed_rows, self.row0, bn, t, splits, scratch, 0 if leave else 1,
-                  *self.unit.args, _stream())
+            args = (code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0), self.silu,
+                    self.packed_rows, self.row0, bn, t, splits, scratch, 0 if leave else 1)
         else:
-            _call("tie_gemm_tc", code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0),
-                  t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0, *self.unit.args, _stream())
+            args = (code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0),
+                    t, bn, splits, scratch, self.silu, 0 if leave else 1, deep, self.packed_rows, self.row0)
+        name = "tie_gemm_tc2" if pair else "tie_gemm_tc"
+        if self.unit is _PLAIN_UNIT:
+            _call(name, *args, _stream())
+        else:
+            _call(name + "_unit", *args, *self.unit.args, _stream())
         if leave:
             return SplitSum(buf, real, M, self.N)
         return out

@@ -24,7 +24,7 @@ import torch
 from .. import ops
 from ..errors import InvalidArgument
 from ..weights.loader import TensorNeed
-from .attention import MAX_SPLITS, NUM_SMS, TMA_DECODE_TABLE_ENTRIES, decode_splits
+from .attention import MAX_SPLITS, NUM_SMS, TMA_DECODE_TABLE_ENTRIES, decode_order, decode_splits
 from .base import CacheNeed, Mixer, StateNeed, build_part, register_part, to_compute
 
 
@@ -150,7 +150,7 @@ class ConvKeyAttention(Mixer):
                 scratch = ctx.ws.flat("attn.split", ops.attention_split_scratch_floats(ctx.max_seqs, H, dim, MAX_SPLITS), torch.float32)
                 counters = ctx.ws.zeros("attn.counters", ctx.max_seqs * G, torch.int32)
                 cluster = max_splits in ops.CLUSTER_SPLITS and n * G * max_splits <= 2 * NUM_SMS
-                ops.attention_decode_kept(q, cache.k, cache.v, attn, *index, H, G, dim, self.scale, ctx.multi_seqs, n, split_keys, max_splits,
+                ops.attention_decode_kept(q, cache.k, cache.v, attn, *index, H, G, dim, self.scale, decode_order(ctx, n * G * max_splits), n, split_keys, max_splits,
                                           scratch, counters, cluster=cluster, **options)
                 return
         longest += self.keep_first

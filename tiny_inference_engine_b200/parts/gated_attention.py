@@ -21,7 +21,7 @@ import torch
 from .. import ops
 from ..errors import InvalidArgument
 from ..weights.loader import TensorNeed
-from .attention import MAX_SPLITS, NUM_SMS, SPLIT_KEYS, decode_splits
+from .attention import MAX_SPLITS, NUM_SMS, SPLIT_KEYS, decode_order, decode_splits
 from .base import CacheNeed, Mixer, build_part, register_part, to_compute
 
 _GATES = {None: None, False: None, True: "channel", "channel": "channel", "head": "head"}
@@ -181,8 +181,8 @@ class GatedWindowAttention(Mixer):
             counters = ctx.ws.zeros("attn.counters", ctx.max_seqs * G, torch.int32)
             cluster = max_splits in ops.CLUSTER_SPLITS and ctx.single_count * G * max_splits <= 2 * NUM_SMS
             ops.attention_decode_tma(q, cache.k, cache.v, attn, ctx.query_start, ctx.context_lens, g.block_tables, H, G, Dh,
-                                     self.scale, ctx.multi_seqs, ctx.single_count, split_keys, max_splits, scratch, counters,
-                                     self.window, cluster=cluster, exact_weights=True)
+                                     self.scale, decode_order(ctx, ctx.single_count * G * max_splits), ctx.single_count, split_keys,
+                                     max_splits, scratch, counters, self.window, cluster=cluster, exact_weights=True)
 
     def _attend_cuda_cores(self, q, attn, ctx, g, cache):
         """float32, or heads of other sizes (keys and values may differ): one warp per (row, head), everything float."""
