@@ -458,7 +458,8 @@ TIE_API int tie_moe_route(const float* logits, long long ld_logits, int tokens, 
 
 TIE_API int tie_moe_align(const int* ids, int pairs, int experts, int block_m, int* sorted, int* tile_expert, int* meta,
                           cudaStream_t s) {
-  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 8 || block_m == 16 || block_m == 64 || block_m == 256),
+  TIE_REQUIRE(experts > 0 && experts <= 4096 && (block_m == 4 || block_m == 8 || block_m == 16 || block_m == 64 || block_m == 128 ||
+               block_m == 256),
               "moe_align: bad sizes experts=%d block_m=%d", experts, block_m);
   if (pairs <= 0) return kOk;
   TIE_LAUNCH(moe_align_kernel, 1, 1024, 2 * experts * sizeof(int), s, ids, pairs, experts, block_m, sorted, tile_expert, meta);

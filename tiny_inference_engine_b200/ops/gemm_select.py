@@ -407,8 +407,9 @@ class BoundGemm:
         if leave:
             buf = partial_scratch(splits * M * self.N)
             scratch = buf.data_ptr()
-        elif splits > 1:
-            buf = _scratch_for(splits * M * self.N, a.device)
+        elif splits > 1:        # added up here: a gated unit's caller brings memory of its own step
+            n = splits * M * self.N
+            buf = partial_scratch(n) if partial_scratch is not None else _scratch_for(n, a.device)
             scratch = buf.data_ptr()
         if pair:
             args = (code, a.data_ptr(), self.w_ptr, out.data_ptr(), M, self.N, self.K, a.stride(0), self.ldw, out.stride(0), self.silu,

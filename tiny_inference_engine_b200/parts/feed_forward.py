@@ -7,8 +7,15 @@ import torch
 
 from .. import ops
 from ..weights.loader import TensorNeed
-from ..ops.gemm_select import GatedUnit
+from ..ops.gemm_select import PAIR_FROM, GatedUnit
 from .base import FeedForward, register_part, to_compute
+
+
+def unit_scratch(part, ctx):
+    """Memory of the step's workspace for the sums of a gated product whose k is split (few tokens)."""
+    if part._unit_capacity is None:
+        part._unit_capacity = ops.partial_capacity(min(ctx.ws.max_rows, PAIR_FROM), part.gate_up.N, part.gate_up.K)
+    return lambda n: ctx.ws.flat("ffn.unit.partial", n, torch.float32, part._unit_capacity)
 
 
 class SwiGLU(FeedForward):
@@ -30,6 +37,7 @@ class SwiGLU(FeedForward):
         self.names = tuple(self.prefix + p.get(k, k + "_proj.weight") for k in ("gate", "up", "down"))
         self.dtype = dtype
         self.w_gate_up = self.w_down = None
+        self._unit_capacity = None
 
     def needs(self):
         g, u, d = self.names
@@ -51,7 +59,7 @@ class SwiGLU(FeedForward):
         T = h.shape[0]
         act = ctx.ws.rows("ffn.act", T, self.inter, self.dtype)
         if self.fused:
-            self.gate_up(h, act)
+            self.gate_up(h, act, unit_scratch(self, ctx))
         else:
             gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
             self.gate_up(h, gu)
@@ -78,7 +86,7 @@ class ClampedGLU(FeedForward):
         self.limit, self.slope, self.up_shift = float(p["limit"]), float(p.get("slope", 1.0)), float(p.get("up_shift", 0.0))
         self.names = tuple(self.prefix + p.get(k, k) for k in ("gate", "up", "down"))
         self.dtype = dtype
-        self._partial_capacity = None
+        self._partial_capacity = self._unit_capacity = None
 
     def needs(self):
         return {self.names[0]: TensorNeed((self.inter, self.hidden)), self.names[1]: TensorNeed((self.inter, self.hidden)),
@@ -101,7 +109,7 @@ class ClampedGLU(FeedForward):
         T = h.shape[0]
         act = ctx.ws.rows("ffn.act", T, self.inter, self.dtype)
         if self.fused:
-            self.gate_up(h, act)
+            self.gate_up(h, act, unit_scratch(self, ctx))
         else:
             gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
             self.gate_up(h, gu)
@@ -135,7 +143,7 @@ class BiasedGLU(FeedForward):
         self.names = tuple(self.prefix + p.get(k, k) for k in ("gate", "up", "down"))
         self.padded = (self.inter + 1 + 7) // 8 * 8          # the unit, the column of ones, zeros
         self.dtype = dtype
-        self._partial_capacity = None
+        self._partial_capacity = self._unit_capacity = None
 
     def needs(self):
         g, u, d = self.names
@@ -165,7 +173,7 @@ class BiasedGLU(FeedForward):
         T = h.shape[0]
         act = ctx.ws.rows("ffn.act1", T, self.padded, self.dtype)
         if self.fused:
-            self.gate_up(h, act[:, :self.inter])
+            self.gate_up(h, act[:, :self.inter], unit_scratch(self, ctx))
         else:
             gu = ctx.ws.rows("ffn.gate_up", T, 2 * self.inter, self.dtype)
             self.gate_up(h, gu)
