@@ -63,6 +63,37 @@ def test_two_layers_are_no_run_and_a_moved_tensor_is_noticed(tmp_path):
     assert fresh.alive() and moved in fresh.table[0][3].tolist() and moved not in runs.table[0][3].tolist()
 
 
+@pytest.mark.parametrize("change", ["none", "tensor", "attribute", "part", "in place", "list", "constant", "plane"])
+def test_a_second_look_at_a_layers_tensors_notices_what_the_first_would(tmp_path, change):
+    """What `spans` took from its last look it takes again only while the layer holds the same tensors at the same addresses."""
+    import copy
+    model, cache, states = _model(tmp_path, num_hidden_layers=4)
+    runs = LayerRuns(model, cache, states)
+    first = runs.spans(1, 0)
+    assert first is not None and runs.spans(1, 0) is first
+    ffn = model.layers[1].ffn
+    if change == "none":
+        assert runs.spans(1, 0) == first
+        return
+    if change == "tensor":
+        ffn.down.w = ffn.down.w.clone()
+    elif change == "attribute":
+        ffn.extra = torch.zeros(3)
+    elif change == "part":
+        model.layers[1].ffn = copy.deepcopy(ffn)
+    elif change == "in place":
+        ffn.down.w.data = ffn.down.w.data.clone()
+    elif change == "list":
+        ffn.names = (*ffn.names, torch.zeros(3))
+    elif change == "constant":
+        ffn.inter = torch.zeros(3)          # a tensor where a number was
+    else:
+        view = cache.layer_cache(1, writes=True)
+        fresh = type("View", (), dict(k=view.k.clone(), v=view.v, group=view.group, writes=view.writes))()
+        cache.layer_cache = lambda owner, writes: fresh
+    assert runs.spans(1, 0) is None
+
+
 def test_the_model_hands_out_runs_after_its_first_forward_and_builds_them_anew_when_a_tensor_is_gone(tmp_path):
     class Ctx:
         layer_hook = None

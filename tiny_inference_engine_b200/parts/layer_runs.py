@@ -18,14 +18,24 @@ from .base import Part
 _PACKAGE = __name__.split(".")[0]
 
 
-def walk_part(obj, tensors: list, scalars: list, seen: set) -> bool:
+def walk_part(obj, tensors: list, scalars: list, seen: set, places: list | None = None) -> bool:
     """Collects, in attribute order, the tensors `obj` and the parts inside it hold, and the sizes and constants
     beside them (names of checkpoint tensors and addresses left out). Layers built alike give lists that differ in
-    the tensors' addresses only. Returns whether every part met says `launches_only`."""
+    the tensors' addresses only. Returns whether every part met says `launches_only`. `places` receives, per object
+    met, what `unchanged` needs to tell that walking it again would meet the same tensors."""
     ok = bool(getattr(obj, "launches_only", False)) if isinstance(obj, Part) else True
     seen.add(id(obj))
+    held = []           # (attribute, its place in a list or None, the list's length or -1, the tensor or object, weakly)
+    if places is not None:
+        places.append((weakref.ref(obj), len(vars(obj)), held))
     for name, v in vars(obj).items():
-        for item in (v if isinstance(v, (list, tuple)) else (v,)):
+        listed = isinstance(v, (list, tuple))
+        if places is not None and listed and not v:
+            held.append((name, None, 0, None))
+        for k, item in enumerate(v if listed else (v,)):
+            if places is not None:
+                kept = isinstance(item, torch.Tensor) or hasattr(item, "__dict__")
+                held.append((name, k if listed else None, len(v) if listed else -1, weakref.ref(item) if kept else None))
             if isinstance(item, torch.Tensor):
                 tensors.append(item)
             elif isinstance(item, (bool, float, torch.dtype)) or item is None:
@@ -41,10 +51,40 @@ def walk_part(obj, tensors: list, scalars: list, seen: set) -> bool:
             elif hasattr(item, "__dict__") and id(item) not in seen and (
                     isinstance(item, Part) or type(item).__module__.split(".")[0] == _PACKAGE):
                 scalars.append((name, type(item).__qualname__))
-                ok = walk_part(item, tensors, scalars, seen) and ok
+                ok = walk_part(item, tensors, scalars, seen, places) and ok
             elif hasattr(item, "__dict__") and id(item) not in seen:
                 ok = False      # an object of unknown kind: what it holds cannot be listed
     return ok
+
+
+def unchanged(places: list) -> bool:
+    """Whether every object that `walk_part` met still has as many attributes and holds the same tensors and objects at the
+    same places, and none where there was none (a fraction of the time of walking them again)."""
+    for ref, count, held in places:
+        obj = ref()
+        if obj is None:
+            return False
+        attributes = vars(obj)
+        if len(attributes) != count:
+            return False
+        for name, k, length, item in held:
+            if name not in attributes:
+                return False
+            v = attributes[name]
+            if isinstance(v, (list, tuple)):
+                if len(v) != length:
+                    return False
+                if length == 0:
+                    continue
+                v = v[k]
+            elif length >= 0:
+                return False
+            if item is None:
+                if isinstance(v, torch.Tensor) or hasattr(v, "__dict__"):
+                    return False
+            elif v is not item():
+                return False
+    return True
 
 
 def _extent_bytes(t: torch.Tensor) -> int:
@@ -76,6 +116,7 @@ class LayerRuns:
         self.model_ref = weakref.ref(model)
         order = model.spec.run_order
         sigs, rows = [], []
+        self._looks: dict[tuple, tuple] = {}    # (entry, start of its run) -> what `spans` found last
         self._held = []     # weak references to the layers' own tensors: one that is gone means the table is stale
         for i in range(len(order)):
             ok, scalars, tensors, view = self._entry(model, cache, i)
@@ -108,23 +149,39 @@ class LayerRuns:
         return all(r() is not None for r in self._held)
 
     @staticmethod
-    def _entry(model, cache, i):
+    def _view(model, cache, i):
+        entry = model.spec.run_order[i]
+        owner = i if entry.cache_of is None else entry.cache_of
+        return cache.layer_cache(owner, writes=entry.cache_of is None) if cache is not None else None
+
+    @staticmethod
+    def _entry(model, cache, i, places: list | None = None):
         """(every part launches only, constants, tensors in slot order: the layer's own, then its cache planes,
         the entry's view of the cache)."""
-        entry = model.spec.run_order[i]
         tensors, scalars = [], []
-        ok = walk_part(model.layers[entry.layer], tensors, scalars, set())
-        owner = i if entry.cache_of is None else entry.cache_of
-        view = cache.layer_cache(owner, writes=entry.cache_of is None) if cache is not None else None
+        ok = walk_part(model.layers[model.spec.run_order[i].layer], tensors, scalars, set(), places)
+        view = LayerRuns._view(model, cache, i)
         tensors += [t for t in ((view.k, view.v) if view is not None else ()) if t is not None]
         return ok, scalars, tensors, view
 
     def spans(self, i: int, start: int):
-        """(address, bytes) per slot of entry i of the run that starts at `start`, looked up afresh; None if
-        the layer's tensors are no longer where the table says (then nothing is repeated)."""
+        """(address, bytes) per slot of entry i of the run that starts at `start`; None if the layer's tensors are no longer
+        where the table says (then nothing is repeated). Looked up afresh, or, where the layer still holds the tensors of the
+        last look, taken from it once their addresses and shapes have been compared."""
         model, cache = self.model_ref(), self.cache_ref() if self.cache_ref is not None else None
         row = self.table[start][i - start]
-        _, _, tensors, _ = self._entry(model, cache, i)
+        known = self._looks.get((i, start))
+        if known is not None and unchanged(known[0]):
+            view = self._view(model, cache, i)
+            tensors = [r() for r in known[1]] + [t for t in ((view.k, view.v) if view is not None else ()) if t is not None]
+            if all(t is not None for t in tensors) and [(t.data_ptr(), t.shape, t.stride()) for t in tensors] == known[2]:
+                return known[3]
+        places: list = []
+        _, _, tensors, view = self._entry(model, cache, i, places)
         if len(tensors) != len(row) or any(t.data_ptr() != int(p) for t, p in zip(tensors, row)):
             return None
-        return [(t.data_ptr(), _extent_bytes(t)) for t in tensors]
+        planes = sum(1 for t in ((view.k, view.v) if view is not None else ()) if t is not None)
+        spans = [(t.data_ptr(), _extent_bytes(t)) for t in tensors]
+        self._looks[i, start] = (places, [weakref.ref(t) for t in tensors[:len(tensors) - planes]],
+                                 [(t.data_ptr(), t.shape, t.stride()) for t in tensors], spans)
+        return spans
