@@ -268,6 +268,39 @@ def test_float_products_by_three_terms_of_infinities_and_large_values(ops, bn, s
     assert (np.abs(got[9] - want[9])[~odd[9]] <= 1e-6 * np.abs(want[9])[~odd[9]]).all()
 
 
+def float_products_both_ways(a, w, bn, splits):
+    """out = a w^T by three terms and by FFMAs (64 x 64 tiles, whole k), and the relative errors of both against 64 bits."""
+    from tiny_inference_engine_b200.ops.library import call
+    M, K, N = *a.shape, w.shape[0]
+    outs = [torch.empty(M, N, device="cuda") for _ in range(2)]
+    for name, out, tile, s in (("tie_gemm_f32_split", outs[0], bn, splits), ("tie_gemm_f32_tiled", outs[1], 1, 1)):
+        call(name, a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, tile, s, torch.cuda.current_stream().cuda_stream)
+    want = a.double() @ w.double().T
+    return outs[0], want, *(float((o.double() - want).norm() / want.norm()) for o in outs)
+
+
+@pytest.mark.parametrize("size", [1.0, 1e-35, 3e-37, 1e-40])
+@pytest.mark.parametrize("bn,splits", [(32, 1), (96, 2)])
+def test_float_products_by_three_terms_of_small_values(ops, bn, splits, size):
+    """Operands whose low bits bfloat16 has no exponent for (below 2^-109), and subnormal ones: no bit of them is lost, the error is
+    no larger than with FFMAs (results near the smallest float round alike in both)."""
+    g = torch.Generator("cuda").manual_seed(3)
+    a, w = (torch.randn(n, 600, device="cuda", generator=g) for n in (130, 100))
+    _, _, terms, ffma = float_products_both_ways(a * size, w, bn, splits)
+    assert terms <= ffma
+
+
+def test_float_products_by_three_terms_whose_partial_sums_overflow(ops):
+    """All terms as large as they get: 2^16 times the products of the low ones adds up to three times the result, beyond the largest
+    float, where the result is below it."""
+    x = (1.0 + 254 / 256 * 2.0 ** -8 + 126 / 128 * 2.0 ** -16) * 2.0 ** 60
+    a = torch.zeros(70, 200, device="cuda")
+    a[:, :64] = x
+    w = torch.full((40, 200), 2.0 * x, device="cuda")
+    out, want, terms, _ = float_products_both_ways(a, w, 32, 1)
+    assert torch.isfinite(out).all() and terms < 1e-6
+
+
 def dense_reference(q, k, v, Hq, Hkv, Dh, n_new, window=0):
     """The last n_new rows of causal attention over all of k, v."""
     n = k.shape[0]

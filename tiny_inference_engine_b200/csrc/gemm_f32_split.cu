@@ -1,12 +1,15 @@
 // 32-bit matrix products on the tensor cores, out[M, N] = a[M, K] . w[N, K]^T with float operands and results.
 //
-// Every float is the sum of three bfloat16 numbers, x = hi + mid + lo, each the rounding of what the ones before it leave over:
-// 8 bits of mantissa three times, 24 in all, so the three are x exactly (down to 2^-133, below which bfloat16 ends). Six of the
-// nine products of terms are formed, the smallest first; what the other three (mid lo, lo mid, lo lo) leave out is below 2^-26 of
-// a product, a quarter of a unit of the float product. The tensor core multiplies the terms exactly; its float accumulator is
-// trusted with 64 k's only: a k-block's sum is then read out of tensor memory and added in registers, to the nearest. Against 64 bits the
+// Every float is the sum of three bfloat16 numbers, x = hi + 2^-8 mid + 2^-16 lo, each the rounding of what the ones before it leave
+// over: 8 bits of mantissa three times, 24 in all. The second and third are held 2^8 and 2^16 up, so that the three are x exactly for
+// every float, subnormal ones too (unscaled, values below 2^-109 lost low bits: bfloat16 ends at 2^-133). Six of the nine products of
+// terms are formed, the smallest first, and the accumulator comes down by 2^8 (scale-input-d) ahead of the next order of magnitude;
+// what the other three (mid lo, lo mid, lo lo) leave out is below 2^-26 of a product, a quarter of a unit of the float product. This is
+// Ozaki's error-free splitting with a fixed number of slices.
+// The tensor core multiplies the terms exactly; its float accumulator is trusted with 64 k's only: a k-block's sum is then read out of
+// tensor memory and added in registers, to the nearest. Against 64 bits the
 // result is off by half of what the FFMA kernel of gemm_simt.cu is, whose accumulators round at every k (the measured figures are
-// in test_float_products_by_three_terms). This is Ozaki's error-free splitting with a fixed number of slices.
+// in test_float_products_by_three_terms).
 //
 // One CTA computes a tile of 128 x BN. Warps 0-15 read both operands' k-block (float, straight from global memory, any size, stride
 // and alignment; the next block's loads are in flight while this one is split), write the six term tiles in the tensor core's
@@ -20,8 +23,9 @@
 // spilled words came from L2 (2,400 cycles). 389 x 3,072 x 1,024: 112 -> 28.6 us, 389 x 1,024 x 1,024: 39.5 -> 15.6, 32 x 1,536 x
 // 1,024: 17.9 -> 10.4, 1,000 x 2,048 x 2,048: 254 -> 74.
 //
-// Infinities and NaN: hi is one, the rest would make NaN of an infinity (inf - inf, inf * 0). The splitting warps look at
-// exponents; a CTA that met one (or a float that rounds to an infinity in bfloat16) computes its tile again with FFMAs.
+// Infinities and NaN: hi is one, and the terms behind it make NaN of every sum of its row or column (inf - inf). So does a float that
+// rounds to an infinity in bfloat16, and partial sums beyond the largest float stay infinite: a thread that ends with a sum that is not
+// finite computes its sums again with FFMAs.
 #include "umma.cuh"
 
 namespace tie {
@@ -54,10 +58,25 @@ __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
-// What is left of a and b beside the bfloat16 pair.
+// What is left of a and b beside the bfloat16 pair, 2^8 up (exact, as is the difference).
 __device__ __forceinline__ void take_off(float& a, float& b, uint32_t pair) {
-  a -= __uint_as_float(pair << 16);
-  b -= __uint_as_float(pair & 0xffff0000u);
+  asm("{\n\t.reg .b64 x, h;\n\t"
+      "mov.b64 x, {%0, %1};\n\t"
+      "mov.b64 h, {%2, %3};\n\t"
+      "fma.rn.f32x2 x, h, %4, x;\n\t"
+      "mul.rn.f32x2 x, x, %5;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(__uint_as_float(pair << 16)), "f"(__uint_as_float(pair & 0xffff0000u)), "l"(0xbf800000bf800000ull), "l"(0x4380000043800000ull));
+}
+// umma_bf16 onto 2^-8 times the accumulator.
+__device__ __forceinline__ void umma_bf16_down8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, 1, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 8;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc)
+      : "memory");
 }
 
 template <int BN>
@@ -73,7 +92,6 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  volatile int* special = abort_flag + 1;            // an operand held an infinity or a NaN
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x % g.splits, tile = blockIdx.x / g.splits;
@@ -90,7 +108,6 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
       mbar_init(acc_empty + b, kFsAdders);
     }
     *abort_flag = 0;
-    *special = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kFsIssuer) {
@@ -138,7 +155,6 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
     } else if (kb_begin < kb_end) {
       load_any(kb_begin);
     }
-    float odd = 0.0f;           // NaN once an infinity, a NaN or what bfloat16 rounds to an infinity came by: its third term is NaN
     uint8_t* const to_a = smem + r0 * 128 + (((chunk >> 1) ^ (r0 & 7)) << 4) + (chunk & 1) * 8;      // (rows of the next step: the same swizzle)
     for (int kb = kb_begin; kb < kb_end; ++kb) {
       const int it = kb - kb_begin, s = it % C::kStages;
@@ -156,7 +172,6 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
             take_off(v.z, v.w, q);
           }
         }
-        odd += (v.x + v.y) + (v.z + v.w);
       };
       if (kb + 1 < min(kb_end, kb_any)) {
 #pragma unroll
@@ -170,7 +185,6 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
         for (int i = 0; i < kRows; ++i) emit(i, next[i]);
         if (kb + 1 < kb_end) load_any(kb + 1);
       }
-      if (odd != odd) *special = 1;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(full + s)) : "memory");
@@ -178,7 +192,7 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
     __syncthreads();
   } else if (warp == kFsIssuer) {
     constexpr uint32_t idesc = instr_desc(BN);
-    // term pairs, the smallest products first: (a, w) with hi 0, mid 1, lo 2
+    // term pairs, the smallest products first: (a, w) with hi 0, mid 1, lo 2; three 2^16 up, two 2^8 up, then the products of hi
     constexpr int kTermA[6] = {2, 0, 1, 1, 0, 0}, kTermW[6] = {0, 2, 1, 0, 1, 0};
     const uint32_t ring_lo = desc_lo_sw128(smem_u32(smem));
     for (int kb = kb_begin; kb < kb_end; ++kb) {
@@ -194,8 +208,10 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
         for (int t = 0; t < 6; ++t) {
 #pragma unroll
           for (int k = 0; k < kFsBK / 16; ++k) {
-            umma_bf16(acc, desc_from_words(a_lo + kTermA[t] * (C::kA >> 4) + 2 * k, kDescHiSw128),
-                      desc_from_words(w_lo + kTermW[t] * (C::kB >> 4) + 2 * k, kDescHiSw128), idesc, t + k > 0 ? 1u : 0u);
+            const uint64_t da = desc_from_words(a_lo + kTermA[t] * (C::kA >> 4) + 2 * k, kDescHiSw128);
+            const uint64_t dw = desc_from_words(w_lo + kTermW[t] * (C::kB >> 4) + 2 * k, kDescHiSw128);
+            if (k == 0 && (t == 3 || t == 5)) umma_bf16_down8(acc, da, dw, idesc);
+            else umma_bf16(acc, da, dw, idesc, t + k > 0 ? 1u : 0u);
           }
         }
         umma_commit(empty + s);
@@ -234,10 +250,13 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     const int row = (warp & 3) * 32 + lane, n1 = n0 + col0;
-    if (*special != 0) {        // with FFMAs, in order of k
+    if (m0 + row < g.M) {
+      bool finite = true;
 #pragma unroll
-      for (int c = 0; c < kCols; ++c) sum[c] = 0.0f;
-      if (m0 + row < g.M) {
+      for (int c = 0; c < kCols; ++c) finite = finite && fabsf(sum[c]) <= 3.402823466e38f;
+      if (!finite) {            // with FFMAs, in order of k
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) sum[c] = 0.0f;
         const float* ar = g.a + static_cast<long long>(m0 + row) * g.lda;
         const int k_end = min(g.K, kb_end * kFsBK);
         for (int k = kb_begin * kFsBK; k < k_end; ++k) {
