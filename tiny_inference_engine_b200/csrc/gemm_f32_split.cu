@@ -7,9 +7,12 @@
 // what the other three (mid lo, lo mid, lo lo) leave out is below 2^-26 of a product, a quarter of a unit of the float product. This is
 // Ozaki's error-free splitting with a fixed number of slices.
 // The tensor core multiplies the terms exactly; its float accumulator is trusted with 64 k's only: a k-block's sum is then read out of
-// tensor memory and added in registers, to the nearest. Against 64 bits the
-// result is off by half of what the FFMA kernel of gemm_simt.cu is, whose accumulators round at every k (the measured figures are
-// in test_float_products_by_three_terms).
+// tensor memory and added in registers, to the nearest. Its additions cut off: sums of one sign came out 0.7 to 1.4 units of 2^-24
+// too small. Every second block's sum is therefore taken 2^-23 larger, in the addition, which leaves a mean of nearly nothing.
+// Relative error against 64 bits, here and with the FFMAs of gemm_simt.cu, at k = 128, 1,024 and 4,096: normal operands 0.8, 1.0, 1.1e-7
+// against 1.5, 2.1, 2.9e-7; operands of one sign 0.4, 0.5, 0.5e-7 against 0.9, 0.7, 0.8e-7 (before the correction 0.9, 1.0, 1.0e-7); operands
+// spread over twelve decades, where a few products make the sum, 0.9, 1.1, 1.2e-7 against 0.7, 1.1, 1.4e-7. With one block of 64 k's nothing
+// evens out (one sign: 0.9e-7 against 0.7e-7): such products stay with the FFMAs.
 //
 // One CTA computes a tile of 128 x BN. Warps 0-15 read both operands' k-block (float, straight from global memory, any size, stride
 // and alignment; the next block's loads are in flight while this one is split), write the six term tiles in the tensor core's
@@ -231,6 +234,7 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
     for (int kb = kb_begin; kb < kb_end; ++kb) {
       const int it = kb - kb_begin, buf = it & 1;
+      const float up = (kb & 1) != 0 ? 1.00000011920928955f : 1.0f;          // 1 + 2^-23
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full + buf, (it >> 1) & 1, abort_flag, g.status, 3) ? 1 : 0)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -244,7 +248,7 @@ __global__ void __launch_bounds__(kFsThreads, 1) gemm_f32_split_kernel(const __g
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + buf)) : "memory");
         }
 #pragma unroll
-        for (int e = 0; e < 16; ++e) sum[c0 + e] += __uint_as_float(r[e]);
+        for (int e = 0; e < 16; ++e) sum[c0 + e] = fmaf(__uint_as_float(r[e]), up, sum[c0 + e]);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

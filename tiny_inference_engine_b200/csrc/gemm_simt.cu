@@ -342,8 +342,8 @@ int launch_gemm(const void* a, const void* w, void* out, int M, int N, int K, lo
 #undef TIE_SMALL_M
   } else if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
     // one product of more than 16 rows by three bfloat16 terms on the tensor cores: a half to a quarter of the FFMAs' time at every size
-    // tried (17 to 1,000 rows, 32 to 32,000 columns, k from 64 on), and nearer to 64 bits; below 64 k's a block is mostly padding
-    if (batch == 1 && M > 16 && K >= 64) return launch_gemm_f32_split_chosen(ap, wp, op, M, N, K, lda, ldw, ldo, s);
+    // tried (17 to 1,000 rows, 32 to 32,000 columns), and nearer to 64 bits from two blocks of 64 k's on (gemm_f32_split.cu)
+    if (batch == 1 && M > 16 && K >= 128) return launch_gemm_f32_split_chosen(ap, wp, op, M, N, K, lda, ldw, ldo, s);
     return launch_gemm_f32(ap, wp, op, M, N, K, lda, ldw, ldo, s, batch, sa, sw, so, -1, 1);
   } else {
     TIE_LAUNCH((gemm_tiled_kernel<TI, TO>), dim3(ceil_div(N, 64), ceil_div(M, 64), batch), 256, 0, s, ap, wp, op, M, N, K, lda, ldw,
