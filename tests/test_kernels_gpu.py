@@ -315,6 +315,17 @@ def test_float_products_are_nearer_to_64_bits_than_ffmas(ops, kind, K):
     assert off(out) <= best
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 512, 1024), (32, 1024, 2048), (24, 16384, 128), (33, 16384, 128), (17, 14208, 320), (17, 24000, 400)])
+def test_float_products_of_few_rows(ops, M, N, K):
+    """Products on either side of the line between the two float kernels, and those whose clusters were taken for more than are resident."""
+    g = torch.Generator("cuda").manual_seed(N)
+    a, w = (torch.randn(n, K, device="cuda", generator=g) for n in (M, N))
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm(a, w, out)
+    want = a.double() @ w.double().T
+    assert float((out.double() - want).norm() / want.norm()) < 4e-7
+
+
 def test_float_products_by_three_terms_whose_partial_sums_overflow(ops):
     """All terms as large as they get: 2^16 times the products of the low ones adds up to three times the result, beyond the largest
     float, where the result is below it."""

@@ -374,9 +374,38 @@ int launch_gemm_f32_split(const float* a, const float* w, float* out, int M, int
   return bn == 64 ? launch_fs<64>(g, s) : launch_fs<96>(g, s);
 }
 
-// The width and the splits with the least estimated time (us: a k-block of a tile, a wave of tiles, a cluster; fitted to a sweep of
-// 90 products of 17 to 1,000 rows: the choice costs 0.3 % more than the best one on average). Clusters only where the tiles leave SMs
-// idle: they never start early.
+// CTAs of the kernel that are resident at once in clusters of `splits` (1, 2, 4 or 8): which GPCs have how many SMs differs from GPU to
+// GPU, so it is asked for, once (148, 132 and 120 for 2, 4 and 8 on one; taken for 128, sixteen clusters of eight ran in two waves: 32 x 512 x
+// 1,024 14.7 us, now 9.2). Every width takes an SM for itself.
+static int resident_ctas(int splits) {
+  static int known[9] = {};
+  if (known[splits] == 0) {
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(148 / splits * splits);
+    cfg.blockDim = dim3(kFsThreads);
+    cfg.dynamicSmemBytes = FsConfig<96>::kSmem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = splits;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (splits == 1 ||
+        cudaFuncSetAttribute(gemm_f32_split_kernel<96>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(FsConfig<96>::kSmem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_f32_split_kernel<96>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = (splits < 4 ? 148 : splits == 4 ? 132 : 96) / splits;
+    }
+    known[splits] = n * splits;
+  }
+  return known[splits];
+}
+
+// The width and the splits with the least estimated time (us: a k-block of a tile, a wave of tiles, a cluster; fitted to a sweep of 18
+// products of 32 to 389 rows, 64 to 6,144 columns, k 128 to 4,096, each launch's weight from memory: the choice costs 0.05 % more
+// than the best one on average, 4 % at most). Clusters only where the tiles leave SMs idle: they never start early.
 int launch_gemm_f32_split_chosen(const float* a, const float* w, float* out, int M, int N, int K, long long lda, long long ldw, long long ldo,
                                  cudaStream_t s) {
   const int k_blocks = ceil_div(K, kFsBK);
@@ -386,9 +415,9 @@ int launch_gemm_f32_split_chosen(const float* a, const float* w, float* out, int
     const long long tiles = static_cast<long long>(ceil_div(M, kFsBM)) * ceil_div(N, bn);
     for (int c = 1; c <= 8; c *= 2) {
       if (c > 1 && (tiles > 148 || k_blocks < c)) break;
-      const int at_once = c < 4 ? 148 : c == 4 ? 144 : 128;
-      const float block = bn == 32 ? 0.77f : bn == 64 ? 1.02f : 1.46f;
-      const float us = ceil_div(tiles * c, at_once) * (ceil_div(k_blocks, c) * block + 4.3f) + (c == 1 ? 0.0f : c == 2 ? 2.2f : c == 4 ? 2.5f : 4.0f);
+      const int at_once = resident_ctas(c);
+      const float block = bn == 32 ? 0.85f : bn == 64 ? 1.0f : 1.35f;
+      const float us = ceil_div(tiles * c, at_once) * (ceil_div(k_blocks, c) * block + 3.6f) + (c == 1 ? 0.0f : c == 2 ? 2.8f : c == 4 ? 3.0f : 4.0f);
       if (width == 0 || us < best) best = us, width = bn, splits = c;
     }
   }

@@ -341,9 +341,13 @@ int launch_gemm(const void* a, const void* w, void* out, int M, int N, int K, lo
 #undef TIE_SMALL_M_ROWS
 #undef TIE_SMALL_M
   } else if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
-    // one product of more than 16 rows by three bfloat16 terms on the tensor cores: a half to a quarter of the FFMAs' time at every size
-    // tried (17 to 1,000 rows, 32 to 32,000 columns), and nearer to 64 bits from two blocks of 64 k's on (gemm_f32_split.cu)
-    if (batch == 1 && M > 16 && K >= 128) return launch_gemm_f32_split_chosen(ap, wp, op, M, N, K, lda, ldw, ldo, s);
+    // One product of more than 16 rows by three bfloat16 terms on the tensor cores: nearer to 64 bits from two blocks of 64 k's on
+    // (gemm_f32_split.cu), and, with the weights read from memory, 17 to 64 rows in 0.4 to 1.06 of the FFMAs' time, more in 0.25 to
+    // 0.75 (64 to 65,536 columns, k 128 to 4,096). Not with up to 32 rows, short k and more than a wave of the widest
+    // tiles: those wait for the weights, which the FFMA kernel's several CTAs an SM keep coming (17 x 16,384 x 256 15.3 us against 16.2, x
+    // 128 8.4 against 11.3; from k 384 on even).
+    const bool streams = M <= 32 && K < 384 && N > 148 * 96;
+    if (batch == 1 && M > 16 && K >= 128 && !streams) return launch_gemm_f32_split_chosen(ap, wp, op, M, N, K, lda, ldw, ldo, s);
     return launch_gemm_f32(ap, wp, op, M, N, K, lda, ldw, ldo, s, batch, sa, sw, so, -1, 1);
   } else {
     TIE_LAUNCH((gemm_tiled_kernel<TI, TO>), dim3(ceil_div(N, 64), ceil_div(M, 64), batch), 256, 0, s, ap, wp, op, M, N, K, lda, ldw,
