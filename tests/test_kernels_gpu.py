@@ -711,6 +711,41 @@ def test_silu_epilogue_from_the_smallest_to_the_largest_gates(ops, transposed):
     assert ((got - want).abs()[near] <= 6 * 2.0 ** -24 * want.abs()[near] * 2).all() and (got - want).abs()[~near].max() < 2e-36
 
 
+@pytest.mark.parametrize("act", [1, 4, 5])
+@pytest.mark.parametrize("kernel", ["pair", "pair transposed", "single", "single transposed", "split k"])
+def test_silu_epilogue_of_gates_that_overflow(ops, kernel, act):
+    """Gates whose sums are infinite or not a number, of every unit with a SiLU (the clamped one without a limit): in kind what
+    g / (1 + exp(-g)) gives, an infinity of the same sign, NaN, or the number."""
+    from tiny_inference_engine_b200.ops import gemm_select
+    M, I, K = 40, 32, 128
+    a = torch.zeros(M, K, dtype=torch.bfloat16)
+    a[:, 0] = torch.tensor([3e38, -3e38, float("nan"), 1e38, -1e38, 104.0, 60.0, 0.0]).to(torch.bfloat16).repeat(5)
+    a[:, 1] = 1.5
+    gate, up = torch.zeros(I, K, dtype=torch.bfloat16), torch.zeros(I, K, dtype=torch.bfloat16)
+    gate[:, 0], up[:, 1] = 2.0, torch.linspace(-1, 1, I).to(torch.bfloat16)
+    w, da, out = ops.interleave_gate_up(gate.cuda(), up.cuda()), a.cuda(), torch.full((M, I), 7.0, device="cuda")
+    zeros, scratch = torch.zeros(I, device="cuda"), torch.empty(2 * M * 2 * I, device="cuda")
+    slope = 1.702 if act == 4 else 1.0
+    unit = (zeros.data_ptr(), zeros.data_ptr(), float("inf"), slope, 0.0, 0, torch.cuda.current_stream().cuda_stream)
+    sizes = (0, da.data_ptr(), w.data_ptr(), out.data_ptr(), M, 2 * I, K, K, K, I)
+    if kernel.startswith("pair"):
+        gemm_select._call("tie_gemm_tc2_unit", *sizes, act, 0, 0, 64, int("transposed" in kernel), 1, 0, 1, *unit)
+    else:
+        t = int(kernel != "single")
+        splits = 2 if kernel == "split k" else 1
+        gemm_select._call("tie_gemm_tc_unit", *sizes, t, 64, splits, scratch.data_ptr() if splits > 1 else 0, act, 1, 0, 0, 0, *unit)
+    torch.cuda.synchronize()
+    gemm_select.check_status()
+    g, u = 2.0 * a[:, :1].float().expand(M, I), (1.5 * up[:, 1].float() + 0.0 * a[:, :1].float())
+    if act == 4:            # its minimum and maximum, like the device's, pass over NaN
+        g, u = torch.fmin(g, torch.tensor(float("inf"))), torch.fmax(u, torch.tensor(-float("inf")))
+    want = g / (1.0 + torch.exp(-slope * g)) * u
+    got = out.cpu()
+    odd = ~torch.isfinite(want)
+    assert odd.sum() == 15 * I and (torch.isnan(got) == torch.isnan(want)).all() and (got[torch.isinf(want)] == want[torch.isinf(want)]).all()
+    assert ((got - want).abs()[~odd] <= 12 * 2.0 ** -24 * want.abs()[~odd] + 1e-37).all()
+
+
 @pytest.mark.parametrize("act", [4, 5, 6])
 @pytest.mark.parametrize("M,I,K", [(5, 48, 1024), (64, 496, 2048), (100, 48, 72), (200, 352, 264), (640, 176, 136)])
 def test_gated_units_in_the_epilogue(ops, M, I, K, act):

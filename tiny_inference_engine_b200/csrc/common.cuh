@@ -121,7 +121,8 @@ __device__ __forceinline__ float squared_relu(float v) {
 // g / (1 + exp(-slope g)). An epilogue evaluates sixteen and more of these side by side, and the branches of `/` keep them from
 // overlapping (the gate/up product of 2,048 tokens waited for its epilogue), so the quotient is formed without any: the
 // hardware's approximate reciprocal, one Newton-Raphson step on it, and one on the quotient by its residual. Denominators
-// above 2^60 are scaled down first, so that no reciprocal is subnormal; where exp(-g) overflows, g * 0 is what g / inf is.
+// above 2^60 are scaled down first, so that no reciprocal is subnormal; where exp(-g) overflows, g * 0 is what g / inf is, and where
+// it is zero, g is what g / 1 is (the residual of an infinite quotient would be NaN).
 __device__ __forceinline__ float silu(float g, float slope = 1.0f) {
   const float e = expf(-slope * g);
   const float scale = e > 1.152921504606847e18f ? 5.421010862427522e-20f : 1.0f;      // 2^60, 2^-64
@@ -131,6 +132,7 @@ __device__ __forceinline__ float silu(float g, float slope = 1.0f) {
   r = fmaf(r, fmaf(-d, r, 1.0f), r);
   float q = n * r;
   q = fmaf(r, fmaf(-d, q, n), q);
+  q = e == 0.0f ? g : q;
   return e > 3.402823466e38f ? g * 0.0f : q;
 }
 
