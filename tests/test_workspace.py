@@ -1,9 +1,14 @@
 """Workspace buffers on the CPU: which are kept, which are let go, and what happens when the device is short of memory; and which steps
 ask for the largest of them, and which go through recurrences in chunks."""
+import threading
+import types
+
 import torch
 
 from tiny_inference_engine_b200.engine.workspace import Workspace
+from tiny_inference_engine_b200.ops import gemm_select
 from tiny_inference_engine_b200.parts import latent_attention
+from tiny_inference_engine_b200.parts.model import Model
 
 
 def test_spare_buffers_are_outgrown_without_a_trace_and_refused_when_memory_is_short(monkeypatch):
@@ -64,3 +69,31 @@ def test_recurrences_go_in_chunks_where_that_was_measured_to_be_faster():
     for lens, heads, dim, vdim in (([2048], 32, 128, 128), ([1021, 510], 16, 128, 128), ([128] * 3, 16, 128, 128), ([1024] + [1] * 8, 16, 64, 64),
                                    ([1021] * 2, 64, 64, 64), ([256], 64, 128, 128), ([128] * 2, 64, 64, 64), ([128], 32, 128, 128)):
         assert pays("head", lens, heads, dim, vdim), (lens, heads, dim, vdim)
+
+
+def test_sums_of_split_products_are_no_other_engines_memory():
+    """Two engines stepping in two threads: a split product whose caller brings no memory uses the step's workspace; outside a step,
+    memory that nothing else holds."""
+    class Step(Model):
+        def __init__(self):
+            pass
+
+        def _forward(self, ctx, cache, states):
+            first = gemm_select._scratch_for(100, "cpu")
+            meet.wait(10)                       # both steps are between their product and its reduction
+            return first, gemm_select._scratch_for(200, "cpu")
+
+    meet, got = threading.Barrier(2), {}
+    spaces = [Workspace(4, "cpu") for _ in range(2)]
+
+    def engine(i):
+        got[i] = Step().forward(types.SimpleNamespace(ws=spaces[i]), None, None)
+    threads = [threading.Thread(target=engine, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got[0][0] is got[0][1] and got[1][0] is got[1][1] and got[0][0].data_ptr() != got[1][0].data_ptr()
+    assert spaces[0].flat("gemm.partial", 1, torch.float32) is got[0][0]
+    outside = [gemm_select._scratch_for(100, "cpu") for _ in range(2)]
+    assert outside[0].data_ptr() != outside[1].data_ptr()

@@ -7,9 +7,11 @@ row strides multiples of 8 elements, 16-byte aligned bases), else on the CUDA co
 """
 from __future__ import annotations
 
+import contextlib
 import functools
 import math
 import os
+import threading
 
 import torch
 
@@ -17,7 +19,6 @@ from ..errors import TieError
 from .library import call as _call, library as _library
 
 NUM_SMS = 148
-_scratch: dict = {}
 
 
 def tc_takes(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
@@ -84,19 +85,26 @@ def plan(M: int, N: int, K: int, split_many: bool = True) -> tuple[int, int, int
     return 0, best[1], best[2]
 
 
-_retired: list = []
+_step = threading.local()
+
+
+@contextlib.contextmanager
+def step_scratch(ws):
+    """While a step is issued by this thread: split products whose caller brings no memory leave their sums in the step's workspace."""
+    before, _step.ws = getattr(_step, "ws", None), ws
+    try:
+        yield
+    finally:
+        _step.ws = before
 
 
 def _scratch_for(numel: int, device) -> torch.Tensor:
-    """Scratch for split products whose caller gave none. An outgrown buffer is kept: a captured CUDA graph
-    may still use its address."""
-    buf = _scratch.get(device)
-    if buf is None or buf.numel() < numel:
-        if buf is not None:
-            _retired.append(buf)
-        buf = torch.empty(max(numel, 1 << 20, 2 * buf.numel() if buf is not None else 0), dtype=torch.float32, device=device)
-        _scratch[device] = buf
-    return buf
+    """Scratch for split products whose caller gave none: the step's own (captured graphs and repeated layers use its address again), or
+    outside a step memory of the call's own stream. None of it is shared, so engines in several threads or streams do not meet in it."""
+    ws = getattr(_step, "ws", None)
+    if ws is not None:
+        return ws.flat("gemm.partial", numel, torch.float32, 1 << 20)
+    return torch.empty(numel, dtype=torch.float32, device=device)
 
 
 @functools.lru_cache(maxsize=None)

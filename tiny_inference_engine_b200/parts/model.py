@@ -9,6 +9,7 @@ import torch
 from ..config.spec import ModelSpec
 from ..errors import InvalidArgument, UnsupportedError
 from ..ops import replay as layer_replay
+from ..ops.gemm_select import step_scratch
 from ..weights.loader import TensorNeed, TensorSource, bind_check
 from .base import BLOCKS, CacheNeed, StateNeed, build_part
 from .layer_runs import LayerRuns, same_handoff
@@ -117,6 +118,10 @@ class Model:
 
     # -- one step over the rows of ctx; returns float32 logits [R, V] or None when no row is wanted
     def forward(self, ctx, cache, states) -> torch.Tensor | None:
+        with step_scratch(ctx.ws):
+            return self._forward(ctx, cache, states)
+
+    def _forward(self, ctx, cache, states) -> torch.Tensor | None:
         T, D = ctx.T, self.spec.hidden_size
         ctx.ws_dtype = self.dtype
         x = ctx.ws.rows("model.x", T, D, torch.float32)
