@@ -175,3 +175,15 @@ def test_pair_kernel_tile_widths_follow_the_waves():
     for M in (512, 700, 1024, 2048, 4096):
         for N in (256, 2560, 4096, 9728, 151936):
             assert gs.pair_width(M, N, 4096, 74) in gs.PAIR_WIDTHS
+
+
+def test_gated_products_split_k_only_where_it_was_measured_faster():
+    """Few tokens, few tiles, above 16 tokens long k; the sums fit the memory that a step keeps for them."""
+    from tiny_inference_engine_b200.ops import gemm_select as gs
+    shapes = ((12288, 2048, 1, 1, 1), (12288, 2048, 4, 3, 1), (10240, 2560, 1, 3, 1), (16384, 2048, 5, 1, 1), (24576, 4096, 1, 1, 1),
+              (3072, 1024, 1, 4, 1), (6144, 4096, 1, 6, 6), (4096, 2048, 2, 8, 4), (96, 136, 1, 1, 1))
+    for N, K, act, few, more in shapes:
+        assert [gs.gated_splits(M, N, K, act) for M in (1, 16)] == [few, few] and gs.gated_splits(64, N, K, act) == more
+        for M in range(1, 66):
+            splits = gs.gated_splits(M, N, K, act)
+            assert splits == 1 or M <= 64 and splits == gs.plan(M, N, K)[2] and splits * M * N <= gs.partial_capacity(64, N, K)

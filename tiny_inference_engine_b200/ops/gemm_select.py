@@ -216,6 +216,18 @@ def _gated(epilogue) -> bool:
     return int(epilogue) in (1, 2, 4, 5, 6)
 
 
+def gated_splits(M: int, N: int, K: int, act: int) -> int:
+    """Into how many parts a gated product's k is cut, the unit formed where the sums are added. In a step the kernels on either side
+    overlap more with the split one, until its sums weigh more than that: up to 16 tokens a split pays from three parts on (decode steps of
+    1 to 16 requests against whole k: 1 to 3 % for 12,288 x 2,048 with a clamped unit, 3 to 5 % for 3,072 and 6,144 x 1,024, 1 % for 10,240 x
+    2,560; but 12,288 x 2,048 with the plain SiLU or ReLU, whose kernel leaves room for the next one, is 2 % slower at one request and even at
+    eight), above from four and with long k (8,192 x 2,048 and longer ones; whole k 2 to 4 % faster for 12,288 x 2,048 with the SiLU
+    at 32 and 64 requests, even or 1 % faster for the others)."""
+    splits = plan(M, N, K)[2]
+    pays = splits >= (3 if act > 2 or K >= 2560 else 4) if M <= 16 else splits >= 4 and K >= 2048
+    return splits if M <= PAIR_FROM and pays else 1
+
+
 class GatedUnit:
     """What a gated unit in a product's epilogue takes beside its code: the clamped unit's limit, slope and shift, the biases of
     the biased ones (float32 [N / 2]), and how many columns stand behind the unit's in the output's rows, a one and zeros."""
@@ -374,10 +386,7 @@ class BoundGemm:
         else:
             t, bn, splits = plan(M, self.N, self.K, self.split_many)
         if self.gated:
-            # few tokens on few tiles: k split like any product's, the unit formed where the sums are added (12,288 columns at 8 tokens,
-            # 96 tiles: whole k 2.5 us slower than three splits, their sum and the unit in kernels of their own; 16,384 columns in two
-            # splits 3 us slower than whole k)
-            splits = splits if M <= PAIR_FROM and splits >= 3 else 1
+            splits = gated_splits(M, self.N, self.K, self.silu) if pair is None else 1
             if not t:
                 bn = max(bn, 32)
         real = _library().tie_gemm_tc_real_splits(self.K, splits) if splits > 1 else 1
