@@ -1,6 +1,7 @@
 """Configuration parsing, the architecture registry and the model description (CPU)."""
 import json
 
+import numpy as np
 import pytest
 
 import plain_qwen3 as plain
@@ -187,3 +188,28 @@ def test_gated_products_split_k_only_where_it_was_measured_faster():
         for M in range(1, 66):
             splits = gs.gated_splits(M, N, K, act)
             assert splits == 1 or M <= 64 and splits == gs.plan(M, N, K)[2] and splits * M * N <= gs.partial_capacity(64, N, K)
+
+
+def test_pair_plans_are_ones_the_kernel_and_the_workspaces_take():
+    """What products of more than 64 tokens run with: a width and a side that the kernel has, real splits whose sums fit the memory that parts keep
+    for them, whole k for those who ask for it, nothing for few tokens or columns; and the estimate's choices where it was mended."""
+    from tiny_inference_engine_b200.ops import gemm_select as gs
+    rng = np.random.default_rng(5)
+    shapes = [(6144, 4096), (4096, 12288), (256, 2048), (24576, 4096), (151936, 2560), (1000, 1000)]
+    shapes += [tuple(int(v) for v in np.exp(rng.uniform(np.log(64), np.log(40000), 2)) // 8 * 8) for _ in range(25)]
+    for N, K in shapes:
+        for M in [1, 64, 65, 96, 128, 129, 256, 257, 384, 512, 2048] + rng.integers(65, 3000, 6).tolist():
+            for split, consumer, gated in ((True, True, False), (True, False, False), (False, False, False), (False, False, True)):
+                plan = gs.pair_plan(M, N, K, 74, split, consumer, gated)
+                if plan is None:
+                    continue
+                transposed, bn, splits = plan
+                assert M > gs.PAIR_FROM and N >= gs.PAIR_MIN_COLUMNS and bn in gs.PAIR_WIDTHS and transposed in (0, 1) and not (transposed and M > 256)
+                k_blocks = -(-K // 64)
+                assert splits == 1 or (split and -(-k_blocks // -(-k_blocks // splits)) == splits)
+                assert splits * M * N <= max(gs.partial_capacity(3000, N, K, True), M * N)
+                if not gated and (M <= 128 or not split):
+                    assert splits * M * N <= max(gs.partial_capacity(3000, N, K, False), M * N)
+            assert M > 64 or gs.pair_plan(M, N, K, 74, True) is None
+    assert gs.pair_plan(192, 8192, 2048, 74, False) == (0, 128, 1) and gs.pair_plan(144, 6144, 4096, 74, False) == (0, 96, 1)
+    assert gs.pair_plan(320, 24576, 4096, 74, False, gated=True) is None and gs.pair_plan(144, 24576, 4096, 74, False, gated=True) == (1, 160, 1)

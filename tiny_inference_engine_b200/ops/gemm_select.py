@@ -133,6 +133,10 @@ PAIR_WIDTHS = (256, 224, 192, 160, 128, 96, 64)
 # float partial sums on their way out. _REDUCE_*: adding them up again, in the kernel that consumes them or in one of its own.
 _PAIR_US_K_BLOCK = {64: 0.190, 96: 0.199, 128: 0.205, 160: 0.213, 192: 0.253, 224: 0.278, 256: 0.321}
 _PAIR_US_LAUNCH, _PAIR_US_TILE, _PAIR_US_TAIL, _PAIR_US_MEGA_PARTIAL = 3.55, 0.92, 1.12, 0.367
+# What the fit does not know of, seen in chains of launches with weights from memory: rows that the transposed side writes in 2-byte pieces (us a
+# column of a tile, once; 8,192 x 2,048 at 192 tokens 13.9 us with tiles of 96 on that side, 13.1 with 128 on the other), and a gated unit of
+# the plain side, which keeps a wave longer (24,576 x 4,096 at 320 tokens: estimated at 61 us, 69.1; one CTA a tile 65.0).
+_PAIR_US_COLUMN_STORES, _PAIR_US_COLUMN_GATED = 0.0098, 0.008
 _REDUCE_US_MEGA_CONSUMER, _REDUCE_US_MEGA, _REDUCE_US_LAUNCH = 0.35, 0.6, 2.2
 # The same for one CTA a tile of 128 rows (`plan`), from the same sweep.
 _SINGLE_US_K_BLOCK, _SINGLE_US_WAVE = {128: 0.237, 256: 0.414}, {128: 1.3, 256: 3.9}
@@ -156,12 +160,16 @@ def _reduce_cost(M: int, N: int, splits: int, consumer: bool) -> float:
     return 0.0 if splits == 1 else mega * _REDUCE_US_MEGA_CONSUMER if consumer else _REDUCE_US_LAUNCH + mega * _REDUCE_US_MEGA
 
 
-def _pair_cost(M: int, N: int, K: int, pairs: int, transposed: int, bn: int, splits: int) -> float:
+def _pair_cost(M: int, N: int, K: int, pairs: int, transposed: int, bn: int, splits: int, gated: bool = False) -> float:
     """Estimated time of the pair kernel: its work items (tiles x splits) go round the pairs in waves."""
     rows, cols = (N, M) if transposed else (M, N)
     waves = math.ceil(math.ceil(rows / 256) * math.ceil(cols / bn) * splits / pairs)
     per = math.ceil(math.ceil(K / 64) / splits)
     out = _PAIR_US_TAIL * bn / 256 + (_PAIR_US_TAIL * bn / 256 + _PAIR_US_MEGA_PARTIAL * splits * M * N / 1e6 if splits > 1 else 0.0)
+    if gated and not transposed:
+        out += waves * bn * _PAIR_US_COLUMN_GATED
+    elif transposed and not gated and splits == 1:
+        out += bn * _PAIR_US_COLUMN_STORES
     # of two that come out alike the wider one: fewer bytes from L2, which counts once the power limit sets the clock
     return (_PAIR_US_LAUNCH + waves * (per * _PAIR_US_K_BLOCK[bn] + _PAIR_US_TILE) + out) * (1.0 + 1e-4 * (256 - bn))
 
@@ -176,12 +184,13 @@ def _single_cost(M: int, N: int, K: int, bn: int, splits: int) -> float:
 
 
 @functools.lru_cache(maxsize=None)
-def pair_plan(M: int, N: int, K: int, pairs: int, split: bool, consumer: bool = False) -> tuple | None:
+def pair_plan(M: int, N: int, K: int, pairs: int, split: bool, consumer: bool = False, gated: bool = False) -> tuple | None:
     """(transposed, tile width, splits) of the pair kernel for out[M, N] = a[M, K] w^T, or None where `plan`'s one CTA a tile is
     as good: up to 64 tokens, few columns, and where its row tiles of 128 save more than pairs do (257 to 384 tokens).
 
     Up to 256 tokens the weights may fill the 256-row side of a tile and the tokens the other (`transposed`). With `split` k may be
-    cut so that every pair has work; `consumer`: whoever reads the product adds the splits (else a kernel of its own does)."""
+    cut so that every pair has work; `consumer`: whoever reads the product adds the splits (else a kernel of its own does). `gated`: the
+    epilogue forms a gated unit."""
     if M <= PAIR_FROM or N < PAIR_MIN_COLUMNS or _NO_PAIR:
         return None
     k_blocks, best = math.ceil(K / 64), None
@@ -196,7 +205,7 @@ def pair_plan(M: int, N: int, K: int, pairs: int, split: bool, consumer: bool = 
                     break
                 if math.ceil(k_blocks / math.ceil(k_blocks / splits)) != splits:
                     continue
-                cost = _pair_cost(M, N, K, pairs, transposed, bn, splits) + _reduce_cost(M, N, splits, consumer)
+                cost = _pair_cost(M, N, K, pairs, transposed, bn, splits, gated) + _reduce_cost(M, N, splits, consumer)
                 if best is None or cost < best[0] - 1e-9:
                     best = (cost, transposed, bn, splits)
     if M > 128:
@@ -264,7 +273,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, transposed=None
     _need(checked or tc_takes(a, w, out),
           "gemm_tc: operands must be bfloat16 with K and row strides multiples of 8, 16-byte aligned")
     forced = not (transposed is None and bn is None and splits is None)
-    p = None if forced or pair is False else pair_plan(M, N, K, resident_pairs(), not silu and K > 0, partial_scratch is not None)
+    p = None if forced or pair is False else pair_plan(M, N, K, resident_pairs(), not silu and K > 0, partial_scratch is not None, _gated(silu))
     if pair and p is None:
         p = (transposed or 0, bn or pair_width(M, N, K, resident_pairs()), splits or 1)
     if p is not None:
@@ -380,7 +389,7 @@ class BoundGemm:
 
     def _plan(self, M: int, consumer: bool):
         # up to 128 tokens k may be split for anyone, above for those who did not ask for the finished product
-        pair = pair_plan(M, self.N, self.K, resident_pairs(), not self.silu and (self.split_many or M <= 128), consumer)
+        pair = pair_plan(M, self.N, self.K, resident_pairs(), not self.silu and (self.split_many or M <= 128), consumer, self.gated)
         if pair is not None:
             t, bn, splits = pair
         else:
