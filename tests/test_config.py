@@ -211,5 +211,6 @@ def test_pair_plans_are_ones_the_kernel_and_the_workspaces_take():
                 if not gated and (M <= 128 or not split):
                     assert splits * M * N <= max(gs.partial_capacity(3000, N, K, False), M * N)
             assert M > 64 or gs.pair_plan(M, N, K, 74, True) is None
+            assert gs.pair_plan(M, N, K, 0, True, True) is None            # a GPU that holds no pair
     assert gs.pair_plan(192, 8192, 2048, 74, False) == (0, 128, 1) and gs.pair_plan(144, 6144, 4096, 74, False) == (0, 96, 1)
     assert gs.pair_plan(320, 24576, 4096, 74, False, gated=True) is None and gs.pair_plan(144, 24576, 4096, 74, False, gated=True) == (1, 160, 1)

@@ -632,6 +632,42 @@ def test_grouped_products_on_the_tensor_cores(tokens):
         assert torch.allclose(partial.view(top, tokens, D), want, rtol=2e-2, atol=2e-2), f"tiles of {block_m}"
 
 
+@pytest.mark.parametrize("kernel", ["pairs", "single SMs"])
+@pytest.mark.parametrize("I,K,dtype", [(144, 200, torch.bfloat16), (272, 72, torch.float32), (16, 8, torch.bfloat16), (40, 136, torch.bfloat16)])
+def test_grouped_products_with_and_without_the_clamped_unit(kernel, I, K, dtype, monkeypatch):
+    """Several tiles of rows and of columns a group, a group without rows, fewer tiles than the buffers hold; on pairs of SMs, and on single
+    ones where the GPU holds no pair. The unit is formed from the float sums of gate and up rows in blocks of sixteen."""
+    from tiny_inference_engine_b200 import ops
+    from tiny_inference_engine_b200.ops import gemm_select
+    if kernel == "single SMs":
+        monkeypatch.setattr(gemm_select, "_pairs", 0)
+    E, tile = 4, ops.GROUPED_TILE
+    group = [0, 0, 1, 3, 3, 3]
+    g = torch.Generator().manual_seed(I)
+    gate, up = ((torch.randn((E, I, K), generator=g) * 3 / K ** 0.5).to(torch.bfloat16).cuda() for _ in range(2))
+    cap = len(group) + 2
+    a = torch.randn((cap * tile, K), generator=g).to(torch.bfloat16).cuda()
+    lists = torch.tensor([len(group)], dtype=torch.int32).cuda(), torch.tensor(group + [99, 99], dtype=torch.int32).cuda()
+    used, rows = len(group) * tile, a.double().view(cap, tile, K)
+    sums = [torch.cat([rows[i] @ w[e].double().T for i, e in enumerate(group)]) for w in (gate, up)]
+    out = torch.full((cap * tile, 2 * I + 8), 7.0, dtype=dtype, device="cuda")
+    ops.gemm_grouped(a, ops.pack_k_blocks(torch.cat([gate, up], 1).reshape(E * 2 * I, K)), out[:, :2 * I], 2 * I, K, *lists)
+    rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 4e-6       # one rounding to the output's type and as much for float sums
+    want = torch.cat(sums, 1)
+    assert (out[:used, :2 * I].double() - want).abs().max() <= rounding * want.abs().max()
+    assert (out[used:] == 7).all() and (out[:, 2 * I:] == 7).all()
+    if I % 16 == 0:
+        both = torch.stack([ops.interleave_gate_up(gate[e], up[e]) for e in range(E)])
+        act = torch.full((cap * tile, I + 8), 7.0, dtype=dtype, device="cuda")
+        ops.gemm_grouped(a, ops.pack_k_blocks(both.reshape(E * 2 * I, K)), act[:, :I], 2 * I, K, *lists, clamped=(2.5, 1.702, 1.0))
+        gv, uv = sums[0].clamp(max=2.5), sums[1].clamp(-2.5, 2.5)
+        want = gv * torch.sigmoid(1.702 * gv) * (uv + 1.0)
+        assert (act[:used, :I].double() - want).abs().max() <= rounding * want.abs().max()
+        assert (act[used:] == 7).all() and (act[:, I:] == 7).all()
+    torch.cuda.synchronize()
+    gemm_select.check_status()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(5, 3, 24, 40, 8), (300, 4, 64, 96, 32), (130, 2, 10, 6, 0), (1000, 16, 128, 64, 64)])
 def test_products_batched_over_heads(shape, dtype):

@@ -60,13 +60,22 @@ template <int BN, bool DEEP> struct TcConfig {
 // memory let the MMAs of the next tile run while the epilogue drains the last one.
 // UNIT: gated units of every kind; else the SiLU and the ReLU only, with 40 registers fewer, which the kernel behind this one needs to
 // get resident beside two of its CTAs (decode steps of 1 and 8 requests were 1 % slower without them).
-template <int BN, typename OutT, bool DEEP, bool UNIT>
+// GROUPED (plain tiling): the row operand is `group_meta[0]` tiles of 256 rows, fewer than the grid was sized for, and row tile t multiplies
+// the weight rows of group `group_of_tile[t]`, `rows_y` each, one group's behind the other's. A kernel ahead of this one writes both.
+template <int BN, typename OutT, bool DEEP, bool UNIT, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, OutT* __restrict__ out,
                float* __restrict__ partial, long long part_stride, long long ldp, int rows_x, int rows_y, int k_blocks,
                int k_blocks_per_split, long long ldo, int transposed, int silu, int tiles_x, int n_tiles, int* status,
-               int w_rows, int w_row0, const __grid_constant__ GatedUnit unit) {
+               int w_rows, int w_row0, const __grid_constant__ GatedUnit unit, const int* __restrict__ group_meta,
+               const int* __restrict__ group_of_tile) {
   pdl_launch_dependents();   // the next kernel may get resident now; it waits for this one at its own pdl_wait()
+  if constexpr (GROUPED) {
+    pdl_wait();
+    const int tiles_y = n_tiles / tiles_x;
+    tiles_x = 2 * group_meta[0];
+    n_tiles = tiles_x * tiles_y;
+  }
   using C = TcConfig<BN, DEEP>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -114,7 +123,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       bool first = true, ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int i0 = (tile % tiles_x) * kBM;
-        const int j0 = (tile / tiles_x) * BN;
+        int j0 = (tile / tiles_x) * BN;
+        if constexpr (GROUPED) j0 += group_of_tile[(tile % tiles_x) >> 1] * rows_y;
         int kb = kb_begin;
         if (first) {
           first = false;
@@ -397,14 +407,14 @@ __global__ void splitk_gated_kernel(const float* __restrict__ partial, long long
 // ---------------------------------------------------------------------------------------------
 // Host side
 
-template <int BN, typename OutT, bool DEEP, bool UNIT>
+template <int BN, typename OutT, bool DEEP, bool UNIT, bool GROUPED = false>
 static int launch_tc_of(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* partial, long long part_stride,
                      long long ldp, int rows_x, int rows_y, int K, long long ldo, int transposed, int silu, int splits, int w_rows,
-                     int w_row0, cudaStream_t s, const GatedUnit& unit) {
+                     int w_row0, cudaStream_t s, const GatedUnit& unit, const int* group_meta = nullptr, const int* group_of_tile = nullptr) {
   using C = TcConfig<BN, DEEP>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, OutT, DEEP, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, OutT, DEEP, UNIT, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(C::kSmem)) != cudaSuccess) {
       set_error("gemm_tc: cannot reserve %zu bytes of shared memory", C::kSmem);
       return kCudaError;
@@ -421,8 +431,9 @@ static int launch_tc_of(const CUtensorMap& mx, const CUtensorMap& my, void* out,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
   const int ctas = DEEP ? (n_tiles * z > sms ? max(1, sms / z) : n_tiles) : n_tiles;
   const dim3 grid(min(ctas, n_tiles), 1, z);
-  TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP, UNIT>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
-             rows_x, rows_y, k_blocks, per_split, ldo, transposed, silu, tiles_x, n_tiles, status_word(), w_rows, w_row0, unit);
+  TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP, UNIT, GROUPED>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
+             rows_x, rows_y, k_blocks, per_split, ldo, transposed, silu, tiles_x, n_tiles, status_word(), w_rows, w_row0, unit, group_meta,
+             group_of_tile);
   return kOk;
 }
 
@@ -543,4 +554,28 @@ TIE_API int tie_gemm_tc_unit(int out_dtype, const void* a, const void* w, void* 
                              cudaStream_t s) {
   return gemm_tc_of(out_dtype, a, w, out, M, N, K, lda, ldw, ldo, transposed, bn, splits, scratch, silu, reduce, deep, w_rows, w_row0,
                     GatedUnit{bias_gate, bias_up, limit, slope, up_shift, ones}, s);
+}
+
+// The grouped product of tie_gemm_tc2_grouped on single SMs, the same arguments: where no pair of SMs holds that kernel.
+TIE_API int tie_gemm_tc_grouped(int out_dtype, const void* a, const void* w, void* out, int M_cap, int N, int K, long long lda, long long ldo,
+                                int w_rows, int epilogue, float limit, float slope, float up_shift, const int* meta, const int* group_of_tile,
+                                cudaStream_t s) {
+  TIE_REQUIRE(M_cap > 0 && M_cap % 256 == 0 && N > 0 && K > 0, "gemm_tc_grouped: bad sizes M=%d (whole tiles of 256) N=%d K=%d", M_cap, N, K);
+  TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && w_rows >= N && w_rows % N == 0, "gemm_tc_grouped: K=%d, lda and the weight's %d rows", K, w_rows);
+  TIE_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0, "gemm_tc_grouped: operands must be 16-byte aligned");
+  TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc_grouped: output dtype code %d", out_dtype);
+  TIE_REQUIRE((epilogue == 0 || epilogue == kEpilogueClamped) && (epilogue == 0 || N % 32 == 0), "gemm_tc_grouped: epilogue %d (N=%d)", epilogue, N);
+  TIE_REQUIRE(meta != nullptr && group_of_tile != nullptr && status_word() != nullptr, "gemm_tc_grouped: no tile list");
+  constexpr int kWidth = 128;
+  CUtensorMap mx, my;
+  TIE_REQUIRE(make_map_bf16(&mx, a, M_cap, K, lda, kBK, kBM) &&
+                  make_map_bf16(&my, w, static_cast<long long>(ceil_div(K, kBK)) * w_rows, kBK, kBK, kBK, kWidth),
+              "gemm_tc_grouped: cuTensorMapEncodeTiled failed (rows %d, K %d)", M_cap, K);
+  const GatedUnit unit{nullptr, nullptr, limit, slope, up_shift, 0};
+#define TIE_TCG_ARGS mx, my, out, nullptr, 0, N, M_cap, N, K, ldo, 0, epilogue, 1, w_rows, 0, s, unit, meta, group_of_tile
+  const int st = out_dtype == TIE_BF16 ? launch_tc_of<kWidth, __nv_bfloat16, true, true, true>(TIE_TCG_ARGS)
+                                       : launch_tc_of<kWidth, float, true, true, true>(TIE_TCG_ARGS);
+#undef TIE_TCG_ARGS
+  if (st != kOk) return st;
+  TIE_RETURN_LAUNCH("gemm_tc_grouped");
 }

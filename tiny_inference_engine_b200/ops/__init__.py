@@ -1222,9 +1222,10 @@ def gemm_grouped(a, w_blocks, out, N: int, K: int, meta, tile_group, clamped=Non
           w_blocks.shape[1] % N == 0 and w_blocks.dtype == torch.bfloat16, "gemm_grouped: weights must be k-blocks of [groups * N, K]")
     _need(out.dim() == 2 and out.stride(1) == 1 and out.shape == (a.shape[0], N if clamped is None else N // 2), "gemm_grouped: out must be [rows, N]")
     limit, slope, up_shift = clamped if clamped is not None else (0.0, 1.0, 0.0)
-    call("tie_gemm_tc2_grouped", dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(), a.shape[0], N, K, a.stride(0), out.stride(0),
-         w_blocks.shape[1], 0 if clamped is None else GATED_CLAMPED, float(limit), float(slope), float(up_shift), meta.data_ptr(),
-         tile_group.data_ptr(), _stream())
+    from .gemm_select import resident_pairs
+    call("tie_gemm_tc2_grouped" if resident_pairs() > 0 else "tie_gemm_tc_grouped", dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(),
+         a.shape[0], N, K, a.stride(0), out.stride(0), w_blocks.shape[1], 0 if clamped is None else GATED_CLAMPED, float(limit), float(slope),
+         float(up_shift), meta.data_ptr(), tile_group.data_ptr(), _stream())
 
 
 # -- layers whose sublayers read the stream side by side, and what stands around them (csrc/parallel_layer.cu)

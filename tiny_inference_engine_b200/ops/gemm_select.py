@@ -145,13 +145,13 @@ _pairs = None
 
 
 def resident_pairs() -> int:
-    """Pairs of SMs that hold the pair kernel at once (asked of the library once; 74 without a GPU, for planning)."""
+    """Pairs of SMs that hold the pair kernel at once: asked of the library once, 0 where there are none or TIE_NO_PAIR_GEMM=1 says not to use
+    any (74 without a GPU, for planning)."""
     global _pairs
     if _pairs is None:
-        try:
-            _pairs = int(_library().tie_gemm_tc2_pairs()) or NUM_SMS // 2
-        except Exception:       # no GPU, no library: plans are still worth looking at
+        if not torch.cuda.is_available():
             return NUM_SMS // 2
+        _pairs = 0 if _NO_PAIR else int(_library().tie_gemm_tc2_pairs())
     return _pairs
 
 
@@ -186,12 +186,12 @@ def _single_cost(M: int, N: int, K: int, bn: int, splits: int) -> float:
 @functools.lru_cache(maxsize=None)
 def pair_plan(M: int, N: int, K: int, pairs: int, split: bool, consumer: bool = False, gated: bool = False) -> tuple | None:
     """(transposed, tile width, splits) of the pair kernel for out[M, N] = a[M, K] w^T, or None where `plan`'s one CTA a tile is
-    as good: up to 64 tokens, few columns, and where its row tiles of 128 save more than pairs do (257 to 384 tokens).
+    as good: up to 64 tokens, few columns, and where its row tiles of 128 save more than pairs do (257 to 384 tokens); and without pairs.
 
     Up to 256 tokens the weights may fill the 256-row side of a tile and the tokens the other (`transposed`). With `split` k may be
     cut so that every pair has work; `consumer`: whoever reads the product adds the splits (else a kernel of its own does). `gated`: the
     epilogue forms a gated unit."""
-    if M <= PAIR_FROM or N < PAIR_MIN_COLUMNS or _NO_PAIR:
+    if M <= PAIR_FROM or N < PAIR_MIN_COLUMNS or pairs < 1:
         return None
     k_blocks, best = math.ceil(K / 64), None
     most = plan(M, N, K, split)[2] if split else 1        # as many sums as one CTA a tile would leave: what their buffers are made for
