@@ -143,6 +143,31 @@ def test_decode_attention_splits_respect_the_kernel_limits():
     assert att.decode_splits(4096, 8, 8, 16, [4096] * 8) == att.decode_splits(4096, 8, 8, 16)
 
 
+def test_decode_attention_evens_out_long_contexts():
+    """Splits of about a place's share where contexts are long: shorter than with all CTAs at once, the limits kept; contexts that are
+    short, or all alike, are split as they were."""
+    from tiny_inference_engine_b200.parts import attention as att
+    lens = [3071 - 2600 * i // 29 for i in range(30)]
+    assert att.decode_splits(3071, 30, 8, 16, lens) == (1536, 2)                # all at once: 2,624 keys
+    assert att.decode_splits(9000, 64, 4, 16, [9000] * 16 + [300] * 48) == (2304, 4)
+    ramp = lambda n, longest: [longest - 7 * longest * i // (8 * n) for i in range(n)]      # noqa: E731
+    # all at once is as good or better where it keeps the places busy, and where the evened splits would come in waves
+    assert att.decode_splits(6000, 12, 8, 16, ramp(12, 6000)) == (1408, 5) and att.decode_splits(9000, 96, 2, 16, ramp(96, 9000)) == (5184, 2)
+    assert att.decode_splits(3071, 24, 8, 16, ramp(24, 3071)) == (1728, 2) and att.decode_splits(1531, 64, 8, 16, [1531] * 16 + [300] * 48) == (1536, 1)
+    shorter = False
+    for n, longest, kv_heads, page in ((30, 3071, 8, 16), (40, 16000, 8, 16), (100, 8200, 4, 8), (64, 40960, 2, 64), (9, 131072, 8, 16), (200, 1023, 8, 16),
+                                       (37, 100000, 1, 8)):
+        for shape in (lambda i: longest - (longest - longest // 7) * i // n, lambda i: longest if i < n // 4 else 70, lambda i: longest):
+            lens = [max(1, shape(i)) for i in range(n)]
+            split_keys, max_splits = att.decode_splits(longest, n, kv_heads, page, lens)
+            assert split_keys % 64 == 0 and 1 <= max_splits <= att.MAX_SPLITS and max_splits * split_keys >= longest
+            assert (split_keys // 64 + 1) * (64 // min(page, 64)) <= att.TMA_DECODE_TABLE_ENTRIES or max_splits == att.MAX_SPLITS
+            at_once = sum(-(-c // split_keys) for c in lens) * kv_heads <= 2 * att.NUM_SMS
+            assert at_once or split_keys >= 14 * 64 or max_splits == 1
+            shorter = shorter or not at_once and max_splits > 1
+    assert shorter
+
+
 def test_matrix_product_plans_are_ones_the_kernel_takes():
     """Whatever the sizes: a tile width the kernel has, splits that leave every split k-blocks to do, k whole where
     the caller asks for it, and no more partial sums than the capacity the parts size their scratch for."""

@@ -216,7 +216,8 @@ class GQAttention(Mixer):
 
 def decode_order(ctx, ctas: int):
     """Which sequences the TMA decode kernel takes in which order: as they stand in the step, or, where its CTAs do not all fit at once,
-    the longest context first. The kernel starts a sequence's heads together, so the last CTAs to start are then the shortest ones
+    as the step lists them: the longest context first, up to eight of them as they stand. The kernel starts a sequence's heads together, so the
+    last CTAs to start are then the shortest ones
     (64 contexts of 1,531 down to 212 keys, 8 kv heads: 36.7 us against 45.1 in any order)."""
     return ctx.single_seqs if ctas > 2 * NUM_SMS else ctx.multi_seqs
 
@@ -247,11 +248,16 @@ def decode_splits(longest: int, sequences: int, kv_heads: int, page_size: int, c
             split_keys += max(64, split_keys // 8 // 64 * 64)
         split_keys = min(split_keys, max(SPLIT_KEYS, -(-longest // 64) * 64))
         # Long contexts: splits about as long as what each place has to do in all, although some CTAs then wait for a place (started
-        # longest first, they fill the gaps that the shorter ones leave: 30 contexts of 3,071 down to 471 keys 38.8 us in halves of
-        # 1,536, 50.4 with all CTAs at once); from 16 tiles a place on, below which the merge and the waiting cost more than that.
-        even = math.ceil(1.1 * int((-(-lens // 64)).sum()) * kv_heads / slots) * 64
-        if even >= 16 * 64 and even < split_keys and longest > 1.25 * even:
-            split_keys = -(-math.ceil(longest / math.ceil(longest / even)) // 64) * 64
+        # longest first, they fill the gaps that the shorter ones leave: 30 contexts of 3,071 down to 471 keys 57.6 us in halves of
+        # 1,536, 63.5 with all CTAs at once). From 16 tiles a place on, only where all CTAs at once leave four tenths of the places' time
+        # unused, and not in splits well below a place's share, which come in waves: of 131 batches (12 to 96 contexts up to 9,000 keys, 2
+        # to 8 kv heads, even, random or a few long ones) the 26 that this takes gain 14 % on average (0.92 to 1.50); the others would
+        # lose 8 % (12 contexts of 6,000 down to 750 keys, 8 kv heads: 49.2 us at once, 63.5 in 328 CTAs for 296 places).
+        share = int((-(-lens // 64)).sum()) * 64 * kv_heads / slots
+        even = math.ceil(1.1 * share / 64) * 64
+        if even >= 16 * 64 and share <= 0.58 * split_keys and longest > 1.25 * even:
+            evened = -(-math.ceil(longest / math.ceil(longest / even)) // 64) * 64
+            split_keys = evened if evened >= 0.95 * share else split_keys
     else:
         want = max(1, slots // max(1, sequences * kv_heads))
         split_keys = max(SPLIT_KEYS, -(-math.ceil(longest / want) // 64) * 64)
