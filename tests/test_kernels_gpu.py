@@ -1170,6 +1170,38 @@ def test_decode_attention_over_long_contexts_with_the_longest_splits(ops, page, 
     assert rel_err(host(out), want) < TOL["bfloat16"] and not counters.any()
 
 
+@pytest.mark.parametrize("split_keys", [128, 1024])
+def test_decode_attention_of_more_ctas_than_places_in_any_order(ops, split_keys):
+    """More CTAs than fit at once: a sequence's heads start together and the list's order says which sequences start first. Each
+    sequence's output has the same bits in any order, also with the sequences as they stand, and in a launch of few CTAs."""
+    from tiny_inference_engine_b200.ops import gemm_select
+    rng = np.random.default_rng(split_keys)
+    Hq, Hkv, Dh, page = 16, 8, 64, 16
+    ctx = [int(c) for c in rng.integers(1, 700, 45)]
+    S, max_splits = len(ctx), -(-max(ctx) // split_keys)
+    assert S * Hkv * max_splits > 2 * 148
+    kc, vc, bt, ks, vs = paged_cache(rng, "bfloat16", ctx, Hkv, Dh, page, sum(-(-c // page) for c in ctx) + 3)
+    q = as_stored(rng.standard_normal((S, Hq * Dh)), "bfloat16")
+    want = np.concatenate([dense_reference(q[i:i + 1], ks[i], vs[i], Hq, Hkv, Dh, 1) for i in range(S)])
+    scratch = torch.empty(ops.attention_split_scratch_floats(S, Hq, Dh, max_splits), device="cuda")
+    counters = torch.zeros(S * Hkv, dtype=torch.int32, device="cuda")
+    args = (dev(q, torch.bfloat16), dev(kc, torch.bfloat16), dev(vc, torch.bfloat16))
+    meta = (dev(np.arange(S + 1), torch.int32), dev(np.array(ctx), torch.int32), dev(bt, torch.int32), Hq, Hkv, Dh, 1 / np.sqrt(Dh))
+    longest_first = np.argsort(-np.array(ctx), kind="stable")
+    orders = [[(0, S)], [(dev(np.arange(S), torch.int32), S)], [(dev(longest_first, torch.int32), S)], [(dev(longest_first[::-1].copy(), torch.int32), S)],
+              [(dev(part.copy(), torch.int32), len(part)) for part in np.array_split(longest_first, 15)]]
+    outs = []
+    for launches in orders:
+        out = torch.full((S, Hq * Dh), float("nan"), device="cuda", dtype=torch.bfloat16)
+        for seqs, n in launches:
+            ops.attention_decode_tma(*args, out, *meta, seqs, n, split_keys, max_splits, scratch, counters)
+        outs.append(out)
+    torch.cuda.synchronize()
+    gemm_select.check_status()
+    assert rel_err(host(outs[0]), want) < TOL["bfloat16"] and not counters.any()
+    assert all(torch.equal(outs[0], out) for out in outs[1:])
+
+
 def test_a_context_beyond_the_splits_a_call_allows_costs_time_or_is_refused_but_never_keys(ops):
     """A caller of the exported kernels who sizes max_splits from something else than the longest context: the
     CUDA-core and cp.async kernels let the last split take the rest (the merge reads no more splits than there

@@ -720,3 +720,26 @@ def test_few_rows_of_experts_on_the_tensor_cores(tokens, E, top, D, I, block_m):
     want = torch.stack([torch.stack([weights[t, s].double() * (w2[int(ids[t, s])].double() @ act[t * top + s].double()) for t in range(tokens)])
                         for s in range(top)])
     assert (partial.double() - want).abs().max() <= 2e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("tokens,E,top,D,I", [(1, 5, 2, 40, 16), (16, 32, 4, 136, 80), (40, 6, 3, 200, 144)])
+@pytest.mark.parametrize("block_m", [4, 8])
+def test_few_rows_of_experts_with_gate_and_up_rows_in_blocks(tokens, E, top, D, I, block_m):
+    """The first product and its unit over an expert's rows in blocks of sixteen (as the grouped product wants them): the same values, bit for
+    bit, as over its gate rows and then its up rows."""
+    from tiny_inference_engine_b200 import ops
+    g = torch.Generator().manual_seed(tokens + E)
+    h = torch.randn((tokens, D), generator=g).to(torch.bfloat16).cuda()
+    gate, up = ((torch.randn((E, I, D), generator=g) * 3 / D ** 0.5).to(torch.bfloat16).cuda() for _ in range(2))
+    stacked = ops.pack_k_blocks(torch.cat([gate, up], 1).reshape(E * 2 * I, D))
+    blocks = ops.pack_k_blocks(torch.stack([ops.interleave_gate_up(gate[e], up[e]) for e in range(E)]).reshape(E * 2 * I, D))
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(tokens)]).to(torch.int32).cuda()
+    tiles = ops.moe_max_tiles(tokens * top, E, block_m)
+    lists = [torch.zeros(n, dtype=torch.int32, device="cuda") for n in (tiles * block_m, tiles, 4)]
+    ops.moe_align(ids, E, block_m, *lists)
+    act = [torch.full((tokens * top, I), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    for a, w, interleaved in zip(act, (stacked, blocks), (False, True)):
+        ops.moe_gemm_glu(h, w, a, top, block_m, *lists, tiles, I, 2.5, 1.702, 1.0, interleaved=interleaved)
+    gv, uv = (torch.stack([w[int(ids[t, s])].double() @ h[t].double() for t in range(tokens) for s in range(top)]) for w in (gate, up))
+    want = gv.clamp(max=2.5) * torch.sigmoid(1.702 * gv.clamp(max=2.5)) * (uv.clamp(-2.5, 2.5) + 1.0)
+    assert (act[1].double() - want).abs().max() <= 2.0 ** -8 * want.abs().max() and torch.equal(act[0], act[1])
