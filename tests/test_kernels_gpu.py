@@ -337,6 +337,30 @@ def test_float_products_by_three_terms_whose_partial_sums_overflow(ops):
     assert torch.isfinite(out).all() and terms < 1e-6
 
 
+def test_a_float_product_may_be_captured_before_any_other_has_run(ops):
+    """In a process of its own: the first product of all inside a graph's capture, as the FFMA kernels allow."""
+    import pathlib
+    import subprocess
+    import sys
+    script = """
+import torch
+from tiny_inference_engine_b200 import ops
+from tiny_inference_engine_b200.ops.library import library
+library()
+a, w, out = (torch.randn(n, k, device="cuda") for n, k in ((64, 512), (96, 512), (64, 96)))
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    ops.gemm(a, w, out)
+graph.replay()
+torch.cuda.synchronize()
+want = a.double() @ w.double().T
+assert float((out.double() - want).norm() / want.norm()) < 4e-7
+"""
+    done = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300,
+                          cwd=pathlib.Path(__file__).resolve().parents[1])
+    assert done.returncode == 0, done.stderr[-2000:]
+
+
 def dense_reference(q, k, v, Hq, Hkv, Dh, n_new, window=0):
     """The last n_new rows of causal attention over all of k, v."""
     n = k.shape[0]

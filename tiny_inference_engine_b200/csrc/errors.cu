@@ -71,7 +71,15 @@ static int* g_status_dev = nullptr;
 
 int* status_word() {
   if (g_status_host == nullptr) {
-    if (cudaHostAlloc(reinterpret_cast<void**>(&g_status_host), sizeof(int), cudaHostAllocMapped) != cudaSuccess) return nullptr;
+    // a kernel's first call may come while the caller captures a graph, when this thread may not allocate unless it says that it means to
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t got = cudaHostAlloc(reinterpret_cast<void**>(&g_status_host), sizeof(int), cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (got != cudaSuccess) {
+      g_status_host = nullptr;
+      return nullptr;
+    }
     *g_status_host = 0;
     if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&g_status_dev), g_status_host, 0) != cudaSuccess) return nullptr;
   }
