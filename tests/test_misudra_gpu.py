@@ -632,16 +632,16 @@ def test_grouped_products_on_the_tensor_cores(tokens):
         assert torch.allclose(partial.view(top, tokens, D), want, rtol=2e-2, atol=2e-2), f"tiles of {block_m}"
 
 
-@pytest.mark.parametrize("kernel", ["pairs", "single SMs"])
+@pytest.mark.parametrize("kernel", ["pairs", "single SMs", "single SMs, few rows"])
 @pytest.mark.parametrize("I,K,dtype", [(144, 200, torch.bfloat16), (272, 72, torch.float32), (16, 8, torch.bfloat16), (40, 136, torch.bfloat16)])
 def test_grouped_products_with_and_without_the_clamped_unit(kernel, I, K, dtype, monkeypatch):
     """Several tiles of rows and of columns a group, a group without rows, fewer tiles than the buffers hold; on pairs of SMs, and on single
-    ones where the GPU holds no pair. The unit is formed from the float sums of gate and up rows in blocks of sixteen."""
+    ones where the GPU holds no pair or groups have few rows. The unit is formed from the float sums of gate and up rows in blocks of sixteen."""
     from tiny_inference_engine_b200 import ops
     from tiny_inference_engine_b200.ops import gemm_select
     if kernel == "single SMs":
         monkeypatch.setattr(gemm_select, "_pairs", 0)
-    E, tile = 4, ops.GROUPED_TILE
+    E, tile = 4, ops.GROUPED_TILE_FEW if "few" in kernel else ops.GROUPED_TILE
     group = [0, 0, 1, 3, 3, 3]
     g = torch.Generator().manual_seed(I)
     gate, up = ((torch.randn((E, I, K), generator=g) * 3 / K ** 0.5).to(torch.bfloat16).cuda() for _ in range(2))
@@ -651,7 +651,7 @@ def test_grouped_products_with_and_without_the_clamped_unit(kernel, I, K, dtype,
     used, rows = len(group) * tile, a.double().view(cap, tile, K)
     sums = [torch.cat([rows[i] @ w[e].double().T for i, e in enumerate(group)]) for w in (gate, up)]
     out = torch.full((cap * tile, 2 * I + 8), 7.0, dtype=dtype, device="cuda")
-    ops.gemm_grouped(a, ops.pack_k_blocks(torch.cat([gate, up], 1).reshape(E * 2 * I, K)), out[:, :2 * I], 2 * I, K, *lists)
+    ops.gemm_grouped(a, ops.pack_k_blocks(torch.cat([gate, up], 1).reshape(E * 2 * I, K)), out[:, :2 * I], 2 * I, K, *lists, tile=tile)
     rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 4e-6       # one rounding to the output's type and as much for float sums
     want = torch.cat(sums, 1)
     assert (out[:used, :2 * I].double() - want).abs().max() <= rounding * want.abs().max()
@@ -659,13 +659,36 @@ def test_grouped_products_with_and_without_the_clamped_unit(kernel, I, K, dtype,
     if I % 16 == 0:
         both = torch.stack([ops.interleave_gate_up(gate[e], up[e]) for e in range(E)])
         act = torch.full((cap * tile, I + 8), 7.0, dtype=dtype, device="cuda")
-        ops.gemm_grouped(a, ops.pack_k_blocks(both.reshape(E * 2 * I, K)), act[:, :I], 2 * I, K, *lists, clamped=(2.5, 1.702, 1.0))
+        ops.gemm_grouped(a, ops.pack_k_blocks(both.reshape(E * 2 * I, K)), act[:, :I], 2 * I, K, *lists, clamped=(2.5, 1.702, 1.0), tile=tile)
         gv, uv = sums[0].clamp(max=2.5), sums[1].clamp(-2.5, 2.5)
         want = gv * torch.sigmoid(1.702 * gv) * (uv + 1.0)
         assert (act[:used, :I].double() - want).abs().max() <= rounding * want.abs().max()
         assert (act[used:] == 7).all() and (act[:, I:] == 7).all()
     torch.cuda.synchronize()
     gemm_select.check_status()
+
+
+@pytest.mark.parametrize("tokens,E,top", [(1, 4, 2), (40, 5, 3), (300, 3, 2), (128, 32, 4)])
+def test_rows_listed_in_tiles_of_either_size_come_back_to_their_tokens(tokens, E, top):
+    """Rows copied into the listed order and their weighted results back, in tiles of 256 and of 128 rows: every pair once, zeros in the padding."""
+    from tiny_inference_engine_b200 import ops
+    g = torch.Generator().manual_seed(tokens)
+    h = torch.randn((tokens, 72), generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(tokens)]).to(torch.int32).cuda()
+    weights = torch.rand((tokens, top), generator=g).cuda()
+    assert ops.grouped_tile(144 * E, E) == ops.GROUPED_TILE and ops.grouped_tile(144 * E - 1, E) == ops.GROUPED_TILE_FEW
+    for tile in (ops.GROUPED_TILE, ops.GROUPED_TILE_FEW):
+        tiles = ops.moe_max_tiles(tokens * top, E, tile)
+        lists = [torch.zeros(n, dtype=torch.int32, device="cuda") for n in (tiles * tile, tiles, 4)]
+        ops.moe_align(ids, E, tile, *lists)
+        xs = torch.full((tiles * tile, 72), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops.moe_gather(h, lists[0], lists[2], top, xs, tile=tile)
+        used = int(lists[2][0]) * tile
+        pair = lists[0][:used].long()
+        assert torch.equal(xs[:used], torch.where((pair >= 0)[:, None], h[pair.clamp(min=0) // top], torch.zeros_like(h[:1]))) and (xs[used:] == 7).all()
+        partial = torch.full((top, tokens, 72), float("nan"), device="cuda")
+        ops.moe_combine(xs, lists[0], lists[2], top, weights.view(-1), partial, tokens, tile=tile)
+        assert torch.equal(partial, weights.T[:, :, None] * h.float()[None])
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -60,20 +60,20 @@ template <int BN, bool DEEP> struct TcConfig {
 // memory let the MMAs of the next tile run while the epilogue drains the last one.
 // UNIT: gated units of every kind; else the SiLU and the ReLU only, with 40 registers fewer, which the kernel behind this one needs to
 // get resident beside two of its CTAs (decode steps of 1 and 8 requests were 1 % slower without them).
-// GROUPED (plain tiling): the row operand is `group_meta[0]` tiles of 256 rows, fewer than the grid was sized for, and row tile t multiplies
-// the weight rows of group `group_of_tile[t]`, `rows_y` each, one group's behind the other's. A kernel ahead of this one writes both.
+// GROUPED (plain tiling): the row operand is `group_meta[0]` tiles of 128 << group_shift rows, fewer than the grid was sized for, and tile t
+// multiplies the weight rows of group `group_of_tile[t]`, `rows_y` each, one group's behind the other's. A kernel ahead of this one writes both.
 template <int BN, typename OutT, bool DEEP, bool UNIT, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, OutT* __restrict__ out,
                float* __restrict__ partial, long long part_stride, long long ldp, int rows_x, int rows_y, int k_blocks,
                int k_blocks_per_split, long long ldo, int transposed, int silu, int tiles_x, int n_tiles, int* status,
                int w_rows, int w_row0, const __grid_constant__ GatedUnit unit, const int* __restrict__ group_meta,
-               const int* __restrict__ group_of_tile) {
+               const int* __restrict__ group_of_tile, int group_shift) {
   pdl_launch_dependents();   // the next kernel may get resident now; it waits for this one at its own pdl_wait()
   if constexpr (GROUPED) {
     pdl_wait();
     const int tiles_y = n_tiles / tiles_x;
-    tiles_x = 2 * group_meta[0];
+    tiles_x = group_meta[0] << group_shift;
     n_tiles = tiles_x * tiles_y;
   }
   using C = TcConfig<BN, DEEP>;
@@ -124,7 +124,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int i0 = (tile % tiles_x) * kBM;
         int j0 = (tile / tiles_x) * BN;
-        if constexpr (GROUPED) j0 += group_of_tile[(tile % tiles_x) >> 1] * rows_y;
+        if constexpr (GROUPED) j0 += group_of_tile[(tile % tiles_x) >> group_shift] * rows_y;
         int kb = kb_begin;
         if (first) {
           first = false;
@@ -410,7 +410,7 @@ __global__ void splitk_gated_kernel(const float* __restrict__ partial, long long
 template <int BN, typename OutT, bool DEEP, bool UNIT, bool GROUPED = false>
 static int launch_tc_of(const CUtensorMap& mx, const CUtensorMap& my, void* out, float* partial, long long part_stride,
                      long long ldp, int rows_x, int rows_y, int K, long long ldo, int transposed, int silu, int splits, int w_rows,
-                     int w_row0, cudaStream_t s, const GatedUnit& unit, const int* group_meta = nullptr, const int* group_of_tile = nullptr) {
+                     int w_row0, cudaStream_t s, const GatedUnit& unit, const int* group_meta = nullptr, const int* group_of_tile = nullptr, int group_shift = 0) {
   using C = TcConfig<BN, DEEP>;
   static bool configured = false;
   if (!configured) {
@@ -433,7 +433,7 @@ static int launch_tc_of(const CUtensorMap& mx, const CUtensorMap& my, void* out,
   const dim3 grid(min(ctas, n_tiles), 1, z);
   TIE_LAUNCH((gemm_tc_kernel<BN, OutT, DEEP, UNIT, GROUPED>), grid, kThreads, C::kSmem, s, mx, my, static_cast<OutT*>(out), partial, part_stride, ldp,
              rows_x, rows_y, k_blocks, per_split, ldo, transposed, silu, tiles_x, n_tiles, status_word(), w_rows, w_row0, unit, group_meta,
-             group_of_tile);
+             group_of_tile, group_shift);
   return kOk;
 }
 
@@ -556,25 +556,30 @@ TIE_API int tie_gemm_tc_unit(int out_dtype, const void* a, const void* w, void* 
                     GatedUnit{bias_gate, bias_up, limit, slope, up_shift, ones}, s);
 }
 
-// The grouped product of tie_gemm_tc2_grouped on single SMs, the same arguments: where no pair of SMs holds that kernel.
+// The grouped product of tie_gemm_tc2_grouped on single SMs, the list's tiles of tile_rows 128 or 256: for groups of few rows (which tiles of 256
+// would mostly pad) and where no pair of SMs holds that kernel.
 TIE_API int tie_gemm_tc_grouped(int out_dtype, const void* a, const void* w, void* out, int M_cap, int N, int K, long long lda, long long ldo,
                                 int w_rows, int epilogue, float limit, float slope, float up_shift, const int* meta, const int* group_of_tile,
-                                cudaStream_t s) {
-  TIE_REQUIRE(M_cap > 0 && M_cap % 256 == 0 && N > 0 && K > 0, "gemm_tc_grouped: bad sizes M=%d (whole tiles of 256) N=%d K=%d", M_cap, N, K);
+                                int tile_rows, cudaStream_t s) {
+  TIE_REQUIRE((tile_rows == 128 || tile_rows == 256) && M_cap > 0 && M_cap % tile_rows == 0 && N > 0 && K > 0,
+              "gemm_tc_grouped: bad sizes M=%d (whole tiles of %d) N=%d K=%d", M_cap, tile_rows, N, K);
   TIE_REQUIRE(K % 8 == 0 && lda % 8 == 0 && w_rows >= N && w_rows % N == 0, "gemm_tc_grouped: K=%d, lda and the weight's %d rows", K, w_rows);
   TIE_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0, "gemm_tc_grouped: operands must be 16-byte aligned");
   TIE_REQUIRE(out_dtype == TIE_BF16 || out_dtype == TIE_F32, "gemm_tc_grouped: output dtype code %d", out_dtype);
   TIE_REQUIRE((epilogue == 0 || epilogue == kEpilogueClamped) && (epilogue == 0 || N % 32 == 0), "gemm_tc_grouped: epilogue %d (N=%d)", epilogue, N);
   TIE_REQUIRE(meta != nullptr && group_of_tile != nullptr && status_word() != nullptr, "gemm_tc_grouped: no tile list");
-  constexpr int kWidth = 128;
+  const int bn = N >= 256 ? 256 : 128;
   CUtensorMap mx, my;
   TIE_REQUIRE(make_map_bf16(&mx, a, M_cap, K, lda, kBK, kBM) &&
-                  make_map_bf16(&my, w, static_cast<long long>(ceil_div(K, kBK)) * w_rows, kBK, kBK, kBK, kWidth),
+                  make_map_bf16(&my, w, static_cast<long long>(ceil_div(K, kBK)) * w_rows, kBK, kBK, kBK, bn),
               "gemm_tc_grouped: cuTensorMapEncodeTiled failed (rows %d, K %d)", M_cap, K);
   const GatedUnit unit{nullptr, nullptr, limit, slope, up_shift, 0};
-#define TIE_TCG_ARGS mx, my, out, nullptr, 0, N, M_cap, N, K, ldo, 0, epilogue, 1, w_rows, 0, s, unit, meta, group_of_tile
-  const int st = out_dtype == TIE_BF16 ? launch_tc_of<kWidth, __nv_bfloat16, true, true, true>(TIE_TCG_ARGS)
-                                       : launch_tc_of<kWidth, float, true, true, true>(TIE_TCG_ARGS);
+  int st = kOk;
+#define TIE_TCG_ARGS mx, my, out, nullptr, 0, N, M_cap, N, K, ldo, 0, epilogue, 1, w_rows, 0, s, unit, meta, group_of_tile, tile_rows == 256
+  if (bn == 128)
+    st = out_dtype == TIE_BF16 ? launch_tc_of<128, __nv_bfloat16, true, true, true>(TIE_TCG_ARGS) : launch_tc_of<128, float, true, true, true>(TIE_TCG_ARGS);
+  else
+    st = out_dtype == TIE_BF16 ? launch_tc_of<256, __nv_bfloat16, true, true, true>(TIE_TCG_ARGS) : launch_tc_of<256, float, true, true, true>(TIE_TCG_ARGS);
 #undef TIE_TCG_ARGS
   if (st != kOk) return st;
   TIE_RETURN_LAUNCH("gemm_tc_grouped");

@@ -13,7 +13,8 @@
 //               expert's weight rows are streamed once, a warp per output column (row-major weights, 4 pairs) or per
 //               sixteen (bfloat16 weights in k-blocks, on the tensor cores).
 //   moe_gather, moe_combine   for prompts in bfloat16: rows copied into the listed order ahead of the grouped products
-//               on the tensor cores (gemm_tc2.cu, tiles of 256 rows), and the weighted results back to their tokens.
+//               on the tensor cores (gemm_tc2.cu in tiles of 256 rows, gemm_tc.cu in tiles of 128 where experts have few), and the weighted
+//               results back to their tokens.
 //   moe_gemm    grouped products on the CUDA cores, one block per (tile of rows, 64 output columns): rows are
 //               gathered through the list, weights are the tile's expert's. `first` reads token rows and writes a
 //               row per pair; `second` reads a row per pair and writes weight * result as the pair's choice-th

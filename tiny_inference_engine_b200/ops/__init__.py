@@ -1185,24 +1185,25 @@ def moe_gemm_glu(a, w, out, top: int, block_m: int, sorted_pairs, tile_expert, m
 
 
 GROUPED_TILE = 256      # rows of a tile of the grouped product on the tensor cores (a pair of SMs)
+GROUPED_TILE_FEW = 128  # the same on single SMs, for groups of few rows
 
 
-def moe_gather(h, sorted_pairs, meta, top: int, out) -> None:
-    """out[r] = h[pair(r) // top] for the rows r listed by `moe_align` with tiles of GROUPED_TILE (zeros where a row pads a
+def moe_gather(h, sorted_pairs, meta, top: int, out, tile: int = GROUPED_TILE) -> None:
+    """out[r] = h[pair(r) // top] for the rows r listed by `moe_align` with tiles of `tile` rows (zeros where a row pads a
     tile); bfloat16, width in whole 16-byte vectors."""
     _dev(h, sorted_pairs, meta, out)
     _need(h.dim() == 2 and h.stride(1) == 1 and out.dim() == 2 and out.is_contiguous() and out.shape[1] == h.shape[1] and
           h.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "moe_gather: bfloat16 rows of one width")
-    call("tie_moe_gather", dtype_code(h), h.data_ptr(), h.stride(0), sorted_pairs.data_ptr(), meta.data_ptr(), GROUPED_TILE, top,
+    call("tie_moe_gather", dtype_code(h), h.data_ptr(), h.stride(0), sorted_pairs.data_ptr(), meta.data_ptr(), tile, top,
          out.data_ptr(), h.shape[1], out.shape[0], _stream())
 
 
-def moe_combine(y, sorted_pairs, meta, top: int, weights, partial, tokens: int) -> None:
+def moe_combine(y, sorted_pairs, meta, top: int, weights, partial, tokens: int, tile: int = GROUPED_TILE) -> None:
     """partial[pair % top][pair // top] = weights[pair] * y[row of the pair] (float32 [top, tokens, width])."""
     _dev(y, sorted_pairs, meta, weights, partial)
     _need(y.dim() == 2 and y.is_contiguous() and y.dtype == torch.bfloat16 and partial.dtype == torch.float32 and
           partial.numel() >= top * tokens * y.shape[1] and weights.dtype == torch.float32, "moe_combine: y bfloat16 rows, partial float32 [top, tokens, width]")
-    call("tie_moe_combine", dtype_code(y), y.data_ptr(), sorted_pairs.data_ptr(), meta.data_ptr(), GROUPED_TILE, top,
+    call("tie_moe_combine", dtype_code(y), y.data_ptr(), sorted_pairs.data_ptr(), meta.data_ptr(), tile, top,
          weights.data_ptr(), partial.data_ptr(), tokens * y.shape[1], y.shape[1], y.shape[0], _stream())
 
 
@@ -1211,21 +1212,32 @@ def gemm_grouped_takes(rows: int, N: int, K: int) -> bool:
     return K % 8 == 0 and N % 8 == 0 and rows % GROUPED_TILE == 0
 
 
-def gemm_grouped(a, w_blocks, out, N: int, K: int, meta, tile_group, clamped=None) -> None:
-    """out[r, :N] = w[group of r's tile] a[r] for the first meta[0] tiles of GROUPED_TILE rows of a; `w_blocks` is the
-    groups' weights one after the other, [groups * N, K], stored in k-blocks (`pack_k_blocks`). `clamped`: (limit, slope, up_shift) of the
+def grouped_tile(pairs: int, experts: int) -> int:
+    """Rows of the grouped products' tiles: pairs of SMs from 144 rows an expert on. With fewer, tiles of 256 rows are padding for the most part and
+    the padded products take longer than the weights' way from memory (steps with 4 of 32 experts of 3,072 x 4,096 in one of three layers,
+    on pairs and on single SMs: 128 tokens 1,192 and 1,036 us, 720 1,875 and 1,740, 1,000 2,217 and 2,135, 1,200 even)."""
+    from .gemm_select import resident_pairs
+    return GROUPED_TILE if pairs >= 144 * experts and resident_pairs() > 0 else GROUPED_TILE_FEW
+
+
+def gemm_grouped(a, w_blocks, out, N: int, K: int, meta, tile_group, clamped=None, tile: int = GROUPED_TILE) -> None:
+    """out[r, :N] = w[group of r's tile] a[r] for the first meta[0] tiles of `tile` rows of a (GROUPED_TILE, or GROUPED_TILE_FEW); `w_blocks` is
+    the groups' weights one after the other, [groups * N, K], stored in k-blocks (`pack_k_blocks`). `clamped`: (limit, slope, up_shift) of the
     clamped gated unit on top (`glu_clamped`); a group's rows are then blocks of 16 gate and 16 up rows and out is [rows, N / 2]."""
     _dev(a, w_blocks, out, meta, tile_group)
-    _need(a.dim() == 2 and a.stride(1) == 1 and a.shape[1] == K and a.dtype == torch.bfloat16 and a.shape[0] % GROUPED_TILE == 0,
-          "gemm_grouped: a must be bfloat16 [whole tiles, K]")
+    _need(a.dim() == 2 and a.stride(1) == 1 and a.shape[1] == K and a.dtype == torch.bfloat16 and tile in (GROUPED_TILE, GROUPED_TILE_FEW) and
+          a.shape[0] % tile == 0, "gemm_grouped: a must be bfloat16 [whole tiles, K]")
     _need(w_blocks.dim() == 3 and w_blocks.is_contiguous() and w_blocks.shape[2] == 64 and w_blocks.shape[0] == (K + 63) // 64 and
           w_blocks.shape[1] % N == 0 and w_blocks.dtype == torch.bfloat16, "gemm_grouped: weights must be k-blocks of [groups * N, K]")
     _need(out.dim() == 2 and out.stride(1) == 1 and out.shape == (a.shape[0], N if clamped is None else N // 2), "gemm_grouped: out must be [rows, N]")
     limit, slope, up_shift = clamped if clamped is not None else (0.0, 1.0, 0.0)
     from .gemm_select import resident_pairs
-    call("tie_gemm_tc2_grouped" if resident_pairs() > 0 else "tie_gemm_tc_grouped", dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(),
-         a.shape[0], N, K, a.stride(0), out.stride(0), w_blocks.shape[1], 0 if clamped is None else GATED_CLAMPED, float(limit), float(slope),
-         float(up_shift), meta.data_ptr(), tile_group.data_ptr(), _stream())
+    args = (dtype_code(out), a.data_ptr(), w_blocks.data_ptr(), out.data_ptr(), a.shape[0], N, K, a.stride(0), out.stride(0), w_blocks.shape[1],
+            0 if clamped is None else GATED_CLAMPED, float(limit), float(slope), float(up_shift), meta.data_ptr(), tile_group.data_ptr())
+    if tile == GROUPED_TILE and resident_pairs() > 0:
+        call("tie_gemm_tc2_grouped", *args, _stream())
+    else:
+        call("tie_gemm_tc_grouped", *args, tile, _stream())
 
 
 # -- layers whose sublayers read the stream side by side, and what stands around them (csrc/parallel_layer.cu)

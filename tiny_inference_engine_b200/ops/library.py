@@ -78,7 +78,7 @@ _SIGNATURES = {
     "tie_moe_gather": [I, P, L, P, P, I, I, P, I, I, P],
     "tie_moe_combine": [I, P, P, P, I, I, P, P, L, I, I, P],
     "tie_gemm_heads_mma": [P, L, I, P, P, L, I, I, I, I, I, P],
-    "tie_gemm_tc_grouped": [I, P, P, P, I, I, I, L, L, I, I, F, F, F, P, P, P],
+    "tie_gemm_tc_grouped": [I, P, P, P, I, I, I, L, L, I, I, F, F, F, P, P, I, P],
     "tie_gemm_tc2_grouped": [I, P, P, P, I, I, I, L, L, I, I, F, F, F, P, P, P],
     "tie_pair_hash_add": [I, P, P, P, P, P, P, P, P, I, L, L, I, I, P],
     "tie_add_row_vector": [P, P, I, I, P],

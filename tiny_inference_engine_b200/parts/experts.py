@@ -118,7 +118,7 @@ class RoutedExperts(FeedForward):
         pairs = T * top
         few = pairs <= 8 * E      # an expert has a few rows: its weights are streamed once
         if self.in_blocks:
-            block_m = 8 if few else ops.GROUPED_TILE
+            block_m = 8 if few else ops.grouped_tile(pairs, E)
         elif few and D % 4 == 0 and I % 4 == 0 and self.dtype == torch.float32:
             block_m = 4
         else:
@@ -131,23 +131,23 @@ class RoutedExperts(FeedForward):
         ops.moe_align(ids, E, block_m, sorted_pairs, tile_expert, meta)
         max_tiles = ops.moe_max_tiles(pairs, E, block_m)
         partial = ctx.ws.flat("moe.partial", rows_cap * D, torch.float32)
-        if block_m == ops.GROUPED_TILE:
+        if self.in_blocks and not few:
             # prompts on the tensor cores: rows copied into the listed order, two grouped products over dense operands,
             # the weighted results back to their tokens
             rows = max_tiles * block_m
-            cap = ops.moe_max_tiles(rows_cap, E, block_m) * block_m
+            cap = ops.moe_max_tiles(rows_cap, E, ops.GROUPED_TILE) * ops.GROUPED_TILE
             xs = ctx.ws.flat("moe.listed", cap * D, self.dtype)[:rows * D].view(rows, D)
-            ops.moe_gather(h, sorted_pairs, meta, top, xs)
+            ops.moe_gather(h, sorted_pairs, meta, top, xs, tile=block_m)
             act = ctx.ws.flat("moe.listed.act", cap * I, self.dtype)[:rows * I].view(rows, I)
             if self.fused:
-                ops.gemm_grouped(xs, self.w_gate_up, act, 2 * I, D, meta, tile_expert, clamped=(self.limit, self.slope, self.up_shift))
+                ops.gemm_grouped(xs, self.w_gate_up, act, 2 * I, D, meta, tile_expert, clamped=(self.limit, self.slope, self.up_shift), tile=block_m)
             else:
                 gu = ctx.ws.flat("moe.listed.gate_up", cap * 2 * I, self.dtype)[:rows * 2 * I].view(rows, 2 * I)
-                ops.gemm_grouped(xs, self.w_gate_up, gu, 2 * I, D, meta, tile_expert)
+                ops.gemm_grouped(xs, self.w_gate_up, gu, 2 * I, D, meta, tile_expert, tile=block_m)
                 ops.glu_clamped(gu, act, self.limit, self.slope, self.up_shift)
             y = xs                                          # the listed inputs are done with
-            ops.gemm_grouped(act, self.w_down, y, D, I, meta, tile_expert)
-            ops.moe_combine(y, sorted_pairs, meta, top, weights.view(-1), partial, T)
+            ops.gemm_grouped(act, self.w_down, y, D, I, meta, tile_expert, tile=block_m)
+            ops.moe_combine(y, sorted_pairs, meta, top, weights.view(-1), partial, T, tile=block_m)
             return ops.SplitSum(partial, top, T, D)
         act = ctx.ws.rows("moe.act", T, top * I, self.dtype).view(pairs, I)
         if self.in_blocks:
